@@ -4,6 +4,7 @@
 // 62-131): fit copies the base into memory the index owns (linear_index.cpp:82 copies into a
 // std::vector; here the copy lands in HBM as zero-padded rows), query returns int64 ids and adds
 // n to the cumulative distance counter per query (linear_index.cpp:108, 123).
+#include <cmath>
 #include <cstdarg>
 #include <cstring>
 #include <algorithm>
@@ -255,6 +256,8 @@ int ann_flat_fit(ann_flat* h, const float* data, int64_t n, int32_t dim, int64_t
         h->base_e4m3 = nullptr;
         h->fac_e4m3 = nullptr;
     }
+    h->bounds_known = false;
+    h->prune_credit_us = 0.0;
     const size_t bytes = sizeof(float) * (size_t)n * dpad;
     cudaError_t e = cudaMalloc(&h->base, bytes);
     if (e != cudaSuccess) {
@@ -303,6 +306,10 @@ int annb::flat_choose_nsplit(int64_t n, int nq, int bq, int64_t* rows_per_split,
 }
 
 extern "C" {
+
+static int flat_exact_pruned(ann_flat* h, ann_workspace* ws, const float* qdev, int nq, int kk, int64_t* ids_dev,
+                             float* dists_dev, cudaStream_t st, bool* done);
+static int flat_check_err(ann_flat* h);
 
 int ann_flat_query(ann_flat* h, ann_workspace* ws, const float* queries, int32_t nq, int64_t ldq, int32_t k,
                    int32_t mode, int32_t mem, int64_t* out_ids, float* out_dists, void* stream) {
@@ -391,7 +398,14 @@ int ann_flat_query(ann_flat* h, ann_workspace* ws, const float* queries, int32_t
 
     // ---- search ----
     const int prec = h->prof.begin(st);
-    if (mode == ANN_MODE_EXACT) {
+    bool pruned = false;
+    if (mode == ANN_MODE_EXACT && h->query_tile == 0) {  // a set tile asks for the scan itself
+        if ((rc = flat_exact_pruned(h, ws, qdev, nq, kk, ids_dev, dists_dev, st, &pruned))) return rc;
+    }
+    if (pruned) {
+        h->prof.mark(prec, st);
+        if (prec >= 0) h->prof.launches += 1;
+    } else if (mode == ANN_MODE_EXACT) {
         float* skey = cv.take<float>((size_t)nq * nsplit * kk);
         int* sid = cv.take<int>((size_t)nq * nsplit * kk);
         float* qpair = cv.take<float>((size_t)(nq + 1) / 2 * 2 * dpad);
@@ -449,6 +463,7 @@ int ann_flat_query(ann_flat* h, ann_workspace* ws, const float* queries, int32_t
         if (out_dists)
             ANN_CUDA_TRY(cudaMemcpyAsync(out_dists, dists_dev, sizeof(float) * (size_t)nq * kk, cudaMemcpyDeviceToHost, st));
         ANN_CUDA_TRY(cudaStreamSynchronize(st));
+        if (pruned) return flat_check_err(h);
     }
     return ANN_OK;
 }
@@ -511,7 +526,10 @@ static int flat_ensure_bf16(ann_flat* h, cudaStream_t st) {
     }
     const int64_t mult = tc_row_mult(h->n);
     int rc = launch_tc_operand(h->base, h->n, h->dim, h->dpad, b, kpad, kTcBase, h->metric, mult, st);
-    if (rc) return rc;
+    if (rc) {
+        cudaFree(b);
+        return rc;
+    }
     ANN_CUDA_TRY(cudaStreamSynchronize(st));
     h->base_bf16 = b;
     h->row_mult = mult;
@@ -557,6 +575,7 @@ struct FlatTc {
     const float2* cfac;
 };
 static int flat_ensure_tc(ann_flat* h, cudaStream_t st, FlatTc* t) {
+    std::lock_guard<std::mutex> lk(h->tc_mu);
     int rc = h->tc_kind == kTcE4M3 ? flat_ensure_e4m3(h, st) : flat_ensure_bf16(h, st);
     if (rc) return rc;
     t->kind = h->tc_kind;
@@ -584,6 +603,177 @@ static int flat_check_err(ann_flat* h) {
         set_error("a device-side wait gave up after its time limit; the results are invalid");
         return ANN_ERR_TIMEOUT;
     }
+    return ANN_OK;
+}
+
+// The BF16 copy and its keys' bounds for the pruned exact scan. Laying them out costs about 0.5 ms + 3.1e-6 us an
+// element (1.7 ms at 1M x 384), a pruned call saves 40 us and up, so a base that is searched only once or twice
+// should not pay: the calls' estimated savings add up (prune_credit_us), and the copy is laid out by the call
+// that brings them to its cost -- at once for a large batch, after a dozen single queries otherwise. Measured, scan
+// / pruned, us a call: 1M x 384: 376 / 259 (1 query), 1121 / 256 (8), 45342 / 967 (1,000); 32768 x 64: 105 / 67
+// (1), 2550 / 172 (1,000). *ok = false (and no error) where the search keeps to the plain scan: not yet laid out,
+// a copy that would take more than half of the free memory, or rows that the bounds do not cover.
+static int flat_ensure_pruned(ann_flat* h, int nq, cudaStream_t st, bool* ok) {
+    *ok = false;
+    std::lock_guard<std::mutex> lk(h->tc_mu);
+    if (!h->bounds_known) {
+        const double elems = (double)h->n * h->dim;
+        h->prune_credit_us += 40.0 + elems * (nq <= 4 ? 0.25e-6 + 0.2e-6 * (nq - 1) : 1.0e-7 * nq);
+        if (!h->base_bf16 && h->prune_credit_us < 500.0 + 3.1e-6 * elems) return ANN_OK;
+        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+        ANN_CUDA_TRY(cudaStreamIsCapturing(st, &cs));
+        if (cs != cudaStreamCaptureStatusNone) return ANN_OK;
+        if (!h->base_bf16) {
+            size_t mfree = 0, mtotal = 0;
+            ANN_CUDA_TRY(cudaMemGetInfo(&mfree, &mtotal));
+            if (sizeof(__nv_bfloat16) * (size_t)h->n * tc_kpad(h->dim, h->metric) > mfree / 2) return ANN_OK;
+        }
+        int rc = flat_ensure_bf16(h, st);
+        if (rc == ANN_ERR_NOMEM) {
+            clear_error();
+            return ANN_OK;
+        }
+        if (rc) return rc;
+        unsigned *d2 = nullptr, h2[2] = {0, 0};
+        if (cudaMalloc(&d2, sizeof(h2)) != cudaSuccess) {
+            cudaGetLastError();
+            return ANN_OK;
+        }
+        rc = launch_base_norms(h->base, h->n, h->dim, h->dpad, d2, st);
+        cudaError_t e = cudaSuccess;
+        if (!rc) e = cudaMemcpyAsync(h2, d2, sizeof(h2), cudaMemcpyDeviceToHost, st);
+        if (!rc && e == cudaSuccess) e = cudaStreamSynchronize(st);
+        cudaFree(d2);
+        if (rc) return rc;
+        ANN_CUDA_TRY(e);
+        float s2, e2;
+        memcpy(&s2, &h2[0], 4);
+        memcpy(&e2, &h2[1], 4);
+        const float c = std::sqrt(s2), r = std::sqrt(e2);
+        h->bounds = PruneBounds{};
+        if (c >= kPruneNormMin && c <= kPruneNormMax && r <= c) h->bounds = PruneBounds{c * 1.001f, r * 1.001f};
+        h->bounds_known = true;
+    }
+    *ok = h->bounds.cmax > 0.f;
+    return ANN_OK;
+}
+
+// The pruned form of the exact scan (flat_prune.cu) for queries qdev [nq, dpad]; *done = false, and nothing
+// written, where the plain scan answers the call.
+static int flat_exact_pruned(ann_flat* h, ann_workspace* ws, const float* qdev, int nq, int kk, int64_t* ids_dev,
+                             float* dists_dev, cudaStream_t st, bool* done) {
+    *done = false;
+    const int64_t n = h->n;
+    const int dpad = h->dpad;
+    if (n < kPruneMinRows || n < 64 * (int64_t)kk || !prune_fits(kk, dpad)) return ANN_OK;
+    bool ok = false;
+    int rc = flat_ensure_pruned(h, nq, st, &ok);
+    if (rc || !ok) return rc;
+    const int bq = std::min(flat_scan_bq(nq), flat_scan_max_bq(kk));
+    const bool stream_form = flat_stream_eligible(bq, kk, dpad);
+    // a sample of about 64 tiles of 256 rows, an eighth of a small base
+    const int64_t full_tiles = n / 256;
+    const int64_t want_tiles = std::min<int64_t>(64, full_tiles / 8);
+    const int stride = (int)(full_tiles / want_tiles);
+    const int64_t S = full_tiles / stride * 256;
+    const int rF = prune_bar_rank(kk, S, n), cap = prune_cap(kk);
+    const int kpad = h->kpad;
+    constexpr int kChunk = 5120;  // queries at a time: 0.5 GB of sampled keys and survivors
+    const int nchunks = (int)ceil_div(nq, kChunk);
+    const int qc = nchunks == 1 ? nq : (int)std::min<int64_t>(kChunk, ceil_div(ceil_div(nq, nchunks), 128) * 128);
+    // the scan of the queries left over: up to one split per SM, its lists bounded to 256 MB
+    int64_t rps = 0;
+    const int ns_plain = flat_choose_nsplit(n, qc, bq, &rps, flat_scan_ctas_per_sm(bq, kk, dpad, h->metric));
+    int nsplit = (int)std::max<int64_t>(ns_plain, std::min<int64_t>(kNumSMs, ((int64_t)256 << 20) / ((int64_t)qc * kk * 8)));
+    rps = ceil_div(ceil_div(n, nsplit), 256) * 256;
+    nsplit = (int)ceil_div(n, rps);
+    Sizer sz;
+    sz.take<__nv_bfloat16>((size_t)qc * kpad);
+    sz.take<float>((size_t)qc * S);
+    for (int i = 0; i < 4; ++i) sz.take<float>((size_t)qc);
+    sz.take<float>((size_t)qc * cap);
+    sz.take<int>((size_t)qc * cap);
+    for (int i = 0; i < 2; ++i) sz.take<int>((size_t)qc);
+    sz.take<int>(1);
+    sz.take<float>((size_t)qc * dpad);
+    sz.take<float>((size_t)(qc + 1) / 2 * 2 * dpad);
+    sz.take<float>((size_t)qc * nsplit * kk);
+    sz.take<int>((size_t)qc * nsplit * kk);
+    if ((rc = ws_reserve_big(ws, sz.bytes()))) {
+        if (rc != ANN_ERR_NOMEM) return rc;
+        clear_error();
+        return ANN_OK;
+    }
+    Carver cv(ws->big);
+    __nv_bfloat16* qb = cv.take<__nv_bfloat16>((size_t)qc * kpad);
+    float* kA = cv.take<float>((size_t)qc * S);
+    float* win = cv.take<float>((size_t)qc);
+    float* tauF = cv.take<float>((size_t)qc);
+    float* tauX = cv.take<float>((size_t)qc);
+    float* tauU = cv.take<float>((size_t)qc);
+    float* fkey = cv.take<float>((size_t)qc * cap);
+    int* fcol = cv.take<int>((size_t)qc * cap);
+    int* rcount = cv.take<int>((size_t)qc);
+    int* list = cv.take<int>((size_t)qc);
+    int* count = cv.take<int>(1);
+    float* qg = cv.take<float>((size_t)qc * dpad);
+    float* qpair = cv.take<float>((size_t)(qc + 1) / 2 * 2 * dpad);
+    float* skey = cv.take<float>((size_t)qc * nsplit * kk);
+    int* sid = cv.take<int>((size_t)qc * nsplit * kk);
+    for (int q0 = 0; q0 < nq; q0 += qc) {
+        const int nc = std::min(qc, nq - q0);
+        const float* q = qdev + (size_t)q0 * dpad;
+        PruneArgs p{};
+        p.base = h->base;
+        p.n = n;
+        p.dim = h->dim;
+        p.dpad = dpad;
+        p.mult = h->row_mult;
+        p.q = q;
+        p.nq = nc;
+        p.k = kk;
+        p.metric = h->metric;
+        p.stream_form = stream_form;
+        p.b = h->bounds;
+        p.win = win;
+        p.tauF = tauF;
+        p.tauX = tauX;
+        p.cap = cap;
+        p.fkey = fkey;
+        p.fcol = fcol;
+        p.rcount = rcount;
+        p.list = list;
+        p.count = count;
+        p.out_ids = ids_dev + (size_t)q0 * kk;
+        p.out_dists = dists_dev ? dists_dev + (size_t)q0 * kk : nullptr;
+        if ((rc = launch_tc_operand(q, nc, h->dim, dpad, qb, kpad, kTcQuery, h->metric, 0, st))) return rc;
+        if ((rc = launch_prune_windows(p, st))) return rc;
+        TcGemmArgs sa{nc, (int)S, kpad, nullptr, kA, S, h->d_err};
+        sa.b_tile_stride = stride;
+        sa.b_rows = n;
+        if ((rc = launch_tc_gemm(qb, h->base_bf16, sa, st))) return rc;
+        if ((rc = launch_sample_bars(kA, (int)S, nc, rF, rF, tauF, tauU, st))) return rc;
+        if ((rc = launch_prune_bars(p, st))) return rc;
+        TcGemmArgs fa{nc, (int)n, kpad, nullptr, nullptr, n, h->d_err};
+        fa.tau = tauX;
+        fa.fkey = fkey;
+        fa.fcol = fcol;
+        fa.row_cap = cap;
+        fa.rcount = rcount;
+        if ((rc = launch_tc_gemm(qb, h->base_bf16, fa, st))) return rc;
+        if ((rc = launch_prune_finish(p, st))) return rc;
+        // the queries on the list, by the plain scan (none, nearly always: the kernels read the count and return)
+        if ((rc = launch_prune_gather(q, dpad, list, count, nc, qg, st))) return rc;
+        FlatScanArgs a{h->base, n, dpad, qg, nc, h->metric, kk, rps, nsplit, skey, sid};
+        a.qpair = qpair;
+        a.nq_dev = count;
+        if ((rc = launch_flat_scan(a, bq, st))) return rc;
+        MergeArgs m{skey, sid, nc, nsplit, kk, kk, h->metric == ANN_METRIC_IP ? 1 : 0, p.out_ids, p.out_dists};
+        m.nq_dev = count;
+        m.out_rows = list;
+        if ((rc = launch_merge_splits(m, st))) return rc;
+    }
+    *done = true;
     return ANN_OK;
 }
 

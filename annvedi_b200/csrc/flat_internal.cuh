@@ -5,6 +5,7 @@
 #include <cuda_bf16.h>
 
 #include "common.cuh"
+#include "flat_prune.cuh"
 #include "runtime.cuh"
 
 struct ann_flat {
@@ -26,6 +27,10 @@ struct ann_flat {
     uint8_t* base_e4m3 = nullptr;        // [n, kpad8] E4M3 operand form, Weyl order, built on first use
     float2* fac_e4m3 = nullptr;          // [n] its per-row key factors
     int kpad8 = 0;                       // dim rounded up to 32
+    std::mutex tc_mu;                    // serialises the first use of the operand forms above
+    annb::PruneBounds bounds;            // of the BF16 copy's keys (cmax 0: the rows are not covered)
+    bool bounds_known = false;
+    double prune_credit_us = 0.0;        // what pruning would have saved the exact searches so far (estimated)
 };
 
 namespace annb {

@@ -1,0 +1,372 @@
+// The exact scan of a query batch with its rows pruned by tensor-core keys.
+//
+// The exact scan (flat_scan.cu) forms every (query, row) distance on the FP32 units: 2 N dim instructions a query,
+// 45.3 ms for 1,000 queries over 1M x 384 with the tensor cores idle (1.07 ms pruned); a single query reads 4 bytes
+// an element (0.37 ms, 0.26 ms pruned). Only about k distances a query are kept. Here the BF16 tensor-core keys (tc_gemm.cu) say which rows can be among them, and
+// only those rows' FP32 distances are formed, with the scan's own sums, so that ids and distances are the scan's
+// bit for bit:
+//   1. a BF16 key differs from the real |x|^2 - 2 x.q (or -x.q) by at most eps (launch_prune_windows);
+//   2. a sampled bar tauF that about a few k keys pass, and a filter pass that keeps every key <= tauF + w,
+//      w = 2 eps + delta, delta covering the rounding of the FP32 distances themselves;
+//   3. per query: T, the k-th smallest kept key, is the k-th smallest of all if T <= tauF. A row whose key exceeds
+//      T + w is farther, in the scan's FP32 arithmetic as in real arithmetic, than the k rows of smallest key, so
+//      the best k by (distance, id) are among the kept keys <= T + w; those rows' distances are formed and the
+//      best k taken.
+// A query that the bound does not cover (norms out of range, NaN), whose bar was too low, or with more survivors
+// than fit goes to a list that the plain scan answers right after, its length read on the device: no step waits
+// for the host.
+#include "common.cuh"
+#include "flat_prune.cuh"
+
+#include <cmath>
+
+#include <cuda_bf16.h>
+
+namespace annb {
+
+namespace {
+
+constexpr int kFinThreads = 256;
+constexpr int kFinWarps = kFinThreads / 32;
+constexpr int kFinPitch = 36;  // floats per staged row of 32: 16-byte reads of 8 rows fall in different banks
+constexpr int kFinStages = 2;
+
+__device__ __forceinline__ uint32_t ord_f32(float f) {
+    const uint32_t u = __float_as_uint(f);
+    return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
+}
+__device__ __forceinline__ float f32_ord(uint32_t o) {
+    return __uint_as_float((o & 0x80000000u) ? (o & 0x7fffffffu) : ~o);
+}
+__device__ __forceinline__ int row_of_pos(int64_t p, int64_t n, int64_t mult) {
+    return (int)(((unsigned __int128)p * (uint64_t)mult) % (uint64_t)n);
+}
+__device__ __forceinline__ void cp_async16_pr(float* smem, const float* gmem) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((unsigned)__cvta_generic_to_shared(smem)), "l"(gmem)
+                 : "memory");
+}
+
+// one warp per row, grid-stride
+__global__ void __launch_bounds__(256) base_norms_kernel(const float* __restrict__ x, int64_t n, int dim, int64_t ld,
+                                                         unsigned* out2) {
+    const int lane = threadIdx.x & 31;
+    unsigned ms = 0, mr = 0;
+    for (int64_t r = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; r < n;
+         r += ((int64_t)gridDim.x * blockDim.x) >> 5) {
+        float s = 0.f, e = 0.f;
+        for (int d = lane; d < dim; d += 32) {
+            const float v = x[r * ld + d];
+            const float t = v - __bfloat162float(__float2bfloat16_rn(v));  // exact
+            s = fmaf(v, v, s);
+            e = fmaf(t, t, e);
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            s += __shfl_xor_sync(0xffffffffu, s, o);
+            e += __shfl_xor_sync(0xffffffffu, e, o);
+        }
+        // non-negative floats order as their bit patterns, NaN above them all (its sign cleared)
+        ms = max(ms, __float_as_uint(s) & 0x7fffffffu);
+        mr = max(mr, __float_as_uint(e) & 0x7fffffffu);
+    }
+    if (lane == 0) {
+        atomicMax(&out2[0], ms);
+        atomicMax(&out2[1], mr);
+    }
+}
+
+// One warp per query: its window w = 2 eps + delta. With x^, q^ the BF16 operands,
+//   |x.q - x^.q^| <= |x - x^| |q| + |x^| |q - q^| <= rmax |q| + (cmax + rmax) |q - q^|,
+// (residual norms taken, not bounded by 2^-9: about 0.4 of that), and the FP32 accumulation of the dim + 3 products
+// (truncating adds allowed for: 2^-21 each, of the terms' absolute sum) adds acc * sum. delta bounds the rounding
+// of two FP32 distances summed over dim terms. The sums taken here are FP32 too: the factor 1.002 covers them.
+__global__ void __launch_bounds__(256) prune_windows_kernel(PruneArgs a) {
+    const int q = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (q >= a.nq) return;
+    float s = 0.f, e = 0.f;
+    for (int d = lane; d < a.dim; d += 32) {
+        const float v = a.q[(int64_t)q * a.dpad + d];
+        const float t = v - __bfloat162float(__float2bfloat16_rn(v));
+        s = fmaf(v, v, s);
+        e = fmaf(t, t, e);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        s += __shfl_xor_sync(0xffffffffu, s, o);
+        e += __shfl_xor_sync(0xffffffffu, e, o);
+    }
+    if (lane != 0) return;
+    const float qn = sqrtf(s), rq = sqrtf(e), cm = a.b.cmax, rm = a.b.rmax;
+    const float acc = (float)(a.dim + 19) * 4.76837158e-7f;  // (dim + 19) 2^-21
+    const float cross = rm * qn + (cm + rm) * rq;
+    const float sum = (cm + rm) * (qn + rq);
+    float w;
+    if (a.metric == ANN_METRIC_L2)
+        w = 2.f * (2.f * cross + acc * (2.f * sum + cm * cm)) + acc * (qn + cm) * (qn + cm);
+    else
+        w = 2.f * (cross + acc * sum) + 2.f * acc * qn * cm;
+    const bool ok = qn <= kPruneNormMax && (qn >= kPruneNormMin || s == 0.f);  // false for NaN
+    a.win[q] = ok ? w * 1.002f : __int_as_float(0x7fffffff);
+}
+
+__global__ void prune_bars_kernel(PruneArgs a) {
+    const int q = blockIdx.x * blockDim.x + threadIdx.x;
+    if (q == 0) *a.count = 0;
+    if (q >= a.nq) return;
+    a.tauX[q] = __fadd_ru(a.tauF[q], a.win[q]);
+    a.rcount[q] = 0;
+}
+
+// The digit (8 bits) of rank `rem` (1-based) of the block's 256-bin histogram: every thread gets the digit, the
+// count below it and the digit's own count. One bin per thread.
+__device__ __forceinline__ void block_pick(const int* hist, int rem, int* sMisc, int* digit, int* before, int* own) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int c = hist[threadIdx.x];
+    int incl = c;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += y;
+    }
+    if (lane == 31) sMisc[warp] = incl;
+    __syncthreads();
+    for (int w = 0; w < warp; ++w) incl += sMisc[w];
+    if (incl - c < rem && rem <= incl) {
+        sMisc[8] = threadIdx.x;
+        sMisc[9] = incl - c;
+        sMisc[10] = c;
+    }
+    __syncthreads();
+    *digit = sMisc[8];
+    *before = sMisc[9];
+    *own = sMisc[10];
+}
+
+// One block per query (file comment, step 3). Bound by the gather of the kept rows (about 500 rows of 1.5 KB a query
+// at 1M x 384, k = 100): each warp takes 32 rows at a time, 128 bytes of each by coalesced asynchronous copies into
+// its own stage, and each lane then sums its own row in the scan's order -- a row's terms are one serial chain, so
+// 32 rows a warp, not 32 lanes a row, keep the FP32 pipe fed.
+//   staged scan: one chain over d; streaming scan: 8 chains (floats 4o .. 4o + 3 of every 32), added pairwise.
+template <bool STREAM, int METRIC>
+__global__ void __launch_bounds__(kFinThreads) prune_finish_kernel(PruneArgs a) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int cap = a.cap, k = a.k, dpad = a.dpad;
+    float* sX = reinterpret_cast<float*>(smem_raw);                                  // [warps][stages][32 pitch]
+    float* sQ = sX + kFinWarps * kFinStages * 32 * kFinPitch;                        // [dpad]
+    unsigned long long* sE = reinterpret_cast<unsigned long long*>(sQ + dpad);       // [cap] (distance, row)
+    uint32_t* sO = reinterpret_cast<uint32_t*>(sE);                                  // [cap] keys, before sE is filled
+    __shared__ int sHist[256];
+    __shared__ int sMisc[12];
+    __shared__ int sN;
+    const int q = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int cnt = a.rcount[q];
+    const float w = a.win[q], tauF = a.tauF[q];
+    const float* fk = a.fkey + (int64_t)q * cap;
+    const int* fc = a.fcol + (int64_t)q * cap;
+    bool fail = cnt > cap || cnt < k || !(w < kInf);
+    float T = 0.f;
+    if (!fail) {  // the k-th smallest kept key: four 8-bit digits
+        for (int i = tid; i < cnt; i += kFinThreads) sO[i] = ord_f32(fk[i]);
+        uint32_t prefix = 0, mask = 0;
+        int rem = k;
+        for (int shift = 24; shift >= 0; shift -= 8) {
+            sHist[tid] = 0;
+            __syncthreads();
+            for (int i = tid; i < cnt; i += kFinThreads)
+                if ((sO[i] & mask) == prefix) atomicAdd(&sHist[(sO[i] >> shift) & 255u], 1);
+            __syncthreads();
+            int d, before, own;
+            block_pick(sHist, rem, sMisc, &d, &before, &own);
+            rem -= before;
+            prefix |= (uint32_t)d << shift;
+            mask |= 255u << shift;
+        }
+        T = f32_ord(prefix);
+        fail = !(T <= tauF);
+    }
+    if (fail) {  // uniform
+        if (tid == 0) a.list[atomicAdd(a.count, 1)] = q;
+        return;
+    }
+    const float lim = __fadd_ru(T, w);  // <= tauX: every key at or below it was kept
+    if (tid == 0) sN = 0;
+    __syncthreads();
+    for (int d = tid; d < dpad; d += kFinThreads) sQ[d] = a.q[(int64_t)q * dpad + d];
+    for (int i = tid; i < cnt; i += kFinThreads)
+        if (fk[i] <= lim) sE[atomicAdd(&sN, 1)] = (unsigned)row_of_pos(fc[i], a.n, a.mult);
+    __syncthreads();
+    const int m = sN;  // >= k
+    float* myX = sX + warp * kFinStages * 32 * kFinPitch;
+    const int nch = dpad / 32;
+    for (int g = warp * 32; g < m; g += kFinWarps * 32) {
+        const int row = (int)(unsigned)sE[min(g + lane, m - 1)];
+        const int rows = min(32, m - g);
+        auto issue = [&](int c) {
+            if (c < nch) {
+                float* dst = myX + (c % kFinStages) * 32 * kFinPitch;
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const int r = 4 * i + (lane >> 3);
+                    const int rr = __shfl_sync(0xffffffffu, row, r);
+                    if (r < rows)
+                        cp_async16_pr(dst + r * kFinPitch + (lane & 7) * 4,
+                                      a.base + (int64_t)rr * dpad + c * 32 + (lane & 7) * 4);
+                }
+            }
+            asm volatile("cp.async.commit_group;\n" ::: "memory");
+        };
+        float acc[STREAM ? 8 : 1];
+#pragma unroll
+        for (int o = 0; o < (STREAM ? 8 : 1); ++o) acc[o] = 0.f;
+        __syncwarp();  // every lane is done with the last group's stages
+        issue(0);
+        for (int c = 0; c < nch; ++c) {
+            issue(c + 1);
+            asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+            __syncwarp();
+            const float* x = myX + (c % kFinStages) * 32 * kFinPitch + lane * kFinPitch;
+            const float* qc = sQ + c * 32;
+#pragma unroll
+            for (int o = 0; o < 8; ++o) {
+                const float4 xv = *reinterpret_cast<const float4*>(x + 4 * o);
+                const float4 qv = *reinterpret_cast<const float4*>(qc + 4 * o);
+                float& s = acc[STREAM ? o : 0];
+                if (METRIC == ANN_METRIC_L2) {
+                    const float d0 = xv.x - qv.x, d1 = xv.y - qv.y, d2 = xv.z - qv.z, d3 = xv.w - qv.w;
+                    s = fmaf(d0, d0, s);
+                    s = fmaf(d1, d1, s);
+                    s = fmaf(d2, d2, s);
+                    s = fmaf(d3, d3, s);
+                } else {
+                    s = fmaf(xv.x, qv.x, s);
+                    s = fmaf(xv.y, qv.y, s);
+                    s = fmaf(xv.z, qv.z, s);
+                    s = fmaf(xv.w, qv.w, s);
+                }
+            }
+            __syncwarp();  // the stage is free for the copies issued next
+        }
+        asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+        float v = acc[0];
+        if (STREAM)
+            v = ((acc[0] + acc[1 % (STREAM ? 8 : 1)]) + (acc[2 % (STREAM ? 8 : 1)] + acc[3 % (STREAM ? 8 : 1)])) +
+                ((acc[4 % (STREAM ? 8 : 1)] + acc[5 % (STREAM ? 8 : 1)]) +
+                 (acc[6 % (STREAM ? 8 : 1)] + acc[7 % (STREAM ? 8 : 1)]));
+        // + 0: a key of -0 orders with +0, by row
+        if (lane < rows)
+            sE[g + lane] = ((unsigned long long)ord_f32((METRIC == ANN_METRIC_L2 ? v : -v) + 0.f) << 32) | (unsigned)row;
+    }
+    __syncthreads();
+    // the k smallest (distance, row): 8-bit digits from the top until a digit ends at the k-th exactly
+    unsigned long long prefix = 0, mask = 0;
+    int rem = k;
+    for (int shift = 56; shift >= 0; shift -= 8) {
+        sHist[tid] = 0;
+        __syncthreads();
+        for (int i = tid; i < m; i += kFinThreads)
+            if ((sE[i] & mask) == prefix) atomicAdd(&sHist[(int)(sE[i] >> shift) & 255], 1);
+        __syncthreads();
+        int d, before, own;
+        block_pick(sHist, rem, sMisc, &d, &before, &own);
+        rem -= before;
+        prefix |= (unsigned long long)d << shift;
+        mask |= 255ull << shift;
+        if (rem == own) break;  // uniform
+    }
+    unsigned long long* sR = reinterpret_cast<unsigned long long*>(sX);  // the best k, then sorted
+    const int p2 = pow2_ceil(k);
+    if (tid == 0) sN = 0;
+    __syncthreads();
+    for (int i = tid; i < m; i += kFinThreads)
+        if ((sE[i] & mask) <= prefix) sR[atomicAdd(&sN, 1)] = sE[i];
+    for (int i = k + tid; i < p2; i += kFinThreads) sR[i] = ~0ull;
+    __syncthreads();
+    for (int size = 2; size <= p2; size <<= 1)
+        for (int stride = size >> 1; stride > 0; stride >>= 1) {
+            for (int t = tid; t < p2 / 2; t += kFinThreads) {
+                const int lo = 2 * t - (t & (stride - 1)), hi = lo + stride;
+                const unsigned long long x = sR[lo], y = sR[hi];
+                if ((x > y) == ((lo & size) == 0)) {
+                    sR[lo] = y;
+                    sR[hi] = x;
+                }
+            }
+            __syncthreads();
+        }
+    for (int e = tid; e < k; e += kFinThreads) {
+        a.out_ids[(int64_t)q * k + e] = (int64_t)(unsigned)sR[e];
+        if (a.out_dists) {
+            const float key = f32_ord((uint32_t)(sR[e] >> 32));
+            a.out_dists[(int64_t)q * k + e] = METRIC == ANN_METRIC_L2 ? key : 0.f - key;
+        }
+    }
+}
+
+__global__ void prune_gather_kernel(const float* __restrict__ q, int dpad, const int* __restrict__ list,
+                                    const int* __restrict__ count, float* __restrict__ qg) {
+    const int n = *count;
+    for (int j = blockIdx.x; j < n; j += gridDim.x)
+        for (int d = threadIdx.x; d < dpad; d += blockDim.x) qg[(int64_t)j * dpad + d] = q[(int64_t)list[j] * dpad + d];
+}
+
+size_t finish_smem(int cap, int dpad) {
+    return sizeof(float) * ((size_t)kFinWarps * kFinStages * 32 * kFinPitch + dpad) + sizeof(unsigned long long) * cap;
+}
+
+}  // namespace
+
+int prune_cap(int k) { return k <= 128 ? 4096 : 8192; }
+bool prune_fits(int k, int dpad) { return k <= 512 && finish_smem(prune_cap(k), dpad) <= 200 * 1024; }
+
+int prune_bar_rank(int k, int64_t S, int64_t n) {
+    // keys of the k best met in the sample: about Poisson(k S / n); the rank past its 1 - 1e-7 quantile
+    const double lam = (double)k * (double)S / (double)n;
+    double term = std::exp(-lam), cdf = term;
+    int r = 1;
+    while (r < k && 1.0 - cdf > 1e-7) {
+        term *= lam / r;
+        cdf += term;
+        ++r;
+    }
+    return r;
+}
+
+int launch_base_norms(const float* x, int64_t n, int dim, int64_t ld, unsigned* out2, cudaStream_t st) {
+    ANN_CUDA_TRY(cudaMemsetAsync(out2, 0, 2 * sizeof(unsigned), st));
+    if (n == 0) return ANN_OK;
+    base_norms_kernel<<<(unsigned)std::min<int64_t>(ceil_div(n, 8), 16 * kNumSMs), 256, 0, st>>>(x, n, dim, ld, out2);
+    ANN_LAUNCH_CHECK();
+    return ANN_OK;
+}
+
+int launch_prune_windows(const PruneArgs& a, cudaStream_t st) {
+    prune_windows_kernel<<<(unsigned)ceil_div(a.nq, 8), 256, 0, st>>>(a);
+    ANN_LAUNCH_CHECK();
+    return ANN_OK;
+}
+
+int launch_prune_bars(const PruneArgs& a, cudaStream_t st) {
+    prune_bars_kernel<<<(unsigned)ceil_div(a.nq, 256), 256, 0, st>>>(a);
+    ANN_LAUNCH_CHECK();
+    return ANN_OK;
+}
+
+int launch_prune_finish(const PruneArgs& a, cudaStream_t st) {
+    ANN_CHECK_ARG(a.k >= 1 && prune_fits(a.k, a.dpad) && a.dpad % 32 == 0 && a.cap == prune_cap(a.k),
+                  "pruned scan: k=%d, padded dim %d", a.k, a.dpad);
+    auto kern = a.metric == ANN_METRIC_L2
+                    ? (a.stream_form ? prune_finish_kernel<true, ANN_METRIC_L2> : prune_finish_kernel<false, ANN_METRIC_L2>)
+                    : (a.stream_form ? prune_finish_kernel<true, ANN_METRIC_IP> : prune_finish_kernel<false, ANN_METRIC_IP>);
+    ANN_CUDA_TRY(smem_optin(reinterpret_cast<const void*>(kern)));
+    kern<<<a.nq, kFinThreads, finish_smem(a.cap, a.dpad), st>>>(a);
+    ANN_LAUNCH_CHECK();
+    return ANN_OK;
+}
+
+int launch_prune_gather(const float* q, int dpad, const int* list, const int* count, int nq, float* qg, cudaStream_t st) {
+    prune_gather_kernel<<<(unsigned)std::min(nq, 2 * kNumSMs), 128, 0, st>>>(q, dpad, list, count, qg);
+    ANN_LAUNCH_CHECK();
+    return ANN_OK;
+}
+
+}  // namespace annb

@@ -85,12 +85,17 @@ __global__ void __launch_bounds__(256) flat_scan_kernel(FlatScanArgs a) {
     const int warp = tid >> 5;
     const int tq = tid / C::WR;
     const int tr = tid % C::WR;
-    const int q0 = blockIdx.x * BQ;
-    const int split = blockIdx.y;
+    const int k = a.k;
+    // one (query tile, split) per CTA; a batch whose size the device knows (nq_dev) runs on a fixed grid instead,
+    // each CTA taking the tiles that exist in turn
+    if (a.nq_dev) a.nq = min(a.nq, *a.nq_dev);
+    const int n_qt = a.nq_dev ? (a.nq + BQ - 1) / BQ : gridDim.x;
+    for (int item = blockIdx.y * gridDim.x + blockIdx.x; item < n_qt * a.nsplit; item += gridDim.x * gridDim.y) {
+    const int q0 = (item % n_qt) * BQ;
+    const int split = item / n_qt;
     const int64_t row_begin = (int64_t)split * a.rows_per_split;
     int64_t row_end = row_begin + a.rows_per_split;
     if (row_end > a.n) row_end = a.n;
-    const int k = a.k;
 
     for (int i = tid; i < BQ; i += C::THREADS) {
         sCnt[i] = 0;
@@ -290,6 +295,8 @@ __global__ void __launch_bounds__(256) flat_scan_kernel(FlatScanArgs a) {
             oi[e] = e < cnt ? sId[ql * cap + e] : kNoId;
         }
     }
+    __syncthreads();  // the next item reuses the stages and the buffers
+    }
 }
 
 // Merge kernel: one CTA (8 warps) per query reduces nsplit sorted lists of kin pairs to the
@@ -301,13 +308,14 @@ __global__ void __launch_bounds__(256) merge_splits_kernel(MergeArgs a) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     float* sKey = reinterpret_cast<float*>(smem_raw);
     int* sId = reinterpret_cast<int*>(sKey + 8 * cap);
-    const int qi = blockIdx.x;
+    if (a.nq_dev && (int)blockIdx.x >= *a.nq_dev) return;  // the whole block
+    const int qi = a.out_rows ? a.out_rows[blockIdx.x] : blockIdx.x;
     const int k = a.k;
     WarpTopK top;
     top.init(sKey + warp * cap, sId + warp * cap, k);
     const int64_t total = (int64_t)a.nsplit * a.kin;
-    const float* ik = a.in_key + (int64_t)qi * total;
-    const int* ii = a.in_id + (int64_t)qi * total;
+    const float* ik = a.in_key + (int64_t)blockIdx.x * total;
+    const int* ii = a.in_id + (int64_t)blockIdx.x * total;
     for (int64_t base = (int64_t)warp * 32; base < total; base += 8 * 32) {
         const int64_t e = base + lane;
         float kv = kInf;
@@ -420,7 +428,9 @@ __global__ void __launch_bounds__(32 * kStreamWarps) flat_stream_kernel(FlatScan
     int* sCount = bufI + kStreamWarps * BQ * cap;                   // [warps][BQ]
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int oct = lane >> 3, o = lane & 7;
+    if (a.nq_dev) a.nq = min(a.nq, *a.nq_dev);
     const int q0 = blockIdx.x * BQ;
+    if (q0 >= a.nq) return;  // the whole CTA: a tile past the queries the device counted
     const int split = blockIdx.y;
     const int64_t row_begin = (int64_t)split * a.rows_per_split;
     const int64_t row_end = min(row_begin + a.rows_per_split, a.n);
@@ -580,6 +590,7 @@ static int launch_scan_t(FlatScanArgs a, int n_qtiles, cudaStream_t st) {
     ANN_CHECK_ARG(smem <= 227 * 1024, "flat scan: %zu bytes of shared memory for k=%d", smem, a.k);
     ANN_CUDA_TRY(smem_optin(reinterpret_cast<const void*>(kern)));
     dim3 grid(n_qtiles, a.nsplit);
+    if (a.nq_dev) grid = dim3((unsigned)std::min<int64_t>((int64_t)n_qtiles * a.nsplit, 2 * kNumSMs), 1);
     kern<<<grid, C::THREADS, smem, st>>>(a);
     ANN_LAUNCH_CHECK();
     return ANN_OK;
@@ -616,7 +627,8 @@ static int dispatch_bq(const FlatScanArgs& a, int bq, int n_qtiles, cudaStream_t
 
 // qpair[(p dpad + d) 2 + h] = s q[2 p + h][d] (s = -1 for L2, +1 for inner products; 0 past nq)
 __global__ void flat_pair_queries_kernel(const float* __restrict__ q, int nq, int dpad, float s,
-                                         float* __restrict__ qpair) {
+                                         float* __restrict__ qpair, const int* __restrict__ nq_dev) {
+    if (nq_dev) nq = min(nq, *nq_dev);
     const int64_t total = (int64_t)((nq + 1) / 2) * dpad * 2;
     for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x) {
         const int h = (int)(e & 1);
@@ -642,7 +654,7 @@ int launch_flat_scan(const FlatScanArgs& a0, int bq, cudaStream_t st) {
     if (a.qpair && bq >= 32 && a.metric == ANN_METRIC_L2 && a.nq > 0) {  // the paired query tile
         const int64_t total = (int64_t)((a.nq + 1) / 2) * a.dpad * 2;
         flat_pair_queries_kernel<<<(unsigned)std::min<int64_t>(ceil_div(total, 256), 8 * kNumSMs), 256, 0, st>>>(
-            a.q, a.nq, a.dpad, a.metric == ANN_METRIC_L2 ? -1.f : 1.f, a.qpair);
+            a.q, a.nq, a.dpad, a.metric == ANN_METRIC_L2 ? -1.f : 1.f, a.qpair, a.nq_dev);
         ANN_LAUNCH_CHECK();
     } else {
         a.qpair = nullptr;

@@ -22,6 +22,9 @@ struct FlatScanArgs {
     // the queries there as interleaved negated pairs and the scan takes two queries a packed FP32
     // instruction, each half rounding as the scalar form (the same distances)
     float* qpair = nullptr;
+    // optional: the number of queries (at most nq) as the device knows it, read by the kernels; tiles past it do
+    // nothing, so a batch counted on the device needs no host round trip
+    const int* nq_dev = nullptr;
 };
 
 struct MergeArgs {
@@ -36,6 +39,8 @@ struct MergeArgs {
     float* out_dists;        // [nq, k] or nullptr
     int* out_id32 = nullptr;   // [nq, k] raw ids (INT_MAX where fewer than k exist), optional
     float* out_key32 = nullptr; // [nq, k] raw keys (+inf where fewer), optional
+    const int* nq_dev = nullptr;   // optional: queries as the device counted them (at most nq)
+    const int* out_rows = nullptr; // optional: input query j writes output row out_rows[j]
 };
 
 // Pipeline depth of the query tiles of 1..8 queries (HBM-bound: four 36 KB stages keep enough bytes
