@@ -17,6 +17,7 @@
 #include "runtime.cuh"
 #include "flat_internal.cuh"
 #include "ivf.cuh"
+#include "tc_filter.cuh"
 #include "tc_gemm.cuh"
 #include "tc_search.cuh"
 #include "radix_select.cuh"
@@ -754,13 +755,8 @@ static int flat_exact_pruned(ann_flat* h, ann_workspace* ws, const float* qdev, 
         if ((rc = launch_tc_gemm(qb, h->base_bf16, sa, st))) return rc;
         if ((rc = launch_sample_bars(kA, (int)S, nc, rF, rF, tauF, tauU, st))) return rc;
         if ((rc = launch_prune_bars(p, st))) return rc;
-        TcGemmArgs fa{nc, (int)n, kpad, nullptr, nullptr, n, h->d_err};
-        fa.tau = tauX;
-        fa.fkey = fkey;
-        fa.fcol = fcol;
-        fa.row_cap = cap;
-        fa.rcount = rcount;
-        if ((rc = launch_tc_gemm(qb, h->base_bf16, fa, st))) return rc;
+        const TcFilterArgs fa{nc, (int)n, kpad, kTcBF16, tauX, fkey, fcol, cap, rcount, nullptr, nullptr, h->d_err};
+        if ((rc = launch_tc_filter(qb, h->base_bf16, fa, st))) return rc;
         if ((rc = launch_prune_finish(p, st))) return rc;
         // the queries on the list, by the plain scan (none, nearly always: the kernels read the count and return)
         if ((rc = launch_prune_gather(q, dpad, list, count, nc, qg, st))) return rc;
@@ -911,23 +907,17 @@ int ann_flat_query_tc(ann_flat* h, ann_workspace* ws, const float* queries, int3
         int* idRc = idR + (size_t)q0 * R;
         bool done = false;
         if (sampled) {
-            const int nwarps = tc_filter_warps(nc, (int)n);
-            const int64_t main_total = ceil_div((int64_t)nc * rF * n, S);
-            const int64_t rerun_total = ceil_div((int64_t)std::min(nc, kRerunBatch) * R * n, S);
-            const int64_t wcap64 = 4 * ceil_div(std::max(main_total, rerun_total), nwarps) + 1024;
-            const int wcap = (int)std::min<int64_t>(wcap64, INT32_MAX / std::max(1, nwarps));
-            const size_t ent = (size_t)nwarps * wcap;
+            // survivors kept per query: about 3 R pass the fast bar (9 R were met over 5,000 queries of a 4M-row
+            // mixture), n R / S the safe bar of a re-run
+            const int cap = (int)std::min<int64_t>(n, 16 * (int64_t)R);
+            const int cap2 = (int)std::min<int64_t>(n, 2 * ceil_div((int64_t)R * n, S) + 1024);
+            const size_t ent = std::max((size_t)nc * cap, (size_t)std::min(nc, kRerunBatch) * cap2);
             Sizer s2;
             s2.take<float>((size_t)nc * S);            // sample keys
-            s2.take<float>(ent);                       // survivors: key, column, row
+            s2.take<float>(ent);                       // survivors: key, position
             s2.take<int>(ent);
-            s2.take<int>(ent);
-            s2.take<float>(ent);                       // grouped: key, id
-            s2.take<int>(ent);
-            s2.take<int>((size_t)nwarps);              // warp counts
             for (int i = 0; i < 3; ++i) s2.take<float>((size_t)nc);  // fast, safe, gathered bars
-            for (int i = 0; i < 3; ++i) s2.take<int>((size_t)nc);    // row counts, cursors, re-run list
-            s2.take<int64_t>((size_t)nc);              // stream offsets
+            for (int i = 0; i < 2; ++i) s2.take<int>((size_t)nc);    // row counts, re-run list
             s2.take<int>(4);                           // flags
             s2.take<unsigned char>((size_t)kRerunBatch * rowb);
             s2.take<float>((size_t)kRerunBatch);
@@ -936,17 +926,11 @@ int ann_flat_query_tc(ann_flat* h, ann_workspace* ws, const float* queries, int3
             float* kA = cb.take<float>((size_t)nc * S);
             float* fkey = cb.take<float>(ent);
             int* fcol = cb.take<int>(ent);
-            int* frow = cb.take<int>(ent);
-            float* gkey = cb.take<float>(ent);
-            int* gid = cb.take<int>(ent);
-            int* wcnt = cb.take<int>((size_t)nwarps);
             float* tauF = cb.take<float>((size_t)nc);
             float* tauS = cb.take<float>((size_t)nc);
             float* tau2 = cb.take<float>((size_t)nc);
             int* rowcnt = cb.take<int>((size_t)nc);
-            int* cursor = cb.take<int>((size_t)nc);
             int* list = cb.take<int>((size_t)nc);
-            int64_t* offs = cb.take<int64_t>((size_t)nc);
             int* flags = cb.take<int>(4);
             unsigned char* A2 = cb.take<unsigned char>((size_t)kRerunBatch * rowb);
             float* rfac2 = cb.take<float>((size_t)kRerunBatch);
@@ -974,39 +958,28 @@ int ann_flat_query_tc(ann_flat* h, ann_workspace* ws, const float* queries, int3
                 if ((rc = launch_radix_select(bar, nc, st))) return rc;
             }
             h->prof.mark(prec, st);
-            auto filter = [&](const void* A, int M, const float* tau, const float* rf) -> int {
-                TcGemmArgs fa{M, (int)n, kpad, nullptr, nullptr, n, h->d_err};
-                fa.kind = t.kind;
-                fa.col_fac = t.cfac;
-                fa.row_fac = rf;
-                fa.tau = tau;
-                fa.fkey = fkey;
-                fa.fcol = fcol;
-                fa.frow = frow;
-                fa.wcount = wcnt;
-                fa.wcap = wcap;
-                int r = launch_tc_gemm(A, t.base, fa, st);
+            auto filter = [&](const void* A, int M, const float* tau, const float* rf, int rcap) -> int {
+                ANN_CUDA_TRY(cudaMemsetAsync(rowcnt, 0, sizeof(int) * (size_t)M, st));
+                const TcFilterArgs fa{M, (int)n, kpad, t.kind, tau, fkey, fcol, rcap, rowcnt, t.cfac, rf, h->d_err};
+                int r = launch_tc_filter(A, t.base, fa, st);
                 if (r) return r;
-                TcGroupArgs ga{fkey, fcol, frow, wcnt, tc_filter_warps(M, (int)n), wcap, M, n, h->row_mult,
-                               rowcnt, offs, cursor, gkey, gid, flags + 1};
-                return launch_tc_group(ga, st);
+                return launch_max_int(rowcnt, M, flags + 1, st);
             };
-            if ((rc = filter(qbc, nc, tauF, rfc))) return rc;
+            if ((rc = filter(qbc, nc, tauF, rfc, cap))) return rc;
             h->prof.mark(prec, st);
             if (prec >= 0) h->prof.filter_launches += 1;
             ANN_CUDA_TRY(cudaMemsetAsync(flags, 0, sizeof(int), st));
             if ((rc = launch_tc_bar_check(rowcnt, nc, R, list, flags, st))) return rc;
-            int hf[2] = {0, 0};  // re-runs, largest warp count
+            int hf[2] = {0, 0};  // re-runs, most survivors of a query
             ANN_CUDA_TRY(cudaMemcpyAsync(hf, flags, sizeof(hf), cudaMemcpyDeviceToHost, st));
             ANN_CUDA_TRY(cudaStreamSynchronize(st));
             int ngemm = 2;
-            if (hf[1] <= wcap) {
+            if (hf[1] <= cap) {
                 RadixSelectArgs sv{};
-                sv.keys = gkey;
-                sv.ld = (int64_t)ent;
-                sv.offs = offs;
+                sv.keys = fkey;
+                sv.ld = cap;
                 sv.lens32 = rowcnt;
-                sv.ids = gid;
+                sv.ids = fcol;
                 sv.R = R;
                 sv.out_key = keyRc;
                 sv.out_id = idRc;
@@ -1016,19 +989,22 @@ int ann_flat_query_tc(ann_flat* h, ann_workspace* ws, const float* queries, int3
                     const int nb = std::min(kRerunBatch, hf[0] - j0);
                     if ((rc = launch_tc_gather(qbc, (int)rowb, list + j0, nb, tauS, A2, tau2, rfc, rfac2, st)))
                         return rc;
-                    if ((rc = filter(A2, nb, tau2, e4 ? rfac2 : nullptr))) return rc;
+                    if ((rc = filter(A2, nb, tau2, e4 ? rfac2 : nullptr, cap2))) return rc;
                     ++ngemm;
                     int hmax = 0;
                     ANN_CUDA_TRY(cudaMemcpyAsync(&hmax, flags + 1, sizeof(int), cudaMemcpyDeviceToHost, st));
                     ANN_CUDA_TRY(cudaStreamSynchronize(st));
-                    if (hmax > wcap) {
+                    if (hmax > cap2) {
                         done = false;
                         break;
                     }
                     RadixSelectArgs sv2 = sv;
+                    sv2.ld = cap2;
                     sv2.out_rows = list + j0;
                     if ((rc = launch_radix_select(sv2, nb, st))) return rc;
                 }
+                // positions of the operand copy -> rows
+                if (done && (rc = launch_tc_map_ids(idRc, (int64_t)nc * R, n, h->row_mult, st))) return rc;
             }
             h->prof.mark(prec, st);
             if (prec >= 0) h->prof.tc_launches += ngemm;

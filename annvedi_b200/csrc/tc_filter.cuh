@@ -1,0 +1,22 @@
+// Launch interface of the dense tensor-core filter pass (tc_filter.cu).
+#pragma once
+#include "tc_gemm.cuh"
+
+namespace annb {
+
+struct TcFilterArgs {
+    int M, N, K;           // A [M, K] queries, B [N, K] base rows in operand form (tc_gemm.cuh); K as launch_tc_gemm takes it
+    int kind;              // kTcBF16 or kTcE4M3
+    const float* tau;      // [M] bars: keys <= tau[m] are kept (NaN: none)
+    float* fkey;           // [M, cap] kept keys of row m, in no particular order
+    int* fcol;             // [M, cap] their columns
+    int cap;
+    int* rcount;           // [M] keys kept (zeroed by the caller); may exceed cap: nothing is written past it
+    const float2* col_fac; // E4M3: per B row, per A row (TcGemmArgs)
+    const float* row_fac;
+    int* err;              // device flag set (to 2) if a bounded wait gives up
+    uint64_t wait_ns = 0;
+};
+int launch_tc_filter(const void* A, const void* B, const TcFilterArgs& a, cudaStream_t st);
+
+}  // namespace annb

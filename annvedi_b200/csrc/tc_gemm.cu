@@ -14,176 +14,24 @@
 //             instruction, 4 per stage); tcgen05.commit frees each stage and publishes each tile;
 //   warps 2.. epilogue: 8 warps, two per TMEM lane quarter (warp w reads lanes 32 * (w % 4)), each
 //             taking half of the 256 columns, for the key-matrix and grouped forms; 16 warps, four
-//             per quarter taking 64 columns each, for the filter form, whose per-key test and
+//             per quarter taking 64 columns each, for the grouped filter form, whose per-key test and
 //             survivor compaction are bound by issue latency at two warps per scheduler.
 //             tcgen05.ld 2 x 32 columns per wait, then either store the keys (transposed through
-//             shared memory into coalesced rows) or, in filter mode, one test per key against the
-//             row's bar (the sign bit of a packed FP32 difference, gathered by funnel shifts);
-//             survivors go to the warp's own region at slots from a warp prefix sum (no atomics,
-//             nothing waits on memory).
+//             shared memory into coalesced rows) or, in the grouped filter mode, one test per key against
+//             its query's bar (the sign bit of a packed FP32 difference, gathered by funnel shifts);
+//             survivors go to the query's own buffer, one atomic per row and 64 columns. (The dense filter
+//             pass, whose survivors are rarer, is tc_filter.cu.)
 // Every mbarrier wait is bounded (about 2 s); a timeout raises a device flag and the CTA winds down.
 #include <cuda.h>
 #include <cuda_fp8.h>
 
 #include "common.cuh"
 #include "tc_gemm.cuh"
+#include "tc_ptx.cuh"
 
 namespace annb {
 
 namespace {
-
-// A k-block is one 128-byte row per operand row: 64 BF16 or 128 E4M3 elements.
-constexpr int kBM = 128, kBN = 256, kBK = 64;
-constexpr int kRowBytes = 128;
-constexpr int kABytes = kBM * kRowBytes;  // 16 KB
-constexpr int kBBytes = kBN * kRowBytes;  // 32 KB
-template <int KIND>
-struct KindOf {
-    static constexpr int kBlockK = KIND == kTcBF16 ? 64 : 128;  // elements per k-block
-    static constexpr int kMmaK = KIND == kTcBF16 ? 16 : 32;     // elements per MMA
-};
-constexpr int kTmemCols = 512;
-
-__device__ __forceinline__ uint32_t su32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-// 4 bytes from global src to shared dst, asynchronously (zeros when !valid: no bytes are read)
-__device__ __forceinline__ void cp_async4(float* dst, const float* src, bool valid) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(su32(dst)), "l"(src), "r"(valid ? 4 : 0)
-                 : "memory");
-}
-__device__ __forceinline__ uint64_t gtimer() {
-    uint64_t t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
-}
-__device__ __forceinline__ void bar_init(uint64_t* b, uint32_t n) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(su32(b)), "r"(n) : "memory");
-}
-__device__ __forceinline__ bool bar_try(uint64_t* b, uint32_t parity) {
-    uint32_t ok;
-    asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
-                 : "=r"(ok)
-                 : "r"(su32(b)), "r"(parity)
-                 : "memory");
-    return ok != 0;
-}
-// try_wait that may suspend the thread for up to 0.1 ms (woken early when the phase completes), so a
-// waiting warp takes few issue slots from the epilogue warps that share its scheduler
-__device__ __forceinline__ bool bar_try_sleep(uint64_t* b, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n selp.u32 %0, 1, 0, p;\n}"
-        : "=r"(ok)
-        : "r"(su32(b)), "r"(parity), "r"(100000u)
-        : "memory");
-    return ok != 0;
-}
-// Waits for the phase; gives up after `limit_ns` (2 s when 0), sets *err = 2 and returns false.
-__device__ __forceinline__ bool bar_wait(uint64_t* b, uint32_t parity, int* err, uint64_t limit_ns = 0) {
-    if (bar_try(b, parity)) return true;
-    const uint64_t limit = limit_ns ? limit_ns : 2000000000ull;
-    const uint64_t t0 = gtimer();
-    while (!bar_try_sleep(b, parity))
-        if (gtimer() - t0 > limit) {
-            if (err) atomicExch(err, 2);
-            return false;
-        }
-    return true;
-}
-__device__ __forceinline__ void bar_arrive(uint64_t* b) {
-    asm volatile("{\n .reg .b64 st;\n mbarrier.arrive.shared::cta.b64 st, [%0];\n}" ::"r"(su32(b)) : "memory");
-}
-__device__ __forceinline__ void bar_expect(uint64_t* b, uint32_t bytes) {
-    asm volatile("{\n .reg .b64 st;\n mbarrier.arrive.expect_tx.shared::cta.b64 st, [%0], %1;\n}" ::"r"(su32(b)),
-                 "r"(bytes)
-                 : "memory");
-}
-__device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* tm, int c0, int c1, uint64_t* bar) {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
-            su32(dst)),
-        "l"(tm), "r"(c0), "r"(c1), "r"(su32(bar))
-        : "memory");
-}
-// Shared-memory matrix descriptor for a K-major tile in the 128-byte swizzle layout (rows of 128 B,
-// 8-row groups 1024 B apart): start address >> 4, leading offset 1 (unused with swizzle), stride
-// offset 1024 >> 4, descriptor version 1, layout type 2 (128-byte swizzle).
-__device__ __forceinline__ uint64_t sw128_desc(const void* p) {
-    const uint64_t addr = (su32(p) >> 4) & 0x3FFFull;
-    return addr | (1ull << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
-}
-// Instruction descriptors: FP32 accumulator (bits 4-5 = 1), A and B K-major, N = 256 (bits 17-22 = N / 8),
-// M = 128 (bits 24-28 = M / 16); A and B types in bits 7-9 and 10-12: BF16 = 1 under kind::f16, E4M3 = 0
-// under kind::f8f6f4.
-constexpr uint32_t kIdescShape = (1u << 4) | ((uint32_t)(kBN >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);
-constexpr uint32_t kIdescBF16 = kIdescShape | (1u << 7) | (1u << 10);
-constexpr uint32_t kIdescE4M3 = kIdescShape;
-// kind::i8: S32 accumulator (bits 4-5 = 2), A signed (bits 7-9 = 1), B unsigned (bits 10-12 = 0)
-constexpr uint32_t kIdescI8 = (2u << 4) | ((uint32_t)(kBN >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24) | (1u << 7);
-
-// One MMA of the 32 bytes of K that follow each descriptor's start: 16 BF16 or 32 E4M3 elements.
-template <int KIND>
-__device__ __forceinline__ void mma_issue(uint32_t tmem_d, uint64_t ad, uint64_t bd, uint32_t accumulate) {
-    if (KIND == kTcBF16)
-        asm volatile(
-            "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-            " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}" ::"r"(tmem_d),
-            "l"(ad), "l"(bd), "r"(kIdescBF16), "r"(accumulate)
-            : "memory");
-    else if (KIND == kTcE4M3)
-        asm volatile(
-            "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-            " tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n}" ::"r"(tmem_d),
-            "l"(ad), "l"(bd), "r"(kIdescE4M3), "r"(accumulate)
-            : "memory");
-    else
-        asm volatile(
-            "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-            " tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n}" ::"r"(tmem_d),
-            "l"(ad), "l"(bd), "r"(kIdescI8), "r"(accumulate)
-            : "memory");
-}
-// An accumulator read from TMEM as a float: FP32 bits, or (kind::i8) an int32 converted (exact below 2^24).
-template <int KIND>
-__device__ __forceinline__ float acc_value(uint32_t r) {
-    return KIND == kTcI8 ? __int2float_rn((int)r) : __uint_as_float(r);
-}
-__device__ __forceinline__ void mma_commit(uint64_t* bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(su32(bar))
-                 : "memory");
-}
-// tcgen05.ld of 32 consecutive columns of the warp's 32 lanes; the registers are valid only after
-// tmem_wait (which names them, so no use is scheduled before the wait).
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,"
-        "%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
-          "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
-          "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-        : "r"(taddr));
-}
-__device__ __forceinline__ void tmem_wait(uint32_t (&r)[32]) {
-    asm volatile("tcgen05.wait::ld.sync.aligned;"
-                 : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]),
-                   "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]),
-                   "+r"(r[15]), "+r"(r[16]), "+r"(r[17]), "+r"(r[18]), "+r"(r[19]), "+r"(r[20]), "+r"(r[21]),
-                   "+r"(r[22]), "+r"(r[23]), "+r"(r[24]), "+r"(r[25]), "+r"(r[26]), "+r"(r[27]), "+r"(r[28]),
-                   "+r"(r[29]), "+r"(r[30]), "+r"(r[31])
-                 :
-                 : "memory");
-}
-// Orders a second register set after the wait already issued for the first.
-__device__ __forceinline__ void tmem_after_wait(uint32_t (&r)[32]) {
-    asm volatile(""
-                 : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]),
-                   "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]),
-                   "+r"(r[15]), "+r"(r[16]), "+r"(r[17]), "+r"(r[18]), "+r"(r[19]), "+r"(r[20]), "+r"(r[21]),
-                   "+r"(r[22]), "+r"(r[23]), "+r"(r[24]), "+r"(r[25]), "+r"(r[26]), "+r"(r[27]), "+r"(r[28]),
-                   "+r"(r[29]), "+r"(r[30]), "+r"(r[31])
-                 :
-                 : "memory");
-}
 
 // A grouped-mode work item: A rows [a0, a0 + am), B rows [b0, b0 + bn).
 struct GroupTile {
@@ -349,8 +197,6 @@ __global__ void __launch_bounds__(epi_threads(EPI), 1) tc_gemm_kernel(const __gr
         const int ew = warp - 2;
         const int col0 = kCols * (ew >> 2);  // this warp's share of the tile's columns
         float* tw = sT + ew * epi_area_floats(EPI);
-        const int64_t wbase = ((int64_t)blockIdx.x * EPI + ew) * a.wcap;
-        int wcount = 0;  // survivors met by this warp (uniform across the warp)
         int64_t acc = 0;
         for (int64_t t = blockIdx.x; t < tiles; t += gridDim.x, ++acc) {
             const int b = (int)(acc & 1);
@@ -383,7 +229,7 @@ __global__ void __launch_bounds__(epi_threads(EPI), 1) tc_gemm_kernel(const __gr
             // so that they land while the MMAs run) into its (otherwise unused) transpose buffer as two arrays
             // (x then y), so that the factors of two adjacent columns load as one float2 broadcast; zeros past
             // the valid columns
-            const bool staged = a.col_fac != nullptr && (kFilterOnly || a.out == nullptr);
+            const bool staged = kFilterOnly && a.col_fac != nullptr;
             float* sfx = tw;
             float* sfy = tw + kCols;
             if (staged) {
@@ -456,7 +302,6 @@ __global__ void __launch_bounds__(epi_threads(EPI), 1) tc_gemm_kernel(const __gr
                 __syncwarp();
             }
             const bool has_an = a.normA != nullptr;  // uniform
-            const bool rowbuf = a.row_cap > 0 && (kFilterOnly || a.out == nullptr);
             // filter keys of the 32 columns from col0 + c + 32 h (raw accumulators r): the row norm, the
             // scale factors, NaN past the tile's valid columns
             auto half_keys = [&](const uint32_t (&r)[32], int h, int c, float (&v)[32]) {
@@ -529,7 +374,7 @@ __global__ void __launch_bounds__(epi_threads(EPI), 1) tc_gemm_kernel(const __gr
                 // per-row buffers: the survivors of the 64 columns under one atomic, so that the lane waits
                 // for one round trip per 64 columns; one 32-column half in registers at a time (the first
                 // half's keys are loaded and made again for their stores)
-                if (rowbuf) {
+                if (kFilterOnly) {
                     uint32_t r[32];
                     float v[32];
                     __syncwarp();  // .sync.aligned loads after the divergent survivor stores of the last step
@@ -572,22 +417,7 @@ __global__ void __launch_bounds__(epi_threads(EPI), 1) tc_gemm_kernel(const __gr
                     }
                     const int nb = n0 + col0 + c + 32 * h;  // output column of v[0]
                     const int lb = col0 + c + 32 * h;       // its column within the tile
-                    if (staged) {  // scaled operands: key = f.y + f.x * (row scale * accumulator), two at a time
-                        const float2 r2 = make_float2(rfac, rfac);
-#pragma unroll
-                        for (int u = 0; u < 32; u += 4) {
-                            const float4 fx = *reinterpret_cast<const float4*>(sfx + c + 32 * h + u);
-                            const float4 fy = *reinterpret_cast<const float4*>(sfy + c + 32 * h + u);
-                            const float2 t0 = __fmul2_rn(r2, make_float2(v[u], v[u + 1]));
-                            const float2 t1 = __fmul2_rn(r2, make_float2(v[u + 2], v[u + 3]));
-                            const float2 k0 = __ffma2_rn(make_float2(fx.x, fx.y), t0, make_float2(fy.x, fy.y));
-                            const float2 k1 = __ffma2_rn(make_float2(fx.z, fx.w), t1, make_float2(fy.z, fy.w));
-                            v[u] = k0.x;
-                            v[u + 1] = k0.y;
-                            v[u + 2] = k1.x;
-                            v[u + 3] = k1.y;
-                        }
-                    } else if (!kFilterOnly && a.col_fac) {
+                    if (a.col_fac) {  // scaled operands: key = f.y + f.x * (row scale * accumulator)
                         const int col = nb + lane;  // output column -> base row (strided sample of 256-row tiles)
                         const int64_t nrow = (int64_t)(col / kBN) * kBN * a.b_tile_stride + col % kBN;
                         const float2 f = col < a.N ? a.col_fac[nrow] : make_float2(0.f, 0.f);
@@ -600,63 +430,26 @@ __global__ void __launch_bounds__(epi_threads(EPI), 1) tc_gemm_kernel(const __gr
                         for (int u = 0; u < 32; ++u)
                             if (lb + u >= ncols) v[u] = __int_as_float(0x7fffffff);
                     }
-                    if (!kFilterOnly && a.out) {
-                        if (a.out_cmin && m < a.M && nb < a.N) {  // the chunk's minimum (NaN columns past N ignored)
-                            float mn = v[0];
+                    if (a.out_cmin && m < a.M && nb < a.N) {  // the chunk's minimum (NaN columns past N ignored)
+                        float mn = v[0];
 #pragma unroll
-                            for (int u = 1; u < 32; ++u) mn = fminf(mn, v[u]);
-                            a.out_cmin[(int64_t)m * ((a.N + 31) / 32) + nb / 32] = mn;
-                        }
-                        // transpose through shared memory so each store covers 32 consecutive columns
-#pragma unroll
-                        for (int u = 0; u < 32; ++u) tw[lane * 33 + u] = v[u];
-                        __syncwarp();
-                        for (int r = 0; r < 32; ++r) {
-                            const int mr = m0 + lane_base + r;
-                            if (mr < a.M && nb + lane < a.N) a.out[(int64_t)mr * a.ldo + nb + lane] = tw[r * 33 + lane];
-                        }
-                        __syncwarp();
-                    } else {
-                        uint32_t msk = half_mask(v);
-                        if (__any_sync(0xffffffffu, msk != 0)) {
-                            const int cnt = __popc(msk);
-                            int incl = cnt;
-#pragma unroll
-                            for (int o = 1; o < 32; o <<= 1) {
-                                const int y = __shfl_up_sync(0xffffffffu, incl, o);
-                                if (lane >= o) incl += y;
-                            }
-                            int slot = wcount + incl - cnt;
-                            wcount += __shfl_sync(0xffffffffu, incl, 31);
-                            while (msk) {
-                                const int u = __ffs(msk) - 1;
-                                msk &= msk - 1;
-                                if (slot < a.wcap) {
-                                    // v[u] for a run-time u: a five-level select tree on u's bits
-                                    float s16[16], s8[8], s4[4], s2[2];
-#pragma unroll
-                                    for (int z = 0; z < 16; ++z) s16[z] = (u & 16) ? v[z + 16] : v[z];
-#pragma unroll
-                                    for (int z = 0; z < 8; ++z) s8[z] = (u & 8) ? s16[z + 8] : s16[z];
-#pragma unroll
-                                    for (int z = 0; z < 4; ++z) s4[z] = (u & 4) ? s8[z + 4] : s8[z];
-#pragma unroll
-                                    for (int z = 0; z < 2; ++z) s2[z] = (u & 2) ? s4[z + 2] : s4[z];
-                                    const float kv = (u & 1) ? s2[1] : s2[0];
-                                    a.fkey[wbase + slot] = kv;
-                                    a.fcol[wbase + slot] = (int)(cbase + lb + u);
-                                    a.frow[wbase + slot] = rq;
-                                }
-                                ++slot;
-                            }
-                        }
+                        for (int u = 1; u < 32; ++u) mn = fminf(mn, v[u]);
+                        a.out_cmin[(int64_t)m * ((a.N + 31) / 32) + nb / 32] = mn;
                     }
+                    // transpose through shared memory so each store covers 32 consecutive columns
+#pragma unroll
+                    for (int u = 0; u < 32; ++u) tw[lane * 33 + u] = v[u];
+                    __syncwarp();
+                    for (int r = 0; r < 32; ++r) {
+                        const int mr = m0 + lane_base + r;
+                        if (mr < a.M && nb + lane < a.N) a.out[(int64_t)mr * a.ldo + nb + lane] = tw[r * 33 + lane];
+                    }
+                    __syncwarp();
                 }
             }
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             bar_arrive(&tempty[b]);
         }
-        if (a.wcount && lane == 0) a.wcount[(int64_t)blockIdx.x * EPI + ew] = wcount;
     }
     __syncthreads();
     if (warp == 1) {
@@ -682,7 +475,9 @@ EncodeTiledFn encode_fn() {
     return fn;
 }
 
-int make_map(CUtensorMap* tm, const void* base, int64_t rows, int cols, int box_rows, int kind) {
+}  // namespace
+
+int tc_make_map(CUtensorMap* tm, const void* base, int64_t rows, int cols, int box_rows, int kind) {
     EncodeTiledFn fn = encode_fn();
     if (!fn) {
         set_error("cuTensorMapEncodeTiled is not available from the driver");
@@ -704,15 +499,11 @@ int make_map(CUtensorMap* tm, const void* base, int64_t rows, int cols, int box_
     return ANN_OK;
 }
 
-}  // namespace
-
 size_t tc_gemm_smem() { return std::max(epi_smem(kKeyEpi), epi_smem(kFilterEpi)); }
 
 int tc_kpad(int dim, int metric) { return (int)ceil_div(dim + (metric == ANN_METRIC_L2 ? 3 : 0), 16) * 16; }
 
 static int tc_grid(int M, int N) { return (int)std::min<int64_t>(ceil_div(M, kBM) * ceil_div(N, kBN), kNumSMs); }
-int tc_filter_warps(int M, int N) { return tc_grid(M, N) * kFilterEpi; }
-int tc_grouped_filter_warps() { return kNumSMs * kFilterEpi; }
 
 template <int KIND, int EPI>
 static cudaError_t run_tc_gemm(const CUtensorMap& tmA, const CUtensorMap& tmB, const TcGemmArgs& a, int grid,
@@ -732,9 +523,8 @@ int launch_tc_gemm(const void* A, const void* B, const TcGemmArgs& a, cudaStream
                   "tensor-core scan: E4M3 / I8 operands need their scale factors (E4M3: no grouping)");
     ANN_CHECK_ARG((reinterpret_cast<uintptr_t>(A) & 15) == 0 && (reinterpret_cast<uintptr_t>(B) & 15) == 0,
                   "tensor-core scan: operands must be 16-byte aligned");
-    ANN_CHECK_ARG(a.out != nullptr || (a.tau && a.fkey && a.fcol &&
-                                       ((a.frow && a.wcount && a.wcap > 0) || (a.row_cap > 0 && a.rcount))),
-                  "tensor-core scan: neither an output matrix nor a filter");
+    ANN_CHECK_ARG(a.out != nullptr || (a.g_item_off && a.tau && a.fkey && a.fcol && a.row_cap > 0 && a.rcount),
+                  "tensor-core scan: neither an output matrix nor a grouped filter");
     ANN_CHECK_ARG(a.g_item_off == nullptr ||
                       (a.g_a_off && a.g_b_off && a.g_total && a.g_lists > 0 &&
                        ((a.out && a.g_dbase && a.tau == nullptr) || (a.out == nullptr && a.tau && a.g_row_query))),
@@ -748,9 +538,9 @@ int launch_tc_gemm(const void* A, const void* B, const TcGemmArgs& a, cudaStream
     ANN_CHECK_ARG(a.g_item_off != nullptr || (ceil_div(a.N, kBN) - 1) * kBN * (int64_t)a.b_tile_stride < b_rows,
                   "tensor-core scan: sample runs past the base");
     CUtensorMap tmA, tmB;
-    int rc = make_map(&tmA, A, a.M, a.K, kBM, a.kind);
+    int rc = tc_make_map(&tmA, A, a.M, a.K, kBM, a.kind);
     if (rc) return rc;
-    rc = make_map(&tmB, B, b_rows, a.K, kBN, a.kind);
+    rc = tc_make_map(&tmB, B, b_rows, a.K, kBN, a.kind);
     if (rc) return rc;
     const int grid = a.g_item_off ? kNumSMs : tc_grid(a.M, a.N);  // grouped: persistent over the items
     const bool filter = a.out == nullptr;
@@ -759,8 +549,7 @@ int launch_tc_gemm(const void* A, const void* B, const TcGemmArgs& a, cudaStream
         e = filter ? run_tc_gemm<kTcBF16, kFilterEpi>(tmA, tmB, a, grid, st)
                    : run_tc_gemm<kTcBF16, kKeyEpi>(tmA, tmB, a, grid, st);
     else if (a.kind == kTcE4M3)
-        e = filter ? run_tc_gemm<kTcE4M3, kFilterEpi>(tmA, tmB, a, grid, st)
-                   : run_tc_gemm<kTcE4M3, kKeyEpi>(tmA, tmB, a, grid, st);
+        e = run_tc_gemm<kTcE4M3, kKeyEpi>(tmA, tmB, a, grid, st);
     else
         e = filter ? run_tc_gemm<kTcI8, kFilterEpi>(tmA, tmB, a, grid, st)
                    : run_tc_gemm<kTcI8, kKeyEpi>(tmA, tmB, a, grid, st);

@@ -18,24 +18,18 @@ enum TcKind { kTcBF16 = 0, kTcE4M3 = 1, kTcI8 = 2 };
 struct TcGemmArgs {
     int M, N, K;           // A [M, K], B [N, K] BF16 row-major; K a multiple of 16
     const float* normA;    // [M] optional per-row addend (|a|^2 turns the L2 key into the squared distance)
-    float* out;            // [M, ldo] keys; null in filter mode
+    float* out;            // [M, ldo] keys; null in the grouped filter mode
     int64_t ldo;
     int* err;              // device flag set (to 2) if a bounded wait gives up
     int b_tile_stride = 1; // B rows of output tile j start at row j * 256 * b_tile_stride (a strided sample)
     int64_t b_rows = 0;    // rows of the B matrix when sampling (0: N)
-    // Filter mode (out == null): keys <= tau[m] are appended, as (key, column, row m), to the region of
-    // the epilogue warp that met them: warp w of the grid owns entries [w * wcap, (w + 1) * wcap) of
-    // fkey / fcol / frow, and wcount[w] receives its count (which may exceed wcap: the caller checks).
+    // Grouped filter mode (out == null): keys <= tau of a row's query are appended, as (key, column), to the query's
+    // buffer: fkey / fcol [query * row_cap + slot] at slot = atomicAdd(&rcount[query], n) -- one atomic per lane per
+    // 64 columns, n its survivors there -- and nothing is written at slots past row_cap (rcount may exceed it: the
+    // caller checks).
     const float* tau = nullptr;
     float* fkey = nullptr;
     int* fcol = nullptr;
-    int* frow = nullptr;
-    int* wcount = nullptr;
-    int wcap = 0;
-    // Filter mode, per-row buffers (row_cap > 0; the grouped form, rows = queries): a survivor of row r goes
-    // to fkey / fcol [r * row_cap + slot] at slot = atomicAdd(&rcount[r], n) -- one atomic per lane per 32
-    // columns, n its survivors there -- and nothing is written at slots past row_cap (rcount[r] may exceed
-    // it: the caller checks).
     int row_cap = 0;
     int* rcount = nullptr;
     // Grouped mode (g_item_off != null; out receives the keys): tile t is work item t of a list-major
@@ -81,10 +75,6 @@ enum TcRole { kTcBase = 0, kTcQuery = 1 };
 // Columns of the BF16 operands for vectors of `dim` FP32 values: the key columns included, rounded up
 // to the 16-column MMA step (the 64-column TMA boxes of the last k-block read zeros past it).
 int tc_kpad(int dim, int metric);
-// Epilogue warps of a filter launch over M x N keys (the size of the wcount array).
-int tc_filter_warps(int M, int N);
-// ... and of a grouped filter launch (persistent over the work items).
-int tc_grouped_filter_warps();
 size_t tc_gemm_smem();
 // The grouped mode's item descriptors (TcGemmArgs::g_item_desc) for items [0, min(item_off[C], cap)): list l's
 // items from item_off[l] (launch_tc_ivf_items), its A rows [a_off[l], a_off[l+1]) and B rows from b_off[l]

@@ -20,64 +20,6 @@ __device__ __forceinline__ int pos_to_row(int64_t p, int64_t n, int64_t mult) {
     return (int)(((unsigned __int128)p * (uint64_t)mult) % (uint64_t)n);
 }
 
-__global__ void tc_count_kernel(TcGroupArgs g) {
-    const int w = blockIdx.x;
-    const int cnt = min(g.wcount[w], g.wcap);
-    const int64_t base = (int64_t)w * g.wcap;
-    for (int e = threadIdx.x; e < cnt; e += blockDim.x) atomicAdd(&g.rowcnt[g.frow[base + e]], 1);
-}
-
-// One block: exclusive scan of rowcnt into offs, cursors zeroed, largest warp count.
-__global__ void __launch_bounds__(1024) tc_scan_kernel(TcGroupArgs g) {
-    __shared__ int64_t sPart[1024];
-    __shared__ int sMax[32];
-    const int per = (g.M + 1023) / 1024;
-    const int r0 = threadIdx.x * per;
-    int64_t local = 0;
-    for (int i = 0; i < per; ++i)
-        if (r0 + i < g.M) local += g.rowcnt[r0 + i];
-    sPart[threadIdx.x] = local;
-    __syncthreads();
-    for (int off = 1; off < 1024; off <<= 1) {
-        const int64_t v = threadIdx.x >= off ? sPart[threadIdx.x - off] : 0;
-        __syncthreads();
-        sPart[threadIdx.x] += v;
-        __syncthreads();
-    }
-    int64_t run = sPart[threadIdx.x] - local;
-    for (int i = 0; i < per; ++i) {
-        const int r = r0 + i;
-        if (r < g.M) {
-            g.offs[r] = run;
-            g.cursor[r] = 0;
-            run += g.rowcnt[r];
-        }
-    }
-    int m = 0;
-    for (int w = threadIdx.x; w < g.nwarps; w += 1024) m = max(m, g.wcount[w]);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
-    if ((threadIdx.x & 31) == 0) sMax[threadIdx.x >> 5] = m;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int r = 0;
-        for (int i = 0; i < 32; ++i) r = max(r, sMax[i]);
-        *g.max_wcount = r;
-    }
-}
-
-__global__ void tc_scatter_kernel(TcGroupArgs g) {
-    const int w = blockIdx.x;
-    const int cnt = min(g.wcount[w], g.wcap);
-    const int64_t base = (int64_t)w * g.wcap;
-    for (int e = threadIdx.x; e < cnt; e += blockDim.x) {
-        const int row = g.frow[base + e];
-        const int64_t at = g.offs[row] + atomicAdd(&g.cursor[row], 1);
-        g.gkey[at] = g.fkey[base + e];
-        g.gid[at] = pos_to_row(g.fcol[base + e], g.n, g.mult);
-    }
-}
-
 __global__ void tc_bar_check_kernel(const int* rowcnt, int M, int R, int* list, int* flags, const int64_t* lens,
                                     int* mark) {
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
@@ -936,19 +878,6 @@ int launch_tc_ivf_pairs(const void* qrows, int row_bytes, const int32_t* pair_va
     tc_ivf_pairs_kernel<<<grid, 256, 0, st>>>(static_cast<const unsigned char*>(qrows), row_bytes, pair_vals,
                                               pair_lists, n_pairs, max_pairs, npc, cand_off, seg_pref, list_off,
                                               static_cast<unsigned char*>(A), dbase, sm);
-    ANN_LAUNCH_CHECK();
-    return ANN_OK;
-}
-
-int launch_tc_group(const TcGroupArgs& g, cudaStream_t st) {
-    if (g.M == 0) return ANN_OK;
-    ANN_CHECK_ARG(g.nwarps > 0 && g.wcap > 0, "survivor grouping: no regions");
-    ANN_CUDA_TRY(cudaMemsetAsync(g.rowcnt, 0, sizeof(int) * (size_t)g.M, st));
-    tc_count_kernel<<<g.nwarps, 256, 0, st>>>(g);
-    ANN_LAUNCH_CHECK();
-    tc_scan_kernel<<<1, 1024, 0, st>>>(g);
-    ANN_LAUNCH_CHECK();
-    tc_scatter_kernel<<<g.nwarps, 256, 0, st>>>(g);
     ANN_LAUNCH_CHECK();
     return ANN_OK;
 }

@@ -1,5 +1,4 @@
-// Helpers of the tensor-core search around the GEMM (tc_search.cu): grouping filter survivors into
-// per-query streams, the bar check and re-run gather, and the row order of the BF16 base copy.
+// Helpers of the tensor-core search around the GEMM (tc_search.cu): the bar check and re-run gather, and the row order of the BF16 base copy.
 #pragma once
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -13,27 +12,6 @@ namespace annb {
 // coprime to n): any 256 consecutive positions cover the rows evenly, so a strided sample of whole
 // tiles is an even sample of the base whatever order the rows came in.
 int64_t tc_row_mult(int64_t n);
-
-struct TcGroupArgs {
-    // filter survivors: warp w holds entries [w * wcap, w * wcap + min(wcount[w], wcap))
-    const float* fkey;
-    const int* fcol;
-    const int* frow;
-    const int* wcount;
-    int nwarps;
-    int wcap;
-    int M;            // rows (queries) of the filter launch
-    int64_t n;        // base rows, for the position -> row map
-    int64_t mult;     // tc_row_mult(n)
-    // outputs
-    int* rowcnt;      // [M] survivors per row
-    int64_t* offs;    // [M] start of row m's stream in gkey / gid
-    int* cursor;      // [M] scratch
-    float* gkey;      // [nwarps * wcap]
-    int* gid;         // [nwarps * wcap] base row ids
-    int* max_wcount;  // [1] largest wcount (an overflow if > wcap)
-};
-int launch_tc_group(const TcGroupArgs& g, cudaStream_t st);
 
 // Rows with fewer than R survivors -- fewer than min(R, lens[row]) where lens is given -- go to list (count in
 // flags[0]); mark[row], if given, is 1 for them and 0 for the others.
