@@ -679,7 +679,7 @@ static int flat_exact_pruned(ann_flat* h, ann_workspace* ws, const float* qdev, 
     const int64_t S = full_tiles / stride * 256;
     const int rF = prune_bar_rank(kk, S, n), cap = prune_cap(kk);
     const int kpad = h->kpad;
-    constexpr int kChunk = 5120;  // queries at a time: 0.5 GB of sampled keys and survivors
+    constexpr int kChunk = 10240;  // queries at a time: 0.4 GB of sampled minima and survivors (k <= 128)
     const int nchunks = (int)ceil_div(nq, kChunk);
     const int qc = nchunks == 1 ? nq : (int)std::min<int64_t>(kChunk, ceil_div(ceil_div(nq, nchunks), 128) * 128);
     // the scan of the queries left over: up to one split per SM, its lists bounded to 256 MB
@@ -690,7 +690,7 @@ static int flat_exact_pruned(ann_flat* h, ann_workspace* ws, const float* qdev, 
     nsplit = (int)ceil_div(n, rps);
     Sizer sz;
     sz.take<__nv_bfloat16>((size_t)qc * kpad);
-    sz.take<float>((size_t)qc * S);
+    sz.take<float>((size_t)qc * (S / 8));
     for (int i = 0; i < 4; ++i) sz.take<float>((size_t)qc);
     sz.take<float>((size_t)qc * cap);
     sz.take<int>((size_t)qc * cap);
@@ -707,7 +707,7 @@ static int flat_exact_pruned(ann_flat* h, ann_workspace* ws, const float* qdev, 
     }
     Carver cv(ws->big);
     __nv_bfloat16* qb = cv.take<__nv_bfloat16>((size_t)qc * kpad);
-    float* kA = cv.take<float>((size_t)qc * S);
+    float* kA = cv.take<float>((size_t)qc * (S / 8));
     float* win = cv.take<float>((size_t)qc);
     float* tauF = cv.take<float>((size_t)qc);
     float* tauX = cv.take<float>((size_t)qc);
@@ -749,11 +749,13 @@ static int flat_exact_pruned(ann_flat* h, ann_workspace* ws, const float* qdev, 
         p.out_dists = dists_dev ? dists_dev + (size_t)q0 * kk : nullptr;
         if ((rc = launch_tc_operand(q, nc, h->dim, dpad, qb, kpad, kTcQuery, h->metric, 0, st))) return rc;
         if ((rc = launch_prune_windows(p, st))) return rc;
-        TcGemmArgs sa{nc, (int)S, kpad, nullptr, kA, S, h->d_err};
+        TcFilterArgs sa{nc, (int)S, kpad, kTcBF16};
+        sa.err = h->d_err;
+        sa.out_min = kA;
         sa.b_tile_stride = stride;
         sa.b_rows = n;
-        if ((rc = launch_tc_gemm(qb, h->base_bf16, sa, st))) return rc;
-        if ((rc = launch_sample_bars(kA, (int)S, nc, rF, rF, tauF, tauU, st))) return rc;
+        if ((rc = launch_tc_sample(qb, h->base_bf16, sa, st))) return rc;
+        if ((rc = launch_warp_bars(kA, nullptr, nullptr, nc, rF, rF, tauF, tauU, st, S / 8))) return rc;
         if ((rc = launch_prune_bars(p, st))) return rc;
         const TcFilterArgs fa{nc, (int)n, kpad, kTcBF16, tauX, fkey, fcol, cap, rcount, nullptr, nullptr, h->d_err};
         if ((rc = launch_tc_filter(qb, h->base_bf16, fa, st))) return rc;
@@ -878,25 +880,28 @@ int ann_flat_query_tc(ann_flat* h, ann_workspace* ws, const float* queries, int3
         if ((rc = launch_pad_rows(queries, nq, h->dim, ldq, qdev, dpad, st))) return rc;
     }
     if ((rc = flat_tc_queries(h, t, qdev, nq, dpad, qb, rfac, st))) return rc;
-    // Sampled bars: keys over a strided sample of S positions of the BF16 copy (an even sample of the
-    // base, by its row order) give each query two bars. The safe bar, its R-th best sampled key, is at
-    // or above its R-th best key over all rows (about n * R / S keys pass it). The fast bar, its rF-th
-    // best sampled key with rF ~ 3 R S / n, lets about 3 R keys pass. The full pass keeps the keys
+    // Sampled bars: keys over a strided sample of S positions of the operand copy (an even sample of the
+    // base, by its row order), of which the smallest of every 8 are kept, give each query two bars. The safe
+    // bar, the R-th smallest of them, is at or above its R-th best key over all rows (a little more than
+    // n R / S keys pass it). The fast bar, the rF-th, lets n rF / S keys pass, rF just past the number of the
+    // R best that a sample holds: fewer than R survivors, about 1 query in 10^7. The full pass keeps the keys
     // under the fast bar; a query with fewer than R survivors (the count is exact) is re-run under its
     // safe bar, so every query ends with its best R keys among its survivors. Small bases, or a
-    // survivor overflow, use the full key matrix.
+    // survivor overflow, use the full key matrix. (With every sampled key written and binned, a tenth of
+    // a 10,000-query call went to the bars: sample and bars 1.59 ms, 0.31 ms from the minima.)
     const int64_t n = h->n;
     const int64_t full_tiles = n / 256;
-    const int64_t want_tiles = std::max<int64_t>(128, ceil_div(16 * (int64_t)R, 256));
+    const int64_t want_tiles = std::max(std::max<int64_t>(128, ceil_div(16 * (int64_t)R, 256)), full_tiles / 64);
     const bool sampled = full_tiles >= 4 * want_tiles;
     const int stride = sampled ? (int)(full_tiles / want_tiles) : 1;
     const int64_t S = sampled ? (full_tiles / stride) * 256 : 0;
-    const int rF = sampled ? (int)std::min<int64_t>(R, std::max<int64_t>(1, ceil_div(3 * (int64_t)R * S, n))) : 0;
+    const int rF = sampled ? prune_bar_rank(R, S, n) : 0;
     constexpr int kRerunBatch = 128;
-    // queries per chunk: ~2 GB of sampled keys, or ~4 GB of full key matrix
+    // queries per chunk: 1 GB of survivors, or ~4 GB of full key matrix
     const int64_t qfull64 = std::max<int64_t>(128, ((int64_t)4 << 30) / (int64_t)(sizeof(float) * n) / 128 * 128);
     const int qfull = (int)std::min<int64_t>(qfull64, 65535);
-    const int qmax = sampled ? (int)std::clamp<int64_t>(((int64_t)2 << 30) / (4 * S) / 128 * 128, 128, 8192) : qfull;
+    const int64_t cap64 = std::min<int64_t>(n, 16 * (int64_t)R);
+    const int qmax = sampled ? (int)std::clamp<int64_t>(((int64_t)1 << 30) / (8 * cap64) / 128 * 128, 128, 16384) : qfull;
     const int nchunks = (int)ceil_div(nq, qmax);
     const int qc = (int)std::min<int64_t>(qmax, ceil_div(ceil_div(nq, nchunks), 128) * 128);
     for (int q0 = 0; q0 < nq; q0 += qc) {
@@ -909,11 +914,11 @@ int ann_flat_query_tc(ann_flat* h, ann_workspace* ws, const float* queries, int3
         if (sampled) {
             // survivors kept per query: about 3 R pass the fast bar (9 R were met over 5,000 queries of a 4M-row
             // mixture), n R / S the safe bar of a re-run
-            const int cap = (int)std::min<int64_t>(n, 16 * (int64_t)R);
+            const int cap = (int)cap64;
             const int cap2 = (int)std::min<int64_t>(n, 2 * ceil_div((int64_t)R * n, S) + 1024);
             const size_t ent = std::max((size_t)nc * cap, (size_t)std::min(nc, kRerunBatch) * cap2);
             Sizer s2;
-            s2.take<float>((size_t)nc * S);            // sample keys
+            s2.take<float>((size_t)nc * (S / 8));      // minima of 8 sampled keys
             s2.take<float>(ent);                       // survivors: key, position
             s2.take<int>(ent);
             for (int i = 0; i < 3; ++i) s2.take<float>((size_t)nc);  // fast, safe, gathered bars
@@ -923,7 +928,7 @@ int ann_flat_query_tc(ann_flat* h, ann_workspace* ws, const float* queries, int3
             s2.take<float>((size_t)kRerunBatch);
             if ((rc = ws_reserve_big(ws, s2.bytes()))) return rc;
             Carver cb(ws->big);
-            float* kA = cb.take<float>((size_t)nc * S);
+            float* kA = cb.take<float>((size_t)nc * (S / 8));
             float* fkey = cb.take<float>(ent);
             int* fcol = cb.take<int>(ent);
             float* tauF = cb.take<float>((size_t)nc);
@@ -937,26 +942,16 @@ int ann_flat_query_tc(ann_flat* h, ann_workspace* ws, const float* queries, int3
 
             // stages 2: sample pass and bars, 3: filter pass, 4: grouping, selections and re-runs
             const int prec = h->prof.begin(st, 2);
-            TcGemmArgs sa{nc, (int)S, kpad, nullptr, kA, S, h->d_err};
-            sa.b_tile_stride = stride;
-            sa.b_rows = n;
-            sa.kind = t.kind;
+            TcFilterArgs sa{nc, (int)S, kpad, t.kind};
             sa.col_fac = t.cfac;
             sa.row_fac = rfc;
-            if ((rc = launch_tc_gemm(qbc, t.base, sa, st))) return rc;
-            if (sample_bars_smem((int)S) <= kSampleBarsMaxSmem) {
-                if ((rc = launch_sample_bars(kA, (int)S, nc, rF, R, tauF, tauS, st))) return rc;
-            } else {
-                RadixSelectArgs bar{};
-                bar.keys = kA;
-                bar.ld = S;
-                bar.R = rF;
-                bar.out_kth = tauF;
-                bar.R2 = R;
-                bar.out_kth2 = tauS;
-                bar.kth_upper = 1;
-                if ((rc = launch_radix_select(bar, nc, st))) return rc;
-            }
+            sa.err = h->d_err;
+            sa.out_min = kA;
+            sa.b_tile_stride = stride;
+            sa.b_rows = n;
+            if ((rc = launch_tc_sample(qbc, t.base, sa, st))) return rc;
+            const int S8 = (int)(S / 8);
+            if ((rc = launch_warp_bars(kA, nullptr, nullptr, nc, rF, R, tauF, tauS, st, S8))) return rc;
             h->prof.mark(prec, st);
             auto filter = [&](const void* A, int M, const float* tau, const float* rf, int rcap) -> int {
                 ANN_CUDA_TRY(cudaMemsetAsync(rowcnt, 0, sizeof(int) * (size_t)M, st));

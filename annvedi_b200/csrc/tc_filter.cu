@@ -145,7 +145,8 @@ struct RingPos {
     }
 };
 
-template <int KIND, int CG>
+// SAMPLE: no bars and no survivors, the minima of 8 columns are written instead.
+template <int KIND, int CG, bool SAMPLE>
 __global__ void __launch_bounds__(kFiThreads, 1) tc_filter_kernel(const __grid_constant__ CUtensorMap tmA,
                                                                  const __grid_constant__ CUtensorMap tmB,
                                                                  const TcFilterArgs a, const FilterShape sh) {
@@ -213,7 +214,8 @@ __global__ void __launch_bounds__(kFiThreads, 1) tc_filter_kernel(const __grid_c
             bool ok = true;
             const uint32_t bytes = CG * (kBSize + (resident ? 0 : kABytes));  // of both CTAs: one barrier counts them
             while (ok && work.next()) {
-                const int arow = work.m * CG * kBM + rank * kBM, brow = work.n * kBN + rank * kBRows;
+                const int arow = work.m * CG * kBM + rank * kBM;
+                const int brow = work.n * kBN * (SAMPLE ? a.b_tile_stride : 1) + rank * kBRows;
                 for (int kb = 0; kb < kt; ++kb, pos.step(nst)) {
                     const int s = pos.s;
                     if (!(ok = bar_wait(&empty[s], pos.ph ^ 1u, a.err, a.wait_ns))) break;
@@ -319,11 +321,11 @@ __global__ void __launch_bounds__(kFiThreads, 1) tc_filter_kernel(const __grid_c
         while (work.next()) {
             const int b = (int)(acc & 1);
             if (work.first) {
-                flush(nq);
+                if (!SAMPLE) flush(nq);
                 row0 = work.m * CG * kBM + rank * kBM + lane_base;
                 const int rq = row0 + lane;
                 const bool valid = rq < a.M;
-                tau = valid ? a.tau[rq] : __int_as_float(0x7fffffff);  // NaN: no key passes
+                if (!SAMPLE) tau = valid ? a.tau[rq] : __int_as_float(0x7fffffff);  // NaN: no key passes
                 if (KIND != kTcBF16) rfac = valid ? a.row_fac[rq] : 1.f;
             }
             const int n0 = work.n * kBN + col0;
@@ -333,7 +335,8 @@ __global__ void __launch_bounds__(kFiThreads, 1) tc_filter_kernel(const __grid_c
                 for (int i = 0; i < kFiCols / 32; ++i) {
                     const int c = n0 + 32 * i + lane;
                     const bool in = c < a.N;
-                    const float* src = reinterpret_cast<const float*>(a.col_fac + (in ? c : 0));
+                    const int64_t brow = SAMPLE ? (int64_t)work.n * kBN * a.b_tile_stride + (c - work.n * kBN) : c;
+                    const float* src = reinterpret_cast<const float*>(a.col_fac + (in ? brow : 0));
                     cp_async4(sfx + 32 * i + lane, src, in);
                     cp_async4(sfy + 32 * i + lane, src + 1, in);
                 }
@@ -366,11 +369,12 @@ __global__ void __launch_bounds__(kFiThreads, 1) tc_filter_kernel(const __grid_c
                             bar_arrive(&tempty[b]);
                     }
                 }
-                if (n0 + h + 32 > a.N) {  // the ragged last tile: columns past N become NaN keys, which pass no bar
+                if (!SAMPLE && n0 + h + 32 > a.N) {  // the ragged last tile: columns past N become NaN keys, which pass no bar
 #pragma unroll
                     for (int u = 0; u < 32; ++u)
                         if (n0 + h + u >= a.N) r[u] = 0x7fffffffu;
                 }
+                float mins[4];
 #pragma unroll
                 for (int g = 0; g < 4; ++g) {
                     float v[8];
@@ -393,6 +397,10 @@ __global__ void __launch_bounds__(kFiThreads, 1) tc_filter_kernel(const __grid_c
                         }
                     }
                     const float mn = min3f(min3f(v[0], v[1], v[2]), min3f(v[3], v[4], v[5]), fminf(v[6], v[7]));
+                    if (SAMPLE) {
+                        mins[g] = mn;
+                        continue;
+                    }
                     if (!__any_sync(0xffffffffu, mn <= tau)) continue;
                     uint32_t mask = 0;  // the lane's survivors of the 8
 #pragma unroll
@@ -418,10 +426,13 @@ __global__ void __launch_bounds__(kFiThreads, 1) tc_filter_kernel(const __grid_c
                         if (nq >= 32) flush(32);
                     }
                 }
+                if (SAMPLE && row0 + lane < a.M)
+                    *reinterpret_cast<float4*>(a.out_min + (int64_t)(row0 + lane) * (a.N / 8) + (n0 + h) / 8) =
+                        make_float4(mins[0], mins[1], mins[2], mins[3]);
             }
             ++acc;
         }
-        flush(nq);
+        if (!SAMPLE) flush(nq);
     }
     __syncthreads();
     if (CG == 2) cluster_sync();  // neither CTA's barriers or accumulators are in use any more
@@ -463,12 +474,12 @@ int resident_clusters(const void* kern, int cg, size_t smem) {
     return n;
 }
 
-template <int KIND, int CG>
+template <int KIND, int CG, bool SAMPLE>
 int run_filter(const void* A, const void* B, const TcFilterArgs& a, cudaStream_t st) {
     CUtensorMap tmA, tmB;
     int rc = tc_make_map(&tmA, A, a.M, a.K, kBM, KIND);
     if (rc) return rc;
-    if ((rc = tc_make_map(&tmB, B, a.N, a.K, kBN / CG, KIND))) return rc;
+    if ((rc = tc_make_map(&tmB, B, SAMPLE ? a.b_rows : a.N, a.K, kBN / CG, KIND))) return rc;
     FilterShape sh{};
     sh.mt = (int)ceil_div(a.M, CG * kBM);
     sh.nt = (int)ceil_div(a.N, kBN);
@@ -481,7 +492,7 @@ int run_filter(const void* A, const void* B, const TcFilterArgs& a, cudaStream_t
     sh.nst = (int)std::min<size_t>(kFiMaxStages, left / (bs + (sh.resident ? 0 : kABytes)));
     const size_t smem = kFiFixed + fac + (size_t)sh.nst * (bs + (sh.resident ? 0 : kABytes)) +
                         (sh.resident ? (size_t)sh.kt * kABytes : 0);
-    auto kern = tc_filter_kernel<KIND, CG>;
+    auto kern = tc_filter_kernel<KIND, CG, SAMPLE>;
     ANN_CUDA_TRY(smem_optin(reinterpret_cast<const void*>(kern)));
     const int64_t tiles = (int64_t)sh.mt * sh.nt;
     const int ncl = (int)std::min<int64_t>(tiles, resident_clusters(reinterpret_cast<const void*>(kern), CG, smem));
@@ -509,18 +520,39 @@ int run_filter(const void* A, const void* B, const TcFilterArgs& a, cudaStream_t
 
 }  // namespace
 
-int launch_tc_filter(const void* A, const void* B, const TcFilterArgs& a, cudaStream_t st) {
+static int check_filter(const void* A, const void* B, const TcFilterArgs& a) {
     const int step = a.kind == kTcBF16 ? 16 : 32;
     ANN_CHECK_ARG(a.kind == kTcBF16 || a.kind == kTcE4M3, "tensor-core filter: element kind %d", a.kind);
     ANN_CHECK_ARG(a.K % step == 0 && a.K > 0, "tensor-core filter: K=%d not a positive multiple of %d", a.K, step);
     ANN_CHECK_ARG(a.kind == kTcBF16 || (a.col_fac && a.row_fac), "tensor-core filter: E4M3 operands need their factors");
     ANN_CHECK_ARG((reinterpret_cast<uintptr_t>(A) & 15) == 0 && (reinterpret_cast<uintptr_t>(B) & 15) == 0,
                   "tensor-core filter: operands must be 16-byte aligned");
-    ANN_CHECK_ARG(a.tau && a.fkey && a.fcol && a.rcount && a.cap > 0, "tensor-core filter: no buffers");
+    return ANN_OK;
+}
+
+// one CTA a tile up to 128 queries: the base is read once either way, and a pair would multiply padding
+template <bool SAMPLE>
+static int dispatch_filter(const void* A, const void* B, const TcFilterArgs& a, cudaStream_t st) {
     if (a.M == 0 || a.N == 0) return ANN_OK;
-    // one CTA a tile up to 128 queries: the base is read once either way, and a pair would multiply padding
-    if (a.kind == kTcBF16) return a.M <= kBM ? run_filter<kTcBF16, 1>(A, B, a, st) : run_filter<kTcBF16, 2>(A, B, a, st);
-    return a.M <= kBM ? run_filter<kTcE4M3, 1>(A, B, a, st) : run_filter<kTcE4M3, 2>(A, B, a, st);
+    if (a.kind == kTcBF16)
+        return a.M <= kBM ? run_filter<kTcBF16, 1, SAMPLE>(A, B, a, st) : run_filter<kTcBF16, 2, SAMPLE>(A, B, a, st);
+    return a.M <= kBM ? run_filter<kTcE4M3, 1, SAMPLE>(A, B, a, st) : run_filter<kTcE4M3, 2, SAMPLE>(A, B, a, st);
+}
+
+int launch_tc_filter(const void* A, const void* B, const TcFilterArgs& a, cudaStream_t st) {
+    const int rc = check_filter(A, B, a);
+    if (rc) return rc;
+    ANN_CHECK_ARG(a.tau && a.fkey && a.fcol && a.rcount && a.cap > 0, "tensor-core filter: no buffers");
+    return dispatch_filter<false>(A, B, a, st);
+}
+
+int launch_tc_sample(const void* A, const void* B, const TcFilterArgs& a, cudaStream_t st) {
+    const int rc = check_filter(A, B, a);
+    if (rc) return rc;
+    ANN_CHECK_ARG(a.out_min && a.N % kBN == 0 && a.b_tile_stride >= 1 &&
+                      ((int64_t)a.N / kBN - 1) * kBN * a.b_tile_stride + kBN <= a.b_rows,
+                  "tensor-core sample: %d columns, stride %d", a.N, a.b_tile_stride);
+    return dispatch_filter<true>(A, B, a, st);
 }
 
 }  // namespace annb

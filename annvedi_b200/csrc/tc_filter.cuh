@@ -16,7 +16,15 @@ struct TcFilterArgs {
     const float* row_fac;
     int* err;              // device flag set (to 2) if a bounded wait gives up
     uint64_t wait_ns = 0;
+    // Sample pass (launch_tc_sample): N sampled columns in whole tiles of 256, tile j holding B rows
+    // j * 256 * b_tile_stride ..; out_min [M, N / 8] receives the smallest key of each 8 columns.
+    float* out_min = nullptr;
+    int b_tile_stride = 1;
+    int64_t b_rows = 0;    // rows of B
 };
 int launch_tc_filter(const void* A, const void* B, const TcFilterArgs& a, cudaStream_t st);
+// The r-th smallest of a row's minima is at or above the r-th smallest of its sampled keys, and close to it while r is
+// a small share of N / 8: bars are taken from the minima, an eighth of the keys to write and read.
+int launch_tc_sample(const void* A, const void* B, const TcFilterArgs& a, cudaStream_t st);
 
 }  // namespace annb

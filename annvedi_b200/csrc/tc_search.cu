@@ -334,8 +334,8 @@ __device__ __forceinline__ void warp_bin_pick(const int* hist, int rank, int* bi
 }
 __global__ void __launch_bounds__(kBarThreads) block_bars_kernel(const float* __restrict__ keys,
                                                                  const int64_t* __restrict__ offs,
-                                                                 const int64_t* __restrict__ lens, int nq, int r1,
-                                                                 int r2, int staged, float* __restrict__ bar1,
+                                                                 const int64_t* __restrict__ lens, int64_t ld, int nq,
+                                                                 int r1, int r2, int staged, float* __restrict__ bar1,
                                                                  float* __restrict__ bar2) {
     extern __shared__ uint32_t smem_bars[];
     __shared__ int sHist[2][256];
@@ -343,8 +343,8 @@ __global__ void __launch_bounds__(kBarThreads) block_bars_kernel(const float* __
     const int q = blockIdx.x;
     if (q >= nq) return;  // the whole block
     const int warp = threadIdx.x >> 5;
-    const int64_t n = lens[q];
-    const float* kq = keys + offs[q];
+    const int64_t n = lens ? lens[q] : ld;
+    const float* kq = keys + (offs ? offs[q] : q * ld);
     const bool in_smem = n <= staged;
     if (in_smem)
         for (int64_t p = threadIdx.x; p < n; p += kBarThreads) smem_bars[p] = ord_key(kq[p]);
@@ -940,10 +940,11 @@ int launch_warp_bars(const float* keys, const int64_t* offs, const int64_t* lens
                      float* bar2, cudaStream_t st, int64_t max_len) {
     if (nq == 0) return ANN_OK;
     ANN_CHECK_ARG(r1 >= 1 && r2 >= 1, "bars: ranks %d, %d", r1, r2);
-    if (max_len > 0) {  // one block per query; streams of up to 6,144 keys (24 KB) staged in shared memory
-        const int staged = (int)std::min<int64_t>(max_len, 6144);
-        block_bars_kernel<<<(unsigned)nq, kBarThreads, (size_t)staged * 4, st>>>(keys, offs, lens, nq, r1, r2, staged,
-                                                                                bar1, bar2);
+    ANN_CHECK_ARG(max_len > 0 || (offs && lens), "bars: streams without offsets need their length");
+    if (max_len > 0) {  // one block per query; streams of up to 8,192 keys (32 KB) staged in shared memory
+        const int staged = (int)std::min<int64_t>(max_len, 8192);
+        block_bars_kernel<<<(unsigned)nq, kBarThreads, (size_t)staged * 4, st>>>(keys, offs, lens, max_len, nq, r1, r2,
+                                                                                staged, bar1, bar2);
     } else {
         warp_bars_kernel<<<(unsigned)ceil_div(nq, 8), 256, 0, st>>>(keys, offs, lens, nq, r1, r2, bar1, bar2);
     }

@@ -73,7 +73,7 @@ int launch_max_int(const int* v, int n, int* out, cudaStream_t st);
 // One warp per query: bar1 / bar2 = the r1-th / r2-th smallest key of keys[offs[q] .. + lens[q]) (exact; +inf
 // where the stream is shorter).
 // With max_len > 0 (a bound of the lens[q]) one block works on each query and streams of up to
-// min(max_len, 6144) keys are staged in shared memory.
+// min(max_len, 8192) keys are staged in shared memory; offs and lens may then be null, for rows of max_len keys each.
 int launch_warp_bars(const float* keys, const int64_t* offs, const int64_t* lens, int nq, int r1, int r2, float* bar1,
                      float* bar2, cudaStream_t st, int64_t max_len = 0);
 // One warp per query: the R smallest (key, id) of the buffer [q * cap, + min(count[q], cap)) as a set (the keys
