@@ -15,6 +15,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "flat_prune.cuh"
 #include "flat_scan.cuh"
 #include "ivf.cuh"
 #include "ivf_batched.cuh"
@@ -140,7 +141,91 @@ static int ivf_finish_lists(ann_ivf* h, cudaStream_t st) {
     return ANN_OK;
 }
 
-// Nearest centroid of every row (exact FP32 scan, k = 1): assign[i] in [0, C).
+// What the assignment by BF16 keys keeps over a fit: the rows in operand form with their norms, buffers for a chunk of
+// keys, and the centroids' operand form and norms, made again each round.
+struct KmeansKeys {
+    bool ok = false;
+    int kpad = 0;
+    int chunk = 0;                   // rows at a time
+    __nv_bfloat16* xb = nullptr;     // [n, kpad]
+    __nv_bfloat16* cb = nullptr;     // [C, kpad]
+    float2* norms = nullptr;         // [n] (norm, residual norm)
+    unsigned* max2 = nullptr;        // [4] largest squared norm and residual norm: of the rows, of the centroids
+    float* keys = nullptr;           // [chunk, C]
+    float* cmin = nullptr;           // [chunk, ceil(C / 32)]
+    int32_t* amb = nullptr;          // [chunk] rows the keys' bound does not cover, and their count
+    int* amb_count = nullptr;
+    int* err = nullptr;
+    ~KmeansKeys() {
+        for (void* p : {(void*)xb, (void*)cb, (void*)norms, (void*)max2, (void*)keys, (void*)cmin, (void*)amb,
+                        (void*)amb_count, (void*)err})
+            if (p) cudaFree(p);
+    }
+};
+
+static bool prune_norm_ok(unsigned bits2) {
+    float s;
+    memcpy(&s, &bits2, 4);
+    s = std::sqrt(s);
+    return s >= kPruneNormMin && s <= kPruneNormMax;
+}
+
+// Lays the rows out for the assignment by keys. k.ok stays false, without an error, where the FP32 scan assigns: small
+// problems (under 65,536 row-centroid pairs both take a few launches), no memory for the copy, or norms that the keys'
+// error bound does not cover (the given centroids' too; those of k-means are rows or means of rows).
+static int kmeans_keys_setup(KmeansKeys& k, const float* x, int64_t n, int dim, int dpad, const float* cent, int C,
+                             bool given, cudaStream_t st) {
+    if (C < 2 || n * (int64_t)C < 65536) return ANN_OK;
+    k.kpad = tc_kpad(dim, ANN_METRIC_L2);
+    const int nch = (int)ceil_div(C, 32);
+    const int64_t per_row = sizeof(float) * ((int64_t)C + nch);
+    k.chunk = (int)std::min<int64_t>(std::min<int64_t>(n, 1 << 20), std::max<int64_t>(128, ((int64_t)256 << 20) / per_row / 128 * 128));
+    const bool mem = cudaMalloc(&k.xb, sizeof(__nv_bfloat16) * (size_t)n * k.kpad) == cudaSuccess &&
+                     cudaMalloc(&k.cb, sizeof(__nv_bfloat16) * (size_t)C * k.kpad) == cudaSuccess &&
+                     cudaMalloc(&k.norms, sizeof(float2) * (size_t)n) == cudaSuccess &&
+                     cudaMalloc(&k.max2, 4 * sizeof(unsigned)) == cudaSuccess &&
+                     cudaMalloc(&k.keys, sizeof(float) * (size_t)k.chunk * C) == cudaSuccess &&
+                     cudaMalloc(&k.cmin, sizeof(float) * (size_t)k.chunk * nch) == cudaSuccess &&
+                     cudaMalloc(&k.amb, sizeof(int32_t) * (size_t)k.chunk) == cudaSuccess &&
+                     cudaMalloc(&k.amb_count, sizeof(int)) == cudaSuccess &&
+                     cudaMalloc(&k.err, sizeof(int)) == cudaSuccess;
+    if (!mem) {
+        cudaGetLastError();
+        return ANN_OK;
+    }
+    int rc = launch_base_norms(x, n, dim, dpad, k.max2, st, k.norms);
+    if (rc || (rc = launch_base_norms(cent, C, dim, dpad, k.max2 + 2, st))) return rc;
+    unsigned h[4] = {0, 0, 0, 0};
+    ANN_CUDA_TRY(cudaMemsetAsync(k.err, 0, sizeof(int), st));
+    ANN_CUDA_TRY(cudaMemcpyAsync(h, k.max2, sizeof(h), cudaMemcpyDeviceToHost, st));
+    ANN_CUDA_TRY(cudaStreamSynchronize(st));
+    if (!prune_norm_ok(h[0]) || (given && !prune_norm_ok(h[2]))) return ANN_OK;
+    if ((rc = launch_tc_operand(x, n, dim, dpad, k.xb, k.kpad, kTcQuery, ANN_METRIC_L2, 0, st))) return rc;
+    k.ok = true;
+    return ANN_OK;
+}
+
+// One round of the assignment by keys (ivf_build.cu).
+static int assign_rows_keys(KmeansKeys& k, const float* x, int64_t n, int dim, int dpad, const float* cent, int C,
+                            int32_t* assign, cudaStream_t st) {
+    int rc = launch_base_norms(cent, C, dim, dpad, k.max2 + 2, st);
+    if (rc) return rc;
+    if ((rc = launch_tc_operand(cent, C, dim, dpad, k.cb, k.kpad, kTcBase, ANN_METRIC_L2, 0, st))) return rc;
+    for (int64_t r0 = 0; r0 < n; r0 += k.chunk) {
+        const int nr = (int)std::min<int64_t>(k.chunk, n - r0);
+        TcGemmArgs g{nr, C, k.kpad, nullptr, k.keys, C, k.err};
+        g.out_cmin = k.cmin;
+        if ((rc = launch_tc_gemm(k.xb + (size_t)r0 * k.kpad, k.cb, g, st))) return rc;
+        ANN_CUDA_TRY(cudaMemsetAsync(k.amb_count, 0, sizeof(int), st));
+        const float* xr = x + r0 * dpad;
+        if ((rc = launch_kmeans_key_assign(k.keys, k.cmin, nr, C, xr, dpad, dim, k.norms + r0, cent, dpad, k.max2 + 2,
+                                           assign + r0, k.amb, k.amb_count, st)))
+            return rc;
+        if ((rc = launch_kmeans_ref_assign(xr, dpad, dim, cent, dpad, C, k.amb, k.amb_count, assign + r0, st))) return rc;
+    }
+    return ANN_OK;
+}
+
 // Nearest centroid of every row, as the reference's kmeans_assign_worker picks it (first minimum of
 // compute_l2_distance, lsh_index_optimized.cpp:32-47): the exact FP32 scan's two nearest per row,
 // certified by the rounding bound of both arithmetics, the near-ties redone in the reference's.
@@ -267,6 +352,7 @@ int ann_ivf_fit(ann_ivf* h, const float* data, int64_t n, int32_t dim, int64_t l
     float* mn = nullptr;
     float* mx = nullptr;
     int32_t* seed_rows = nullptr;
+    KmeansKeys kk;
     int rc = ANN_OK;
 #define FIT_TRY(x)          \
     do {                    \
@@ -290,13 +376,13 @@ int ann_ivf_fit(ann_ivf* h, const float* data, int64_t n, int32_t dim, int64_t l
         FIT_TRY(dmalloc(&idx, n));
         FIT_TRY(dmalloc(&order, n));
         FIT_TRY(dmalloc(&h->list_off, C + 1));
-        FIT_CUDA(cudaMemsetAsync(X, 0, sizeof(float) * (size_t)n * dpad, st));
+        if (dpad != dim) FIT_CUDA(cudaMemsetAsync(X, 0, sizeof(float) * (size_t)n * dpad, st));
         FIT_CUDA(cudaMemcpy2DAsync(X, sizeof(float) * dpad, data, sizeof(float) * ld, sizeof(float) * dim, n, kind, st));
         FIT_CUDA(cudaMemsetAsync(h->centroids, 0, sizeof(float) * (size_t)C * dpad, st));
         // rand_indices of run_kmeans: std::shuffle(iota(n), std::mt19937(1337)) (:553-555), the same
         // libstdc++ algorithm the reference runs. Row rand_indices[c] seeds list c (:557-561); row
         // rand_indices[(c * 37) % n] reseeds it whenever it ends an update empty (:608-613).
-        {
+        if (!centroids) {
             std::vector<int32_t> perm((size_t)n);
             std::iota(perm.begin(), perm.end(), 0);
             std::shuffle(perm.begin(), perm.end(), std::mt19937(1337));
@@ -315,20 +401,25 @@ int ann_ivf_fit(ann_ivf* h, const float* data, int64_t n, int32_t dim, int64_t l
         } else {
             FIT_TRY(launch_gather_rows(X, C, dpad, seed_rows, h->centroids, dpad, st));
         }
-        // iota for the sort values
-        {
-            std::vector<int32_t> io((size_t)n);
-            for (int64_t i = 0; i < n; ++i) io[i] = (int32_t)i;
-            FIT_CUDA(cudaMemcpyAsync(idx, io.data(), sizeof(int32_t) * n, cudaMemcpyHostToDevice, st));
-            FIT_CUDA(cudaStreamSynchronize(st));
-        }
+        FIT_TRY(launch_iota(idx, n, st));  // the sort values
+        // sort keys below C have few bits; a given assignment is sorted whole
+        int c_bits = 1;
+        while (c_bits < 31 && ((int64_t)1 << c_bits) < C) ++c_bits;
+        size_t tmp_few = 0;
         FIT_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tmp_bytes, a_raw, a_sorted, idx, order, (int)n, 0, 32, st));
+        FIT_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tmp_few, a_raw, a_sorted, idx, order, (int)n, 0, c_bits, st));
+        tmp_bytes = std::max(tmp_bytes, tmp_few);
         FIT_CUDA(cudaMalloc(&tmp, tmp_bytes));
         const bool given_assign = assign != nullptr;
         const int iters = (centroids || given_assign) ? 0 : kmeans_iters;
+        if (!given_assign) FIT_TRY(kmeans_keys_setup(kk, X, n, dim, dpad, h->centroids, C, centroids != nullptr, st));
+        auto assign_round = [&]() -> int {
+            if (kk.ok) return assign_rows_keys(kk, X, n, dim, dpad, h->centroids, C, a_raw, st);
+            return assign_rows(X, n, dim, dpad, h->centroids, C, a_raw, &h->ws, st);
+        };
         for (int it = 0; it < iters; ++it) {
-            FIT_TRY(assign_rows(X, n, dim, dpad, h->centroids, C, a_raw, &h->ws, st));
-            FIT_CUDA(cub::DeviceRadixSort::SortPairs(tmp, tmp_bytes, a_raw, a_sorted, idx, order, (int)n, 0, 32, st));
+            FIT_TRY(assign_round());
+            FIT_CUDA(cub::DeviceRadixSort::SortPairs(tmp, tmp_bytes, a_raw, a_sorted, idx, order, (int)n, 0, c_bits, st));
             FIT_TRY(launch_list_offsets(a_sorted, n, C, h->list_off, st));
             FIT_TRY(launch_kmeans_update(X, dpad, dim, order, h->list_off, C, h->centroids, dpad, seed_rows + C, n,
                                          fit_threads, st));
@@ -338,9 +429,10 @@ int ann_ivf_fit(ann_ivf* h, const float* data, int64_t n, int32_t dim, int64_t l
         if (given_assign) {
             FIT_CUDA(cudaMemcpyAsync(a_raw, assign, sizeof(int32_t) * n, kind, st));
         } else if (iters == 0) {
-            FIT_TRY(assign_rows(X, n, dim, dpad, h->centroids, C, a_raw, &h->ws, st));
+            FIT_TRY(assign_round());
         }
-        FIT_CUDA(cub::DeviceRadixSort::SortPairs(tmp, tmp_bytes, a_raw, a_sorted, idx, order, (int)n, 0, 32, st));
+        FIT_CUDA(cub::DeviceRadixSort::SortPairs(tmp, tmp_bytes, a_raw, a_sorted, idx, order, (int)n, 0,
+                                                 given_assign ? 32 : c_bits, st));
         FIT_TRY(launch_list_offsets(a_sorted, n, C, h->list_off, st));
         // reorder rows, SQ8 train / encode over the reordered rows
         FIT_TRY(dmalloc(&h->original, (size_t)n * dpad));
@@ -362,6 +454,15 @@ int ann_ivf_fit(ann_ivf* h, const float* data, int64_t n, int32_t dim, int64_t l
         h->C = C;
         FIT_TRY(ivf_finish_lists(h, st));
         FIT_CUDA(cudaStreamSynchronize(st));
+        if (kk.ok) {
+            int gave_up = 0;
+            FIT_CUDA(cudaMemcpy(&gave_up, kk.err, sizeof(int), cudaMemcpyDeviceToHost));
+            if (gave_up) {
+                set_error("ann_ivf_fit: a device-side wait gave up after its time limit");
+                rc = ANN_ERR_TIMEOUT;
+                goto fail;
+            }
+        }
     }
 fail:
     for (void* p : {(void*)X, (void*)a_raw, (void*)a_sorted, (void*)idx, (void*)order, tmp, (void*)mn, (void*)mx,

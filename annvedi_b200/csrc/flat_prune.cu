@@ -48,7 +48,7 @@ __device__ __forceinline__ void cp_async16_pr(float* smem, const float* gmem) {
 
 // one warp per row, grid-stride
 __global__ void __launch_bounds__(256) base_norms_kernel(const float* __restrict__ x, int64_t n, int dim, int64_t ld,
-                                                         unsigned* out2) {
+                                                         unsigned* out2, float2* __restrict__ rows) {
     const int lane = threadIdx.x & 31;
     unsigned ms = 0, mr = 0;
     for (int64_t r = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; r < n;
@@ -65,6 +65,7 @@ __global__ void __launch_bounds__(256) base_norms_kernel(const float* __restrict
             s += __shfl_xor_sync(0xffffffffu, s, o);
             e += __shfl_xor_sync(0xffffffffu, e, o);
         }
+        if (rows && lane == 0) rows[r] = make_float2(sqrtf(s), sqrtf(e));
         // non-negative floats order as their bit patterns, NaN above them all (its sign cleared)
         ms = max(ms, __float_as_uint(s) & 0x7fffffffu);
         mr = max(mr, __float_as_uint(e) & 0x7fffffffu);
@@ -331,10 +332,10 @@ int prune_bar_rank(int k, int64_t S, int64_t n) {
     return r;
 }
 
-int launch_base_norms(const float* x, int64_t n, int dim, int64_t ld, unsigned* out2, cudaStream_t st) {
+int launch_base_norms(const float* x, int64_t n, int dim, int64_t ld, unsigned* out2, cudaStream_t st, float2* rows) {
     ANN_CUDA_TRY(cudaMemsetAsync(out2, 0, 2 * sizeof(unsigned), st));
     if (n == 0) return ANN_OK;
-    base_norms_kernel<<<(unsigned)std::min<int64_t>(ceil_div(n, 8), 16 * kNumSMs), 256, 0, st>>>(x, n, dim, ld, out2);
+    base_norms_kernel<<<(unsigned)std::min<int64_t>(ceil_div(n, 8), 16 * kNumSMs), 256, 0, st>>>(x, n, dim, ld, out2, rows);
     ANN_LAUNCH_CHECK();
     return ANN_OK;
 }

@@ -19,8 +19,9 @@ constexpr float kPruneNormMin = 1e-12f, kPruneNormMax = 1e15f;
 constexpr int64_t kPruneMinRows = 32768;
 
 // out2 = bit patterns (uint32) of {largest squared norm, largest squared residual norm} over rows [n, dim] of
-// stride ld; a NaN anywhere leaves a NaN pattern.
-int launch_base_norms(const float* x, int64_t n, int dim, int64_t ld, unsigned* out2, cudaStream_t st);
+// stride ld; a NaN anywhere leaves a NaN pattern. rows (optional): each row's norm and residual norm.
+int launch_base_norms(const float* x, int64_t n, int dim, int64_t ld, unsigned* out2, cudaStream_t st,
+                      float2* rows = nullptr);
 
 struct PruneArgs {
     const float* base;  // [n, dpad]

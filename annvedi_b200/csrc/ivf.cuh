@@ -109,6 +109,9 @@ int launch_query_order(const int32_t* probes, int npc, int nq, int C, int32_t* o
 int launch_add_offset(int64_t* v, int64_t n, int64_t add, cudaStream_t st);  // v[i] += add
 // k-means of the reference (ivf_build.cu): certification of the fast two nearest centroids, the
 // reference arithmetic for the queued near-ties, and the ThreadPool-chunk-ordered update.
+int launch_kmeans_key_assign(const float* keys, const float* cmin, int n, int C, const float* x, int ldx, int dim,
+                             const float2* norms, const float* cent, int ldc, const unsigned* cnorm2, int32_t* assign,
+                             int32_t* amb, int* amb_count, cudaStream_t st);
 int launch_kmeans_certify(const float* key2, const int* id2, int64_t n, float margin, int32_t* assign, int32_t* amb,
                           int* amb_count, cudaStream_t st);
 int launch_kmeans_ref_assign(const float* x, int ldx, int dim, const float* cent, int ldc, int C, const int32_t* amb,

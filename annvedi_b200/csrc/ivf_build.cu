@@ -4,11 +4,13 @@
 // * k-means, the reference's run_kmeans (:551-616) reproduced bit for bit for a given ThreadPool
 //   size T (the reference sizes its pool from hardware_concurrency(), :140):
 //   - assignment (:32-47): each row goes to the first centroid with the smallest
-//     compute_l2_distance. The exact FP32 scan (flat_scan.cu) finds each row's two nearest
+//     compute_l2_distance. BF16 tensor-core keys leave, per row, the centroids inside the keys' error
+//     window; one takes the row, of several the reference's own arithmetic (refmath.cuh) decides, first
+//     minimum kept (kmeans_key_assign_kernel). Vectors whose norms the window does not cover, and small
+//     problems: the exact FP32 scan (flat_scan.cu) finds each row's two nearest
 //     centroids; when the second is farther than the first by more than the two arithmetics'
-//     combined rounding bound, the first is also the reference's choice (kmeans_certify_kernel).
-//     The remaining rows -- near-ties -- are recomputed against every centroid with the
-//     reference's own arithmetic (refmath.cuh), first minimum kept (kmeans_ref_assign_kernel).
+//     combined rounding bound, the first is also the reference's choice (kmeans_certify_kernel), and
+//     the near-ties are recomputed against every centroid (kmeans_ref_assign_kernel).
 //   - update (:60-73, :594-613): per list, each ThreadPool chunk's rows summed in row order from
 //     0.0f, the chunk sums added in chunk order from 0.0f, then multiplied by the float reciprocal
 //     of the count (the compiled reference's form of the division); an empty list takes row
@@ -19,6 +21,7 @@
 //   when the range is <= 1e-8, offset = min (or 0), code = clamp(round((x - offset) / scale)) with
 //   a true division and round-half-away-from-zero.
 #include "common.cuh"
+#include "flat_prune.cuh"
 #include "ivf.cuh"
 #include "refmath.cuh"
 
@@ -257,49 +260,177 @@ __global__ void __launch_bounds__(256) kmeans_ref_assign_kernel(const float* __r
     }
 }
 
-// One CTA per list, thread d on component d: the list's rows (order[off[c]..off[c+1]), ascending
-// ids) are summed per ThreadPool chunk -- chunk t of `active` covers [t*q + min(t, r), ...) with
-// q = n / active, r = n % active (src/thread_pool.h:93-124) -- and the chunk sums are added in
-// chunk order; chunks without rows of the list add 0.0f, which changes nothing. Then the sum times
-// the float reciprocal of the count; an empty list copies row reseed_rows[c].
-__global__ void kmeans_update_kernel(const float* __restrict__ x, int ldx, int dim, const int32_t* __restrict__ order,
-                                     const int64_t* __restrict__ off, float* __restrict__ cent, int ldc,
-                                     const int32_t* __restrict__ reseed_rows, int64_t q, int64_t r) {
-    const int c = blockIdx.x;
-    const int64_t b = off[c], e = off[c + 1];
-    const int64_t big = r * (q + 1);  // rows of the chunks one element longer
-    for (int d = threadIdx.x; d < dim; d += blockDim.x) {
-        if (e == b) {
-            cent[(int64_t)c * ldc + d] = x[(int64_t)reseed_rows[c] * ldx + d];
-            continue;
+// compute_l2_distance (ref_l2_f32) of the group's row pieces xr against centroid c, its pieces all loaded before the
+// first is used: the loop's loads, one a step, made each distance a chain of L2 round trips. dim <= 16 kRefPieces.
+constexpr int kRefPieces = 32;
+__device__ __forceinline__ float ref_l2_pieces(const float (&xr)[kRefPieces], const float* __restrict__ x,
+                                               const float* __restrict__ c, int dim) {
+    const int lane = threadIdx.x & 15;
+    const int full16 = dim >> 4;
+    float cv[kRefPieces];
+#pragma unroll
+    for (int i = 0; i < kRefPieces; ++i) cv[i] = i < full16 ? c[i * 16 + lane] : 0.f;
+    float acc = 0.f;
+#pragma unroll
+    for (int i = 0; i < kRefPieces; ++i)
+        if (i < full16) {
+            const float diff = __fsub_rn(xr[i], cv[i]);
+            acc = __fadd_rn(acc, __fmul_rn(diff, diff));
         }
-        float acc = 0.f, s = 0.f;
-        int64_t bound = -1;  // first row past the current chunk
-        constexpr int U = 8;
-        for (int64_t i0 = b; i0 < e; i0 += U) {
-            int32_t rows[U];
-            float v[U];
+    return ref_l2_tail(ref_fold16(acc), x, c, dim);
+}
+
+// Assignment from BF16 keys (tc_gemm.cuh) of every (row, centroid), keys [rows, C], and their 32-centroid chunk minima:
+// one warp per row. A centroid whose key exceeds the row's smallest by more than w = 2 eps + delta (eps: the keys'
+// error; delta: the rounding of two distances in the reference's arithmetic) is farther than that of the smallest key in
+// the reference's arithmetic too. One centroid within w takes the row; of several, the first minimum of the
+// reference's distances does, as it would among all. Rows that the bound does not cover are queued.
+// Bound by the latency of a row's chain of reads (minima, keys, then the 2-4 distances of a row whose cluster several
+// lists split): 111 us a round at 50k x 384 and 256 lists, where the scan of the two nearest, its merge and the
+// near-ties against every centroid took 2.2 ms.
+__global__ void __launch_bounds__(256) kmeans_key_assign_kernel(const float* __restrict__ keys,
+                                                                const float* __restrict__ cmin, int n, int C,
+                                                                const float* __restrict__ x, int ldx, int dim,
+                                                                const float2* __restrict__ norms,
+                                                                const float* __restrict__ cent, int ldc,
+                                                                const unsigned* __restrict__ cnorm2,
+                                                                int32_t* __restrict__ assign, int32_t* __restrict__ amb,
+                                                                int* __restrict__ amb_count) {
+    const int i = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (i >= n) return;  // the whole warp
+    const float2 nr = norms[i];
+    const float xn = nr.x * 1.001f, xe = nr.y * 1.001f;
+    const float cm = sqrtf(__uint_as_float(cnorm2[0])) * 1.001f, rm = sqrtf(__uint_as_float(cnorm2[1])) * 1.001f;
+    const float acc = (float)(dim + 19) * 4.76837158e-7f;  // (dim + 19) 2^-21
+    const float cross = rm * xn + (cm + rm) * xe;
+    const float w = 1.002f * (2.f * (2.f * cross + acc * (2.f * (cm + rm) * (xn + xe) + cm * cm)) +
+                              acc * (xn + cm) * (xn + cm));
+    const bool covered = xn <= kPruneNormMax && (xn >= kPruneNormMin || nr.x == 0.f) && cm <= kPruneNormMax &&
+                         cm >= kPruneNormMin;  // false for NaN
+    const int nch = (C + 31) >> 5;
+    const float* kr = keys + (int64_t)i * C;
+    const float* cr = cmin + (int64_t)i * nch;
+    float T = kInf;
+    for (int c = lane; c < nch; c += 32) T = fminf(T, cr[c]);
 #pragma unroll
-            for (int u = 0; u < U; ++u) rows[u] = i0 + u < e ? order[i0 + u] : -1;
+    for (int o = 16; o > 0; o >>= 1) T = fminf(T, __shfl_xor_sync(0xffffffffu, T, o));
+    const float lim = __fadd_ru(T, w);
+    if (!covered || !(lim < kInf)) {
+        if (lane == 0) amb[atomicAdd(amb_count, 1)] = i;
+        return;
+    }
+    // the centroids within the window, chunk by chunk: counted first, then (several) their distances in turn
+    int count = 0, only = 0;
+    for (int c0 = 0; c0 < nch; c0 += 32) {
+        unsigned cm32 = __ballot_sync(0xffffffffu, c0 + lane < nch && cr[c0 + lane] <= lim);
+        while (cm32) {
+            const int ch = c0 + __ffs(cm32) - 1;
+            cm32 &= cm32 - 1;
+            const int c = ch * 32 + lane;
+            const unsigned hit = __ballot_sync(0xffffffffu, c < C && kr[c] <= lim);
+            if (hit) only = ch * 32 + __ffs(hit) - 1;
+            count += __popc(hit);
+        }
+    }
+    if (count == 1) {
+        if (lane == 0) assign[i] = only;
+        return;
+    }
+    const float* xr = x + (int64_t)i * ldx;
+    const int g = lane >> 4, l16 = lane & 15;
+    const bool pieces = dim <= 16 * kRefPieces;
+    float xp[kRefPieces];
 #pragma unroll
-            for (int u = 0; u < U; ++u) v[u] = rows[u] >= 0 ? x[(int64_t)rows[u] * ldx + d] : 0.f;
-#pragma unroll
-            for (int u = 0; u < U; ++u) {
-                if (rows[u] < 0) break;
-                if (rows[u] >= bound) {  // a new chunk starts: fold the finished one in
-                    acc = __fadd_rn(acc, s);
-                    s = 0.f;
-                    const int64_t rr = rows[u];
-                    const int64_t t = rr < big ? rr / (q + 1) : r + (rr - big) / q;
-                    bound = (t + 1) * q + min(t + 1, r);
+    for (int p = 0; p < kRefPieces; ++p) xp[p] = pieces && p < (dim >> 4) ? xr[p * 16 + l16] : 0.f;
+    float best = FLT_MAX;
+    int bc = INT_MAX;
+    for (int c0 = 0; c0 < nch; c0 += 32) {
+        unsigned cm32 = __ballot_sync(0xffffffffu, c0 + lane < nch && cr[c0 + lane] <= lim);
+        while (cm32) {
+            const int ch = c0 + __ffs(cm32) - 1;
+            cm32 &= cm32 - 1;
+            const int c = ch * 32 + lane;
+            unsigned hit = __ballot_sync(0xffffffffu, c < C && kr[c] <= lim);
+            while (hit) {  // two centroids at a time, one per 16-lane group
+                const int ca = ch * 32 + __ffs(hit) - 1;
+                hit &= hit - 1;
+                const bool two = hit != 0;
+                const int cb = two ? ch * 32 + __ffs(hit) - 1 : ca;
+                hit &= hit - 1;
+                const int cc = g ? cb : ca;
+                const float* cp = cent + (int64_t)cc * ldc;
+                const float d = pieces ? ref_l2_pieces(xp, xr, cp, dim) : ref_l2_f32(xr, cp, dim, NoEmit{});
+                if ((g == 0 || two) && d < best) {  // ascending centroids: the first minimum stays
+                    best = d;
+                    bc = cc;
                 }
-                s = __fadd_rn(s, v[u]);
             }
         }
-        acc = __fadd_rn(acc, s);
-        const float rc = __fdiv_rn(1.0f, (float)(e - b));
-        cent[(int64_t)c * ldc + d] = __fmul_rn(acc, rc);
     }
+    const float ob = __shfl_xor_sync(0xffffffffu, best, 16);
+    const int oc = __shfl_xor_sync(0xffffffffu, bc, 16);
+    if (ob < best || (ob == best && oc < bc)) bc = oc;
+    if (lane == 0) assign[i] = bc == INT_MAX ? 0 : bc;
+}
+
+// The list's rows (order[off[c]..off[c+1]), ascending ids) are summed per ThreadPool chunk -- chunk t of `active` covers
+// [t*q + min(t, r), ...) with q = n / active, r = n % active (src/thread_pool.h:93-124) -- and the chunk sums are added
+// in chunk order; chunks without rows of the list add 0.0f, which changes nothing. Then the sum times the float
+// reciprocal of the count; an empty list copies row reseed_rows[c].
+// CTA (list, 32 components); warp w sums chunks w, w + 16, ... (a chunk's rows in order: one serial chain per
+// component, so the chunks are the parallelism), then warp 0 adds the 16 chunk sums in order. With one thread a
+// component for the whole list, a list's rows were one chain of dependent gathers: 255 us a round at 50k x 384 and 256
+// lists, 65 us now.
+constexpr int kUpdWarps = 16;
+__global__ void __launch_bounds__(32 * kUpdWarps) kmeans_update_kernel(const float* __restrict__ x, int ldx, int dim,
+                                                                      const int32_t* __restrict__ order,
+                                                                      const int64_t* __restrict__ off,
+                                                                      float* __restrict__ cent, int ldc,
+                                                                      const int32_t* __restrict__ reseed_rows,
+                                                                      int64_t q, int64_t r, int active) {
+    __shared__ float sSum[kUpdWarps][32];
+    const int c = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int d = blockIdx.y * 32 + lane;
+    const bool in = d < dim;
+    const int64_t b = off[c], e = off[c + 1];
+    if (e == b) {
+        if (warp == 0 && in) cent[(int64_t)c * ldc + d] = x[(int64_t)reseed_rows[c] * ldx + d];
+        return;
+    }
+    auto lower = [&](int64_t row) {  // first position of [b, e) whose row is >= row
+        int64_t lo = b, hi = e;
+        while (lo < hi) {
+            const int64_t mid = (lo + hi) >> 1;
+            if (order[mid] < row)
+                lo = mid + 1;
+            else
+                hi = mid;
+        }
+        return lo;
+    };
+    float acc = 0.f;  // warp 0
+    for (int t0 = 0; t0 < active; t0 += kUpdWarps) {
+        const int64_t t = t0 + warp;
+        float s = 0.f;
+        if (t < active) {
+            const int64_t i1 = lower((t + 1) * q + min(t + 1, r));
+            constexpr int U = 8;
+            for (int64_t i0 = lower(t * q + min(t, r)); i0 < i1; i0 += U) {
+                float v[U];
+#pragma unroll
+                for (int u = 0; u < U; ++u) v[u] = i0 + u < i1 && in ? x[(int64_t)order[i0 + u] * ldx + d] : 0.f;
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+                    if (i0 + u < i1) s = __fadd_rn(s, v[u]);
+            }
+        }
+        sSum[warp][lane] = s;
+        __syncthreads();
+        if (warp == 0)
+            for (int w = 0; w < kUpdWarps; ++w) acc = __fadd_rn(acc, sSum[w][lane]);
+        __syncthreads();
+    }
+    if (warp == 0 && in) cent[(int64_t)c * ldc + d] = __fmul_rn(acc, __fdiv_rn(1.0f, (float)(e - b)));
 }
 
 int launch_kmeans_certify(const float* key2, const int* id2, int64_t n, float margin, int32_t* assign, int32_t* amb,
@@ -323,9 +454,18 @@ int launch_kmeans_update(const float* x, int ldx, int dim, const int32_t* order,
                          cudaStream_t st) {
     ANN_CHECK_ARG(num_threads >= 1 && n >= 1, "k-means update: %d threads over %lld rows", num_threads, (long long)n);
     const int64_t active = std::min<int64_t>(num_threads, n);  // run_parallel's actual_threads
-    const int threads = (int)std::min<int64_t>(1024, ceil_div(dim, 32) * 32);
-    kmeans_update_kernel<<<C, threads, 0, st>>>(x, ldx, dim, order, off, centroids, ldc, reseed_rows, n / active,
-                                                n % active);
+    kmeans_update_kernel<<<dim3(C, (unsigned)ceil_div(dim, 32)), 32 * kUpdWarps, 0, st>>>(
+        x, ldx, dim, order, off, centroids, ldc, reseed_rows, n / active, n % active, (int)active);
+    ANN_LAUNCH_CHECK();
+    return ANN_OK;
+}
+
+int launch_kmeans_key_assign(const float* keys, const float* cmin, int n, int C, const float* x, int ldx, int dim,
+                             const float2* norms, const float* cent, int ldc, const unsigned* cnorm2, int32_t* assign,
+                             int32_t* amb, int* amb_count, cudaStream_t st) {
+    if (n == 0) return ANN_OK;
+    kmeans_key_assign_kernel<<<(unsigned)ceil_div(n, 8), 256, 0, st>>>(keys, cmin, n, C, x, ldx, dim, norms, cent, ldc,
+                                                                      cnorm2, assign, amb, amb_count);
     ANN_LAUNCH_CHECK();
     return ANN_OK;
 }

@@ -27,24 +27,11 @@ __device__ __forceinline__ float ref_fold16(float lane_val) {
 // Number of checkpoint values (checkpoints + the final fold) for `dim`.
 __host__ __device__ inline int ref_num_checkpoints(int dim) { return dim / 16 / 6 + 1; }
 
-// FP32 distance between x and q (both `dim` floats), computed by the calling 16-thread group.
-// Calls emit(c, value) for checkpoint c = 0..ref_num_checkpoints(dim)-1 (the last is the final
-// fold before the remainder). Returns the full distance in every lane of the group. All 32 lanes of
-// the warp must call it together (both halves run a group each).
-template <class Emit>
-__device__ __forceinline__ float ref_l2_f32(const float* __restrict__ x, const float* __restrict__ q, int dim,
-                                            Emit&& emit) {
+// The full distance from the fold `sum` of the full 16-chunks: the remainder (dim % 16) added by the group's first
+// lane, the result in every lane of the group.
+__device__ __forceinline__ float ref_l2_tail(float sum, const float* __restrict__ x, const float* __restrict__ q, int dim) {
     const int lane = threadIdx.x & 15;
     const int full16 = dim >> 4;
-    float acc = 0.f;
-    int cp = 0;
-    for (int c = 0; c < full16; ++c) {
-        const float diff = __fsub_rn(x[c * 16 + lane], q[c * 16 + lane]);
-        acc = __fadd_rn(acc, __fmul_rn(diff, diff));
-        if (c % 6 == 5) emit(cp++, ref_fold16(acc));
-    }
-    float sum = ref_fold16(acc);
-    emit(cp, sum);
     if (lane == 0) {
         int i = full16 * 16;
         if (dim - i >= 8) {
@@ -65,6 +52,27 @@ __device__ __forceinline__ float ref_l2_f32(const float* __restrict__ x, const f
         }
     }
     return __shfl_sync(0xffffffffu, sum, 0, 16);
+}
+
+// FP32 distance between x and q (both `dim` floats), computed by the calling 16-thread group.
+// Calls emit(c, value) for checkpoint c = 0..ref_num_checkpoints(dim)-1 (the last is the final
+// fold before the remainder). Returns the full distance in every lane of the group. All 32 lanes of
+// the warp must call it together (both halves run a group each).
+template <class Emit>
+__device__ __forceinline__ float ref_l2_f32(const float* __restrict__ x, const float* __restrict__ q, int dim,
+                                            Emit&& emit) {
+    const int lane = threadIdx.x & 15;
+    const int full16 = dim >> 4;
+    float acc = 0.f;
+    int cp = 0;
+    for (int c = 0; c < full16; ++c) {
+        const float diff = __fsub_rn(x[c * 16 + lane], q[c * 16 + lane]);
+        acc = __fadd_rn(acc, __fmul_rn(diff, diff));
+        if (c % 6 == 5) emit(cp++, ref_fold16(acc));
+    }
+    float sum = ref_fold16(acc);
+    emit(cp, sum);
+    return ref_l2_tail(sum, x, q, dim);
 }
 
 // SQ8 distance sum_d (code[d]*scale[d] - qs[d])^2, the reference's arithmetic.
