@@ -1,0 +1,89 @@
+// Block-wide selection of the k smallest (key, id) pairs, held as 64-bit words (ordered key bits, then id).
+#pragma once
+#include <stdint.h>
+
+#include "common.cuh"
+
+namespace annb {
+
+// The order-preserving integer image of a float (no NaN) and back.
+__device__ __forceinline__ uint32_t ord_f32(float f) {
+    const uint32_t u = __float_as_uint(f);
+    return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
+}
+__device__ __forceinline__ float f32_ord(uint32_t o) {
+    return __uint_as_float((o & 0x80000000u) ? (o & 0x7fffffffu) : ~o);
+}
+// The digit (8 bits) of rank `rem` (1-based) of the block's 256-bin histogram: every thread gets the digit, the
+// count below it and the digit's own count. One bin per thread of the first 256; sMisc: 12 ints.
+__device__ __forceinline__ void block_pick(const int* hist, int rem, int* sMisc, int* digit, int* before, int* own) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int c = threadIdx.x < 256 ? hist[threadIdx.x] : 0;
+    int incl = c;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += y;
+    }
+    if (lane == 31 && warp < 8) sMisc[warp] = incl;
+    __syncthreads();
+    for (int w = 0; w < min(warp, 8); ++w) incl += sMisc[w];
+    if (threadIdx.x < 256 && incl - c < rem && rem <= incl) {
+        sMisc[8] = threadIdx.x;
+        sMisc[9] = incl - c;
+        sMisc[10] = c;
+    }
+    __syncthreads();
+    *digit = sMisc[8];
+    *before = sMisc[9];
+    *own = sMisc[10];
+}
+
+// The k smallest of a set of distinct words are those with (word & mask) <= prefix.
+struct SelectBound {
+    unsigned long long prefix, mask;
+    __device__ __forceinline__ bool in(unsigned long long w) const { return (w & mask) <= prefix; }
+};
+
+// The bound of the k smallest (1 <= k <= m) of the words at(0..m): 8-bit digits from the top until one ends at the k-th
+// exactly. Whole block of >= 256 threads; sHist: 256 ints, sMisc: 12 ints. Ends with a barrier passed.
+template <class At>
+__device__ __forceinline__ SelectBound block_select_bound(At&& at, int m, int k, int* sHist, int* sMisc) {
+    SelectBound b{0, 0};
+    int rem = k;
+    for (int shift = 56; shift >= 0; shift -= 8) {
+        if (threadIdx.x < 256) sHist[threadIdx.x] = 0;
+        __syncthreads();
+        for (int i = threadIdx.x; i < m; i += blockDim.x) {
+            const unsigned long long w = at(i);
+            if ((w & b.mask) == b.prefix) atomicAdd(&sHist[(int)(w >> shift) & 255], 1);
+        }
+        __syncthreads();
+        int d, before, own;
+        block_pick(sHist, rem, sMisc, &d, &before, &own);
+        rem -= before;
+        b.prefix |= (unsigned long long)d << shift;
+        b.mask |= 255ull << shift;
+        if (rem == own) break;  // uniform
+    }
+    return b;
+}
+
+// Ascending bitonic sort of n words (a power of two) in shared memory by the block; starts and ends with a barrier.
+__device__ __forceinline__ void block_sort_u64(unsigned long long* w, int n) {
+    __syncthreads();
+    for (int size = 2; size <= n; size <<= 1)
+        for (int stride = size >> 1; stride > 0; stride >>= 1) {
+            for (int t = threadIdx.x; t < n / 2; t += blockDim.x) {
+                const int lo = 2 * t - (t & (stride - 1)), hi = lo + stride;
+                const unsigned long long x = w[lo], y = w[hi];
+                if ((x > y) == ((lo & size) == 0)) {
+                    w[lo] = y;
+                    w[hi] = x;
+                }
+            }
+            __syncthreads();
+        }
+}
+
+}  // namespace annb

@@ -341,7 +341,7 @@ int ann_flat_query(ann_flat* h, ann_workspace* ws, const float* queries, int32_t
     const bool need_pad = host || (mode == ANN_MODE_EXACT && (ldq != dpad || (reinterpret_cast<uintptr_t>(queries) & 15)));
 
     // ---- plan the scratch: [padded queries][device outputs][search scratch] ----
-    int bq = 0, nsplit = 0, qc = 0, ncp = 0;
+    int bq = 0, nsplit = 0, qc = 0, ncp = 0, nseg = 0;
     int64_t rps = 0;
     Sizer sz;
     if (need_pad) sz.take<float>((size_t)nq * dpad);
@@ -364,14 +364,15 @@ int ann_flat_query(ann_flat* h, ann_workspace* ws, const float* queries, int32_t
         }
     } else {
         ncp = compat_num_checkpoints(h->dim);
-        const size_t per_q = sizeof(float) * (size_t)h->n * (ncp + 2) + (size_t)8 * kk;
+        nseg = (int)ceil_div(h->n, compat_seg_rows(h->n));
+        const size_t per_q = sizeof(float) * (size_t)h->n * (ncp + 2) + (size_t)nseg * (64 * 4 + (size_t)kk * 8);
         const size_t budget = (size_t)1 << 30;
-        qc = (int)std::max<size_t>(1, std::min<size_t>((size_t)nq, budget / per_q));
+        qc = (int)std::min<size_t>(32768, std::max<size_t>(1, std::min<size_t>((size_t)nq, budget / per_q)));
         sz.take<float>((size_t)qc * h->n);
         sz.take<float>((size_t)qc * h->n * ncp);
         sz.take<float>((size_t)qc * h->n);
-        sz.take<float>((size_t)qc * kk);
-        sz.take<int>((size_t)qc * kk);
+        sz.take<float>((size_t)qc * nseg * 64);
+        sz.take<unsigned long long>((size_t)qc * nseg * kk);
     }
     int rc = ws_reserve_device(ws, sz.bytes());
     if (rc) return rc;
@@ -447,8 +448,8 @@ int ann_flat_query(ann_flat* h, ann_workspace* ws, const float* queries, int32_t
         a.D = cv.take<float>((size_t)qc * h->n);
         a.P = cv.take<float>((size_t)qc * h->n * ncp);
         a.T = cv.take<float>((size_t)qc * h->n);
-        a.kbuf = cv.take<float>((size_t)qc * kk);
-        a.ibuf = cv.take<int>((size_t)qc * kk);
+        a.seg_heap = cv.take<float>((size_t)qc * nseg * 64);
+        a.seg_best = cv.take<unsigned long long>((size_t)qc * nseg * kk);
         a.out_ids = ids_dev;
         a.out_dists = dists_dev;
         for (int q0 = 0; q0 < nq; q0 += qc) {

@@ -14,20 +14,26 @@
 // compiled reference too: one fused 8-wide chunk folded the same way, then scalar fused steps.
 // It writes the full distance D[q][i] and the checkpoint values P[q][c][i].
 //
-// Pass 2 (compat_threshold_kernel) is one warp per query walking the rows in order: the running
-// 64-heap is replayed only at insertions (rows with D < T, which are rare once T settles), and each
-// row's threshold T_i is recorded. Pass 3 (compat_values_kernel), parallel over rows, picks v_i from D,
-// P and T_i. The k best (v_i, i) pairs come from the radix selection (the exact set, ties by row) and
-// a sort of those k.
+// Pass 2, the thresholds: T_i is a prefix order statistic, so the rows are cut into up to 128 segments. Each
+// segment's `lim` smallest distances are found on their own (compat_segments_kernel), merged into the heap the
+// reference holds at every segment's first row (compat_prefix_kernel), and one warp a segment walks its rows from
+// there, replaying insertions (rows with D < T, rare once T settles) and recording each row's threshold
+// (compat_threshold_kernel). As one walk of all rows by one warp this took 248 of a query's 436 us at 100k x 384; what
+// bounds it now is the first segment's walk, about 240 insertions of 290 clocks each (37 us).
+// Pass 3 (compat_values_kernel) picks v_i from D, P and T_i, and each segment's k best (v_i, i) by block; the k best of
+// those, sorted, are the result (compat_final_kernel).
+#include <cfloat>
+
+#include "block_select.cuh"
 #include "common.cuh"
 #include "compat.cuh"
-#include "flat_scan.cuh"
-#include "radix_select.cuh"
 #include "refmath.cuh"
 
 namespace annb {
 
-// grid: (row blocks, query groups); block: 256 threads = 16 rows x 16 lanes.
+// grid: (row blocks, query groups); block: 256 threads = 16 rows x 16 lanes. PIECES: the row's 16-chunks held in
+// registers (dim <= 16 PIECES; 0: any dim), so that a row's loads are in flight together.
+template <int PIECES>
 __global__ void __launch_bounds__(256) compat_partials_kernel(CompatArgs a, int q_begin) {
     extern __shared__ float sQ[];  // [QG][dim]
     const int grp = threadIdx.x >> 4;
@@ -41,12 +47,21 @@ __global__ void __launch_bounds__(256) compat_partials_kernel(CompatArgs a, int 
         const int64_t row = r0 + grp;
         const bool valid = row < a.n;
         const float* x = a.base + (valid ? row : 0) * a.ldb;
+        float xr[PIECES > 0 ? PIECES : 1];  // the row's full 16-chunks, loaded once for the queries
+#pragma unroll
+        for (int c = 0; c < PIECES; ++c) xr[c] = c < (a.dim >> 4) ? x[c * 16 + (threadIdx.x & 15)] : 0.f;
         for (int qq = 0; qq < nqg; ++qq) {
             const int64_t qi = qg0 + qq - q_begin;  // index within this chunk of queries
             float* P = a.P + (int64_t)qi * ncp * a.n + row;
-            const float d = ref_l2_f32(x, sQ + qq * a.dim, a.dim, [&](int c, float v) {
+            auto emit = [&](int c, float v) {
                 if (leader && valid) P[(int64_t)c * a.n] = v;
-            });
+            };
+            const float* qv = sQ + qq * a.dim;
+            float d;
+            if constexpr (PIECES > 0)
+                d = ref_l2_f32_pieces(xr, x, qv, a.dim, emit);
+            else
+                d = ref_l2_f32(x, qv, a.dim, emit);
             if (leader && valid) a.D[(int64_t)qi * a.n + row] = d;
         }
     }
@@ -54,37 +69,35 @@ __global__ void __launch_bounds__(256) compat_partials_kernel(CompatArgs a, int 
 
 constexpr int kCompatAhead = 8;  // 32-row steps of distances loaded ahead of the walk
 
-__global__ void __launch_bounds__(128) compat_threshold_kernel(CompatArgs a, int q_begin) {
-    constexpr int WARPS = 4;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int qi = blockIdx.x * WARPS + warp;  // within chunk
-    if (q_begin + qi >= a.q_end) return;       // the whole warp; no block barrier follows
-    const int lim = a.k < 64 ? a.k : 64;
-    const int64_t n = a.n;
-    const float* D = a.D + (int64_t)qi * n;
-    float* T = a.T + (int64_t)qi * n;
+constexpr int kCompatWarps = 4;
+
+int64_t compat_seg_rows(int64_t n) { return ceil_div(ceil_div(n, kCompatMaxSegs), 1024) * 1024; }
+
+// Walks rows [begin, end) of D through the heap in row order; out(i, T_i, valid) per row.
+template <class Out>
+__device__ __forceinline__ void compat_walk(const float* __restrict__ D, int64_t begin, int64_t end, WarpHeap64& heap,
+                                            Out&& out) {
+    const int lane = threadIdx.x & 31;
     const float inf = __int_as_float(0x7f800000);
-    WarpHeap64 heap;
-    heap.init(lim);
-    float Tcur = 3.402823466e+38f;  // FLT_MAX until the heap holds lim distances
+    float Tcur = heap.worst();
     float nxt[kCompatAhead];
 #pragma unroll
     for (int j = 0; j < kCompatAhead; ++j) {
-        const int64_t i = (int64_t)j * 32 + lane;
-        nxt[j] = i < n ? D[i] : inf;
+        const int64_t i = begin + (int64_t)j * 32 + lane;
+        nxt[j] = i < end ? D[i] : inf;
     }
-    for (int64_t base = 0; base < n; base += 32 * kCompatAhead) {
+    for (int64_t base = begin; base < end; base += 32 * kCompatAhead) {
         float cur[kCompatAhead];
 #pragma unroll
         for (int j = 0; j < kCompatAhead; ++j) {
             cur[j] = nxt[j];
             const int64_t i = base + 32 * kCompatAhead + (int64_t)j * 32 + lane;
-            nxt[j] = i < n ? D[i] : inf;
+            nxt[j] = i < end ? D[i] : inf;
         }
 #pragma unroll
         for (int j = 0; j < kCompatAhead; ++j) {
             const int64_t i = base + (int64_t)j * 32 + lane;
-            const bool valid = i < n;
+            const bool valid = i < end;
             const float d = cur[j];
             // rows enter the heap in row order; a row's threshold is the heap's before its own insertion
             float myT = Tcur;
@@ -98,31 +111,159 @@ __global__ void __launch_bounds__(128) compat_threshold_kernel(CompatArgs a, int
                 if (lane > l0) myT = Tcur;
                 last = l0;
             }
-            if (valid) T[i] = myT;
+            out(i, myT, valid);
         }
     }
 }
 
-// v_i = d_i when d_i < T_i, else the first checkpoint value >= T_i (d_i if none), written over T_i.
-__global__ void __launch_bounds__(256) compat_values_kernel(CompatArgs a, int q_count) {
-    const int64_t n = a.n;
-    for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < (int64_t)q_count * n;
-         e += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t qi = e / n, i = e - qi * n;
-        const float d = a.D[e];
-        const float t = a.T[e];
+// (v, row) as one word; NaN orders after +inf.
+__device__ __forceinline__ unsigned long long compat_word(float v, int64_t row) {
+    if (v != v) v = __int_as_float(0x7fffffff);
+    return ((unsigned long long)ord_f32(v + 0.f) << 32) | (unsigned)row;
+}
+
+// One block per (segment, query): the segment's `lim` smallest distances, ascending (FLT_MAX where fewer than lim are
+// below it, as the heap's empty slots).
+__global__ void __launch_bounds__(256) compat_segments_kernel(CompatArgs a) {
+    __shared__ int sHist[256];
+    __shared__ int sMisc[12];
+    __shared__ int sN;
+    __shared__ unsigned long long sR[64];
+    const int s = blockIdx.x, qi = blockIdx.y;
+    const float* D = a.D + (int64_t)qi * a.n + (int64_t)s * a.seg_rows;
+    const int m = (int)a.seg_rows;  // the last, shorter segment's list serves no later one and is not made
+    const int lim = a.k < 64 ? a.k : 64;
+    if (threadIdx.x == 0) sN = 0;
+    if (threadIdx.x < 64) sR[threadIdx.x] = ~0ull;
+    __syncthreads();
+    auto at = [&](int i) { return compat_word(D[i], i); };
+    const SelectBound b = block_select_bound(at, m, lim, sHist, sMisc);
+    for (int i = threadIdx.x; i < m; i += 256) {
+        const unsigned long long w = at(i);
+        if (b.in(w)) sR[atomicAdd(&sN, 1)] = w;
+    }
+    block_sort_u64(sR, 64);
+    if (threadIdx.x < 64) {
+        const float v = threadIdx.x < lim ? f32_ord((uint32_t)(sR[threadIdx.x] >> 32)) : FLT_MAX;
+        a.seg_heap[((int64_t)qi * a.nseg + s) * 64 + threadIdx.x] = v < FLT_MAX ? v : FLT_MAX;  // inf, NaN: never held
+    }
+}
+
+// One warp per query: seg_heap[s] := the heap the reference holds at segment s's first row, the `lim` smallest of the
+// earlier segments' lists. Two ascending lists a, b of 64 values: min(a[i], b[63 - i]) are the 64 smallest, a bitonic
+// sequence, which six exchange steps sort. Lane l holds values l and l + 32. The lists are staged in shared memory by
+// the block first: a list's load from L2 takes longer than its merge.
+__global__ void __launch_bounds__(256) compat_prefix_kernel(CompatArgs a) {
+    __shared__ float sL[kCompatMaxSegs * 64];
+    const int lane = threadIdx.x & 31, qi = blockIdx.x;
+    const int lim = a.k < 64 ? a.k : 64;
+    float* L = a.seg_heap + (int64_t)qi * a.nseg * 64;
+    for (int i = threadIdx.x; i < (a.nseg - 1) * 64; i += 256) sL[i] = L[i];  // the last segment has no list
+    __syncthreads();
+    if (threadIdx.x >= 32) return;
+    float lo = FLT_MAX, hi = FLT_MAX;
+    for (int s = 0; s < a.nseg; ++s) {
+        L[s * 64 + lane] = lo;
+        L[s * 64 + lane + 32] = hi;
+        if (s + 1 >= a.nseg) break;
+        const float b0 = sL[s * 64 + lane], b1 = sL[s * 64 + lane + 32];
+        // value i meets value 63 - i: lane l's lo meets lane 31 - l's hi, and its hi meets that lane's lo
+        lo = fminf(lo, __shfl_xor_sync(0xffffffffu, b1, 31));
+        hi = fminf(hi, __shfl_xor_sync(0xffffffffu, b0, 31));
+        const float t = fminf(lo, hi);  // step 32
+        hi = fmaxf(lo, hi);
+        lo = t;
+#pragma unroll
+        for (int d = 16; d > 0; d >>= 1) {
+            const float ol = __shfl_xor_sync(0xffffffffu, lo, d), oh = __shfl_xor_sync(0xffffffffu, hi, d);
+            const bool low = (lane & d) == 0;
+            lo = low ? fminf(lo, ol) : fmaxf(lo, ol);
+            hi = low ? fminf(hi, oh) : fmaxf(hi, oh);
+        }
+        if (lane >= lim) lo = FLT_MAX;
+        if (lane + 32 >= lim) hi = FLT_MAX;
+    }
+}
+
+// One warp per (segment, query): each row's threshold, from the segment's starting heap.
+__global__ void __launch_bounds__(32 * kCompatWarps) compat_threshold_kernel(CompatArgs a) {
+    const int s = blockIdx.x * kCompatWarps + (threadIdx.x >> 5), lane = threadIdx.x & 31, qi = blockIdx.y;
+    if (s >= a.nseg) return;  // the whole warp
+    WarpHeap64 heap;
+    heap.init(a.k < 64 ? a.k : 64);
+    if (s > 0) {
+        const float* L = a.seg_heap + ((int64_t)qi * a.nseg + s) * 64;
+        heap.lo = L[lane];
+        heap.hi = L[lane + 32];
+    }
+    const int64_t begin = (int64_t)s * a.seg_rows;
+    float* T = a.T + (int64_t)qi * a.n;
+    compat_walk(a.D + (int64_t)qi * a.n, begin, min(a.n, begin + a.seg_rows), heap, [&](int64_t i, float t, bool valid) {
+        if (valid) T[i] = t;
+    });
+}
+
+// v_i = d_i when d_i < T_i, else the first checkpoint value >= T_i (d_i if none), written over T_i; then the segment's
+// best min(k, rows) (v_i, i), in no order. One block per (segment, query).
+__global__ void __launch_bounds__(256) compat_values_kernel(CompatArgs a) {
+    __shared__ int sHist[256];
+    __shared__ int sMisc[12];
+    __shared__ int sN;
+    const int s = blockIdx.x, qi = blockIdx.y;
+    const int64_t n = a.n, begin = (int64_t)s * a.seg_rows;
+    const int m = (int)min(a.seg_rows, n - begin);
+    const float* D = a.D + (int64_t)qi * n + begin;
+    float* T = a.T + (int64_t)qi * n + begin;
+    const float* P0 = a.P + (int64_t)qi * a.ncp * n + begin;
+    for (int e = threadIdx.x; e < m; e += 256) {
+        const float d = D[e];
+        const float t = T[e];
         float v = d;
         if (!(d < t)) {
-            const float* P = a.P + qi * a.ncp * n + i;
             for (int c = 0; c < a.ncp; ++c) {
-                const float p = P[(int64_t)c * n];
+                const float p = P0[(int64_t)c * n + e];
                 if (p >= t) {
                     v = p;
                     break;
                 }
             }
         }
-        a.T[e] = v;
+        T[e] = v;
+    }
+    if (threadIdx.x == 0) sN = 0;
+    __syncthreads();
+    const int kk = min(a.k, m);
+    auto at = [&](int i) { return compat_word(T[i], begin + i); };
+    const SelectBound b = block_select_bound(at, m, kk, sHist, sMisc);
+    unsigned long long* out = a.seg_best + ((int64_t)qi * a.nseg + s) * a.k;
+    for (int i = threadIdx.x; i < m; i += 256) {
+        const unsigned long long w = at(i);
+        if (b.in(w)) out[atomicAdd(&sN, 1)] = w;
+    }
+    for (int i = kk + threadIdx.x; i < a.k; i += 256) out[i] = ~0ull;
+}
+
+// The k best of the segments' best, in order. One block per query.
+__global__ void __launch_bounds__(512) compat_final_kernel(CompatArgs a, int q_begin) {
+    __shared__ int sHist[256];
+    __shared__ int sMisc[12];
+    __shared__ int sN;
+    __shared__ unsigned long long sR[512];
+    const int qi = blockIdx.x;
+    const unsigned long long* w = a.seg_best + (int64_t)qi * a.nseg * a.k;
+    const int m = a.nseg * a.k;
+    if (threadIdx.x == 0) sN = 0;
+    __syncthreads();
+    const SelectBound b = block_select_bound([&](int i) { return w[i]; }, m, a.k, sHist, sMisc);
+    const int p2 = pow2_ceil(a.k);
+    for (int i = threadIdx.x; i < m; i += 512)
+        if (b.in(w[i])) sR[atomicAdd(&sN, 1)] = w[i];
+    for (int i = a.k + threadIdx.x; i < p2; i += 512) sR[i] = ~0ull;
+    block_sort_u64(sR, p2);
+    const int64_t o = (int64_t)(q_begin + qi) * a.k;
+    for (int e = threadIdx.x; e < a.k; e += 512) {
+        if (a.out_ids) a.out_ids[o + e] = (int64_t)(unsigned)sR[e];
+        if (a.out_dists) a.out_dists[o + e] = f32_ord((uint32_t)(sR[e] >> 32));
     }
 }
 
@@ -134,26 +275,29 @@ int launch_compat(CompatArgs a, int q_begin, int q_count, cudaStream_t st) {
     if (q_count <= 0 || a.n == 0) return ANN_OK;
     a.q_end = q_begin + q_count;
     const size_t smem = sizeof(float) * kCompatQG * a.dim;
-    ANN_CUDA_TRY(smem_optin(reinterpret_cast<const void*>(compat_partials_kernel)));
+    ANN_CHECK_ARG(a.k <= a.n, "reference mode: k=%d above n", a.k);
+    a.seg_rows = compat_seg_rows(a.n);
+    a.nseg = (int)ceil_div(a.n, a.seg_rows);
+    auto partials = a.dim <= 512 ? compat_partials_kernel<32> : compat_partials_kernel<0>;
+    ANN_CUDA_TRY(smem_optin(reinterpret_cast<const void*>(partials)));
     const int64_t rblocks = std::min<int64_t>(ceil_div(a.n, 16), kNumSMs * 8);
     dim3 g1((unsigned)rblocks, (unsigned)ceil_div(q_count, kCompatQG));
-    compat_partials_kernel<<<g1, 256, smem, st>>>(a, q_begin);
+    partials<<<g1, 256, smem, st>>>(a, q_begin);
     ANN_LAUNCH_CHECK();
-    compat_threshold_kernel<<<(unsigned)ceil_div(q_count, 4), 128, 0, st>>>(a, q_begin);
+    const dim3 gw((unsigned)ceil_div(a.nseg, kCompatWarps), (unsigned)q_count);
+    if (a.nseg > 1) {
+        compat_segments_kernel<<<dim3(a.nseg - 1, (unsigned)q_count), 256, 0, st>>>(a);
+        ANN_LAUNCH_CHECK();
+        compat_prefix_kernel<<<(unsigned)q_count, 256, 0, st>>>(a);
+        ANN_LAUNCH_CHECK();
+    }
+    compat_threshold_kernel<<<gw, 32 * kCompatWarps, 0, st>>>(a);
     ANN_LAUNCH_CHECK();
-    compat_values_kernel<<<(unsigned)std::min<int64_t>(ceil_div((int64_t)q_count * a.n, 256), 16 * kNumSMs), 256, 0,
-                           st>>>(a, q_count);
+    compat_values_kernel<<<dim3(a.nseg, (unsigned)q_count), 256, 0, st>>>(a);
     ANN_LAUNCH_CHECK();
-    RadixSelectArgs rs{};
-    rs.keys = a.T;
-    rs.ld = a.n;
-    rs.R = a.k;
-    rs.out_key = a.kbuf;
-    rs.out_id = a.ibuf;
-    int rc = launch_radix_select(rs, q_count, st);
-    if (rc) return rc;
-    return launch_sort_topk(a.kbuf, a.ibuf, q_count, a.k, 0, a.out_ids ? a.out_ids + (int64_t)q_begin * a.k : nullptr,
-                            a.out_dists ? a.out_dists + (int64_t)q_begin * a.k : nullptr, st);
+    compat_final_kernel<<<(unsigned)q_count, 512, 0, st>>>(a, q_begin);
+    ANN_LAUNCH_CHECK();
+    return ANN_OK;
 }
 
 }  // namespace annb

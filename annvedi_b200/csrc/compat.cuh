@@ -20,11 +20,17 @@ struct CompatArgs {
     float* D;           // [chunk, n] scratch: full distances
     float* P;           // [chunk, ncp, n] scratch: checkpoint values
     float* T;           // [chunk, n] scratch: each row's heap threshold, then its ranking value
-    float* kbuf;        // [chunk, k] scratch: the selected values
-    int* ibuf;          // [chunk, k] scratch: their rows
+    float* seg_heap;    // [chunk, segments, 64] scratch: each segment's smallest distances
+    unsigned long long* seg_best;  // [chunk, segments, k] scratch: each segment's best (value, row)
     int64_t* out_ids;   // [nq, k]
     float* out_dists;   // [nq, k] ranking values, or nullptr
+    int64_t seg_rows;   // set by launch_compat
+    int nseg;
 };
+
+// Rows of a segment (a multiple of 1024), and with it ceil(n / rows) <= kCompatMaxSegs segments.
+constexpr int kCompatMaxSegs = 128;
+int64_t compat_seg_rows(int64_t n);
 
 int compat_num_checkpoints(int dim);
 // Runs queries [q_begin, q_begin + q_count) using D/P scratch sized for q_count queries.

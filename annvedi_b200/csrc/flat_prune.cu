@@ -15,6 +15,7 @@
 // A query that the bound does not cover (norms out of range, NaN), whose bar was too low, or with more survivors
 // than fit goes to a list that the plain scan answers right after, its length read on the device: no step waits
 // for the host.
+#include "block_select.cuh"
 #include "common.cuh"
 #include "flat_prune.cuh"
 
@@ -31,13 +32,6 @@ constexpr int kFinWarps = kFinThreads / 32;
 constexpr int kFinPitch = 36;  // floats per staged row of 32: 16-byte reads of 8 rows fall in different banks
 constexpr int kFinStages = 2;
 
-__device__ __forceinline__ uint32_t ord_f32(float f) {
-    const uint32_t u = __float_as_uint(f);
-    return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
-}
-__device__ __forceinline__ float f32_ord(uint32_t o) {
-    return __uint_as_float((o & 0x80000000u) ? (o & 0x7fffffffu) : ~o);
-}
 __device__ __forceinline__ int row_of_pos(int64_t p, int64_t n, int64_t mult) {
     return (int)(((unsigned __int128)p * (uint64_t)mult) % (uint64_t)n);
 }
@@ -116,31 +110,6 @@ __global__ void prune_bars_kernel(PruneArgs a) {
     if (q >= a.nq) return;
     a.tauX[q] = __fadd_ru(a.tauF[q], a.win[q]);
     a.rcount[q] = 0;
-}
-
-// The digit (8 bits) of rank `rem` (1-based) of the block's 256-bin histogram: every thread gets the digit, the
-// count below it and the digit's own count. One bin per thread.
-__device__ __forceinline__ void block_pick(const int* hist, int rem, int* sMisc, int* digit, int* before, int* own) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int c = hist[threadIdx.x];
-    int incl = c;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += y;
-    }
-    if (lane == 31) sMisc[warp] = incl;
-    __syncthreads();
-    for (int w = 0; w < warp; ++w) incl += sMisc[w];
-    if (incl - c < rem && rem <= incl) {
-        sMisc[8] = threadIdx.x;
-        sMisc[9] = incl - c;
-        sMisc[10] = c;
-    }
-    __syncthreads();
-    *digit = sMisc[8];
-    *before = sMisc[9];
-    *own = sMisc[10];
 }
 
 // One block per query (file comment, step 3). Bound by the gather of the kept rows (about 500 rows of 1.5 KB a query
@@ -258,42 +227,15 @@ __global__ void __launch_bounds__(kFinThreads) prune_finish_kernel(PruneArgs a) 
             sE[g + lane] = ((unsigned long long)ord_f32((METRIC == ANN_METRIC_L2 ? v : -v) + 0.f) << 32) | (unsigned)row;
     }
     __syncthreads();
-    // the k smallest (distance, row): 8-bit digits from the top until a digit ends at the k-th exactly
-    unsigned long long prefix = 0, mask = 0;
-    int rem = k;
-    for (int shift = 56; shift >= 0; shift -= 8) {
-        sHist[tid] = 0;
-        __syncthreads();
-        for (int i = tid; i < m; i += kFinThreads)
-            if ((sE[i] & mask) == prefix) atomicAdd(&sHist[(int)(sE[i] >> shift) & 255], 1);
-        __syncthreads();
-        int d, before, own;
-        block_pick(sHist, rem, sMisc, &d, &before, &own);
-        rem -= before;
-        prefix |= (unsigned long long)d << shift;
-        mask |= 255ull << shift;
-        if (rem == own) break;  // uniform
-    }
+    const SelectBound bound = block_select_bound([&](int i) { return sE[i]; }, m, k, sHist, sMisc);
     unsigned long long* sR = reinterpret_cast<unsigned long long*>(sX);  // the best k, then sorted
     const int p2 = pow2_ceil(k);
     if (tid == 0) sN = 0;
     __syncthreads();
     for (int i = tid; i < m; i += kFinThreads)
-        if ((sE[i] & mask) <= prefix) sR[atomicAdd(&sN, 1)] = sE[i];
+        if (bound.in(sE[i])) sR[atomicAdd(&sN, 1)] = sE[i];
     for (int i = k + tid; i < p2; i += kFinThreads) sR[i] = ~0ull;
-    __syncthreads();
-    for (int size = 2; size <= p2; size <<= 1)
-        for (int stride = size >> 1; stride > 0; stride >>= 1) {
-            for (int t = tid; t < p2 / 2; t += kFinThreads) {
-                const int lo = 2 * t - (t & (stride - 1)), hi = lo + stride;
-                const unsigned long long x = sR[lo], y = sR[hi];
-                if ((x > y) == ((lo & size) == 0)) {
-                    sR[lo] = y;
-                    sR[hi] = x;
-                }
-            }
-            __syncthreads();
-        }
+    block_sort_u64(sR, p2);
     for (int e = tid; e < k; e += kFinThreads) {
         a.out_ids[(int64_t)q * k + e] = (int64_t)(unsigned)sR[e];
         if (a.out_dists) {

@@ -75,6 +75,27 @@ __device__ __forceinline__ float ref_l2_f32(const float* __restrict__ x, const f
     return ref_l2_tail(sum, x, q, dim);
 }
 
+// ref_l2_f32 with x's full 16-chunks already in registers (xr[c] = x[16 c + lane], dim <= 16 P): the row's loads are in
+// flight together, and a row is read once for several q.
+template <int P, class Emit>
+__device__ __forceinline__ float ref_l2_f32_pieces(const float (&xr)[P], const float* __restrict__ x,
+                                                   const float* __restrict__ q, int dim, Emit&& emit) {
+    const int lane = threadIdx.x & 15;
+    const int full16 = dim >> 4;
+    float acc = 0.f;
+    int cp = 0;
+#pragma unroll
+    for (int c = 0; c < P; ++c)
+        if (c < full16) {
+            const float diff = __fsub_rn(xr[c], q[c * 16 + lane]);
+            acc = __fadd_rn(acc, __fmul_rn(diff, diff));
+            if (c % 6 == 5) emit(cp++, ref_fold16(acc));
+        }
+    const float sum = ref_fold16(acc);
+    emit(cp, sum);
+    return ref_l2_tail(sum, x, q, dim);
+}
+
 // SQ8 distance sum_d (code[d]*scale[d] - qs[d])^2, the reference's arithmetic.
 template <class Emit>
 __device__ __forceinline__ float ref_l2_sq8(const uint8_t* __restrict__ code, const float* __restrict__ qs,
