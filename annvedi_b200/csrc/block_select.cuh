@@ -86,4 +86,30 @@ __device__ __forceinline__ void block_sort_u64(unsigned long long* w, int n) {
         }
 }
 
+// The word of a distance and its row; NaN orders after +inf, -0 with +0.
+__device__ __forceinline__ unsigned long long select_word(float v, int64_t row) {
+    if (v != v) v = __int_as_float(0x7fffffff);
+    return ((unsigned long long)ord_f32(v + 0.f) << 32) | (unsigned)row;
+}
+
+// Rows of a segment when n rows are selected from in up to kSelectSegs segments (a multiple of 1024).
+constexpr int kSelectSegs = 128;
+inline int64_t select_seg_rows(int64_t n) { return ceil_div(ceil_div(n, kSelectSegs), 1024) * 1024; }
+
+// The segment's best min(k, m) of the values T[0..m) of rows row0.., as words in no order into out[0..k), the rest
+// filled with ~0. Whole block; sN: one int.
+__device__ __forceinline__ void segment_select(const float* T, int64_t row0, int m, int k, unsigned long long* out,
+                                               int* sHist, int* sMisc, int* sN) {
+    if (threadIdx.x == 0) *sN = 0;
+    __syncthreads();
+    const int kk = min(k, m);
+    auto at = [&](int i) { return select_word(T[i], row0 + i); };
+    const SelectBound b = block_select_bound(at, m, kk, sHist, sMisc);
+    for (int i = threadIdx.x; i < m; i += blockDim.x) {
+        const unsigned long long w = at(i);
+        if (b.in(w)) out[atomicAdd(sN, 1)] = w;
+    }
+    for (int i = kk + threadIdx.x; i < k; i += blockDim.x) out[i] = ~0ull;
+}
+
 }  // namespace annb

@@ -11,6 +11,7 @@
 #include <atomic>
 #include <vector>
 
+#include "block_select.cuh"
 #include "common.cuh"
 #include "compat.cuh"
 #include "flat_scan.cuh"
@@ -364,7 +365,7 @@ int ann_flat_query(ann_flat* h, ann_workspace* ws, const float* queries, int32_t
         }
     } else {
         ncp = compat_num_checkpoints(h->dim);
-        nseg = (int)ceil_div(h->n, compat_seg_rows(h->n));
+        nseg = (int)ceil_div(h->n, select_seg_rows(h->n));
         const size_t per_q = sizeof(float) * (size_t)h->n * (ncp + 2) + (size_t)nseg * (64 * 4 + (size_t)kk * 8);
         const size_t budget = (size_t)1 << 30;
         qc = (int)std::min<size_t>(32768, std::max<size_t>(1, std::min<size_t>((size_t)nq, budget / per_q)));

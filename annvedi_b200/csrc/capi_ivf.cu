@@ -58,7 +58,7 @@ struct ann_ivf {
     __nv_bfloat16* cent_bf16 = nullptr;  // [C, kpad] BF16 operand form of the centroids
     float2* sq8_fac = nullptr;           // [n] (1, reconstructed |x|^2) of the SQ8 rows (codes on the tensor cores)
     int kpad = 0;
-    float cent_norm_max = 0.f;           // the largest centroid norm (the coarse ranking's key error bound)
+    PruneBounds cent_bounds;             // of the centroids' norms (the coarse ranking's key error bound)
     std::mutex tc_mu;
     int64_t query_count = 0;
     // query options (ann_ivf_set_option)
@@ -90,7 +90,7 @@ static void ivf_free_state(ann_ivf* h) {
         if (p) cudaFree(p);
     h->base_bf16 = nullptr;
     h->cent_bf16 = nullptr;
-    h->cent_norm_max = 0.f;
+    h->cent_bounds = PruneBounds{};
     h->sq8_fac = nullptr;
     h->proj = h->projT = h->lsh_mean = nullptr;
     h->tab_off = nullptr;
@@ -752,6 +752,7 @@ struct IvfQueryCfg {
     int k, npc, R, nsplit, num_threads, bqc, nsplit_c, ncp;
     int64_t max_c, ub, rps_c;
     bool ref, coarse_flat, batched, tc, lsh;
+    bool coarse_keys;  // exact mode: the coarse scan pruned by tensor-core keys
     bool i8;          // the tensor-core form over the SQ8 codes (int8 x uint8 MMA) instead of BF16 rows
     bool shard;       // ANN_QUERY_SHARD: streams short of k are not widened to every row
     bool fallback;    // a query's stream can fall short of k points and become every row
@@ -764,40 +765,43 @@ struct IvfQueryCfg {
 // Operand forms of the tensor-core forms, built once: BF16 centroids (the coarse ranking of both), and the BF16
 // list-ordered rows (ANN_MODE_TC) or the SQ8 rows' reconstructed norms (ANN_MODE_TC_SQ8, whose B operand is the
 // codes themselves).
+static int ivf_ensure_cent(ann_ivf* h, cudaStream_t st) {  // under tc_mu
+    if (h->cent_bf16) return ANN_OK;
+    const int kpad = tc_kpad(h->dim, ANN_METRIC_L2);
+    const size_t bytes = (sizeof(__nv_bfloat16) * (size_t)h->C * kpad + 255) / 256 * 256;
+    char* cb = nullptr;  // the operand rows, then two words for their norms
+    if (cudaMalloc(&cb, bytes + 256) != cudaSuccess) {
+        cudaGetLastError();
+        set_error("tensor-core IVF: cannot allocate the BF16 centroids");
+        return ANN_ERR_NOMEM;
+    }
+    __nv_bfloat16* rows = reinterpret_cast<__nv_bfloat16*>(cb);
+    unsigned* d2 = reinterpret_cast<unsigned*>(cb + bytes);
+    unsigned h2[2] = {0, 0};
+    int rc = launch_tc_operand(h->centroids, h->C, h->dim, h->dpad, rows, kpad, kTcBase, ANN_METRIC_L2, 0, st);
+    if (!rc) rc = launch_base_norms(h->centroids, h->C, h->dim, h->dpad, d2, st);
+    cudaError_t e = cudaSuccess;
+    if (!rc) e = cudaMemcpyAsync(h2, d2, sizeof(h2), cudaMemcpyDeviceToHost, st);
+    if (!rc && e == cudaSuccess) e = cudaStreamSynchronize(st);
+    if (rc || e != cudaSuccess) {
+        cudaFree(cb);
+        if (rc) return rc;
+        set_error("tensor-core IVF: %s", cudaGetErrorString(e));
+        return ANN_ERR_CUDA;
+    }
+    float s2, e2;
+    memcpy(&s2, &h2[0], 4);
+    memcpy(&e2, &h2[1], 4);
+    h->cent_bounds = PruneBounds{std::sqrt(s2) * 1.001f, std::sqrt(e2) * 1.001f};
+    h->cent_bf16 = rows;
+    h->kpad = kpad;
+    return ANN_OK;
+}
 static int ivf_ensure_tc(ann_ivf* h, bool i8, cudaStream_t st) {
     std::lock_guard<std::mutex> lk(h->tc_mu);
     const int kpad = tc_kpad(h->dim, ANN_METRIC_L2);
-    int rc = ANN_OK;
-    if (!h->cent_bf16) {
-        __nv_bfloat16* cb = nullptr;
-        if (cudaMalloc(&cb, sizeof(__nv_bfloat16) * (size_t)h->C * kpad) != cudaSuccess) {
-            cudaGetLastError();
-            set_error("tensor-core IVF: cannot allocate the BF16 centroids");
-            return ANN_ERR_NOMEM;
-        }
-        if ((rc = launch_tc_operand(h->centroids, h->C, h->dim, h->dpad, cb, kpad, kTcBase, ANN_METRIC_L2, 0, st))) {
-            cudaFree(cb);
-            return rc;
-        }
-        ANN_CUDA_TRY(cudaStreamSynchronize(st));
-        // the largest centroid norm, from a host copy of the (small) centroid table
-        std::vector<float> hc((size_t)h->C * h->dpad);
-        const cudaError_t ce = cudaMemcpy(hc.data(), h->centroids, sizeof(float) * hc.size(), cudaMemcpyDeviceToHost);
-        if (ce != cudaSuccess) {
-            cudaFree(cb);
-            set_error("tensor-core IVF: %s", cudaGetErrorString(ce));
-            return ANN_ERR_CUDA;
-        }
-        double mx = 0.0;
-        for (int c = 0; c < h->C; ++c) {
-            double s2 = 0.0;
-            for (int d = 0; d < h->dim; ++d) s2 += (double)hc[(size_t)c * h->dpad + d] * hc[(size_t)c * h->dpad + d];
-            mx = std::max(mx, s2);
-        }
-        h->cent_norm_max = (float)(std::sqrt(mx) * (1.0 + 1e-6));
-        h->cent_bf16 = cb;
-        h->kpad = kpad;
-    }
+    int rc = ivf_ensure_cent(h, st);
+    if (rc) return rc;
     if (!i8 && !h->base_bf16) {
         __nv_bfloat16* b = nullptr;
         const cudaError_t e = cudaMalloc(&b, sizeof(__nv_bfloat16) * (size_t)h->n * kpad);
@@ -866,10 +870,12 @@ static size_t ivf_scratch(const ann_ivf* h, const IvfQueryCfg& c, int nq) {
         sz.take<int>((size_t)nq * h->T * std::max(1, lsh_p));
     }
     if (c.lsh_keys) sz.take<float>((size_t)nq * c.ub_cand);
-    if (c.tc) {
+    if (c.tc || c.coarse_keys) {
         sz.take<float>((size_t)nq * h->C);  // BF16 coarse keys
         sz.take<float>((size_t)nq * ceil_div(h->C, 32));  // their 32-centroid chunk minima
         sz.take<__nv_bfloat16>((size_t)nq * h->kpad);
+    }
+    if (c.tc) {
         sz.take<unsigned char>((size_t)nq * c.npc * tc_pair_row_bytes(h));
         sz.take<int8_t>((size_t)nq * h->dpad8);  // int8 query weights and factors (ANN_MODE_TC_SQ8)
         sz.take<float>((size_t)nq);
@@ -879,6 +885,8 @@ static size_t ivf_scratch(const ann_ivf* h, const IvfQueryCfg& c, int nq) {
         sz.take<int4>((size_t)tc_items_bound((int64_t)nq * c.npc, (int)h->C, h->sizes_desc[0]));
     }
     sz.take<int32_t>((size_t)nq);  // re-rank query order
+    sz.take<int32_t>((size_t)nq);  // queries set apart (every row), and their count
+    sz.take<int32_t>(1);
     sz.take<int64_t>(1);           // an every-row stream: its length
     sz.take<int32_t>(1);           // and its segment flag
     return sz.off;
@@ -1085,9 +1093,10 @@ static int ivf_query_device(ann_ivf* h, ann_workspace* ws, const IvfQueryCfg& c,
     uint32_t* lsig = c.lsh ? cv.take<uint32_t>((size_t)nq * h->T) : nullptr;
     int* lpert = c.lsh ? cv.take<int>((size_t)nq * h->T * std::max(1, lsh_p)) : nullptr;
     float* lkeys = c.lsh_keys ? cv.take<float>((size_t)nq * c.ub_cand) : nullptr;
-    float* ckeys = c.tc ? cv.take<float>((size_t)nq * h->C) : nullptr;
-    float* ckmin = c.tc ? cv.take<float>((size_t)nq * ceil_div(h->C, 32)) : nullptr;
-    __nv_bfloat16* qb = c.tc ? cv.take<__nv_bfloat16>((size_t)nq * h->kpad) : nullptr;
+    const bool ck = c.tc || c.coarse_keys;
+    float* ckeys = ck ? cv.take<float>((size_t)nq * h->C) : nullptr;
+    float* ckmin = ck ? cv.take<float>((size_t)nq * ceil_div(h->C, 32)) : nullptr;
+    __nv_bfloat16* qb = ck ? cv.take<__nv_bfloat16>((size_t)nq * h->kpad) : nullptr;
     unsigned char* Apk = c.tc ? cv.take<unsigned char>((size_t)nq * c.npc * tc_pair_row_bytes(h)) : nullptr;
     int8_t* q8 = c.tc ? cv.take<int8_t>((size_t)nq * h->dpad8) : nullptr;
     float* qfac = c.tc ? cv.take<float>((size_t)nq) : nullptr;
@@ -1097,6 +1106,8 @@ static int ivf_query_device(ann_ivf* h, ann_workspace* ws, const IvfQueryCfg& c,
     const int64_t items_cap = c.tc ? tc_items_bound((int64_t)nq * c.npc, (int)h->C, h->sizes_desc[0]) : 0;
     int4* titem_desc = c.tc ? cv.take<int4>((size_t)items_cap) : nullptr;
     int32_t* qorder = cv.take<int32_t>((size_t)nq);
+    int32_t* apart = cv.take<int32_t>((size_t)nq);
+    int32_t* apart_count = cv.take<int32_t>(1);
     int64_t* every_len = cv.take<int64_t>(1);
     int32_t* every_seg = cv.take<int32_t>(1);
 
@@ -1125,14 +1136,14 @@ static int ivf_query_device(ann_ivf* h, ann_workspace* ws, const IvfQueryCfg& c,
     int rc;
     const int prec = h->prof.begin(st);
     // 1. coarse ranking
-    if (c.tc) {
+    if (c.tc || c.coarse_keys) {
         // BF16 keys to every centroid, then the exact FP32 order of the best npc + 16
         if ((rc = launch_tc_operand(qdev, nq, h->dim, h->dpad, qb, h->kpad, kTcQuery, ANN_METRIC_L2, 0, st))) return rc;
         TcGemmArgs ca{nq, h->C, h->kpad, nullptr, ckeys, h->C, h->d_err};
         ca.out_cmin = ckmin;  // and each query's 32-centroid chunk minima, which let the ranking skip chunks
         if ((rc = launch_tc_gemm(qb, h->cent_bf16, ca, st))) return rc;
         if ((rc = launch_tc_coarse(ckeys, h->C, nq, h->C, c.npc, 16, qdev, h->centroids, h->dpad, probes, st,
-                                   h->cent_norm_max, h->dim, ckmin)))
+                                   h->cent_bounds.cmax, h->cent_bounds.rmax, h->dim, ckmin, c.coarse_keys)))
             return rc;
         if (c.i8 && (rc = launch_tc_sq8_query(qdev, nq, h->dim, h->dpad, h->scale, h->offset, q8, h->dpad8, qfac, st)))
             return rc;
@@ -1147,6 +1158,20 @@ static int ivf_query_device(ann_ivf* h, ann_workspace* ws, const IvfQueryCfg& c,
         if ((rc = launch_select_topk(Dc, h->C, nullptr, nq, c.npc, nullptr, pkey, probes, st))) return rc;
     }
     h->prof.mark(prec, st);
+    // The queries whose stream is every row (fewer than k candidates, :453-457): in reference mode they do
+    // not fit the per-query scratch of L = ub positions, and in a large exact batch one CTA would scan all
+    // n rows. The main pass sees them as empty streams; each is redone below on its own, split over the
+    // whole GPU. (Small exact batches already split every query that widely and skip the host read.)
+    // Batched passes have the plan list them (apart) and read their number with the batch set-up's totals, so one
+    // such query costs its own scan and no second set-up and pass of the batch (10,000 queries with one: 2.09 ms a
+    // call, 1.18 ms now).
+    const bool every_row_apart = c.fallback && (c.ref || c.nsplit < kEveryRowMinSplit);
+    const bool plan_apart = every_row_apart && c.batched;
+    if (plan_apart) {
+        a.apart = apart;
+        a.apart_count = apart_count;
+        ANN_CUDA_TRY(cudaMemsetAsync(apart_count, 0, sizeof(int32_t), st));
+    }
     // 2. plan: whole lists, or the LSH buckets' explicit streams (signatures first, their own stage)
     LshCandArgs la{};
     if (c.lsh) {
@@ -1179,43 +1204,40 @@ static int ivf_query_device(ann_ivf* h, ann_workspace* ws, const IvfQueryCfg& c,
         return rc;
     }
     h->prof.mark(prec, st);
-    // The queries whose stream is every row (fewer than k candidates, :453-457): in reference mode they do
-    // not fit the per-query scratch of L = ub positions, and in a large exact batch one CTA would scan all
-    // n rows. The main pass sees them as empty streams; each is redone below on its own, split over the
-    // whole GPU. (Small exact batches already split every query that widely and skip the host read.)
     std::vector<int> every_row;
+    int32_t* every_list = apart;  // the same on the device (exact mode)
     auto take_every_row = [&]() -> int {
         std::vector<int32_t> ns(nq);
         ANN_CUDA_TRY(cudaMemcpyAsync(ns.data(), n_seg, sizeof(int32_t) * (size_t)nq, cudaMemcpyDeviceToHost, st));
         ANN_CUDA_TRY(cudaStreamSynchronize(st));
         for (int i = 0; i < nq; ++i)
             if (ns[i] < 0) every_row.push_back(i);
-        if (!every_row.empty()) {
-            int r = launch_clear_every_row(a.plan, st);
-            if (r) return r;
-            const int64_t len = h->n;
-            const int32_t seg = -1;
-            ANN_CUDA_TRY(cudaMemcpyAsync(every_len, &len, sizeof(len), cudaMemcpyHostToDevice, st));
-            ANN_CUDA_TRY(cudaMemcpyAsync(every_seg, &seg, sizeof(seg), cudaMemcpyHostToDevice, st));
-            ANN_CUDA_TRY(cudaStreamSynchronize(st));  // the host values above live on this frame
-        }
+        if (every_row.empty()) return ANN_OK;
+        const int r = launch_clear_every_row(a.plan, st);
+        if (r) return r;
+        const int64_t len = h->n;
+        const int32_t seg = -1;
+        ANN_CUDA_TRY(cudaMemcpyAsync(every_len, &len, sizeof(len), cudaMemcpyHostToDevice, st));
+        ANN_CUDA_TRY(cudaMemcpyAsync(every_seg, &seg, sizeof(seg), cudaMemcpyHostToDevice, st));
+        ANN_CUDA_TRY(cudaMemcpyAsync(every_list, every_row.data(), sizeof(int32_t) * every_row.size(),
+                                     cudaMemcpyHostToDevice, st));
+        ANN_CUDA_TRY(cudaStreamSynchronize(st));  // the host values above live on this frame
         return ANN_OK;
     };
-    const bool every_row_apart = c.fallback && (c.ref || c.nsplit < kEveryRowMinSplit);
-    // batched passes learn of every-row queries from the batch set-up's own host read (below), so the common
-    // case takes no extra round trip here
-    if (every_row_apart && !(c.batched && !c.ref) && (rc = take_every_row())) return rc;
+    if (every_row_apart && !plan_apart && (rc = take_every_row())) return rc;
     // 3. SQ8 pass -> best R per query
     bool done = false;
     if (!c.ref && c.batched) {
         IvfBatchArgs b{};
-        int64_t tot_local[3] = {0, 0, 0};
+        int64_t tot_local[4] = {0, 0, 0, 0};
         int64_t* tot = tot_local;
         // The sampled path needs none of the set-up's totals to run: they land in page-locked words and are read
-        // after its own synchronisation (a batch with every-row queries, rare, is then set up again and redone).
+        // after its own synchronisation.
         const bool sampled = c.tc && nq >= h->sampled_min_queries;
         if (sampled && (rc = ws_pinned(ws, &tot))) return rc;
-        tot[0] = tot[1] = tot[2] = 0;
+        tot[0] = tot[1] = tot[2] = tot[3] = 0;
+        if (plan_apart)
+            ANN_CUDA_TRY(cudaMemcpyAsync(&tot[3], apart_count, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
         auto run_sampled = [&](bool* ok) -> int {
             return ivf_tc_sampled(h, ws, c, a, b, tc_operands(h, c, qb, q8, qfac, pfac), Apk, titem, titem_desc,
                                   items_cap, keyR, idR, prec, ok, st);
@@ -1224,11 +1246,7 @@ static int ivf_query_device(ann_ivf* h, ann_workspace* ws, const IvfQueryCfg& c,
         if ((rc = batched_prepare(a, bscratch, c.sort_tmp, c.scan_tmp, &b, tot, st, !sampled))) return rc;
         if (sampled && (rc = run_sampled(&sampled_done))) return rc;  // synchronises st: tot is current
         if (tot[2] != 0) sampled_done = false;
-        if (tot[2] != 0 && every_row_apart) {  // every-row queries: set apart, then the batch set up again
-            if ((rc = take_every_row())) return rc;
-            if ((rc = batched_prepare(a, bscratch, c.sort_tmp, c.scan_tmp, &b, tot, st))) return rc;
-            if (tot[2] == 0 && sampled && (rc = run_sampled(&sampled_done))) return rc;
-        }
+        if (plan_apart) every_row.resize((size_t)(int)tot[3]);  // the plan has listed them in every_list
         done = sampled_done;
         if (tot[2] == 0 && !sampled_done) {  // no query fell back to scanning every row
             if ((rc = ws_reserve_big(ws, sizeof(float) * (size_t)std::max<int64_t>(tot[1], 1)))) return rc;
@@ -1339,11 +1357,34 @@ static int ivf_query_device(ann_ivf* h, ann_workspace* ws, const IvfQueryCfg& c,
     const int kr = h->prof.kbegin(st);
     if ((rc = launch_ivf_rerank(a, keyR, idR, c.ref ? 1 : 0, st))) return rc;
     h->prof.kend(kr, kKernRerank, st);
-    if (!every_row.empty()) {
+    if (!every_row.empty() && !c.ref) {
+        // the keys of every row for several queries at a time (256 MB of them), the best R of each by segments, and
+        // the re-rank: 4 launches. A scan with fused selection took 512 us a query at 1M x 384 and R = 100, its
+        // merge 346 us; the keys take 100 us, the selection 40 us.
+        const size_t words_q = rows_select_words(h->n, c.R);
+        const size_t per_q = sizeof(float) * (size_t)h->n + 8 * words_q;
+        const int group = (int)std::max<size_t>(1, std::min<size_t>(4096, ((size_t)256 << 20) / per_q));
+        for (size_t e0 = 0; e0 < every_row.size(); e0 += group) {
+            const int ne = (int)std::min<size_t>(group, every_row.size() - e0);
+            Sizer es;
+            es.take<float>((size_t)ne * h->n);
+            es.take<unsigned long long>((size_t)ne * words_q);
+            if ((rc = ws_reserve_big(ws, es.bytes()))) return rc;
+            Carver ec(ws->big);
+            float* D = ec.take<float>((size_t)ne * h->n);
+            unsigned long long* words = ec.take<unsigned long long>((size_t)ne * words_q);
+            IvfQueryArgs b = a;
+            b.plan.nq = ne;
+            b.plan.cand_ids = nullptr;
+            b.qorder = every_list + e0;
+            if ((rc = launch_set_every_row(a.plan, b.qorder, ne, h->n, st))) return rc;
+            if ((rc = launch_ivf_sq8_dists(b, D, h->n, st))) return rc;
+            if ((rc = launch_rows_select(D, h->n, ne, c.R, b.qorder, words, keyR, idR, st))) return rc;
+            if ((rc = launch_ivf_rerank(b, keyR, idR, 0, st))) return rc;
+        }
+    } else if (!every_row.empty()) {
         const int64_t L = h->n;
-        const int nsp = (int)std::min<int64_t>(2 * kNumSMs, std::max<int64_t>(1, ceil_div(L, 2048)));
-        const size_t need = c.ref ? sizeof(float) * (size_t)L * (c.ncp + 2) : (size_t)8 * nsp * c.R;
-        if ((rc = ws_reserve_big(ws, need))) return rc;
+        if ((rc = ws_reserve_big(ws, sizeof(float) * (size_t)L * (c.ncp + 2)))) return rc;
         float* big = reinterpret_cast<float*>(ws->big);
         for (int q : every_row) {
             IvfQueryArgs b = a;
@@ -1360,24 +1401,13 @@ static int ivf_query_device(ann_ivf* h, ann_workspace* ws, const IvfQueryCfg& c,
             b.out_dists = dists_dev ? dists_dev + (size_t)q * c.k : nullptr;
             float* kq = keyR + (size_t)q * c.R;
             int* iq = idR + (size_t)q * c.R;
-            if (c.ref) {
-                b.L = L;
-                b.D = big;
-                b.V = big + L;
-                b.P = big + 2 * L;
-                if ((rc = launch_ivf_ref_sq8(b, L, st))) return rc;
-                if ((rc = launch_select_topk(b.V, L, b.plan.n_cands, 1, c.R, &b.plan, kq, iq, st, nullptr, true))) return rc;
-            } else {
-                b.nsplit = nsp;
-                b.keyR = big;
-                b.idR = reinterpret_cast<int*>(big + (size_t)nsp * c.R);
-                if ((rc = launch_ivf_sq8_scan(b, st))) return rc;
-                MergeArgs m{b.keyR, b.idR, 1, nsp, c.R, c.R, 0, nullptr, nullptr};
-                m.out_id32 = iq;
-                m.out_key32 = kq;
-                if ((rc = launch_merge_splits(m, st))) return rc;
-            }
-            if ((rc = launch_ivf_rerank(b, kq, iq, c.ref ? 1 : 0, st))) return rc;
+            b.L = L;
+            b.D = big;
+            b.V = big + L;
+            b.P = big + 2 * L;
+            if ((rc = launch_ivf_ref_sq8(b, L, st))) return rc;
+            if ((rc = launch_select_topk(b.V, L, b.plan.n_cands, 1, c.R, &b.plan, kq, iq, st, nullptr, true))) return rc;
+            if ((rc = launch_ivf_rerank(b, kq, iq, 1, st))) return rc;
         }
     }
     h->prof.mark(prec, st);
@@ -1459,6 +1489,21 @@ int ann_ivf_query(ann_ivf* h, ann_workspace* ws, const float* queries, int32_t n
     c.coarse_flat = !c.ref && c.npc <= 512;
     c.batched = !c.ref && !c.lsh && (c.tc || nq >= kBatchedMinQueries);
     if (c.tc && (rc0 = ivf_ensure_tc(h, c.i8, st))) return rc0;
+    // The exact form's coarse scan of a batch by keys (the probes are the scan's): from a GEMM and the few distances
+    // inside the keys' window instead of every (query, centroid) distance on the FP32 units. 2,000 queries over 2,048
+    // centroids at dim 384: 425 us scanned (with the merge), 60 us by keys; below 32 queries (which may be captured)
+    // and a few hundred centroids the scan is a launch or two of 30 us and stays. 128 MB of keys at most.
+    if (!c.ref && !c.tc && c.batched && c.coarse_flat && h->C >= 256 && tc_coarse_chunked((int)h->C, c.npc, h->dpad) &&
+        (int64_t)nq * h->C <= (int64_t)1 << 25) {
+        std::lock_guard<std::mutex> lk(h->tc_mu);
+        rc0 = ivf_ensure_cent(h, st);
+        if (rc0 == ANN_ERR_NOMEM)
+            clear_error();
+        else if (rc0)
+            return rc0;
+        else
+            c.coarse_keys = h->cent_bounds.cmax >= kPruneNormMin && h->cent_bounds.cmax <= kPruneNormMax;
+    }
     const int dpad = h->dpad;
     const bool host = mem == ANN_MEM_HOST;
 

@@ -71,8 +71,6 @@ constexpr int kCompatAhead = 8;  // 32-row steps of distances loaded ahead of th
 
 constexpr int kCompatWarps = 4;
 
-int64_t compat_seg_rows(int64_t n) { return ceil_div(ceil_div(n, kCompatMaxSegs), 1024) * 1024; }
-
 // Walks rows [begin, end) of D through the heap in row order; out(i, T_i, valid) per row.
 template <class Out>
 __device__ __forceinline__ void compat_walk(const float* __restrict__ D, int64_t begin, int64_t end, WarpHeap64& heap,
@@ -116,12 +114,6 @@ __device__ __forceinline__ void compat_walk(const float* __restrict__ D, int64_t
     }
 }
 
-// (v, row) as one word; NaN orders after +inf.
-__device__ __forceinline__ unsigned long long compat_word(float v, int64_t row) {
-    if (v != v) v = __int_as_float(0x7fffffff);
-    return ((unsigned long long)ord_f32(v + 0.f) << 32) | (unsigned)row;
-}
-
 // One block per (segment, query): the segment's `lim` smallest distances, ascending (FLT_MAX where fewer than lim are
 // below it, as the heap's empty slots).
 __global__ void __launch_bounds__(256) compat_segments_kernel(CompatArgs a) {
@@ -136,7 +128,7 @@ __global__ void __launch_bounds__(256) compat_segments_kernel(CompatArgs a) {
     if (threadIdx.x == 0) sN = 0;
     if (threadIdx.x < 64) sR[threadIdx.x] = ~0ull;
     __syncthreads();
-    auto at = [&](int i) { return compat_word(D[i], i); };
+    auto at = [&](int i) { return select_word(D[i], i); };
     const SelectBound b = block_select_bound(at, m, lim, sHist, sMisc);
     for (int i = threadIdx.x; i < m; i += 256) {
         const unsigned long long w = at(i);
@@ -154,7 +146,7 @@ __global__ void __launch_bounds__(256) compat_segments_kernel(CompatArgs a) {
 // sequence, which six exchange steps sort. Lane l holds values l and l + 32. The lists are staged in shared memory by
 // the block first: a list's load from L2 takes longer than its merge.
 __global__ void __launch_bounds__(256) compat_prefix_kernel(CompatArgs a) {
-    __shared__ float sL[kCompatMaxSegs * 64];
+    __shared__ float sL[kSelectSegs * 64];
     const int lane = threadIdx.x & 31, qi = blockIdx.x;
     const int lim = a.k < 64 ? a.k : 64;
     float* L = a.seg_heap + (int64_t)qi * a.nseg * 64;
@@ -230,17 +222,7 @@ __global__ void __launch_bounds__(256) compat_values_kernel(CompatArgs a) {
         }
         T[e] = v;
     }
-    if (threadIdx.x == 0) sN = 0;
-    __syncthreads();
-    const int kk = min(a.k, m);
-    auto at = [&](int i) { return compat_word(T[i], begin + i); };
-    const SelectBound b = block_select_bound(at, m, kk, sHist, sMisc);
-    unsigned long long* out = a.seg_best + ((int64_t)qi * a.nseg + s) * a.k;
-    for (int i = threadIdx.x; i < m; i += 256) {
-        const unsigned long long w = at(i);
-        if (b.in(w)) out[atomicAdd(&sN, 1)] = w;
-    }
-    for (int i = kk + threadIdx.x; i < a.k; i += 256) out[i] = ~0ull;
+    segment_select(T, begin, m, a.k, a.seg_best + ((int64_t)qi * a.nseg + s) * a.k, sHist, sMisc, &sN);
 }
 
 // The k best of the segments' best, in order. One block per query.
@@ -276,7 +258,7 @@ int launch_compat(CompatArgs a, int q_begin, int q_count, cudaStream_t st) {
     a.q_end = q_begin + q_count;
     const size_t smem = sizeof(float) * kCompatQG * a.dim;
     ANN_CHECK_ARG(a.k <= a.n, "reference mode: k=%d above n", a.k);
-    a.seg_rows = compat_seg_rows(a.n);
+    a.seg_rows = select_seg_rows(a.n);
     a.nseg = (int)ceil_div(a.n, a.seg_rows);
     auto partials = a.dim <= 512 ? compat_partials_kernel<32> : compat_partials_kernel<0>;
     ANN_CUDA_TRY(smem_optin(reinterpret_cast<const void*>(partials)));

@@ -28,10 +28,6 @@ struct CompatArgs {
     int nseg;
 };
 
-// Rows of a segment (a multiple of 1024), and with it ceil(n / rows) <= kCompatMaxSegs segments.
-constexpr int kCompatMaxSegs = 128;
-int64_t compat_seg_rows(int64_t n);
-
 int compat_num_checkpoints(int dim);
 // Runs queries [q_begin, q_begin + q_count) using D/P scratch sized for q_count queries.
 int launch_compat(CompatArgs a, int q_begin, int q_count, cudaStream_t st);

@@ -70,11 +70,7 @@ __global__ void __launch_bounds__(256) base_norms_kernel(const float* __restrict
     }
 }
 
-// One warp per query: its window w = 2 eps + delta. With x^, q^ the BF16 operands,
-//   |x.q - x^.q^| <= |x - x^| |q| + |x^| |q - q^| <= rmax |q| + (cmax + rmax) |q - q^|,
-// (residual norms taken, not bounded by 2^-9: about 0.4 of that), and the FP32 accumulation of the dim + 3 products
-// (truncating adds allowed for: 2^-21 each, of the terms' absolute sum) adds acc * sum. delta bounds the rounding
-// of two FP32 distances summed over dim terms. The sums taken here are FP32 too: the factor 1.002 covers them.
+// One warp per query: its window w = 2 eps + delta (key_window_l2 / _ip).
 __global__ void __launch_bounds__(256) prune_windows_kernel(PruneArgs a) {
     const int q = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (q >= a.nq) return;
@@ -91,17 +87,11 @@ __global__ void __launch_bounds__(256) prune_windows_kernel(PruneArgs a) {
         e += __shfl_xor_sync(0xffffffffu, e, o);
     }
     if (lane != 0) return;
-    const float qn = sqrtf(s), rq = sqrtf(e), cm = a.b.cmax, rm = a.b.rmax;
-    const float acc = (float)(a.dim + 19) * 4.76837158e-7f;  // (dim + 19) 2^-21
-    const float cross = rm * qn + (cm + rm) * rq;
-    const float sum = (cm + rm) * (qn + rq);
-    float w;
-    if (a.metric == ANN_METRIC_L2)
-        w = 2.f * (2.f * cross + acc * (2.f * sum + cm * cm)) + acc * (qn + cm) * (qn + cm);
-    else
-        w = 2.f * (cross + acc * sum) + 2.f * acc * qn * cm;
+    const float qn = sqrtf(s), rq = sqrtf(e);
+    const float w = a.metric == ANN_METRIC_L2 ? key_window_l2(qn, rq, a.b.cmax, a.b.rmax, a.dim)
+                                              : key_window_ip(qn, rq, a.b.cmax, a.b.rmax, a.dim);
     const bool ok = qn <= kPruneNormMax && (qn >= kPruneNormMin || s == 0.f);  // false for NaN
-    a.win[q] = ok ? w * 1.002f : __int_as_float(0x7fffffff);
+    a.win[q] = ok ? w : __int_as_float(0x7fffffff);
 }
 
 __global__ void prune_bars_kernel(PruneArgs a) {

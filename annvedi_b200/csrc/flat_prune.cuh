@@ -18,6 +18,23 @@ constexpr float kPruneNormMin = 1e-12f, kPruneNormMax = 1e15f;
 // 105 us), and the sample (an eighth of a small base) still holds enough rows for the bar.
 constexpr int64_t kPruneMinRows = 32768;
 
+// The window of the BF16 keys (tc_gemm.cuh) of vector q against rows x: 2 eps + delta. With x^, q^ the BF16 operands,
+//   |x.q - x^.q^| <= |x - x^| |q| + |x^| |q - q^| <= rmax |q| + (cmax + rmax) |q - q^|,
+// (residual norms taken, not bounded by 2^-9: about 0.4 of that), and the FP32 accumulation of the dim + 3 products
+// (truncating adds allowed for: 2^-21 each, of the terms' absolute sum) adds acc * sum. delta bounds the rounding
+// of two FP32 distances summed over dim terms. The norms passed in are FP32 sums too: the factor 1.002 covers them.
+// qn, rq: |q| and |q - q^|; cm, rm: upper bounds of |x| and |x - x^|.
+__host__ __device__ __forceinline__ float key_window_l2(float qn, float rq, float cm, float rm, int dim) {
+    const float acc = (float)(dim + 19) * 4.76837158e-7f;  // (dim + 19) 2^-21
+    const float cross = rm * qn + (cm + rm) * rq;
+    return 1.002f * (2.f * (2.f * cross + acc * (2.f * (cm + rm) * (qn + rq) + cm * cm)) + acc * (qn + cm) * (qn + cm));
+}
+__host__ __device__ __forceinline__ float key_window_ip(float qn, float rq, float cm, float rm, int dim) {
+    const float acc = (float)(dim + 19) * 4.76837158e-7f;
+    const float cross = rm * qn + (cm + rm) * rq;
+    return 1.002f * (2.f * (cross + acc * (cm + rm) * (qn + rq)) + 2.f * acc * qn * cm);
+}
+
 // out2 = bit patterns (uint32) of {largest squared norm, largest squared residual norm} over rows [n, dim] of
 // stride ld; a NaN anywhere leaves a NaN pattern. rows (optional): each row's norm and residual norm.
 int launch_base_norms(const float* x, int64_t n, int dim, int64_t ld, unsigned* out2, cudaStream_t st,

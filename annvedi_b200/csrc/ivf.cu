@@ -19,6 +19,7 @@
 //
 // Layout in HBM: codes [n, dpad8] uint8 and original rows [n, dpad] FP32, both in list order, so a
 // list is one contiguous byte range; per-dimension scale/offset zero-padded past dim.
+#include "block_select.cuh"
 #include "common.cuh"
 #include "ivf.cuh"
 #include "refmath.cuh"
@@ -54,12 +55,14 @@ __global__ void ivf_plan_kernel(IvfQueryArgs a) {
     }
     pref[j] = cands;
     if (cands < a.k && !a.no_fallback) {
-        p.n_seg[q] = -1;
         cands = a.ix.n;
+        if (a.apart) a.apart[atomicAdd(a.apart_count, 1)] = q;
+        p.n_seg[q] = a.apart ? 0 : -1;
+        p.n_cands[q] = a.apart ? 0 : cands;
     } else {
         p.n_seg[q] = j;
+        p.n_cands[q] = cands;
     }
-    p.n_cands[q] = cands;
     if (a.ndist) atomicAdd(a.ndist, (unsigned long long)cands);
 }
 
@@ -231,7 +234,7 @@ __global__ void __launch_bounds__(256) ivf_sq8_dists_kernel(IvfQueryArgs a, floa
     const int dpad8 = a.ix.dpad8;
     float* sQs = sh_qs;
     float* sSc = sh_qs + dpad8;
-    const int q = blockIdx.x, tid = threadIdx.x;
+    const int q = a.qorder ? a.qorder[blockIdx.x] : blockIdx.x, tid = threadIdx.x;
     const float* qv = a.q + (int64_t)q * a.ldq;
     for (int d = tid; d < dpad8; d += 256) {
         sQs[d] = d < a.ix.dim ? __fsub_rn(qv[d], a.ix.offset[d]) : 0.f;
@@ -243,7 +246,7 @@ __global__ void __launch_bounds__(256) ivf_sq8_dists_kernel(IvfQueryArgs a, floa
     const int half = dpad8 >> 1;
     const float* qs = sQs + h * half;
     const float* sc = sSc + h * half;
-    float* Dq = D + (int64_t)q * ld;
+    float* Dq = D + (int64_t)blockIdx.x * ld;
     for (int64_t p0 = (int64_t)blockIdx.y * kSq8Tile; p0 < L; p0 += (int64_t)gridDim.y * kSq8Tile) {
         const int64_t p = p0 + r;
         const bool valid = p < L;
@@ -286,7 +289,9 @@ int launch_ivf_sq8_dists(const IvfQueryArgs& a, float* D, int64_t ld, cudaStream
     ANN_CHECK_ARG(a.ix.dpad8 % 32 == 0, "sq8 keys: code stride %d not a multiple of 32", a.ix.dpad8);
     const size_t smem = sizeof(float) * 2 * a.ix.dpad8;
     ANN_CUDA_TRY(smem_optin(reinterpret_cast<const void*>(ivf_sq8_dists_kernel)));
-    const int slices = (int)std::min<int64_t>(8, std::max<int64_t>(1, ceil_div(ld, kSq8Tile)));
+    // eight slices a query, more where few long streams would leave the chip idle
+    const int64_t want = std::max<int64_t>(8, ceil_div(8 * kNumSMs, a.plan.nq));
+    const int slices = (int)std::min<int64_t>(std::min<int64_t>(want, 65535), std::max<int64_t>(1, ceil_div(ld, kSq8Tile)));
     ivf_sq8_dists_kernel<<<dim3(a.plan.nq, slices), 256, smem, st>>>(a, D, ld);
     ANN_LAUNCH_CHECK();
     return ANN_OK;
@@ -532,6 +537,61 @@ int launch_select_topk(const float* keys, int64_t ld, const int64_t* lens, int n
     if (plan) p = *plan;
     select_topk_kernel<<<nq, warps * 32, smem, st>>>(keys, ld, offs, lens, kout, p, plan ? 1 : 0, out_key, out_id,
                                                       set_only ? 1 : 0);
+    ANN_LAUNCH_CHECK();
+    return ANN_OK;
+}
+
+// ---- the best R rows of whole rows of keys -------------------------------------------------------------
+// One block per (segment of seg_rows keys, list entry): the segment's best R (key, row).
+__global__ void __launch_bounds__(256) rows_segment_kernel(const float* __restrict__ D, int64_t n, int64_t seg_rows, int R,
+                                                           unsigned long long* __restrict__ best) {
+    __shared__ int sHist[256];
+    __shared__ int sMisc[12];
+    __shared__ int sN;
+    const int64_t r0 = (int64_t)blockIdx.x * seg_rows;
+    segment_select(D + (int64_t)blockIdx.y * n + r0, r0, (int)min(seg_rows, n - r0), R,
+                   best + ((int64_t)blockIdx.y * gridDim.x + blockIdx.x) * R, sHist, sMisc, &sN);
+}
+
+// One block per list entry: the best k <= R of its segments' best, in no order, to row rows[entry] of out_key / out_id,
+// padded to R with (+inf, kNoId).
+__global__ void __launch_bounds__(512) rows_final_kernel(const unsigned long long* __restrict__ best, int m, int k, int R,
+                                                         const int32_t* __restrict__ rows, float* __restrict__ out_key,
+                                                         int* __restrict__ out_id) {
+    __shared__ int sHist[256];
+    __shared__ int sMisc[12];
+    __shared__ int sN;
+    const unsigned long long* w = best + (int64_t)blockIdx.x * m;
+    const int64_t o = (int64_t)rows[blockIdx.x] * R;
+    if (threadIdx.x == 0) sN = 0;
+    __syncthreads();
+    const SelectBound b = block_select_bound([&](int i) { return w[i]; }, m, k, sHist, sMisc);
+    for (int i = k + threadIdx.x; i < R; i += 512) {
+        out_key[o + i] = kInf;
+        out_id[o + i] = kNoId;
+    }
+    for (int i = threadIdx.x; i < m; i += 512) {
+        if (!b.in(w[i])) continue;
+        const int at = atomicAdd(&sN, 1);
+        out_key[o + at] = f32_ord((uint32_t)(w[i] >> 32));
+        out_id[o + at] = (int)(unsigned)w[i];
+    }
+}
+
+size_t rows_select_words(int64_t n, int R) {
+    return (size_t)ceil_div(n, select_seg_rows(n)) * (size_t)std::min<int64_t>(R, n);
+}
+
+int launch_rows_select(const float* D, int64_t n, int count, int R, const int32_t* rows, unsigned long long* words,
+                       float* out_key, int* out_id, cudaStream_t st) {
+    if (count == 0) return ANN_OK;
+    ANN_CHECK_ARG(R >= 1 && n >= 1 && count <= 65535, "row selection: R=%d, %d entries", R, count);
+    const int k = (int)std::min<int64_t>(R, n);
+    const int64_t seg = select_seg_rows(n);
+    const int nseg = (int)ceil_div(n, seg);
+    rows_segment_kernel<<<dim3(nseg, (unsigned)count), 256, 0, st>>>(D, n, seg, k, words);
+    ANN_LAUNCH_CHECK();
+    rows_final_kernel<<<(unsigned)count, 512, 0, st>>>(words, nseg * k, k, R, rows, out_key, out_id);
     ANN_LAUNCH_CHECK();
     return ANN_OK;
 }
@@ -830,6 +890,21 @@ __global__ void clear_every_row_kernel(IvfPlan plan) {
 int launch_clear_every_row(const IvfPlan& plan, cudaStream_t st) {
     if (plan.nq == 0) return ANN_OK;
     clear_every_row_kernel<<<(unsigned)ceil_div(plan.nq, 256), 256, 0, st>>>(plan);
+    ANN_LAUNCH_CHECK();
+    return ANN_OK;
+}
+
+__global__ void set_every_row_kernel(IvfPlan plan, const int32_t* __restrict__ list, int count, int64_t n) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < count) {
+        plan.n_seg[list[i]] = -1;
+        plan.n_cands[list[i]] = n;
+    }
+}
+
+int launch_set_every_row(const IvfPlan& plan, const int32_t* list, int count, int64_t n, cudaStream_t st) {
+    if (count == 0) return ANN_OK;
+    set_every_row_kernel<<<(unsigned)ceil_div(count, 256), 256, 0, st>>>(plan, list, count, n);
     ANN_LAUNCH_CHECK();
     return ANN_OK;
 }

@@ -61,6 +61,8 @@ struct IvfQueryArgs {
     int k;
     int R;                     // candidates kept for the FP32 re-rank
     int64_t max_cands;         // cap on the candidate stream (INT64_MAX = none)
+    int32_t* apart;            // plan: queries whose stream is every row are listed here and get an empty stream
+    int* apart_count;          //   (NULL: they get the stream of every row)
     int no_fallback;           // a shard of the lists: a stream short of k stays as it is (no every-row scan)
     int nsplit;                // CTAs per query in the exact SQ8 scan
     int num_threads;           // reference mode: the reference ThreadPool size
@@ -76,7 +78,8 @@ struct IvfQueryArgs {
     int metric;                // re-rank metric: ANN_METRIC_L2 (default) or ANN_METRIC_IP
     int64_t* out_ids;          // [nq, k]
     float* out_dists;          // [nq, k]
-    const int32_t* qorder;     // re-rank: CTA b takes query qorder[b] (NULL: query b)
+    const int32_t* qorder;     // whole-stream SQ8 keys and re-rank: CTA b takes query qorder[b] (NULL: query b); the
+                               // keys go to row b
 };
 
 int launch_ivf_plan(const IvfQueryArgs& a, cudaStream_t st);
@@ -87,6 +90,11 @@ int launch_ivf_ref_sq8(const IvfQueryArgs& a, int64_t Lmax, cudaStream_t st);
 int launch_select_topk(const float* keys, int64_t ld_keys, const int64_t* lens, int nq, int kout,
                        const IvfPlan* plan, float* out_key, int* out_id, cudaStream_t st,
                        const int64_t* offs = nullptr, bool set_only = false);
+// The best R (key, row) of each of `count` rows of n keys D[e * n + row], in no order, into row rows[e] of
+// out_key / out_id, padded with (+inf, kNoId) where n < R; words: count * rows_select_words(n, R) scratch.
+size_t rows_select_words(int64_t n, int R);
+int launch_rows_select(const float* D, int64_t n, int count, int R, const int32_t* rows, unsigned long long* words,
+                       float* out_key, int* out_id, cudaStream_t st);
 int launch_ivf_rerank(const IvfQueryArgs& a, const float* keyR, const int* idR, int reference, cudaStream_t st);
 int launch_ref_centroid_dists(const IvfView& ix, const float* q, int64_t ldq, int nq, float* Dc, cudaStream_t st);
 
@@ -102,6 +110,8 @@ int launch_list_offsets(const int32_t* sorted_assign, int64_t n, int C, int64_t*
 int launch_iota(int32_t* v, int64_t n, cudaStream_t st);                 // v[i] = i
 // Every query whose stream is every row (n_seg < 0) becomes an empty stream: n_seg = n_cands = 0.
 int launch_clear_every_row(const IvfPlan& plan, cudaStream_t st);
+// The listed queries get the stream of every row: n_seg = -1, n_cands = n.
+int launch_set_every_row(const IvfPlan& plan, const int32_t* list, int count, int64_t n, cudaStream_t st);
 // order[0..nq) = the queries grouped by their first probed list (probes[q * npc], in [0, C)), so that
 // neighbouring re-rank CTAs gather rows of the same lists; one CTA, C <= kQueryOrderMaxLists.
 constexpr int kQueryOrderMaxLists = 32768;

@@ -301,10 +301,7 @@ __global__ void __launch_bounds__(256) kmeans_key_assign_kernel(const float* __r
     const float2 nr = norms[i];
     const float xn = nr.x * 1.001f, xe = nr.y * 1.001f;
     const float cm = sqrtf(__uint_as_float(cnorm2[0])) * 1.001f, rm = sqrtf(__uint_as_float(cnorm2[1])) * 1.001f;
-    const float acc = (float)(dim + 19) * 4.76837158e-7f;  // (dim + 19) 2^-21
-    const float cross = rm * xn + (cm + rm) * xe;
-    const float w = 1.002f * (2.f * (2.f * cross + acc * (2.f * (cm + rm) * (xn + xe) + cm * cm)) +
-                              acc * (xn + cm) * (xn + cm));
+    const float w = key_window_l2(xn, xe, cm, rm, dim);
     const bool covered = xn <= kPruneNormMax && (xn >= kPruneNormMin || nr.x == 0.f) && cm <= kPruneNormMax &&
                          cm >= kPruneNormMin;  // false for NaN
     const int nch = (C + 31) >> 5;

@@ -2,7 +2,10 @@
 // the row order of the BF16 base copy.
 #include <numeric>
 
+#include <cuda_bf16.h>
+
 #include "common.cuh"
+#include "flat_prune.cuh"
 #include "tc_search.cuh"
 
 namespace annb {
@@ -557,27 +560,35 @@ constexpr int kCoarseChunks = 16;  // dims up to 512 take the register path of t
 // nch = ceil(C / 32) <= 64, for npc <= 32 and dpad <= 32 kCoarseChunks (cmax > 0).
 //  1. bar = the npc-th smallest chunk minimum (total order by (minimum, chunk); +inf when npc > nch): each
 //     of those npc chunks holds a key <= bar, so the npc-th smallest key T is <= bar.
-//  2. The window lim = bar + 2 eps + delta (the keys' certified error, as below): a centroid whose key
+//  2. The window lim = bar + 2 eps + delta (the keys' certified error, key_window_l2): a centroid whose key
 //     exceeds lim exceeds T + 2 eps + delta, so its exact distance exceeds those of the npc centroids of
 //     smallest key, and it is not among the best npc.
 //  3. Every key <= lim (found in the chunks whose minimum is <= lim) gets its exact FP32 distance, and the
 //     best npc by (distance, id) are kept, lane j holding the j-th: no candidate buffer and no sort.
+// SCAN: the distances are those of the staged exact scan (flat_scan.cu: one chain over d a centroid), so that the
+// ranking is its ranking bit for bit; the centroids inside the window (about 2 npc) are taken 32 at a time, one a lane.
+template <bool SCAN>
 __device__ __forceinline__ void coarse_by_chunks(const float* __restrict__ kr, const float* __restrict__ cq, int C,
                                                  int npc, const float* __restrict__ qv,
                                                  const float* __restrict__ cent, int dpad, int dim, float cmax,
-                                                 int32_t* __restrict__ pout) {
+                                                 float rmax, int32_t* __restrict__ pout, int* sList) {
     const int lane = threadIdx.x & 31;
     const int nch = (C + 31) >> 5;
     const float a0 = lane < nch ? cq[lane] : kInf, a1 = lane + 32 < nch ? cq[lane + 32] : kInf;
     float qr[kCoarseChunks];
-    float s2 = 0.f;
+    float s2 = 0.f, e2 = 0.f;
 #pragma unroll
     for (int i = 0; i < kCoarseChunks; ++i) {
         qr[i] = lane + 32 * i < dpad ? qv[lane + 32 * i] : 0.f;
+        const float t = qr[i] - __bfloat162float(__float2bfloat16_rn(qr[i]));
         s2 = fmaf(qr[i], qr[i], s2);
+        e2 = fmaf(t, t, e2);
     }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s2 += __shfl_xor_sync(0xffffffffu, s2, o);
+    for (int o = 16; o > 0; o >>= 1) {
+        s2 += __shfl_xor_sync(0xffffffffu, s2, o);
+        e2 += __shfl_xor_sync(0xffffffffu, e2, o);
+    }
     float bar = kInf;
     if (npc <= nch) {  // lane l holds chunks l and l + 32; ranks among the 64 (padding +inf, sorted last)
         int r0 = 0, r1 = 0;
@@ -593,11 +604,10 @@ __device__ __forceinline__ void coarse_by_chunks(const float* __restrict__ kr, c
         const float b1 = __shfl_sync(0xffffffffu, a1, s1 ? __ffs(s1) - 1 : 0);
         bar = s0 ? b0 : (s1 ? b1 : kInf);  // no rank npc - 1 only with NaN minima: every chunk
     }
-    const float qn = sqrtf(s2) * 1.0001f;
-    const float acc = (float)(dim + 3) * 4.76837158e-7f;  // (dim + 3) 2^-21
-    const float eps = qn * cmax * (7.8125e-3f * 1.05f + 2.1f * acc) + cmax * cmax * acc;
-    const float delta = acc * (qn + cmax) * (qn + cmax);
-    const float lim = bar + 2.f * eps + delta;
+    const float qn = sqrtf(s2), w = key_window_l2(qn, sqrtf(e2), cmax, rmax, dim);
+    // a query that the bound does not cover (NaN, norms out of range) takes every centroid
+    const bool all = !(qn <= kPruneNormMax && (qn >= kPruneNormMin || s2 == 0.f) && w < kInf);
+    const float lim = all ? kInf : __fadd_ru(bar, w);
     float bd = kInf;  // lane j < npc: the j-th best (distance, id) so far
     int bi = kNoId;
     auto insert = [&](float d, int id) {  // warp-uniform (d, id)
@@ -614,8 +624,32 @@ __device__ __forceinline__ void coarse_by_chunks(const float* __restrict__ kr, c
             }
         }
     };
-    unsigned c0m = __ballot_sync(0xffffffffu, lane < nch && !(a0 > lim));
-    unsigned c1m = __ballot_sync(0xffffffffu, lane + 32 < nch && !(a1 > lim));
+    int held = 0;  // SCAN: centroids waiting in sList (uniform)
+    auto eval_held = [&]() {  // one centroid a lane: its distance as one chain over d, then the insertions in turn
+        __syncwarp();
+        const int id = lane < held ? sList[lane] : 0;
+        const float* x = cent + (int64_t)id * dpad;
+        float acc = 0.f;
+        for (int d0 = 0; d0 < dpad; d0 += 32) {
+            float4 v[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) v[u] = *reinterpret_cast<const float4*>(x + d0 + 4 * u);
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                const float4 q4 = *reinterpret_cast<const float4*>(qv + d0 + 4 * u);
+                const float t0 = v[u].x - q4.x, t1 = v[u].y - q4.y, t2 = v[u].z - q4.z, t3 = v[u].w - q4.w;
+                acc = fmaf(t0, t0, acc);
+                acc = fmaf(t1, t1, acc);
+                acc = fmaf(t2, t2, acc);
+                acc = fmaf(t3, t3, acc);
+            }
+        }
+        for (int j = 0; j < held; ++j) insert(__shfl_sync(0xffffffffu, acc, j), __shfl_sync(0xffffffffu, id, j));
+        held = 0;
+        __syncwarp();
+    };
+    unsigned c0m = __ballot_sync(0xffffffffu, lane < nch && (all || !(a0 > lim)));
+    unsigned c1m = __ballot_sync(0xffffffffu, lane + 32 < nch && (all || !(a1 > lim)));
     while (c0m | c1m) {  // four chunks' loads in flight
         int ch[4];
 #pragma unroll
@@ -638,8 +672,13 @@ __device__ __forceinline__ void coarse_by_chunks(const float* __restrict__ kr, c
         }
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
-            unsigned hit = __ballot_sync(0xffffffffu, ch[u] >= 0 && ch[u] * 32 + lane < C && v[u] <= lim);
-            while (hit) {  // two centroids at a time, all their pieces loaded before use; per lane the sum
+            unsigned hit = __ballot_sync(0xffffffffu, ch[u] >= 0 && ch[u] * 32 + lane < C && (all || v[u] <= lim));
+            if (SCAN) {
+                if (held + __popc(hit) > 32) eval_held();
+                if (hit >> lane & 1u) sList[held + __popc(hit & ((1u << lane) - 1u))] = ch[u] * 32 + lane;
+                held += __popc(hit);
+            }
+            while (!SCAN && hit) {  // two centroids at a time, all their pieces loaded before use; per lane the sum
                            // runs over d = lane, lane + 32, ... as in the kernel below
                 const int ca = ch[u] * 32 + __ffs(hit) - 1;
                 hit &= hit - 1;
@@ -674,15 +713,16 @@ __device__ __forceinline__ void coarse_by_chunks(const float* __restrict__ kr, c
             }
         }
     }
-    if (lane < npc) pout[lane] = bi != kNoId ? bi : 0;
+    if (SCAN && held > 0) eval_held();
+    if (lane < npc) pout[lane] = SCAN || bi != kNoId ? bi : 0;
 }
 
 // one warp per query; CMIN: the keys' 32-column chunk minima are given, and coarse_by_chunks ranks the query
-template <bool CMIN>
+template <bool CMIN, bool SCAN>
 __global__ void __launch_bounds__(128) tc_coarse_kernel(const float* __restrict__ keys, int64_t ldk, int nq, int C,
                                                        int npc, int m, const float* __restrict__ q,
                                                        const float* __restrict__ cent, int dpad, int32_t* probes,
-                                                       float cmax, int dim, const float* __restrict__ cmin) {
+                                                       float cmax, float rmax, int dim, const float* __restrict__ cmin) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int cap = topk_cap(m);
@@ -691,8 +731,10 @@ __global__ void __launch_bounds__(128) tc_coarse_kernel(const float* __restrict_
     const int qi = blockIdx.x * 4 + warp;
     if (qi >= nq) return;
     if (CMIN) {
-        coarse_by_chunks(keys + (int64_t)qi * ldk, cmin + (int64_t)qi * ((C + 31) >> 5), C, npc, q + (int64_t)qi * dpad,
-                         cent, dpad, dim, cmax, probes + (int64_t)qi * npc);
+        __shared__ int sList[4][32];
+        coarse_by_chunks<SCAN>(keys + (int64_t)qi * ldk, cmin + (int64_t)qi * ((C + 31) >> 5), C, npc,
+                               q + (int64_t)qi * dpad, cent, dpad, dim, cmax, rmax, probes + (int64_t)qi * npc,
+                               sList[warp]);
         return;
     }
     WarpTopK top;
@@ -827,17 +869,21 @@ __global__ void __launch_bounds__(128) tc_coarse_kernel(const float* __restrict_
 
 }  // namespace
 
+bool tc_coarse_chunked(int C, int npc, int dpad) { return C <= 64 * 32 && npc <= 32 && dpad <= 32 * kCoarseChunks; }
+
 int launch_tc_coarse(const float* keys, int64_t ldk, int nq, int C, int npc, int margin, const float* q,
-                     const float* centroids, int dpad, int32_t* probes, cudaStream_t st, float cmax, int dim,
-                     const float* cmin) {
+                     const float* centroids, int dpad, int32_t* probes, cudaStream_t st, float cmax, float rmax, int dim,
+                     const float* cmin, bool scan) {
     if (nq == 0) return ANN_OK;
     const int m = std::min(C, npc + margin);
     ANN_CHECK_ARG(npc >= 1 && npc <= m && m <= 1024, "tensor-core coarse ranking: npc=%d, m=%d", npc, m);
     const size_t smem = (size_t)4 * 2 * topk_cap(m) * 4;
-    const bool chunks = cmin != nullptr && C <= 64 * 32 && npc <= 32 && cmax > 0.f && dpad <= 32 * kCoarseChunks;
-    auto kern = chunks ? tc_coarse_kernel<true> : tc_coarse_kernel<false>;
+    const bool chunks = cmin != nullptr && cmax > 0.f && tc_coarse_chunked(C, npc, dpad);
+    ANN_CHECK_ARG(!scan || chunks, "tensor-core coarse ranking: C=%d, npc=%d, padded dim %d", C, npc, dpad);
+    auto kern = chunks ? (scan ? tc_coarse_kernel<true, true> : tc_coarse_kernel<true, false>)
+                       : tc_coarse_kernel<false, false>;
     ANN_CUDA_TRY(smem_optin(reinterpret_cast<const void*>(kern)));
-    kern<<<(unsigned)ceil_div(nq, 4), 128, smem, st>>>(keys, ldk, nq, C, npc, m, q, centroids, dpad, probes, cmax,
+    kern<<<(unsigned)ceil_div(nq, 4), 128, smem, st>>>(keys, ldk, nq, C, npc, m, q, centroids, dpad, probes, cmax, rmax,
                                                        dim > 0 ? dim : dpad, cmin);
     ANN_LAUNCH_CHECK();
     return ANN_OK;

@@ -87,13 +87,17 @@ int launch_tc_compact_rows(const int* list, const int* count, int max_count, con
 // Coarse ranking of the tensor-core IVF form from BF16 keys [nq, C] (ldk per row): per query, the best
 // m = min(C, npc + margin) centroids by key, their exact FP32 squared distances (FP32 queries and
 // centroids, row stride dpad), and the best npc of those by (distance, id) into probes [nq, npc],
-// best first. With cmax > 0 (the largest centroid norm; dim the vectors' dimension) only the candidates whose
+// best first. With cmax > 0 (upper bounds of the centroids' norms and of their BF16 residuals' norms, cmax and rmax;
+// dim the vectors' dimension) only the candidates whose
 // key lies within the keys' certified error window of the npc-th key get exact distances: the others cannot
 // be among the best npc, so the result is the same. cmin (optional): the keys' 32-column chunk minima
-// [nq, ceil(C / 32)] (TcGemmArgs::out_cmin); with C <= 2,048 and m <= 32, only the chunks at or below a bar
-// taken from them are read, with the same result.
+// [nq, ceil(C / 32)] (TcGemmArgs::out_cmin); where tc_coarse_chunked, only the chunks at or below a bar
+// taken from them are read, with the same result. scan (tc_coarse_chunked sizes, with cmin and cmax): the distances
+// are the staged exact scan's, so that probes are those of the exact scan over the centroids (INT_MAX where a query
+// compares with none).
+bool tc_coarse_chunked(int C, int npc, int dpad);
 int launch_tc_coarse(const float* keys, int64_t ldk, int nq, int C, int npc, int margin, const float* q,
                      const float* centroids, int dpad, int32_t* probes, cudaStream_t st, float cmax = 0.f,
-                     int dim = 0, const float* cmin = nullptr);
+                     float rmax = 0.f, int dim = 0, const float* cmin = nullptr, bool scan = false);
 
 }  // namespace annb
