@@ -6,8 +6,8 @@
 // code once per query; here a work item is (list, up to 32 of the queries probing it, a range of up to
 // kItemRows of its rows): the rows stream through shared memory in tiles of 256 rows x 32 dimensions,
 // are decoded once (the exact integer of each code, FP32) and scored against the item's queries with a
-// register-tiled micro-kernel (8 queries x 4 rows per thread, two fused multiply-adds per element
-// pair). Each distance lands at its position in its query's candidate stream (the positions the plan
+// register-tiled micro-kernel (8 queries x 4, 2 or 1 rows per thread by the item's queries, two fused
+// multiply-adds per element pair). Each distance lands at its position in its query's candidate stream (the positions the plan
 // assigns, lsh_index_optimized.cpp:372-405 order), so a per-query selection and the FP32 re-rank
 // follow unchanged. Items are taken from a global counter by a persistent grid (uneven list lengths and
 // query counts balance dynamically).
@@ -28,11 +28,9 @@ namespace annb {
 
 namespace {
 
-constexpr int kBQ = 32, kTQ = 8, kTR = 4;
+constexpr int kBQ = 32, kTQ = 8;
 constexpr int kThreads = 256;
-constexpr int kWQ = kBQ / kTQ;       // 4 query groups
-constexpr int kWR = kThreads / kWQ;  // 64 row groups
-constexpr int kBR = kWR * kTR;       // 256 rows per tile
+constexpr int kBR = 256;             // rows per tile
 constexpr int kKC = 32;              // dimensions per step
 constexpr int kPitch = kKC + 4;      // floats
 
@@ -76,22 +74,141 @@ __global__ void shift_queries_kernel(const float* q, int nq, int dpad, int dim, 
     }
 }
 
-__global__ void __launch_bounds__(kThreads, 2) ivf_batched_kernel(IvfBatchArgs a) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int dpad = a.ix.dpad, dpad8 = a.ix.dpad8;
-    float* sQ = reinterpret_cast<float*>(smem_raw);                 // [kBQ][dpad] shifted queries
-    float* sX = sQ + (size_t)kBQ * dpad;                             // [kBR][kPitch] decoded rows
-    float* sScale = sX + (size_t)kBR * kPitch;                       // [dpad]
-    unsigned char* sRaw = reinterpret_cast<unsigned char*>(sScale + dpad);  // [2][kBR][kKC] codes
-    int64_t* sBase = reinterpret_cast<int64_t*>(sRaw + 2 * kBR * kKC);     // [kBQ] D position of row 0
-    int* sItem = reinterpret_cast<int*>(sBase + kBQ);
+// The shared memory of a CTA.
+struct ItemSmem {
+    float* q;            // [kBQ][dpad] shifted queries
+    float* x;            // [kBR][kPitch] decoded rows
+    float* scale;        // [dpad]
+    unsigned char* raw;  // [2][kBR][kKC] codes
+    int64_t* base;       // [kBQ] D position of row 0
+};
 
+// One work item: rows [r_begin, r_end) against nqi <= 8 WQ queries. WQ query groups of 8 queries; a thread holds 8
+// queries x TR = WQ rows, so that an item of few queries spreads its rows over all threads instead of multiplying
+// padding: at 2,000 queries x 8 lists over 2,048 lists a list has about 7 queries beside its own cluster's, and 32-query
+// tiles did 1.8 times the useful work. Warps whose rows or queries lie past the item's skip the sums.
+template <int WQ>
+__device__ __forceinline__ void score_item(const IvfBatchArgs& a, const ItemSmem& sm, int64_t r_begin, int64_t r_end,
+                                           int nqi) {
+    constexpr int TR = WQ, WR = kThreads / WQ;
+    static_assert(WR * TR == kBR, "a tile's rows");
+    const int dpad = a.ix.dpad, dpad8 = a.ix.dpad8;
     const int tid = threadIdx.x;
-    const int tq = tid / kWR, tr = tid % kWR;
-    for (int d = tid; d < dpad; d += kThreads) sScale[d] = a.ix.scale[d];
+    const int tq = tid / WR, tr = tid % WR;
     const int nkc = dpad8 / kKC;  // code chunks (>= dpad / kKC; extra chunks hold zero codes and scale)
     const int half_kc = nkc / 2;  // first chunk of the high half of the padded code row (dpad8 / 2)
+    const int64_t ntiles = ceil_div(r_end - r_begin, kBR);
+    const int64_t nsteps = ntiles * nkc;
+    auto issue = [&](int64_t step) {
+        if (step < nsteps) {
+            const int64_t t = step / nkc;
+            const int kc = (int)(step % nkc);
+            unsigned char* dst = sm.raw + (size_t)(step & 1) * kBR * kKC;
+            for (int c = tid; c < kBR * 2; c += kThreads) {  // 256 rows x 2 pieces of 16 codes
+                const int r = c >> 1, piece = c & 1;
+                const int64_t row = r_begin + t * kBR + r;
+                const bool ok = row < r_end;
+                cp16(dst + r * kKC + piece * 16, a.ix.codes + (ok ? row : r_begin) * dpad8 + kc * kKC + piece * 16, ok);
+            }
+        }
+        cp_commit();
+    };
+    issue(0);
+    float acc[kTQ][TR], lowh[kTQ][TR];
+#pragma unroll
+    for (int j = 0; j < kTQ; ++j)
+#pragma unroll
+        for (int i = 0; i < TR; ++i) acc[j][i] = lowh[j][i] = 0.f;
+    int kc = 0;
+    int64_t t0 = r_begin;  // first row of the tile
+    for (int64_t step = 0; step < nsteps; ++step) {
+        cp_wait0();
+        __syncthreads();  // raw codes of this step (and the queries) landed; last step's reads are done
+        issue(step + 1);
+        const int rows = (int)min((int64_t)kBR, r_end - t0);  // of this tile
+        // decode the rows' 32 codes: the exact integer of each byte
+        {
+            const unsigned char* raw = sm.raw + (size_t)(step & 1) * kBR * kKC;
+            for (int e = tid; e < rows * (kKC / 4); e += kThreads) {
+                const int r = e / (kKC / 4), w4 = e % (kKC / 4);
+                const uint32_t w = *reinterpret_cast<const uint32_t*>(raw + r * kKC + w4 * 4);
+                float4 v;
+                v.x = __fsub_rn(__uint_as_float(__byte_perm(w, 0x4B000000u, 0x7540u)), 8388608.f);
+                v.y = __fsub_rn(__uint_as_float(__byte_perm(w, 0x4B000000u, 0x7541u)), 8388608.f);
+                v.z = __fsub_rn(__uint_as_float(__byte_perm(w, 0x4B000000u, 0x7542u)), 8388608.f);
+                v.w = __fsub_rn(__uint_as_float(__byte_perm(w, 0x4B000000u, 0x7543u)), 8388608.f);
+                *reinterpret_cast<float4*>(sm.x + r * kPitch + w4 * 4) = v;
+            }
+        }
+        __syncthreads();
+        const bool busy = tq * kTQ < nqi && (tr & ~31) < rows;  // uniform across the warp (WR is a multiple of 32)
+        if (kc == half_kc) {  // the high half starts: keep the low half's sums apart
+#pragma unroll
+            for (int j = 0; j < kTQ; ++j)
+#pragma unroll
+                for (int i = 0; i < TR; ++i) {
+                    lowh[j][i] = acc[j][i];
+                    acc[j][i] = 0.f;
+                }
+        }
+        if (busy && kc * kKC < dpad) {
+            const float* qbase = sm.q + kc * kKC;
+#pragma unroll
+            for (int kk = 0; kk < kKC; kk += 4) {
+                float4 xv[TR], qv[kTQ];
+                const float4 sc = *reinterpret_cast<const float4*>(sm.scale + kc * kKC + kk);
+#pragma unroll
+                for (int i = 0; i < TR; ++i) xv[i] = *reinterpret_cast<const float4*>(sm.x + (tr + i * WR) * kPitch + kk);
+#pragma unroll
+                for (int j = 0; j < kTQ; ++j)
+                    qv[j] = *reinterpret_cast<const float4*>(qbase + (size_t)(tq * kTQ + j) * dpad + kk);
+#pragma unroll
+                for (int j = 0; j < kTQ; ++j)
+#pragma unroll
+                    for (int i = 0; i < TR; ++i) {
+                        const float d0 = __fmaf_rn(xv[i].x, sc.x, -qv[j].x);
+                        const float d1 = __fmaf_rn(xv[i].y, sc.y, -qv[j].y);
+                        const float d2 = __fmaf_rn(xv[i].z, sc.z, -qv[j].z);
+                        const float d3 = __fmaf_rn(xv[i].w, sc.w, -qv[j].w);
+                        acc[j][i] = __fmaf_rn(d0, d0, acc[j][i]);
+                        acc[j][i] = __fmaf_rn(d1, d1, acc[j][i]);
+                        acc[j][i] = __fmaf_rn(d2, d2, acc[j][i]);
+                        acc[j][i] = __fmaf_rn(d3, d3, acc[j][i]);
+                    }
+            }
+        }
+        if (++kc == nkc) {
+            kc = 0;
+#pragma unroll
+            for (int j = 0; j < kTQ; ++j) {
+                const int qq = tq * kTQ + j;
+#pragma unroll
+                for (int i = 0; i < TR; ++i) {
+                    const int64_t row = t0 + tr + i * WR;
+                    if (qq < nqi && row < r_end) a.D[sm.base[qq] + row] = __fadd_rn(lowh[j][i], acc[j][i]);
+                    acc[j][i] = 0.f;
+                    lowh[j][i] = 0.f;
+                }
+            }
+            t0 += kBR;
+        }
+    }
+    cp_wait0();
+}
 
+__global__ void __launch_bounds__(kThreads, 2) ivf_batched_kernel(IvfBatchArgs a) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int dpad = a.ix.dpad;
+    ItemSmem sm;
+    sm.q = reinterpret_cast<float*>(smem_raw);
+    sm.x = sm.q + (size_t)kBQ * dpad;
+    sm.scale = sm.x + (size_t)kBR * kPitch;
+    sm.raw = reinterpret_cast<unsigned char*>(sm.scale + dpad);
+    sm.base = reinterpret_cast<int64_t*>(sm.raw + 2 * kBR * kKC);
+    int* sItem = reinterpret_cast<int*>(sm.base + kBQ);
+
+    const int tid = threadIdx.x;
+    for (int d = tid; d < dpad; d += kThreads) sm.scale[d] = a.ix.scale[d];
     while (true) {
         __syncthreads();
         if (tid == 0) sItem[0] = (int)atomicAdd(a.counter, 1u);
@@ -116,13 +233,14 @@ __global__ void __launch_bounds__(kThreads, 2) ivf_batched_kernel(IvfBatchArgs a
         const int64_t lstart = a.ix.list_off[l];
         const int64_t r_begin = lstart + rr * kItemRows;
         const int64_t r_end = min(a.ix.list_off[l + 1], r_begin + kItemRows);
-        // the item's queries: shifted query rows and the stream position of this list's row 0
-        for (int e = tid; e < kBQ * (dpad / 4); e += kThreads) {
+        // the item's queries (zeros up to a multiple of 8): shifted query rows and the stream position of this list's row 0
+        const int nq8 = (nqi + kTQ - 1) / kTQ * kTQ;
+        for (int e = tid; e < nq8 * (dpad / 4); e += kThreads) {
             const int qq = e / (dpad / 4), piece = e % (dpad / 4);
             const bool ok = qq < nqi;
             const int32_t v = ok ? a.pair_vals[q0 + qq] : 0;
             const int qi = v / a.plan.npc;
-            cp16(sQ + (size_t)qq * dpad + piece * 4, a.qs + (int64_t)qi * dpad + piece * 4, ok);
+            cp16(sm.q + (size_t)qq * dpad + piece * 4, a.qs + (int64_t)qi * dpad + piece * 4, ok);
         }
         cp_commit();
         if (tid < kBQ) {
@@ -132,103 +250,14 @@ __global__ void __launch_bounds__(kThreads, 2) ivf_batched_kernel(IvfBatchArgs a
                 const int qi = v / a.plan.npc, j = v % a.plan.npc;
                 base = a.cand_off[qi] + a.plan.seg_pref[(int64_t)qi * (a.plan.npc + 1) + j] - lstart;
             }
-            sBase[tid] = base;
+            sm.base[tid] = base;
         }
-        const int64_t ntiles = ceil_div(r_end - r_begin, kBR);
-        const int64_t nsteps = ntiles * nkc;
-        auto issue = [&](int64_t step) {
-            if (step < nsteps) {
-                const int64_t t = step / nkc;
-                const int kc = (int)(step % nkc);
-                unsigned char* dst = sRaw + (size_t)(step & 1) * kBR * kKC;
-                for (int c = tid; c < kBR * 2; c += kThreads) {  // 256 rows x 2 pieces of 16 codes
-                    const int r = c >> 1, piece = c & 1;
-                    const int64_t row = r_begin + t * kBR + r;
-                    const bool ok = row < r_end;
-                    cp16(dst + r * kKC + piece * 16, a.ix.codes + (ok ? row : r_begin) * dpad8 + kc * kKC + piece * 16, ok);
-                }
-            }
-            cp_commit();
-        };
-        issue(0);
-        float acc[kTQ][kTR], lowh[kTQ][kTR];
-#pragma unroll
-        for (int j = 0; j < kTQ; ++j)
-#pragma unroll
-            for (int i = 0; i < kTR; ++i) acc[j][i] = lowh[j][i] = 0.f;
-        for (int64_t step = 0; step < nsteps; ++step) {
-            cp_wait0();
-            __syncthreads();  // raw codes of this step (and the queries) landed; last step's reads are done
-            issue(step + 1);
-            const int kc = (int)(step % nkc);
-            // decode 256 rows x 32 codes: code * scale, exact integer from the byte first
-            {
-                const unsigned char* raw = sRaw + (size_t)(step & 1) * kBR * kKC;
-                for (int e = tid; e < kBR * (kKC / 4); e += kThreads) {
-                    const int r = e / (kKC / 4), w4 = e % (kKC / 4);
-                    const uint32_t w = *reinterpret_cast<const uint32_t*>(raw + r * kKC + w4 * 4);
-                    const int d0 = kc * kKC + w4 * 4;
-                    float4 v;
-                    (void)d0;
-                    v.x = __fsub_rn(__uint_as_float(__byte_perm(w, 0x4B000000u, 0x7540u)), 8388608.f);
-                    v.y = __fsub_rn(__uint_as_float(__byte_perm(w, 0x4B000000u, 0x7541u)), 8388608.f);
-                    v.z = __fsub_rn(__uint_as_float(__byte_perm(w, 0x4B000000u, 0x7542u)), 8388608.f);
-                    v.w = __fsub_rn(__uint_as_float(__byte_perm(w, 0x4B000000u, 0x7543u)), 8388608.f);
-                    *reinterpret_cast<float4*>(sX + r * kPitch + w4 * 4) = v;
-                }
-            }
-            __syncthreads();
-            if (kc == half_kc) {  // the high half starts: keep the low half's sums apart
-#pragma unroll
-                for (int j = 0; j < kTQ; ++j)
-#pragma unroll
-                    for (int i = 0; i < kTR; ++i) {
-                        lowh[j][i] = acc[j][i];
-                        acc[j][i] = 0.f;
-                    }
-            }
-            if (kc * kKC < dpad) {
-                const float* qbase = sQ + kc * kKC;
-#pragma unroll
-                for (int kk = 0; kk < kKC; kk += 4) {
-                    float4 xv[kTR], qv[kTQ];
-                    const float4 sc = *reinterpret_cast<const float4*>(sScale + kc * kKC + kk);
-#pragma unroll
-                    for (int i = 0; i < kTR; ++i) xv[i] = *reinterpret_cast<const float4*>(sX + (tr + i * kWR) * kPitch + kk);
-#pragma unroll
-                    for (int j = 0; j < kTQ; ++j)
-                        qv[j] = *reinterpret_cast<const float4*>(qbase + (size_t)(tq * kTQ + j) * dpad + kk);
-#pragma unroll
-                    for (int j = 0; j < kTQ; ++j)
-#pragma unroll
-                        for (int i = 0; i < kTR; ++i) {
-                            const float d0 = __fmaf_rn(xv[i].x, sc.x, -qv[j].x);
-                            const float d1 = __fmaf_rn(xv[i].y, sc.y, -qv[j].y);
-                            const float d2 = __fmaf_rn(xv[i].z, sc.z, -qv[j].z);
-                            const float d3 = __fmaf_rn(xv[i].w, sc.w, -qv[j].w);
-                            acc[j][i] = __fmaf_rn(d0, d0, acc[j][i]);
-                            acc[j][i] = __fmaf_rn(d1, d1, acc[j][i]);
-                            acc[j][i] = __fmaf_rn(d2, d2, acc[j][i]);
-                            acc[j][i] = __fmaf_rn(d3, d3, acc[j][i]);
-                        }
-                }
-            }
-            if (kc == nkc - 1) {
-                const int64_t t = step / nkc;
-#pragma unroll
-                for (int j = 0; j < kTQ; ++j) {
-                    const int qq = tq * kTQ + j;
-#pragma unroll
-                    for (int i = 0; i < kTR; ++i) {
-                        const int64_t row = r_begin + t * kBR + tr + i * kWR;
-                        if (qq < nqi && row < r_end) a.D[sBase[qq] + row] = __fadd_rn(lowh[j][i], acc[j][i]);
-                        acc[j][i] = 0.f;
-                        lowh[j][i] = 0.f;
-                    }
-                }
-            }
-        }
-        cp_wait0();
+        if (nqi <= kTQ)
+            score_item<1>(a, sm, r_begin, r_end, nqi);
+        else if (nqi <= 2 * kTQ)
+            score_item<2>(a, sm, r_begin, r_end, nqi);
+        else
+            score_item<4>(a, sm, r_begin, r_end, nqi);
     }
 }
 
