@@ -751,7 +751,9 @@ constexpr int kEveryRowMinSplit = 8;      // exact batches split fewer ways redo
 struct IvfQueryCfg {
     int k, npc, R, nsplit, num_threads, bqc, nsplit_c, ncp;
     int64_t max_c, ub, rps_c;
+    int64_t small_keys;  // a bound of the batch's candidates: any npc lists a query
     bool ref, coarse_flat, batched, tc, lsh;
+    bool small_tc;     // a small tensor-core batch, set up by one CTA without a host round trip
     bool coarse_keys;  // exact mode: the coarse scan pruned by tensor-core keys
     bool i8;          // the tensor-core form over the SQ8 codes (int8 x uint8 MMA) instead of BF16 rows
     bool shard;       // ANN_QUERY_SHARD: streams short of k are not widened to every row
@@ -1063,6 +1065,20 @@ static int ivf_tc_sampled(ann_ivf* h, ann_workspace* ws, const IvfQueryCfg& c, c
     return ANN_OK;
 }
 
+// The arrays of a small batch's set-up, within batched_scratch_bytes' room (its pair arrays and offsets are a subset);
+// b->total_items holds the number of pairs.
+static void small_setup_carve(void* scratch, int nq, int npc, IvfBatchArgs* b, TcSmallSetup* s) {
+    Carver cv(scratch);
+    s->pair_vals = cv.take<int32_t>((size_t)nq * npc);
+    s->pair_lists = cv.take<int32_t>((size_t)nq * npc);
+    s->cand_off = cv.take<int64_t>((size_t)nq + 1);
+    s->n_pairs = cv.take<int64_t>(1);
+    b->pair_vals = s->pair_vals;
+    b->pair_lists = s->pair_lists;
+    b->cand_off = s->cand_off;
+    b->total_items = s->n_pairs;
+}
+
 // All stages for nq device-resident padded queries; scratch carved from `base`.
 static int ivf_query_device(ann_ivf* h, ann_workspace* ws, const IvfQueryCfg& c, char* base, const float* qdev,
                             int nq, int64_t* ids_dev, float* dists_dev, cudaStream_t st) {
@@ -1200,7 +1216,7 @@ static int ivf_query_device(ann_ivf* h, ann_workspace* ws, const IvfQueryCfg& c,
         if ((rc = launch_lsh_candidates(la, st))) return rc;
         a.plan.cand_ids = cand;
         a.plan.cand_ld = c.ub_cand;
-    } else if ((rc = launch_ivf_plan(a, st))) {
+    } else if (!c.small_tc && (rc = launch_ivf_plan(a, st))) {
         return rc;
     }
     h->prof.mark(prec, st);
@@ -1243,7 +1259,15 @@ static int ivf_query_device(ann_ivf* h, ann_workspace* ws, const IvfQueryCfg& c,
                                   items_cap, keyR, idR, prec, ok, st);
         };
         bool sampled_done = false;
-        if ((rc = batched_prepare(a, bscratch, c.sort_tmp, c.scan_tmp, &b, tot, st, !sampled))) return rc;
+        if (c.small_tc) {  // no totals on the host: the streams' keys fit their bound
+            TcSmallSetup ss{};
+            small_setup_carve(bscratch, nq, c.npc, &b, &ss);
+            ss.total_items = titem + h->C;
+            ss.desc = titem_desc;
+            ss.cap = items_cap;
+            if ((rc = launch_tc_small_setup(a, ss, st))) return rc;
+            tot[1] = c.small_keys;
+        } else if ((rc = batched_prepare(a, bscratch, c.sort_tmp, c.scan_tmp, &b, tot, st, !sampled))) return rc;
         if (sampled && (rc = run_sampled(&sampled_done))) return rc;  // synchronises st: tot is current
         if (tot[2] != 0) sampled_done = false;
         if (plan_apart) every_row.resize((size_t)(int)tot[3]);  // the plan has listed them in every_list
@@ -1259,20 +1283,22 @@ static int ivf_query_device(ann_ivf* h, ann_workspace* ws, const IvfQueryCfg& c,
                 TcIvfSampleMaps maps;
                 maps.qfac = op.qfac;
                 maps.pfac = op.pfac;
-                if ((rc = launch_tc_ivf_pairs(op.qrows, op.row_bytes, b.pair_vals, b.pair_lists, b.lq_off + h->C,
-                                              max_pairs, c.npc, b.cand_off, a.plan.seg_pref, h->list_off, Apk, dbase,
-                                              st, maps)))
+                const int64_t* n_pairs = c.small_tc ? b.total_items : b.lq_off + h->C;
+                if ((rc = launch_tc_ivf_pairs(op.qrows, op.row_bytes, b.pair_vals, b.pair_lists, n_pairs, max_pairs, c.npc,
+                                              b.cand_off, a.plan.seg_pref, h->list_off, Apk, dbase, st, maps)))
                     return rc;
-                if ((rc = launch_tc_ivf_items(b.lq_off, h->list_off, h->C, titem, st))) return rc;
-                if ((rc = launch_tc_item_descs(titem, (int)h->C, b.lq_off, h->list_off, nullptr, titem_desc, items_cap,
-                                               st)))
-                    return rc;
+                if (!c.small_tc) {
+                    if ((rc = launch_tc_ivf_items(b.lq_off, h->list_off, h->C, titem, st))) return rc;
+                    if ((rc = launch_tc_item_descs(titem, (int)h->C, b.lq_off, h->list_off, nullptr, titem_desc,
+                                                   items_cap, st)))
+                        return rc;
+                }
                 TcGemmArgs g{(int)max_pairs, (int)h->n, op.K, nullptr, D, 0, h->d_err};
                 g.kind = op.kind;
                 g.col_fac = op.col_fac;
                 g.row_fac = op.pfac;
                 g.g_item_off = titem;
-                g.g_a_off = b.lq_off;
+                g.g_a_off = c.small_tc ? h->list_off : b.lq_off;  // (small: the descriptors alone are read)
                 g.g_b_off = h->list_off;
                 g.g_dbase = dbase;
                 g.g_total = titem + h->C;
@@ -1525,6 +1551,13 @@ int ann_ivf_query(ann_ivf* h, ann_workspace* ws, const float* queries, int32_t n
         c.rps_c = ceil_div(ceil_div(h->C, c.nsplit_c), 256) * 256;
         c.nsplit_c = (int)ceil_div(h->C, c.rps_c);
     }
+    // One CTA sets up a small tensor-core batch whose queries are sure to find k rows: up to 1,024 pairs and 64 MB of
+    // stream keys, sized by the largest lists. One query x 4 lists at 1M x 384: 154 us a call by the batch's ten
+    // launches and a wait for their totals, 110 us.
+    // (A cap below k could end a stream short of k after all.)
+    c.small_keys = (int64_t)qc * c.npc * h->sizes_desc[0];
+    c.small_tc = c.tc && nq < h->sampled_min_queries && !c.fallback && (c.shard || c.max_c >= k) &&
+                 (int64_t)qc * c.npc <= kSmallSetupPairs && c.small_keys <= ((int64_t)16 << 20);
     if (c.batched) c.bscratch = batched_scratch_bytes(qc, c.npc, h->C, &c.sort_tmp, &c.scan_tmp);
     Sizer head;
     head.take<float>((size_t)nq * dpad);

@@ -35,6 +35,19 @@ int launch_tc_ivf_items(const int64_t* lq_off, const int64_t* list_off, int C, i
 int launch_tc_item_lists(const int64_t* item_off, int C, int32_t* item_list, int64_t cap, cudaStream_t st);
 // Work items of a grouped batch at most: (pairs / 128 + C) x (largest list / 256 + 1).
 inline int64_t tc_items_bound(int64_t pairs, int C, int64_t largest) { return (pairs / 128 + C) * (largest / 256 + 1); }
+// Set-up of a small tensor-core batch (nq * npc <= kSmallSetupPairs, every query's lists known to hold k rows or more) by
+// one CTA: the plan (launch_ivf_plan), the pairs sorted by list, the candidate offsets and the work items' descriptors.
+constexpr int kSmallSetupPairs = 1024;
+struct TcSmallSetup {
+    int32_t* pair_vals;   // [nq * npc] as IvfBatchArgs
+    int32_t* pair_lists;
+    int64_t* n_pairs;     // [1]
+    int64_t* cand_off;    // [nq + 1]
+    int64_t* total_items; // [1]
+    int4* desc;           // [cap]
+    int64_t cap;
+};
+int launch_tc_small_setup(const IvfQueryArgs& a, const TcSmallSetup& s, cudaStream_t st);
 // For each valid pair i (< lq_off[C]; pairs grouped by list, pair_vals = q * npc + j, pair_lists = the
 // list): A[i] = qb[q] (kpad BF16 columns) and dbase[i] = cand_off[q] + seg_pref[q][j] - list_off[list],
 // the stream position of the list's row 0 in the candidate array.
