@@ -15,10 +15,12 @@
 //     passes its bar; survivors are queued per warp and go out 32 at a time (an atomic a survivor as it is met
 //     made each wait for the one before: 10,000 clocks a tile). The accumulator is released as soon as it is in
 //     registers.
-// Measured: 5,120 queries x 1M x 384 3.24 ms with no survivors, 0.38 us per 64 columns of K and a tile (1.63 PFLOP/s,
-// the measured BF16 burst) plus 0.5 us a tile, 3.48 ms with 1.2 survivors per 1,000 keys (3.48 ms before with the
-// survivors in 20 bytes each and two grouping kernels after it, 0.28 ms); E4M3, 5,000 queries x 4M x 256 6.5 ms from
-// 9.1 ms. Ring depth, chunk size and whether the query tile is resident change the BF16 time by under 1%.
+//   * the MMA issuer's loop is kept short (see there): at 66 instructions' latency a k-block it, not the tensor cores,
+//     set the rate.
+// Measured at 5,120 queries x 1M x 384: 2.48 ms with no survivors (1.65 PFLOP/s; 1.81 at K = 512, cuBLAS's measured burst
+// is 1.69), 2.65 ms with 1.2 survivors per 1,000 keys, where the plain tiling took 3.48 ms and grouped its survivors in
+// 0.28 ms more; E4M3 at dim 256 1.29 ms (2.04 PFLOP/s; 2.3 ms before, by the 4M-row case). With the first issue loop
+// 3.24 ms, and neither ring depth, chunk size nor residency of the query tile changed that by 1%.
 // Batches of up to 128 queries are bound by reading the base once and keep one CTA a tile (CG = 1).
 //
 //   warp 0      base-row producer (TMA, 128-byte swizzle);  warp 18: query-tile producer (resident form)
@@ -51,6 +53,7 @@ struct FilterShape {
     int nb;             // base tiles of a chunk
     int nst;            // ring stages
     int resident;       // the query tile stays in shared memory
+    int a_box;          // query rows copied a tile: 128, or the batch rounded up to 8 when smaller
 };
 
 __device__ __forceinline__ float min3f(float a, float b, float c) {
@@ -80,15 +83,18 @@ __device__ __forceinline__ void fi_tma(void* dst, const CUtensorMap* tm, int c0,
 }
 // Arrival on `bar` of every CTA of the tile once the MMAs issued so far are done.
 template <int CG>
-__device__ __forceinline__ void fi_commit(uint64_t* bar) {
+__device__ __forceinline__ void fi_commit_at(uint32_t bar) {
     if (CG == 2)
         asm volatile(
-            "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(
-                su32(bar)),
+            "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar),
             "h"((uint16_t)3)
             : "memory");
     else
-        mma_commit(bar);
+        mma_commit_at(bar);
+}
+template <int CG>
+__device__ __forceinline__ void fi_commit(uint64_t* bar) {
+    fi_commit_at<CG>(su32(bar));
 }
 __device__ __forceinline__ void cluster_sync() {
     asm volatile("barrier.cluster.arrive;" ::: "memory");
@@ -170,7 +176,7 @@ __global__ void __launch_bounds__(kFiThreads, 1) tc_filter_kernel(const __grid_c
     unsigned char* sQueue = reinterpret_cast<unsigned char*>(full) + 512;                  // [warps][kFiQueueBytes]
     float* sFac = reinterpret_cast<float*>(sQueue + kFiEpi * kFiQueueBytes);               // [warps][2][kFiCols]
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;  // warp: known uniform
     const int rank = CG == 2 ? (int)(blockIdx.x & 1) : 0;  // clusters are pairs of consecutive CTAs
     const int k_last = (a.K - (kt - 1) * kBlockK) / kMmaK;  // MMAs of the last k-block
 
@@ -212,7 +218,8 @@ __global__ void __launch_bounds__(kFiThreads, 1) tc_filter_kernel(const __grid_c
         if (lane == 0) {  // base rows (and, when not resident, the query rows of the same k-block)
             RingPos pos;
             bool ok = true;
-            const uint32_t bytes = CG * (kBSize + (resident ? 0 : kABytes));  // of both CTAs: one barrier counts them
+            const uint32_t a_bytes = (uint32_t)sh.a_box * kRowBytes;
+            const uint32_t bytes = CG * (kBSize + (resident ? 0u : a_bytes));  // of both CTAs: one barrier counts them
             while (ok && work.next()) {
                 const int arow = work.m * CG * kBM + rank * kBM;
                 const int brow = work.n * kBN * (SAMPLE ? a.b_tile_stride : 1) + rank * kBRows;
@@ -239,7 +246,7 @@ __global__ void __launch_bounds__(kFiThreads, 1) tc_filter_kernel(const __grid_c
                 if (!work.first) continue;
                 if (!(ok = bar_wait(aempty, (uint32_t)((run & 1) ^ 1), a.err, a.wait_ns))) break;
                 for (int kb = 0; kb < kt; ++kb) {
-                    if (rank == 0) bar_expect(&afull[kb], CG * kABytes);
+                    if (rank == 0) bar_expect(&afull[kb], CG * (uint32_t)sh.a_box * kRowBytes);
                     const uint32_t fb = CG == 2 ? leader_addr(&afull[kb]) : su32(&afull[kb]);
                     fi_tma<CG>(sA + (size_t)kb * kABytes, &tmA, kb * kBlockK, work.m * CG * kBM + rank * kBM, fb);
                 }
@@ -252,42 +259,60 @@ __global__ void __launch_bounds__(kFiThreads, 1) tc_filter_kernel(const __grid_c
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            if (rank == 0) {  // MMA issuer
-                int acc = 0, run = -1;
-                RingPos pos;
-                bool ok = true;
-                while (ok && work.next()) {
-                    const int b = (int)(acc & 1);
-                    if (work.first) ++run;
-                    if (!(ok = bar_wait(&tempty[b], (uint32_t)(((acc >> 1) & 1) ^ 1), a.err, a.wait_ns))) break;
+        if (rank == 0) {  // MMA issuer
+            // One thread issues 4 MMAs a k-block of 512 clocks between the epilogue warps of its scheduler, so its
+            // instructions count: the warp runs the loop as one (uniform registers feed the MMAs), one elected lane
+            // issues, and descriptors and barrier addresses are stepped, not made again. (Made again by a lone lane, a
+            // k-block took 750 clocks and a tile 1,000 more, whatever the operand kind.)
+            int acc = 0, run = -1;
+            RingPos pos;
+            bool ok = true;
+            const bool leader = elect_one();
+            const uint64_t da0 = sw128_desc(sA), db0 = sw128_desc(sB);
+            const uint32_t full_a = su32(full), empty_a = su32(empty), afull_a = su32(afull), tempty_a = su32(tempty);
+            constexpr int kMmas = kBlockK / kMmaK;
+            while (ok && work.next()) {
+                const int b = acc & 1;
+                if (work.first) ++run;
+                if (!(ok = bar_wait_warp(tempty_a + 8u * b, (uint32_t)(((acc >> 1) & 1) ^ 1), a.err, a.wait_ns))) break;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint32_t d = tmem + (uint32_t)(b * kBN);
+                const bool wait_a = resident && work.first;
+                uint64_t da = da0;  // resident: steps with kb
+                for (int kb = 0; kb < kt; ++kb) {
+                    const uint32_t s = (uint32_t)pos.s;
+                    if (wait_a && !(ok = bar_wait_warp(afull_a + 8u * kb, (uint32_t)(run & 1), a.err, a.wait_ns))) break;
+                    if (!(ok = bar_wait_warp(full_a + 8u * s, pos.ph, a.err, a.wait_ns))) break;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    const uint32_t d = tmem + (uint32_t)(b * kBN);
-                    for (int kb = 0; kb < kt; ++kb, pos.step(nst)) {
-                        const int s = pos.s;
-                        if (resident && work.first &&
-                            !(ok = bar_wait(&afull[kb], (uint32_t)(run & 1), a.err, a.wait_ns)))
-                            break;
-                        if (!(ok = bar_wait(&full[s], pos.ph, a.err, a.wait_ns))) break;
-                        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                        const unsigned char* pa = sA + (size_t)(resident ? kb : s) * kABytes;
-                        const unsigned char* pb = sB + (size_t)s * kBSize;
-                        const int nk = kb == kt - 1 ? k_last : kBlockK / kMmaK;
+                    const uint64_t ad = resident ? da : da0 + s * (uint32_t)(kABytes >> 4);
+                    const uint64_t bd = db0 + s * (uint32_t)(kBSize >> 4);
+                    if (leader) {
+                        if (kb + 1 < kt || k_last == kMmas) {
+                            mma_issue<KIND, CG>(d, ad, bd, kb ? 1u : 0u);
 #pragma unroll
-                        for (int k = 0; k < kBlockK / kMmaK; ++k)
-                            if (k < nk)
-                                mma_issue<KIND, CG>(d, sw128_desc(pa + k * 32), sw128_desc(pb + k * 32), (kb | k) ? 1u : 0u);
-                        fi_commit<CG>(&empty[s]);
+                            for (int k = 1; k < kMmas; ++k) mma_issue<KIND, CG>(d, ad + 2u * k, bd + 2u * k, 1u);
+                        } else {
+                            for (int k = 0; k < k_last; ++k)
+                                mma_issue<KIND, CG>(d, ad + 2u * k, bd + 2u * k, (kb | k) ? 1u : 0u);
+                        }
+                        fi_commit_at<CG>(empty_a + 8u * s);
                     }
-                    if (!ok) break;
+                    __syncwarp();
+                    da += (uint32_t)(kABytes >> 4);
+                    pos.step(nst);
+                }
+                if (!ok) break;
+                if (leader) {
                     if (resident && work.last) fi_commit<CG>(aempty);
                     fi_commit<CG>(&tfull[b]);
-                    ++acc;
                 }
-                fi_commit<CG>(done);
+                __syncwarp();
+                ++acc;
             }
-            bar_wait(done, 0, nullptr);  // every MMA issued has completed before TMEM is released
+            if (leader) fi_commit<CG>(done);
+            __syncwarp();
         }
+        bar_wait_warp(su32(done), 0, nullptr, 0);  // every MMA issued has completed before TMEM is released
     } else {  // epilogue
         const int lane_base = 32 * (warp & 3), ew = warp - 2;
         const int col0 = kFiCols * (ew >> 2);
@@ -477,17 +502,20 @@ int resident_clusters(const void* kern, int cg, size_t smem) {
 template <int KIND, int CG, bool SAMPLE>
 int run_filter(const void* A, const void* B, const TcFilterArgs& a, cudaStream_t st) {
     CUtensorMap tmA, tmB;
-    int rc = tc_make_map(&tmA, A, a.M, a.K, kBM, KIND);
+    FilterShape sh{};
+    // Rows past the batch are not copied (their products, of whatever the shared memory holds, meet NaN bars): a box that
+    // is mostly zero fill takes longer than the rows it holds (one query over 1M x 384: 152 us, 117 us for 128 queries).
+    sh.a_box = CG == 1 ? (int)std::min<int64_t>(kBM, ceil_div(a.M, 8) * 8) : kBM;
+    int rc = tc_make_map(&tmA, A, a.M, a.K, sh.a_box, KIND);
     if (rc) return rc;
     if ((rc = tc_make_map(&tmB, B, SAMPLE ? a.b_rows : a.N, a.K, kBN / CG, KIND))) return rc;
-    FilterShape sh{};
     sh.mt = (int)ceil_div(a.M, CG * kBM);
     sh.nt = (int)ceil_div(a.N, kBN);
     sh.kt = (int)ceil_div(a.K, KindOf<KIND>::kBlockK);
     const size_t fac = KIND == kTcBF16 ? 0 : (size_t)kFiEpi * 2 * kFiCols * 4;
     const size_t room = kFiSmemMax - kFiFixed - fac, bs = (size_t)kBN / CG * kRowBytes;
-    // the query tile stays where at least four ring stages fit beside it
-    sh.resident = sh.kt <= kFiMaxKt && (size_t)sh.kt * kABytes + 4 * bs <= room;
+    // the query tile stays where at least three (32 KB) or four (16 KB) ring stages fit beside it
+    sh.resident = sh.kt <= kFiMaxKt && (size_t)sh.kt * kABytes + (CG == 1 ? 3 : 4) * bs <= room;
     const size_t left = sh.resident ? room - (size_t)sh.kt * kABytes : room;
     sh.nst = (int)std::min<size_t>(kFiMaxStages, left / (bs + (sh.resident ? 0 : kABytes)));
     const size_t smem = kFiFixed + fac + (size_t)sh.nst * (bs + (sh.resident ? 0 : kABytes)) +

@@ -98,7 +98,7 @@ __global__ void __launch_bounds__(epi_threads(EPI), 1) tc_gemm_kernel(const __gr
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + 1);
     float* sT = reinterpret_cast<float*>(smem + kStages * (kABytes + kBBytes) + 256);  // [EPI warps][area]
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;  // warp: known uniform
     constexpr int kBlockK = KindOf<KIND>::kBlockK, kMmaK = KindOf<KIND>::kMmaK;
     const int mt = (int)ceil_div(a.M, kBM), nt = (int)ceil_div(a.N, kBN), kt = (int)ceil_div(a.K, kBlockK);
     const int k16_last = (a.K - (kt - 1) * kBlockK) / kMmaK;  // MMAs of the last k-block
@@ -163,35 +163,52 @@ __global__ void __launch_bounds__(epi_threads(EPI), 1) tc_gemm_kernel(const __gr
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {  // MMA issuer
-            int64_t it = 0, acc = 0;
-            bool ok = true;
-            for (int64_t t = blockIdx.x; t < tiles && ok; t += gridDim.x, ++acc) {
-                const int b = (int)(acc & 1);
-                const uint32_t aph = (uint32_t)((acc >> 1) & 1);
-                if (!(ok = bar_wait(&tempty[b], aph ^ 1u, a.err, a.wait_ns))) break;
+        // MMA issuer: the warp runs the loop as one and an elected lane issues, so that uniform registers feed the MMAs
+        // and descriptors and barrier addresses are stepped; the loop's instructions, issued between the epilogue warps'
+        // of the same scheduler, otherwise bound the MMA rate (tc_filter.cu)
+        int64_t acc = 0;
+        int s = 0;
+        uint32_t ph = 0;
+        bool ok = true;
+        const bool leader = elect_one();
+        const uint64_t da0 = sw128_desc(sA), db0 = sw128_desc(sB);
+        const uint32_t full_a = su32(full), empty_a = su32(empty), tempty_a = su32(tempty), tfull_a = su32(tfull);
+        constexpr int kMmas = kBlockK / kMmaK;
+        for (int64_t t = blockIdx.x; t < tiles && ok; t += gridDim.x, ++acc) {
+            const int b = (int)(acc & 1);
+            if (!(ok = bar_wait_warp(tempty_a + 8u * b, (uint32_t)(((acc >> 1) & 1) ^ 1), a.err, a.wait_ns))) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t d = tmem + (uint32_t)(b * kBN);
+            for (int kb = 0; kb < kt; ++kb) {
+                if (!(ok = bar_wait_warp(full_a + 8u * s, ph, a.err, a.wait_ns))) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t d = tmem + (uint32_t)(b * kBN);
-                for (int kb = 0; kb < kt; ++kb, ++it) {
-                    const int s = (int)(it % kStages);
-                    const uint32_t ph = (uint32_t)((it / kStages) & 1);
-                    if (!(ok = bar_wait(&full[s], ph, a.err, a.wait_ns))) break;
-                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint64_t ad = da0 + (uint32_t)s * (uint32_t)(kABytes >> 4);
+                const uint64_t bd = db0 + (uint32_t)s * (uint32_t)(kBBytes >> 4);
+                if (leader) {
                     // the last k-block's box runs past K (zero fill); its zero columns are not multiplied
-                    const int n16 = kb == kt - 1 ? k16_last : kBlockK / kMmaK;
+                    if (kb + 1 < kt || k16_last == kMmas) {
+                        mma_issue<KIND>(d, ad, bd, kb ? 1u : 0u);
 #pragma unroll
-                    for (int k16 = 0; k16 < kBlockK / kMmaK; ++k16)
-                        if (k16 < n16)
-                            mma_issue<KIND>(d, sw128_desc(sA + s * kABytes + k16 * 32),
-                                            sw128_desc(sB + s * kBBytes + k16 * 32), (kb | k16) ? 1u : 0u);
-                    mma_commit(&empty[s]);
+                        for (int k = 1; k < kMmas; ++k) mma_issue<KIND>(d, ad + 2u * k, bd + 2u * k, 1u);
+                    } else {
+                        for (int k = 0; k < k16_last; ++k)
+                            mma_issue<KIND>(d, ad + 2u * k, bd + 2u * k, (kb | k) ? 1u : 0u);
+                    }
+                    mma_commit_at(empty_a + 8u * s);
                 }
-                mma_commit(&tfull[b]);
+                __syncwarp();
+                if (++s == kStages) {
+                    s = 0;
+                    ph ^= 1u;
+                }
             }
-            // every MMA issued has completed before TMEM is released
-            mma_commit(done);
-            bar_wait(done, 0, nullptr);
+            if (leader) mma_commit_at(tfull_a + 8u * b);
+            __syncwarp();
         }
+        // every MMA issued has completed before TMEM is released
+        if (leader) mma_commit(done);
+        __syncwarp();
+        bar_wait_warp(su32(done), 0, nullptr, 0);
     } else {  // epilogue warps 2..9
         const int lane_base = 32 * (warp & 3);
         const int ew = warp - 2;

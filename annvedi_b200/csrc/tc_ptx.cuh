@@ -58,6 +58,15 @@ __device__ __forceinline__ bool bar_try_sleep(uint64_t* b, uint32_t parity) {
         : "memory");
     return ok != 0;
 }
+// bar_wait by shared-memory address (for loops that step it).
+__device__ __forceinline__ bool bar_try_at(uint32_t b, uint32_t parity) {
+    uint32_t ok;
+    asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
+                 : "=r"(ok)
+                 : "r"(b), "r"(parity)
+                 : "memory");
+    return ok != 0;
+}
 // Waits for the phase; gives up after `limit_ns` (2 s when 0), sets *err = 2 and returns false.
 __device__ __forceinline__ bool bar_wait(uint64_t* b, uint32_t parity, int* err, uint64_t limit_ns = 0) {
     if (bar_try(b, parity)) return true;
@@ -65,6 +74,18 @@ __device__ __forceinline__ bool bar_wait(uint64_t* b, uint32_t parity, int* err,
     const uint64_t t0 = gtimer();
     while (!bar_try_sleep(b, parity))
         if (gtimer() - t0 > limit) {
+            if (err) atomicExch(err, 2);
+            return false;
+        }
+    return true;
+}
+// The whole (converged) warp waits; every lane gets the same answer.
+__device__ __forceinline__ bool bar_wait_warp(uint32_t b, uint32_t parity, int* err, uint64_t limit_ns) {
+    if (__all_sync(0xffffffffu, bar_try_at(b, parity))) return true;
+    const uint64_t limit = limit_ns ? limit_ns : 2000000000ull;
+    const uint64_t t0 = gtimer();
+    while (!__all_sync(0xffffffffu, bar_try_at(b, parity)))
+        if (__any_sync(0xffffffffu, gtimer() - t0 > limit)) {
             if (err) atomicExch(err, 2);
             return false;
         }
@@ -107,49 +128,42 @@ constexpr uint32_t kIdescI8 = (2u << 4) | ((uint32_t)(kBN >> 3) << 17) | ((uint3
 
 // One MMA of the 32 bytes of K that follow each descriptor's start: 16 BF16 or 32 E4M3 elements. CG = 2: both CTAs of
 // the pair take part, each with its 128 rows of A, its half of B's rows and the accumulator rows of its A.
+#define ANN_MMA(cg, kind, idesc)                                                  \
+    asm volatile(                                                                 \
+        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"                             \
+        " tcgen05.mma.cta_group::" cg ".kind::" kind " [%0], %1, %2, %3, p;\n}" ::"r"(tmem_d), \
+        "l"(ad), "l"(bd), "r"(idesc), "r"(accumulate)                             \
+        : "memory")
 template <int KIND, int CG = 1>
 __device__ __forceinline__ void mma_issue(uint32_t tmem_d, uint64_t ad, uint64_t bd, uint32_t accumulate) {
     static_assert(KIND != kTcI8 || CG == 1, "int8 operands: one CTA");
-    if (KIND == kTcBF16 && CG == 1)
-        asm volatile(
-            "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-            " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}" ::"r"(tmem_d),
-            "l"(ad), "l"(bd), "r"(kIdescBF16<1>), "r"(accumulate)
-            : "memory");
-    else if (KIND == kTcBF16)
-        asm volatile(
-            "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-            " tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n}" ::"r"(tmem_d),
-            "l"(ad), "l"(bd), "r"(kIdescBF16<2>), "r"(accumulate)
-            : "memory");
-    else if (KIND == kTcE4M3 && CG == 1)
-        asm volatile(
-            "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-            " tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n}" ::"r"(tmem_d),
-            "l"(ad), "l"(bd), "r"(kIdescE4M3<1>), "r"(accumulate)
-            : "memory");
-    else if (KIND == kTcE4M3)
-        asm volatile(
-            "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-            " tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], %1, %2, %3, p;\n}" ::"r"(tmem_d),
-            "l"(ad), "l"(bd), "r"(kIdescE4M3<2>), "r"(accumulate)
-            : "memory");
+    if constexpr (KIND == kTcBF16 && CG == 1)
+        ANN_MMA("1", "f16", kIdescBF16<1>);
+    else if constexpr (KIND == kTcBF16)
+        ANN_MMA("2", "f16", kIdescBF16<2>);
+    else if constexpr (KIND == kTcE4M3 && CG == 1)
+        ANN_MMA("1", "f8f6f4", kIdescE4M3<1>);
+    else if constexpr (KIND == kTcE4M3)
+        ANN_MMA("2", "f8f6f4", kIdescE4M3<2>);
     else
-        asm volatile(
-            "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-            " tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n}" ::"r"(tmem_d),
-            "l"(ad), "l"(bd), "r"(kIdescI8), "r"(accumulate)
-            : "memory");
+        ANN_MMA("1", "i8", kIdescI8);
+}
+#undef ANN_MMA
+// One lane of the (converged) warp, the same at every call.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t ok;
+    asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}" : "=r"(ok));
+    return ok != 0;
 }
 // An accumulator read from TMEM as a float: FP32 bits, or (kind::i8) an int32 converted (exact below 2^24).
 template <int KIND>
 __device__ __forceinline__ float acc_value(uint32_t r) {
     return KIND == kTcI8 ? __int2float_rn((int)r) : __uint_as_float(r);
 }
-__device__ __forceinline__ void mma_commit(uint64_t* bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(su32(bar))
-                 : "memory");
+__device__ __forceinline__ void mma_commit_at(uint32_t bar) {
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
+__device__ __forceinline__ void mma_commit(uint64_t* bar) { mma_commit_at(su32(bar)); }
 // tcgen05.ld of 32 consecutive columns of the warp's 32 lanes; the registers are valid only after
 // tmem_wait (which names them, so no use is scheduled before the wait).
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
