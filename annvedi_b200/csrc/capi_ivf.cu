@@ -20,6 +20,7 @@
 #include "ivf.cuh"
 #include "ivf_batched.cuh"
 #include "ivf_lsh.cuh"
+#include "ivf_prune.cuh"
 #include "radix_select.cuh"
 #include "refmath.cuh"
 #include "runtime.cuh"
@@ -59,6 +60,13 @@ struct ann_ivf {
     float2* sq8_fac = nullptr;           // [n] (1, reconstructed |x|^2) of the SQ8 rows (codes on the tensor cores)
     int kpad = 0;
     PruneBounds cent_bounds;             // of the centroids' norms (the coarse ranking's key error bound)
+    // the pruned exact selection (ivf_prune.cu): the codes' FP16 operand rows, the bound of their norms (0: the keys'
+    // error bound does not cover these rows), their scale and the time that pruned calls are estimated to save, in us
+    __half* code_f16 = nullptr;
+    float code_cmax = 0.f, code_g = 1.f;
+    bool codes_known = false;
+    double prune_credit_us = 0.0;
+    int prune_failed = 0;  // batches in a row that it could not settle
     std::mutex tc_mu;
     int64_t query_count = 0;
     // query options (ann_ivf_set_option)
@@ -86,11 +94,16 @@ struct ann_ivf {
 static void ivf_free_state(ann_ivf* h) {
     for (void* p : {(void*)h->centroids, (void*)h->original, (void*)h->codes, (void*)h->scale, (void*)h->offset,
                     (void*)h->r2o, (void*)h->list_off, (void*)h->base_bf16, (void*)h->cent_bf16, (void*)h->proj,
-                    (void*)h->projT, (void*)h->lsh_mean, (void*)h->tab_off, (void*)h->tab_ids, (void*)h->sq8_fac})
+                    (void*)h->projT, (void*)h->lsh_mean, (void*)h->tab_off, (void*)h->tab_ids, (void*)h->sq8_fac, (void*)h->code_f16})
         if (p) cudaFree(p);
     h->base_bf16 = nullptr;
     h->cent_bf16 = nullptr;
     h->cent_bounds = PruneBounds{};
+    h->code_f16 = nullptr;
+    h->code_cmax = 0.f;
+    h->codes_known = false;
+    h->prune_failed = 0;
+    h->prune_credit_us = 0.0;
     h->sq8_fac = nullptr;
     h->proj = h->projT = h->lsh_mean = nullptr;
     h->tab_off = nullptr;
@@ -787,6 +800,8 @@ struct IvfQueryCfg {
     bool ref, coarse_flat, batched, tc, lsh;
     bool small_tc;     // a small tensor-core batch, set up by one CTA without a host round trip
     bool coarse_keys;  // exact mode: the coarse scan pruned by tensor-core keys
+    double saved_us;   // by a pruned selection, estimated
+    bool pruned;       // exact mode: the SQ8 selection pruned by tensor-core keys
     bool i8;          // the tensor-core form over the SQ8 codes (int8 x uint8 MMA) instead of BF16 rows
     bool shard;       // ANN_QUERY_SHARD: streams short of k are not widened to every row
     bool fallback;    // a query's stream can fall short of k points and become every row
@@ -868,6 +883,66 @@ static int ivf_ensure_tc(ann_ivf* h, bool i8, cudaStream_t st) {
     return ANN_OK;
 }
 
+// The codes' operand rows for the pruned exact selection, laid out by the call that brings the estimated savings of
+// the calls so far (saved_us for this one) to its cost, as the linear index's copy (flat_ensure_pruned). A batch that
+// the selection could not settle ran both passes: the next 16 take the batched pass alone (ivf_prune_settled; the
+// credit goes below zero and each of them adds its estimate), then 32, up to 1,024. *ok = false (and no error) where this call does.
+static int ivf_ensure_codes(ann_ivf* h, double saved_us, cudaStream_t st, bool* ok) {
+    *ok = false;
+    std::lock_guard<std::mutex> lk(h->tc_mu);
+    if (!h->codes_known) {
+        h->prune_credit_us += saved_us;
+        const int kpad = tc_kpad(h->dim, ANN_METRIC_L2);
+        if (h->prune_credit_us < 500.0 + 1.5e-6 * (double)h->n * h->dim) return ANN_OK;
+        size_t mfree = 0, mtotal = 0;
+        ANN_CUDA_TRY(cudaMemGetInfo(&mfree, &mtotal));
+        const size_t bytes = (sizeof(__nv_bfloat16) * (size_t)h->n * kpad + 255) / 256 * 256;
+        if (bytes > mfree / 2) return ANN_OK;
+        char* cb = nullptr;  // the operand rows, then a word for their largest norm
+        if (cudaMalloc(&cb, bytes + 256) != cudaSuccess) {
+            cudaGetLastError();
+            return ANN_OK;
+        }
+        unsigned* d2 = reinterpret_cast<unsigned*>(cb + bytes);
+        unsigned h2 = 0;
+        int rc = launch_sq8_max_norm(h->view(), d2, st);
+        cudaError_t e = cudaSuccess;
+        if (!rc) e = cudaMemcpyAsync(&h2, d2, sizeof(h2), cudaMemcpyDeviceToHost, st);
+        if (!rc && e == cudaSuccess) e = cudaStreamSynchronize(st);
+        float s2;
+        memcpy(&s2, &h2, 4);
+        const float c = std::sqrt(s2);
+        const bool covered = !rc && e == cudaSuccess && c >= kPruneNormMin && c <= kPruneNormMax;
+        if (covered) {
+            h->code_g = std::exp2(-std::floor(std::log2(c)));
+            rc = launch_sq8_operand(h->view(), h->code_g, reinterpret_cast<__half*>(cb), kpad, st);
+            if (!rc) e = cudaStreamSynchronize(st);
+        }
+        if (rc || e != cudaSuccess || !covered) cudaFree(cb);
+        if (rc) return rc;
+        if (e != cudaSuccess) {
+            set_error("pruned SQ8 selection: %s", cudaGetErrorString(e));
+            return ANN_ERR_CUDA;
+        }
+        if (covered) {
+            h->code_f16 = reinterpret_cast<__half*>(cb);
+            h->code_cmax = c * 1.001f;
+        }
+        h->prune_credit_us = 0.0;
+        h->codes_known = true;
+    }
+    if (h->prune_credit_us < 0.0)
+        h->prune_credit_us += saved_us;
+    else
+        *ok = h->code_cmax > 0.f;
+    return ANN_OK;
+}
+static void ivf_prune_settled(ann_ivf* h, bool settled, double saved_us) {
+    std::lock_guard<std::mutex> lk(h->tc_mu);
+    if (!settled) h->prune_credit_us = -16.0 * saved_us * (1 << std::min(h->prune_failed, 6));
+    h->prune_failed = settled ? 0 : h->prune_failed + 1;
+}
+
 // Operand rows of the pairs: BF16 (kpad columns) or int8 weights (dpad8 bytes).
 static int64_t tc_pair_row_bytes(const ann_ivf* h) {
     return std::max<int64_t>(2 * (int64_t)tc_kpad(h->dim, ANN_METRIC_L2), h->dpad8);
@@ -937,6 +1012,9 @@ static size_t ivf_scratch(const ann_ivf* h, const IvfQueryCfg& c, int nq) {
 // (warp_select_kernel: the keys below the R-th, then equal ones by increasing row), as the key-stream path
 // selects them, without writing the stream. Returns with *done = false (and no output) when a query's
 // buffer overflowed.
+// pruned: the exact selection of ivf_prune.cu by the same passes -- one bar per query, of the rank that leaves fewer than
+// R keys at or below it once in 10^7 queries, plus the keys' window, no second filter pass, and the survivors' SQ8
+// distances in place of the selection by key; *done = false where that leaves a query.
 struct TcOperands {
     const void* qrows;     // the queries' operand rows
     int row_bytes;
@@ -961,7 +1039,7 @@ constexpr int kRowCapFactor = 16;
 static int ivf_tc_sampled(ann_ivf* h, ann_workspace* ws, const IvfQueryCfg& c, const IvfQueryArgs& a,
                           const IvfBatchArgs& b, const TcOperands& op, unsigned char* Apk, int64_t* titem,
                           int4* titem_desc, int64_t items_cap, float* keyR, int* idR, int prec, bool* done,
-                          cudaStream_t st) {
+                          cudaStream_t st, bool pruned = false) {
     *done = false;
     const int nq = a.plan.nq, npc = c.npc, C = (int)h->C, R = c.R;
     const int64_t max_pairs = (int64_t)nq * npc;
@@ -970,8 +1048,9 @@ static int ivf_tc_sampled(ann_ivf* h, ann_workspace* ws, const IvfQueryCfg& c, c
     const int64_t head_max = ceil_div(largest, div);
     const int64_t s_bound = (int64_t)nq * npc * head_max;  // sample keys at most
     const int64_t scap = tc_items_bound(max_pairs, C, head_max);
-    const int rF = (int)std::min<int64_t>(R, std::max<int64_t>(1, ceil_div(3 * (int64_t)R, div)));
-    const int cap = kRowCapFactor * R;
+    const int rF = pruned ? prune_bar_rank(R, ((int64_t)1 << 24) / div, (int64_t)1 << 24)
+                          : (int)std::min<int64_t>(R, std::max<int64_t>(1, ceil_div(3 * (int64_t)R, div)));
+    const int cap = pruned ? ivf_prune_cap(R) : kRowCapFactor * R;
     size_t scan_tmp = 0;
     ANN_CUDA_TRY(cub::DeviceScan::ExclusiveSum(nullptr, scan_tmp, (int64_t*)nullptr, (int64_t*)nullptr, nq + 1, st));
     Sizer sz;
@@ -990,6 +1069,13 @@ static int ivf_tc_sampled(ann_ivf* h, ann_workspace* ws, const IvfQueryCfg& c, c
     sz.take<int>((size_t)nq * cap);
     for (int i = 0; i < 3; ++i) sz.take<int>((size_t)nq);    // counts, re-run list, marks
     sz.take<int>(4);                             // flags
+    if (pruned) {  // what the tensor-core form carves beside this
+        sz.take<__half>((size_t)nq * op.K);
+        sz.take<float2>((size_t)nq);
+        sz.take<unsigned char>((size_t)max_pairs * op.row_bytes);
+        sz.take<int64_t>((size_t)C + 1);
+        sz.take<int4>((size_t)items_cap);
+    }
     int rc = ws_reserve_big(ws, sz.bytes());
     if (rc) return rc;
     Carver cv(ws->big);
@@ -1012,6 +1098,34 @@ static int ivf_tc_sampled(ann_ivf* h, ann_workspace* ws, const IvfQueryCfg& c, c
     int* list = cv.take<int>((size_t)nq);
     int* mark = cv.take<int>((size_t)nq);
     int* flags = cv.take<int>(4);
+    IvfPruneArgs pa{};
+    const void* qrows = op.qrows;
+    if (pruned) {
+        pa.ix = a.ix;
+        pa.plan = a.plan;
+        pa.q = a.q;
+        pa.ldq = a.ldq;
+        pa.R = R;
+        pa.cmax = h->code_cmax;
+        pa.g = h->code_g;
+        pa.qop = cv.take<__half>((size_t)nq * op.K);
+        pa.kpad = op.K;
+        pa.win = cv.take<float2>((size_t)nq);
+        pa.tauF = tauF;
+        pa.tauX = tauR;
+        pa.cap = cap;
+        pa.fkey = skey;
+        pa.frow = srow;
+        pa.rcount = scount;
+        pa.fails = flags;
+        pa.keyR = keyR;
+        pa.idR = idR;
+        Apk = cv.take<unsigned char>((size_t)max_pairs * op.row_bytes);
+        titem = cv.take<int64_t>((size_t)C + 1);
+        titem_desc = cv.take<int4>((size_t)items_cap);
+        if ((rc = launch_ivf_prune_queries(pa, st))) return rc;
+        qrows = pa.qop;
+    }
 
     // sample streams: heads of the probed lists, each query's stream offsets
     if ((rc = launch_tc_ivf_sample_plan(a.plan, h->list_off, C, div, lcap, sseg, slen, st))) return rc;
@@ -1025,7 +1139,7 @@ static int ivf_tc_sampled(ann_ivf* h, ann_workspace* ws, const IvfQueryCfg& c, c
     maps.sdbase = sdbase;
     maps.qfac = op.qfac;
     maps.pfac = op.pfac;
-    if ((rc = launch_tc_ivf_pairs(op.qrows, op.row_bytes, b.pair_vals, b.pair_lists, b.lq_off + C, max_pairs, npc,
+    if ((rc = launch_tc_ivf_pairs(qrows, op.row_bytes, b.pair_vals, b.pair_lists, b.lq_off + C, max_pairs, npc,
                                   b.cand_off, a.plan.seg_pref, h->list_off, Apk, nullptr, st, maps)))
         return rc;
     // 1. sample pass: keys of the list heads into the sample streams; the two bars per query
@@ -1045,7 +1159,9 @@ static int ivf_tc_sampled(ann_ivf* h, ann_workspace* ws, const IvfQueryCfg& c, c
     gs.g_item_desc = sitem_desc;
     if ((rc = launch_tc_gemm(Apk, op.B, gs, st))) return rc;
     int kt = h->prof.kbegin(st);
-    if ((rc = launch_warp_bars(SK, soff, slen, nq, rF, R, tauF, tauS, st, (int64_t)npc * head_max))) return rc;
+    if ((rc = launch_warp_bars(SK, soff, slen, nq, rF, pruned ? rF : R, tauF, pruned ? tauR : tauS, st,
+                               (int64_t)npc * head_max)))
+        return rc;
     h->prof.kend(kt, kKernBars, st);
     // 2. filter pass over every row of the probed lists into the queries' buffers
     if ((rc = launch_tc_ivf_items(b.lq_off, h->list_off, C, titem, st))) return rc;
@@ -1073,6 +1189,19 @@ static int ivf_tc_sampled(ann_ivf* h, ann_workspace* ws, const IvfQueryCfg& c, c
         h->prof.kend(k0, kKernKeys, st);
         return r;
     };
+    if (pruned) {
+        if ((rc = launch_ivf_prune_bars(pa, st))) return rc;
+        if ((rc = filter(pa.tauX, nullptr))) return rc;
+        h->prof.mark(prec, st);
+        kt = h->prof.kbegin(st);
+        if ((rc = launch_ivf_prune_finish(pa, st))) return rc;
+        h->prof.kend(kt, kKernSelect, st);
+        int fails = 0;
+        ANN_CUDA_TRY(cudaMemcpyAsync(&fails, pa.fails, sizeof(int), cudaMemcpyDeviceToHost, st));
+        ANN_CUDA_TRY(cudaStreamSynchronize(st));
+        *done = fails == 0;
+        return ANN_OK;
+    }
     ANN_CUDA_TRY(cudaMemsetAsync(scount, 0, sizeof(int) * (size_t)nq, st));
     if ((rc = filter(tauF, nullptr))) return rc;
     h->prof.mark(prec, st);
@@ -1281,12 +1410,25 @@ static int ivf_query_device(ann_ivf* h, ann_workspace* ws, const IvfQueryCfg& c,
         int64_t* tot = tot_local;
         // The sampled path needs none of the set-up's totals to run: they land in page-locked words and are read
         // after its own synchronisation.
-        const bool sampled = c.tc && nq >= h->sampled_min_queries;
+        const bool sampled = c.pruned || (c.tc && nq >= h->sampled_min_queries);
         if (sampled && (rc = ws_pinned(ws, &tot))) return rc;
         tot[0] = tot[1] = tot[2] = tot[3] = 0;
         if (plan_apart)
             ANN_CUDA_TRY(cudaMemcpyAsync(&tot[3], apart_count, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
         auto run_sampled = [&](bool* ok) -> int {
+            if (c.pruned) {
+                const int kpad = tc_kpad(h->dim, ANN_METRIC_L2);
+                const TcOperands op{nullptr, 2 * kpad, h->code_f16, kpad, kTcF16, nullptr, nullptr, nullptr};
+                const int64_t cap = tc_items_bound((int64_t)nq * c.npc, (int)h->C, h->sizes_desc[0]);
+                int r = ivf_tc_sampled(h, ws, c, a, b, op, nullptr, nullptr, nullptr, cap, keyR, idR, prec, ok, st, true);
+                if (r == ANN_ERR_NOMEM) {  // the batched pass may need less
+                    clear_error();
+                    r = ANN_OK;
+                    ANN_CUDA_TRY(cudaStreamSynchronize(st));
+                }
+                if (!r) ivf_prune_settled(h, *ok, c.saved_us);
+                return r;
+            }
             return ivf_tc_sampled(h, ws, c, a, b, tc_operands(h, c, qb, q8, qfac, pfac), Apk, titem, titem_desc,
                                   items_cap, keyR, idR, prec, ok, st);
         };
@@ -1562,6 +1704,20 @@ int ann_ivf_query(ann_ivf* h, ann_workspace* ws, const float* queries, int32_t n
         else
             c.coarse_keys = h->cent_bounds.cmax >= kPruneNormMin && h->cent_bounds.cmax <= kPruneNormMax;
     }
+    // The exact form's SQ8 selection by keys, where it is estimated to save 60 us: it takes the sum of every candidate
+    // off the FP32 units (1.3e-7 us a term at 1M x 384, of lists of the mean size), and adds its launches (60 us) and
+    // the distances formed apart (1.4e-4 us each of nq R). Measured, every distance / by keys, us a call: 1M x 384, 8 of
+    // 2,048 lists: 777 / 570 (1,000 queries, R = 100), 1130 / 933 (2,000, R = 400), 1726 / 988 (5,000, R = 100), and
+    // 2068 / 1008 (2,000, R = 400, list sizes by a power law); 2 probed: 1044 / 932 (5,000, R = 100), 770 / 848 (2,000,
+    // R = 400: not taken); 500k x 768, 8 of 1,024: 1844 / 938 (2,000, R = 100); 200k x 96, 8 of 512: 642 / 583 (5,000,
+    // R = 100), 402 / 442 (2,000: not taken).
+    const int64_t pairs = (int64_t)nq * c.npc;
+    c.saved_us = 1.3e-7 * (double)pairs * ((double)h->n / h->C) * h->dim - 60.0 - 1.4e-4 * (double)nq * c.R;
+    if (!c.ref && !c.tc && c.batched && c.saved_us >= 60.0 && ivf_prune_fits(c.R, c.npc, h->dpad8) &&
+        pairs * tc_kpad(h->dim, ANN_METRIC_L2) <= (int64_t)1 << 29 && pairs * ceil_div(h->sizes_desc[0], h->sample_div) <= (int64_t)1 << 28 &&
+        (int64_t)nq * ivf_prune_cap(c.R) <= (int64_t)1 << 27 &&
+        (rc0 = ivf_ensure_codes(h, c.saved_us, st, &c.pruned)))
+        return rc0;
     const int dpad = h->dpad;
     const bool host = mem == ANN_MEM_HOST;
 

@@ -501,12 +501,14 @@ int tc_make_map(CUtensorMap* tm, const void* base, int64_t rows, int cols, int b
         return ANN_ERR_CUDA;
     }
     const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
-    const int esize = kind == kTcBF16 ? 2 : 1;
+    const int esize = tc_16bit(kind) ? 2 : 1;
     const cuuint64_t strides[1] = {(cuuint64_t)cols * esize};
     const cuuint32_t box[2] = {(cuuint32_t)(kRowBytes / esize), (cuuint32_t)box_rows};
     const cuuint32_t estr[2] = {1, 1};
-    const CUresult r = fn(tm, kind == kTcBF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_UINT8, 2,
-                          const_cast<void*>(base), dims, strides, box, estr,
+    const CUtensorMapDataType type = kind == kTcBF16  ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16
+                                     : kind == kTcF16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16
+                                                      : CU_TENSOR_MAP_DATA_TYPE_UINT8;
+    const CUresult r = fn(tm, type, 2, const_cast<void*>(base), dims, strides, box, estr,
                           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) {
@@ -532,11 +534,11 @@ static cudaError_t run_tc_gemm(const CUtensorMap& tmA, const CUtensorMap& tmB, c
 }
 
 int launch_tc_gemm(const void* A, const void* B, const TcGemmArgs& a, cudaStream_t st) {
-    const int step = a.kind == kTcBF16 ? 16 : 32;
-    ANN_CHECK_ARG(a.kind == kTcBF16 || a.kind == kTcE4M3 || a.kind == kTcI8, "tensor-core scan: element kind %d",
-                  a.kind);
+    const int step = tc_16bit(a.kind) ? 16 : 32;
+    ANN_CHECK_ARG(tc_16bit(a.kind) || a.kind == kTcE4M3 || a.kind == kTcI8, "tensor-core scan: element kind %d", a.kind);
+    ANN_CHECK_ARG(a.kind != kTcF16 || a.g_item_off, "tensor-core scan: FP16 operands are grouped");
     ANN_CHECK_ARG(a.K % step == 0 && a.K > 0, "tensor-core scan: K=%d not a positive multiple of %d", a.K, step);
-    ANN_CHECK_ARG(a.kind == kTcBF16 || (a.col_fac && a.row_fac && (a.g_item_off == nullptr || a.kind == kTcI8)),
+    ANN_CHECK_ARG(tc_16bit(a.kind) || (a.col_fac && a.row_fac && (a.g_item_off == nullptr || a.kind == kTcI8)),
                   "tensor-core scan: E4M3 / I8 operands need their scale factors (E4M3: no grouping)");
     ANN_CHECK_ARG((reinterpret_cast<uintptr_t>(A) & 15) == 0 && (reinterpret_cast<uintptr_t>(B) & 15) == 0,
                   "tensor-core scan: operands must be 16-byte aligned");
@@ -565,6 +567,9 @@ int launch_tc_gemm(const void* A, const void* B, const TcGemmArgs& a, cudaStream
     if (a.kind == kTcBF16)
         e = filter ? run_tc_gemm<kTcBF16, kFilterEpi>(tmA, tmB, a, grid, st)
                    : run_tc_gemm<kTcBF16, kKeyEpi>(tmA, tmB, a, grid, st);
+    else if (a.kind == kTcF16)
+        e = filter ? run_tc_gemm<kTcF16, kFilterEpi>(tmA, tmB, a, grid, st)
+                   : run_tc_gemm<kTcF16, kKeyEpi>(tmA, tmB, a, grid, st);
     else if (a.kind == kTcE4M3)
         e = run_tc_gemm<kTcE4M3, kKeyEpi>(tmA, tmB, a, grid, st);
     else

@@ -13,7 +13,9 @@ namespace annb {
 // Smaller keys are better in both metrics.
 // kTcI8: A int8, B uint8 (tcgen05.mma.kind::i8, exact int32 accumulation): the SQ8 codes of an IVF index as
 // they are stored, against an int8 query weight; the key is col_fac[n].y + col_fac[n].x * row_fac[m] * acc.
-enum TcKind { kTcBF16 = 0, kTcE4M3 = 1, kTcI8 = 2 };
+// kTcF16: A and B FP16, otherwise as BF16 (grouped modes).
+enum TcKind { kTcBF16 = 0, kTcE4M3 = 1, kTcI8 = 2, kTcF16 = 3 };
+constexpr bool tc_16bit(int kind) { return kind == kTcBF16 || kind == kTcF16; }
 
 struct TcGemmArgs {
     int M, N, K;           // A [M, K], B [N, K] BF16 row-major; K a multiple of 16

@@ -13,15 +13,15 @@ int tc_make_map(CUtensorMap* tm, const void* base, int64_t rows, int cols, int b
 
 namespace {
 
-// A k-block is one 128-byte row per operand row: 64 BF16 or 128 E4M3 elements.
+// A k-block is one 128-byte row per operand row: 64 BF16 / FP16 or 128 E4M3 elements.
 constexpr int kBM = 128, kBN = 256, kBK = 64;
 constexpr int kRowBytes = 128;
 constexpr int kABytes = kBM * kRowBytes;  // 16 KB
 constexpr int kBBytes = kBN * kRowBytes;  // 32 KB
 template <int KIND>
 struct KindOf {
-    static constexpr int kBlockK = KIND == kTcBF16 ? 64 : 128;  // elements per k-block
-    static constexpr int kMmaK = KIND == kTcBF16 ? 16 : 32;     // elements per MMA
+    static constexpr int kBlockK = tc_16bit(KIND) ? 64 : 128;  // elements per k-block
+    static constexpr int kMmaK = tc_16bit(KIND) ? 16 : 32;     // elements per MMA
 };
 constexpr int kTmemCols = 512;
 
@@ -114,8 +114,8 @@ __device__ __forceinline__ uint64_t sw128_desc(const void* p) {
     return addr | (1ull << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
 }
 // Instruction descriptors: FP32 accumulator (bits 4-5 = 1), A and B K-major, N = 256 (bits 17-22 = N / 8),
-// M = 128 (bits 24-28 = M / 16); A and B types in bits 7-9 and 10-12: BF16 = 1 under kind::f16, E4M3 = 0
-// under kind::f8f6f4.
+// M = 128 (bits 24-28 = M / 16); A and B types in bits 7-9 and 10-12: BF16 = 1 and FP16 = 0 under kind::f16,
+// E4M3 = 0 under kind::f8f6f4.
 // (CG = 2, two CTAs a tile: M = 256)
 template <int CG>
 constexpr uint32_t kIdescShape = (1u << 4) | ((uint32_t)(kBN >> 3) << 17) | ((uint32_t)(CG * kBM >> 4) << 24);
@@ -123,6 +123,7 @@ template <int CG>
 constexpr uint32_t kIdescBF16 = kIdescShape<CG> | (1u << 7) | (1u << 10);
 template <int CG>
 constexpr uint32_t kIdescE4M3 = kIdescShape<CG>;
+constexpr uint32_t kIdescF16 = kIdescShape<1>;
 // kind::i8: S32 accumulator (bits 4-5 = 2), A signed (bits 7-9 = 1), B unsigned (bits 10-12 = 0)
 constexpr uint32_t kIdescI8 = (2u << 4) | ((uint32_t)(kBN >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24) | (1u << 7);
 
@@ -136,7 +137,7 @@ constexpr uint32_t kIdescI8 = (2u << 4) | ((uint32_t)(kBN >> 3) << 17) | ((uint3
         : "memory")
 template <int KIND, int CG = 1>
 __device__ __forceinline__ void mma_issue(uint32_t tmem_d, uint64_t ad, uint64_t bd, uint32_t accumulate) {
-    static_assert(KIND != kTcI8 || CG == 1, "int8 operands: one CTA");
+    static_assert((KIND != kTcI8 && KIND != kTcF16) || CG == 1, "int8 and FP16 operands: one CTA");
     if constexpr (KIND == kTcBF16 && CG == 1)
         ANN_MMA("1", "f16", kIdescBF16<1>);
     else if constexpr (KIND == kTcBF16)
@@ -145,6 +146,8 @@ __device__ __forceinline__ void mma_issue(uint32_t tmem_d, uint64_t ad, uint64_t
         ANN_MMA("1", "f8f6f4", kIdescE4M3<1>);
     else if constexpr (KIND == kTcE4M3)
         ANN_MMA("2", "f8f6f4", kIdescE4M3<2>);
+    else if constexpr (KIND == kTcF16)
+        ANN_MMA("1", "f16", kIdescF16);
     else
         ANN_MMA("1", "i8", kIdescI8);
 }
