@@ -808,7 +808,7 @@ struct IvfQueryCfg {
     bool lsh_keys;    // exact LSH batch: SQ8 keys of the whole streams, then selection
     int64_t ub_cand;  // longest explicit candidate stream (LSH buckets; a fallback to every row needs none)
     int n_probes;
-    size_t sort_tmp, scan_tmp, bscratch;
+    size_t bscratch;
 };
 
 // Operand forms of the tensor-core forms, built once: BF16 centroids (the coarse ranking of both), and the BF16
@@ -1037,9 +1037,9 @@ constexpr int kKernKeys = 0, kKernBars = 1, kKernSelect = 2, kKernRerank = 3;
 constexpr int kRowCapFactor = 16;
 
 static int ivf_tc_sampled(ann_ivf* h, ann_workspace* ws, const IvfQueryCfg& c, const IvfQueryArgs& a,
-                          const IvfBatchArgs& b, const TcOperands& op, unsigned char* Apk, int64_t* titem,
-                          int4* titem_desc, int64_t items_cap, float* keyR, int* idR, int prec, bool* done,
-                          cudaStream_t st, bool pruned = false) {
+                          IvfBatchArgs* bp, void* bscratch, int64_t* tot, const TcOperands& op, unsigned char* Apk,
+                          int64_t* titem, int4* titem_desc, int64_t items_cap, float* keyR, int* idR, int prec,
+                          bool* done, cudaStream_t st, bool pruned = false) {
     *done = false;
     const int nq = a.plan.nq, npc = c.npc, C = (int)h->C, R = c.R;
     const int64_t max_pairs = (int64_t)nq * npc;
@@ -1051,14 +1051,11 @@ static int ivf_tc_sampled(ann_ivf* h, ann_workspace* ws, const IvfQueryCfg& c, c
     const int rF = pruned ? prune_bar_rank(R, ((int64_t)1 << 24) / div, (int64_t)1 << 24)
                           : (int)std::min<int64_t>(R, std::max<int64_t>(1, ceil_div(3 * (int64_t)R, div)));
     const int cap = pruned ? ivf_prune_cap(R) : kRowCapFactor * R;
-    size_t scan_tmp = 0;
-    ANN_CUDA_TRY(cub::DeviceScan::ExclusiveSum(nullptr, scan_tmp, (int64_t*)nullptr, (int64_t*)nullptr, nq + 1, st));
     Sizer sz;
     sz.take<int64_t>((size_t)C);                 // list heads
     sz.take<int64_t>((size_t)max_pairs);         // sseg
     sz.take<int64_t>((size_t)nq + 1);            // slen
     sz.take<int64_t>((size_t)nq + 1);            // soff
-    sz.take<char>(scan_tmp);
     sz.take<int64_t>((size_t)C + 1);             // sample items
     sz.take<int4>((size_t)scap);
     sz.take<int64_t>((size_t)max_pairs);         // sdbase
@@ -1083,7 +1080,6 @@ static int ivf_tc_sampled(ann_ivf* h, ann_workspace* ws, const IvfQueryCfg& c, c
     int64_t* sseg = cv.take<int64_t>((size_t)max_pairs);
     int64_t* slen = cv.take<int64_t>((size_t)nq + 1);
     int64_t* soff = cv.take<int64_t>((size_t)nq + 1);
-    void* stmp = cv.take<char>(scan_tmp);
     int64_t* sitem = cv.take<int64_t>((size_t)C + 1);
     int4* sitem_desc = cv.take<int4>((size_t)scap);
     int64_t* sdbase = cv.take<int64_t>((size_t)max_pairs);
@@ -1127,24 +1123,27 @@ static int ivf_tc_sampled(ann_ivf* h, ann_workspace* ws, const IvfQueryCfg& c, c
         qrows = pa.qop;
     }
 
-    // sample streams: heads of the probed lists, each query's stream offsets
-    if ((rc = launch_tc_ivf_sample_plan(a.plan, h->list_off, C, div, lcap, sseg, slen, st))) return rc;
-    ANN_CUDA_TRY(cudaMemsetAsync(slen + nq, 0, sizeof(int64_t), st));
-    size_t tb = scan_tmp;
-    ANN_CUDA_TRY(cub::DeviceScan::ExclusiveSum(stmp, tb, slen, soff, nq + 1, st));
-    TcIvfSampleMaps maps;
-    maps.row_query = rowq;
-    maps.soff = soff;
-    maps.sseg = sseg;
-    maps.sdbase = sdbase;
-    maps.qfac = op.qfac;
-    maps.pfac = op.pfac;
-    if ((rc = launch_tc_ivf_pairs(qrows, op.row_bytes, b.pair_vals, b.pair_lists, b.lq_off + C, max_pairs, npc,
-                                  b.cand_off, a.plan.seg_pref, h->list_off, Apk, nullptr, st, maps)))
-        return rc;
+    // the batch's set-up, with the sample streams (the heads of the probed lists), the pairs' operand rows and the tiles
+    IvfBatchTiles tiles;
+    tiles.titem = titem;
+    tiles.div = div;
+    tiles.lcap = lcap;
+    tiles.sitem = sitem;
+    tiles.sseg = sseg;
+    tiles.slen = slen;
+    tiles.soff = soff;
+    tiles.qrows = qrows;
+    tiles.row_bytes = op.row_bytes;
+    tiles.A = Apk;
+    tiles.row_query = rowq;
+    tiles.sdbase = sdbase;
+    tiles.qfac = op.qfac;
+    tiles.pfac = op.pfac;
+    if ((rc = batched_prepare(a, bscratch, bp, tot, st, false, tiles))) return rc;
+    const IvfBatchArgs& b = *bp;
+    const TcItemDescs descs[2] = {{sitem, lcap, sitem_desc, scap}, {titem, nullptr, titem_desc, items_cap}};
+    if ((rc = launch_tc_item_descs(descs, 2, C, b.lq_off, h->list_off, st))) return rc;
     // 1. sample pass: keys of the list heads into the sample streams; the two bars per query
-    if ((rc = launch_tc_ivf_items(b.lq_off, h->list_off, C, sitem, st, lcap))) return rc;
-    if ((rc = launch_tc_item_descs(sitem, C, b.lq_off, h->list_off, lcap, sitem_desc, scap, st))) return rc;
     TcGemmArgs gs{(int)max_pairs, (int)h->n, op.K, nullptr, SK, 0, h->d_err};
     gs.kind = op.kind;
     gs.col_fac = op.col_fac;
@@ -1164,8 +1163,6 @@ static int ivf_tc_sampled(ann_ivf* h, ann_workspace* ws, const IvfQueryCfg& c, c
         return rc;
     h->prof.kend(kt, kKernBars, st);
     // 2. filter pass over every row of the probed lists into the queries' buffers
-    if ((rc = launch_tc_ivf_items(b.lq_off, h->list_off, C, titem, st))) return rc;
-    if ((rc = launch_tc_item_descs(titem, C, b.lq_off, h->list_off, nullptr, titem_desc, items_cap, st))) return rc;
     auto filter = [&](const float* tau, const int* skip_if_zero) -> int {
         TcGemmArgs g{(int)max_pairs, (int)h->n, op.K, nullptr, nullptr, 0, h->d_err};
         g.skip_if_zero = skip_if_zero;
@@ -1413,24 +1410,22 @@ static int ivf_query_device(ann_ivf* h, ann_workspace* ws, const IvfQueryCfg& c,
         const bool sampled = c.pruned || (c.tc && nq >= h->sampled_min_queries);
         if (sampled && (rc = ws_pinned(ws, &tot))) return rc;
         tot[0] = tot[1] = tot[2] = tot[3] = 0;
-        if (plan_apart)
-            ANN_CUDA_TRY(cudaMemcpyAsync(&tot[3], apart_count, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
         auto run_sampled = [&](bool* ok) -> int {
             if (c.pruned) {
                 const int kpad = tc_kpad(h->dim, ANN_METRIC_L2);
                 const TcOperands op{nullptr, 2 * kpad, h->code_f16, kpad, kTcF16, nullptr, nullptr, nullptr};
                 const int64_t cap = tc_items_bound((int64_t)nq * c.npc, (int)h->C, h->sizes_desc[0]);
-                int r = ivf_tc_sampled(h, ws, c, a, b, op, nullptr, nullptr, nullptr, cap, keyR, idR, prec, ok, st, true);
+                int r = ivf_tc_sampled(h, ws, c, a, &b, bscratch, tot, op, nullptr, nullptr, nullptr, cap, keyR, idR, prec,
+                                       ok, st, true);
                 if (r == ANN_ERR_NOMEM) {  // the batched pass may need less
                     clear_error();
-                    r = ANN_OK;
-                    ANN_CUDA_TRY(cudaStreamSynchronize(st));
+                    r = batched_prepare(a, bscratch, &b, tot, st);
                 }
                 if (!r) ivf_prune_settled(h, *ok, c.saved_us);
                 return r;
             }
-            return ivf_tc_sampled(h, ws, c, a, b, tc_operands(h, c, qb, q8, qfac, pfac), Apk, titem, titem_desc,
-                                  items_cap, keyR, idR, prec, ok, st);
+            return ivf_tc_sampled(h, ws, c, a, &b, bscratch, tot, tc_operands(h, c, qb, q8, qfac, pfac), Apk, titem,
+                                  titem_desc, items_cap, keyR, idR, prec, ok, st);
         };
         bool sampled_done = false;
         if (c.small_tc) {  // no totals on the host: the streams' keys fit their bound
@@ -1441,8 +1436,13 @@ static int ivf_query_device(ann_ivf* h, ann_workspace* ws, const IvfQueryCfg& c,
             ss.cap = items_cap;
             if ((rc = launch_tc_small_setup(a, ss, st))) return rc;
             tot[1] = c.small_keys;
-        } else if ((rc = batched_prepare(a, bscratch, c.sort_tmp, c.scan_tmp, &b, tot, st, !sampled))) return rc;
-        if (sampled && (rc = run_sampled(&sampled_done))) return rc;  // synchronises st: tot is current
+        } else if (sampled) {
+            if ((rc = run_sampled(&sampled_done))) return rc;  // synchronises st: tot is current
+        } else {
+            IvfBatchTiles tiles;
+            tiles.titem = titem;
+            if ((rc = batched_prepare(a, bscratch, &b, tot, st, true, tiles))) return rc;
+        }
         if (tot[2] != 0) sampled_done = false;
         if (plan_apart) every_row.resize((size_t)(int)tot[3]);  // the plan has listed them in every_list
         done = sampled_done;
@@ -1454,19 +1454,13 @@ static int ivf_query_device(ann_ivf* h, ann_workspace* ws, const IvfQueryCfg& c,
                 // query's stream by radix selection
                 const TcOperands op = tc_operands(h, c, qb, q8, qfac, pfac);
                 const int64_t max_pairs = (int64_t)nq * c.npc;
-                TcIvfSampleMaps maps;
-                maps.qfac = op.qfac;
-                maps.pfac = op.pfac;
                 const int64_t* n_pairs = c.small_tc ? b.total_items : b.lq_off + h->C;
                 if ((rc = launch_tc_ivf_pairs(op.qrows, op.row_bytes, b.pair_vals, b.pair_lists, n_pairs, max_pairs, c.npc,
-                                              b.cand_off, a.plan.seg_pref, h->list_off, Apk, dbase, st, maps)))
+                                              b.cand_off, a.plan.seg_pref, h->list_off, Apk, dbase, st, op.qfac,
+                                              op.pfac)))
                     return rc;
-                if (!c.small_tc) {
-                    if ((rc = launch_tc_ivf_items(b.lq_off, h->list_off, h->C, titem, st))) return rc;
-                    if ((rc = launch_tc_item_descs(titem, (int)h->C, b.lq_off, h->list_off, nullptr, titem_desc,
-                                                   items_cap, st)))
-                        return rc;
-                }
+                const TcItemDescs descs{titem, nullptr, titem_desc, items_cap};
+                if (!c.small_tc && (rc = launch_tc_item_descs(&descs, 1, h->C, b.lq_off, h->list_off, st))) return rc;
                 TcGemmArgs g{(int)max_pairs, (int)h->n, op.K, nullptr, D, 0, h->d_err};
                 g.kind = op.kind;
                 g.col_fac = op.col_fac;
@@ -1746,7 +1740,7 @@ int ann_ivf_query(ann_ivf* h, ann_workspace* ws, const float* queries, int32_t n
     c.small_keys = (int64_t)qc * c.npc * h->sizes_desc[0];
     c.small_tc = c.tc && nq < h->sampled_min_queries && !c.fallback && (c.shard || c.max_c >= k) &&
                  (int64_t)qc * c.npc <= kSmallSetupPairs && c.small_keys <= ((int64_t)16 << 20);
-    if (c.batched) c.bscratch = batched_scratch_bytes(qc, c.npc, h->C, &c.sort_tmp, &c.scan_tmp);
+    if (c.batched) c.bscratch = batched_scratch_bytes(qc, c.npc, h->C);
     Sizer head;
     head.take<float>((size_t)nq * dpad);
     if (host) {

@@ -9,7 +9,7 @@
 //     key = |y|^2 - 2 sum_d (code_d - 127.5) f16(scale_d u_d), all of it scaled by powers of two into FP16's range. Centred
 //     so, the keys' error does not grow with the data's distance from the origin. FP16 and not BF16: a list of 40,000
 //     rows around one centre holds its best 400 so densely that BF16's window (0.0095 at unit norms) kept several
-//     thousand more, FP16's (0.0025) a few hundred;
+//     thousand more, FP16's (0.0024) a few hundred;
 //   * the heads of the probed lists give a sampled bar per query (as the tensor-core form's), the grouped filter pass keeps
 //     the keys up to the bar plus the window, and if the R-th smallest kept key is within the bar, the best R by
 //     (distance, stream position) are among the keys up to it plus the window.

@@ -582,28 +582,28 @@ int launch_tc_gemm(const void* A, const void* B, const TcGemmArgs& a, cudaStream
 
 namespace {
 // desc[t] for the items of list l = blockIdx.x (strided): the tile group_tile would derive for item t.
-__global__ void tc_item_descs_kernel(const int64_t* __restrict__ item_off, int C, const int64_t* __restrict__ a_off,
-                                     const int64_t* __restrict__ b_off, const int64_t* __restrict__ b_len,
-                                     int4* __restrict__ desc, int64_t cap) {
+__global__ void tc_item_descs_kernel(TcItemDescs s0, TcItemDescs s1, int C, const int64_t* __restrict__ a_off,
+                                     const int64_t* __restrict__ b_off) {
+    const TcItemDescs s = blockIdx.y ? s1 : s0;
     for (int l = blockIdx.x; l < C; l += gridDim.x) {
         const int64_t np = a_off[l + 1] - a_off[l];
-        const int64_t nr = b_len ? b_len[l] : b_off[l + 1] - b_off[l];
+        const int64_t nr = s.b_len ? s.b_len[l] : b_off[l + 1] - b_off[l];
         const int64_t npt = (np + kBM - 1) / kBM;
-        for (int64_t t = item_off[l] + threadIdx.x; t < item_off[l + 1] && t < cap; t += blockDim.x) {
-            const int64_t local = t - item_off[l];
+        for (int64_t t = s.item_off[l] + threadIdx.x; t < s.item_off[l + 1] && t < s.cap; t += blockDim.x) {
+            const int64_t local = t - s.item_off[l];
             const int64_t g = local % npt, rt = local / npt;
-            desc[t] = make_int4((int)(a_off[l] + g * kBM), (int)(b_off[l] + rt * kBN),
-                                (int)min((int64_t)kBM, np - g * kBM), (int)min((int64_t)kBN, nr - rt * kBN));
+            s.desc[t] = make_int4((int)(a_off[l] + g * kBM), (int)(b_off[l] + rt * kBN),
+                                  (int)min((int64_t)kBM, np - g * kBM), (int)min((int64_t)kBN, nr - rt * kBN));
         }
     }
 }
 }  // namespace
 
-int launch_tc_item_descs(const int64_t* item_off, int C, const int64_t* a_off, const int64_t* b_off,
-                         const int64_t* b_len, int4* desc, int64_t cap, cudaStream_t st) {
-    ANN_CHECK_ARG(C >= 1, "tensor-core grouping: no lists");
-    tc_item_descs_kernel<<<(unsigned)std::min(C, 4 * kNumSMs), 128, 0, st>>>(item_off, C, a_off, b_off, b_len, desc,
-                                                                             cap);
+int launch_tc_item_descs(const TcItemDescs* sets, int n_sets, int C, const int64_t* a_off, const int64_t* b_off,
+                         cudaStream_t st) {
+    ANN_CHECK_ARG(C >= 1 && (n_sets == 1 || n_sets == 2), "tensor-core grouping: %d lists, %d sets", C, n_sets);
+    const dim3 grid((unsigned)std::min(C, 4 * kNumSMs), (unsigned)n_sets);
+    tc_item_descs_kernel<<<grid, 128, 0, st>>>(sets[0], sets[n_sets - 1], C, a_off, b_off);
     ANN_LAUNCH_CHECK();
     return ANN_OK;
 }

@@ -79,10 +79,16 @@ enum TcRole { kTcBase = 0, kTcQuery = 1 };
 int tc_kpad(int dim, int metric);
 size_t tc_gemm_smem();
 // The grouped mode's item descriptors (TcGemmArgs::g_item_desc) for items [0, min(item_off[C], cap)): list l's
-// items from item_off[l] (launch_tc_ivf_items), its A rows [a_off[l], a_off[l+1]) and B rows from b_off[l]
-// (b_len[l] of them when given, else to b_off[l+1]).
-int launch_tc_item_descs(const int64_t* item_off, int C, const int64_t* a_off, const int64_t* b_off,
-                         const int64_t* b_len, int4* desc, int64_t cap, cudaStream_t st);
+// items from item_off[l], its A rows [a_off[l], a_off[l+1]) and B rows from b_off[l] (b_len[l] of them when given, else to
+// b_off[l+1]). Up to two sets, of the same lists, in one launch.
+struct TcItemDescs {
+    const int64_t* item_off;
+    const int64_t* b_len;
+    int4* desc;
+    int64_t cap;
+};
+int launch_tc_item_descs(const TcItemDescs* sets, int n_sets, int C, const int64_t* a_off, const int64_t* b_off,
+                         cudaStream_t st);
 int launch_tc_gemm(const void* A, const void* B, const TcGemmArgs& a, cudaStream_t st);
 // Runs one small GEMM whose producer issues no copies, with every wait limited to wait_ns, and returns the
 // device flag it left (2: a bounded wait gave up, as it must); the flag is cleared afterwards.

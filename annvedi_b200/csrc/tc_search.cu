@@ -61,43 +61,11 @@ __global__ void tc_unpermute_kernel(const float* keys, int64_t n, int64_t mult, 
         out[(int64_t)q * n + pos_to_row(p, n, mult)] = keys[(int64_t)q * n + p];
 }
 
-__global__ void __launch_bounds__(1024) tc_ivf_items_kernel(const int64_t* lq_off, const int64_t* list_off, int C,
-                                                            int64_t* item_off, const int64_t* list_len) {
-    __shared__ int64_t sPart[1024];
-    const int per = (C + 1023) / 1024;
-    const int l0 = threadIdx.x * per;
-    auto items = [&](int l) -> int64_t {
-        const int64_t np = lq_off[l + 1] - lq_off[l];
-        const int64_t nr = list_len ? list_len[l] : list_off[l + 1] - list_off[l];
-        return (np == 0 || nr == 0) ? 0 : ((np + 127) / 128) * ((nr + 255) / 256);
-    };
-    int64_t local = 0;
-    for (int i = 0; i < per; ++i)
-        if (l0 + i < C) local += items(l0 + i);
-    sPart[threadIdx.x] = local;
-    __syncthreads();
-    for (int off = 1; off < 1024; off <<= 1) {
-        const int64_t v = threadIdx.x >= off ? sPart[threadIdx.x - off] : 0;
-        __syncthreads();
-        sPart[threadIdx.x] += v;
-        __syncthreads();
-    }
-    int64_t run = sPart[threadIdx.x] - local;
-    for (int i = 0; i < per; ++i) {
-        const int l = l0 + i;
-        if (l < C) {
-            item_off[l] = run;
-            run += items(l);
-        }
-    }
-    if (threadIdx.x == 1023) item_off[C] = sPart[1023];
-}
-
 // one warp per pair
 __global__ void tc_ivf_pairs_kernel(const unsigned char* qrows, int row_bytes, const int32_t* pair_vals,
                                     const int32_t* pair_lists, const int64_t* n_pairs, int64_t max_pairs, int npc,
                                     const int64_t* cand_off, const int64_t* seg_pref, const int64_t* list_off,
-                                    unsigned char* A, int64_t* dbase, TcIvfSampleMaps sm) {
+                                    unsigned char* A, int64_t* dbase, const float* qfac, float* pfac) {
     const int64_t np = min(*n_pairs, max_pairs);
     const int lane = threadIdx.x & 31;
     for (int64_t i = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; i < np;
@@ -108,29 +76,10 @@ __global__ void tc_ivf_pairs_kernel(const unsigned char* qrows, int row_bytes, c
         uint4* dst = reinterpret_cast<uint4*>(A + (size_t)i * row_bytes);
         for (int c = lane; c < row_bytes / 16; c += 32) dst[c] = src[c];
         if (lane == 0) {
-            if (sm.pfac) sm.pfac[i] = sm.qfac[q];
-            if (dbase) dbase[i] = cand_off[q] + seg_pref[(int64_t)q * (npc + 1) + j] - list_off[pair_lists[i]];
-            if (sm.row_query) sm.row_query[i] = q;
-            // the grouped epilogue adds the tile's absolute list row, as for dbase
-            if (sm.sdbase) sm.sdbase[i] = sm.soff[q] + sm.sseg[(int64_t)q * npc + j] - list_off[pair_lists[i]];
+            if (pfac) pfac[i] = qfac[q];
+            dbase[i] = cand_off[q] + seg_pref[(int64_t)q * (npc + 1) + j] - list_off[pair_lists[i]];
         }
     }
-}
-
-// One thread per query: the sample stream of its probed lists (the first lcap[l] rows of each), the
-// segment starts sseg[q][j] and its length slen[q]; the candidates' count comes from the plan.
-__global__ void tc_ivf_sample_plan_kernel(IvfPlan p, const int64_t* __restrict__ lcap, int64_t* __restrict__ sseg,
-                                          int64_t* __restrict__ slen) {
-    const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= p.nq) return;
-    const int ns = p.n_seg[q];
-    int64_t run = 0;
-    for (int j = 0; j < p.npc; ++j) {
-        sseg[(int64_t)q * p.npc + j] = run;
-        const int l = p.probes[(int64_t)q * p.npc + j];
-        if (j < ns && l >= 0) run += lcap[l];
-    }
-    slen[q] = run;
 }
 
 // One warp per query: the int8 weights of the SQ8 tensor-core key. w_d = -2 scale_d (q_d - offset_d), so that
@@ -529,12 +478,6 @@ __global__ void __launch_bounds__(256) warp_select_kernel(const float* __restric
     }
 }
 
-// lcap[l] = ceil(size_l / div): the sampled head of list l
-__global__ void tc_ivf_list_caps_kernel(const int64_t* __restrict__ list_off, int C, int div, int64_t* __restrict__ lcap) {
-    const int l = blockIdx.x * blockDim.x + threadIdx.x;
-    if (l < C) lcap[l] = (list_off[l + 1] - list_off[l] + div - 1) / div;
-}
-
 // tauR[q] = tauS[q] for the queries marked for a re-run, else -inf (no key passes)
 __global__ void tc_rerun_bars_kernel(const int* __restrict__ mark, const float* __restrict__ tauS, int nq,
                                      float* __restrict__ tauR, int* __restrict__ rcount) {
@@ -890,30 +833,6 @@ int launch_tc_coarse(const float* keys, int64_t ldk, int nq, int C, int npc, int
     return ANN_OK;
 }
 
-int launch_tc_ivf_items(const int64_t* lq_off, const int64_t* list_off, int C, int64_t* item_off, cudaStream_t st,
-                        const int64_t* list_len) {
-    ANN_CHECK_ARG(C >= 1, "tensor-core IVF: no lists");
-    tc_ivf_items_kernel<<<1, 1024, 0, st>>>(lq_off, list_off, C, item_off, list_len);
-    ANN_LAUNCH_CHECK();
-    return ANN_OK;
-}
-
-namespace {
-// item_list[t] = l for every item t of list l (t < cap)
-__global__ void tc_item_lists_kernel(const int64_t* __restrict__ item_off, int C, int32_t* __restrict__ item_list,
-                                     int64_t cap) {
-    for (int l = blockIdx.x; l < C; l += gridDim.x)
-        for (int64_t t = item_off[l] + threadIdx.x; t < item_off[l + 1] && t < cap; t += blockDim.x) item_list[t] = l;
-}
-}  // namespace
-
-int launch_tc_item_lists(const int64_t* item_off, int C, int32_t* item_list, int64_t cap, cudaStream_t st) {
-    ANN_CHECK_ARG(C >= 1, "tensor-core IVF: no lists");
-    tc_item_lists_kernel<<<(unsigned)std::min(C, 4 * kNumSMs), 128, 0, st>>>(item_off, C, item_list, cap);
-    ANN_LAUNCH_CHECK();
-    return ANN_OK;
-}
-
 namespace {
 // Exclusive prefix of v over the block's 1,024 threads; *total = the sum. sPart: 1,024 words.
 __device__ __forceinline__ int64_t block_prefix(int64_t v, int64_t* sPart, int64_t* total) {
@@ -1024,14 +943,14 @@ int launch_tc_small_setup(const IvfQueryArgs& a, const TcSmallSetup& s, cudaStre
 int launch_tc_ivf_pairs(const void* qrows, int row_bytes, const int32_t* pair_vals, const int32_t* pair_lists,
                         const int64_t* n_pairs, int64_t max_pairs, int npc, const int64_t* cand_off,
                         const int64_t* seg_pref, const int64_t* list_off, void* A, int64_t* dbase, cudaStream_t st,
-                        const TcIvfSampleMaps& sm) {
+                        const float* qfac, float* pfac) {
     if (max_pairs == 0) return ANN_OK;
     ANN_CHECK_ARG(row_bytes % 16 == 0, "tensor-core IVF: operand rows of %d bytes", row_bytes);
-    ANN_CHECK_ARG((sm.pfac == nullptr) == (sm.qfac == nullptr), "tensor-core IVF: pair factors need query factors");
+    ANN_CHECK_ARG((pfac == nullptr) == (qfac == nullptr), "tensor-core IVF: pair factors need query factors");
     const int grid = (int)std::min<int64_t>(ceil_div(max_pairs * 32, 256), 16 * kNumSMs);
     tc_ivf_pairs_kernel<<<grid, 256, 0, st>>>(static_cast<const unsigned char*>(qrows), row_bytes, pair_vals,
                                               pair_lists, n_pairs, max_pairs, npc, cand_off, seg_pref, list_off,
-                                              static_cast<unsigned char*>(A), dbase, sm);
+                                              static_cast<unsigned char*>(A), dbase, qfac, pfac);
     ANN_LAUNCH_CHECK();
     return ANN_OK;
 }
@@ -1040,17 +959,6 @@ int launch_tc_bar_check(const int* rowcnt, int M, int R, int* list, int* flags, 
                         int* mark) {
     if (M == 0) return ANN_OK;
     tc_bar_check_kernel<<<(unsigned)ceil_div(M, 256), 256, 0, st>>>(rowcnt, M, R, list, flags, lens, mark);
-    ANN_LAUNCH_CHECK();
-    return ANN_OK;
-}
-
-int launch_tc_ivf_sample_plan(const IvfPlan& p, const int64_t* list_off, int C, int div, int64_t* lcap, int64_t* sseg,
-                              int64_t* slen, cudaStream_t st) {
-    ANN_CHECK_ARG(C >= 1 && div >= 1, "IVF sample plan: %d lists, 1/%d", C, div);
-    tc_ivf_list_caps_kernel<<<(unsigned)ceil_div(C, 256), 256, 0, st>>>(list_off, C, div, lcap);
-    ANN_LAUNCH_CHECK();
-    if (p.nq == 0) return ANN_OK;
-    tc_ivf_sample_plan_kernel<<<(unsigned)ceil_div(p.nq, 128), 128, 0, st>>>(p, lcap, sseg, slen);
     ANN_LAUNCH_CHECK();
     return ANN_OK;
 }

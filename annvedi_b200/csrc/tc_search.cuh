@@ -26,13 +26,7 @@ int launch_tc_map_ids(int* ids, int64_t count, int64_t n, int64_t mult, cudaStre
 int launch_tc_unpermute(const float* keys, int nq, int64_t n, int64_t mult, float* out, cudaStream_t st);
 
 // IVF batches on the tensor cores (a list-major grouping of (query, list) pairs, ivf_batched.cu):
-// items per list = ceil(pairs / 128) x ceil(rows / 256), exclusively scanned into item_off[0..C]
-// (item_off[C] = all items). One block.
-// With list_len, list l counts list_len[l] rows (a capped head of each list) instead of its size.
-int launch_tc_ivf_items(const int64_t* lq_off, const int64_t* list_off, int C, int64_t* item_off, cudaStream_t st,
-                        const int64_t* list_len = nullptr);
-// item_list[t] = the list of work item t (item_off [C + 1] from launch_tc_ivf_items), for t < cap.
-int launch_tc_item_lists(const int64_t* item_off, int C, int32_t* item_list, int64_t cap, cudaStream_t st);
+// ceil(pairs / 128) x ceil(rows / 256) work items per list, pair tiles fastest.
 // Work items of a grouped batch at most: (pairs / 128 + C) x (largest list / 256 + 1).
 inline int64_t tc_items_bound(int64_t pairs, int C, int64_t largest) { return (pairs / 128 + C) * (largest / 256 + 1); }
 // Set-up of a small tensor-core batch (nq * npc <= kSmallSetupPairs, every query's lists known to hold k rows or more) by
@@ -51,22 +45,12 @@ int launch_tc_small_setup(const IvfQueryArgs& a, const TcSmallSetup& s, cudaStre
 // For each valid pair i (< lq_off[C]; pairs grouped by list, pair_vals = q * npc + j, pair_lists = the
 // list): A[i] = qb[q] (kpad BF16 columns) and dbase[i] = cand_off[q] + seg_pref[q][j] - list_off[list],
 // the stream position of the list's row 0 in the candidate array.
-// Optional maps of the sampled form: row_query[i] = q; sdbase[i] = soff[q] + sseg[q][j] - list_off[list]
-// (the sample-stream position of the list's row 0, as dbase is for the candidate stream).
 // With qfac / pfac (the int8 form), pfac[i] = qfac[q].
-struct TcIvfSampleMaps {
-    int32_t* row_query = nullptr;
-    const int64_t* soff = nullptr;
-    const int64_t* sseg = nullptr;  // [nq, npc]
-    int64_t* sdbase = nullptr;
-    const float* qfac = nullptr;
-    float* pfac = nullptr;
-};
 // qrows: the queries' operand rows of row_bytes each (BF16 kpad columns, or int8 weights); A: the pairs' rows.
 int launch_tc_ivf_pairs(const void* qrows, int row_bytes, const int32_t* pair_vals, const int32_t* pair_lists,
                         const int64_t* n_pairs, int64_t max_pairs, int npc, const int64_t* cand_off,
                         const int64_t* seg_pref, const int64_t* list_off, void* A, int64_t* dbase, cudaStream_t st,
-                        const TcIvfSampleMaps& sm = TcIvfSampleMaps{});
+                        const float* qfac = nullptr, float* pfac = nullptr);
 // SQ8 codes on the tensor cores (kind::i8): the int8 query weights rint(-2 scale_d (q_d - offset_d) * 127 / max)
 // [nq, ldo] (zero past dim) with their factor qfac = max / 127, and per row fac = (1, sum_d (code_d scale_d)^2);
 // the key fac.y + qfac * sum_d code_d a_d is the SQ8 distance less |q - offset|^2, up to the weights' rounding.
@@ -74,10 +58,6 @@ int launch_tc_sq8_query(const float* q, int nq, int dim, int ldq, const float* s
                         int ldo, float* qfac, cudaStream_t st);
 int launch_tc_sq8_norms(const uint8_t* codes, int64_t n, int dim, int ldc, const float* scale, float2* fac,
                         cudaStream_t st);
-// The sampled heads of the lists, lcap[l] = ceil(size_l / div), and each query's sample stream over its
-// probed lists: segment starts sseg [nq, npc] and length slen [nq].
-int launch_tc_ivf_sample_plan(const IvfPlan& p, const int64_t* list_off, int C, int div, int64_t* lcap, int64_t* sseg,
-                              int64_t* slen, cudaStream_t st);
 // tauR[q] = mark[q] ? tauS[q] : -inf; with rcount, the marked queries' counts are reset to 0.
 int launch_tc_rerun_bars(const int* mark, const float* tauS, int nq, float* tauR, cudaStream_t st,
                          int* rcount = nullptr);
