@@ -693,7 +693,7 @@ static int flat_exact_pruned(ann_flat* h, ann_workspace* ws, const float* qdev, 
     Sizer sz;
     sz.take<__nv_bfloat16>((size_t)qc * kpad);
     sz.take<float>((size_t)qc * (S / 8));
-    for (int i = 0; i < 4; ++i) sz.take<float>((size_t)qc);
+    for (int i = 0; i < 3; ++i) sz.take<float>((size_t)qc);
     sz.take<float>((size_t)qc * cap);
     sz.take<int>((size_t)qc * cap);
     for (int i = 0; i < 2; ++i) sz.take<int>((size_t)qc);
@@ -713,7 +713,6 @@ static int flat_exact_pruned(ann_flat* h, ann_workspace* ws, const float* qdev, 
     float* win = cv.take<float>((size_t)qc);
     float* tauF = cv.take<float>((size_t)qc);
     float* tauX = cv.take<float>((size_t)qc);
-    float* tauU = cv.take<float>((size_t)qc);
     float* fkey = cv.take<float>((size_t)qc * cap);
     int* fcol = cv.take<int>((size_t)qc * cap);
     int* rcount = cv.take<int>((size_t)qc);
@@ -740,7 +739,6 @@ static int flat_exact_pruned(ann_flat* h, ann_workspace* ws, const float* qdev, 
         p.b = h->bounds;
         p.win = win;
         p.tauF = tauF;
-        p.tauX = tauX;
         p.cap = cap;
         p.fkey = fkey;
         p.fcol = fcol;
@@ -749,16 +747,14 @@ static int flat_exact_pruned(ann_flat* h, ann_workspace* ws, const float* qdev, 
         p.count = count;
         p.out_ids = ids_dev + (size_t)q0 * kk;
         p.out_dists = dists_dev ? dists_dev + (size_t)q0 * kk : nullptr;
-        if ((rc = launch_tc_operand(q, nc, h->dim, dpad, qb, kpad, kTcQuery, h->metric, 0, st))) return rc;
-        if ((rc = launch_prune_windows(p, st))) return rc;
+        if ((rc = launch_prune_queries(p, qb, kpad, st))) return rc;
         TcFilterArgs sa{nc, (int)S, kpad, kTcBF16};
         sa.err = h->d_err;
         sa.out_min = kA;
         sa.b_tile_stride = stride;
         sa.b_rows = n;
         if ((rc = launch_tc_sample(qb, h->base_bf16, sa, st))) return rc;
-        if ((rc = launch_warp_bars(kA, nullptr, nullptr, nc, rF, rF, tauF, tauU, st, S / 8))) return rc;
-        if ((rc = launch_prune_bars(p, st))) return rc;
+        if ((rc = launch_bars(kA, nullptr, nullptr, nc, rF, rF, tauF, tauX, st, S / 8, win))) return rc;
         const TcFilterArgs fa{nc, (int)n, kpad, kTcBF16, tauX, fkey, fcol, cap, rcount, nullptr, nullptr, h->d_err};
         if ((rc = launch_tc_filter(qb, h->base_bf16, fa, st))) return rc;
         if ((rc = launch_prune_finish(p, st))) return rc;
@@ -953,7 +949,7 @@ int ann_flat_query_tc(ann_flat* h, ann_workspace* ws, const float* queries, int3
             sa.b_rows = n;
             if ((rc = launch_tc_sample(qbc, t.base, sa, st))) return rc;
             const int S8 = (int)(S / 8);
-            if ((rc = launch_warp_bars(kA, nullptr, nullptr, nc, rF, R, tauF, tauS, st, S8))) return rc;
+            if ((rc = launch_bars(kA, nullptr, nullptr, nc, rF, R, tauF, tauS, st, S8))) return rc;
             h->prof.mark(prec, st);
             auto filter = [&](const void* A, int M, const float* tau, const float* rf, int rcap) -> int {
                 ANN_CUDA_TRY(cudaMemsetAsync(rowcnt, 0, sizeof(int) * (size_t)M, st));

@@ -1158,7 +1158,7 @@ static int ivf_tc_sampled(ann_ivf* h, ann_workspace* ws, const IvfQueryCfg& c, c
     gs.g_item_desc = sitem_desc;
     if ((rc = launch_tc_gemm(Apk, op.B, gs, st))) return rc;
     int kt = h->prof.kbegin(st);
-    if ((rc = launch_warp_bars(SK, soff, slen, nq, rF, pruned ? rF : R, tauF, pruned ? tauR : tauS, st,
+    if ((rc = launch_bars(SK, soff, slen, nq, rF, pruned ? rF : R, tauF, pruned ? tauR : tauS, st,
                                (int64_t)npc * head_max)))
         return rc;
     h->prof.kend(kt, kKernBars, st);

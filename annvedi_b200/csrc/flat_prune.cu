@@ -5,7 +5,7 @@
 // an element (0.37 ms, 0.26 ms pruned). Only about k distances a query are kept. Here the BF16 tensor-core keys (tc_gemm.cu) say which rows can be among them, and
 // only those rows' FP32 distances are formed, with the scan's own sums, so that ids and distances are the scan's
 // bit for bit:
-//   1. a BF16 key differs from the real |x|^2 - 2 x.q (or -x.q) by at most eps (launch_prune_windows);
+//   1. a BF16 key differs from the real |x|^2 - 2 x.q (or -x.q) by at most eps (launch_prune_queries);
 //   2. a sampled bar tauF that about a few k keys pass, and a filter pass that keeps every key <= tauF + w,
 //      w = 2 eps + delta, delta covering the rounding of the FP32 distances themselves;
 //   3. per query: T, the k-th smallest kept key, is the k-th smallest of all if T <= tauF. A row whose key exceeds
@@ -27,8 +27,6 @@ namespace annb {
 
 namespace {
 
-constexpr int kFinThreads = 256;
-constexpr int kFinWarps = kFinThreads / 32;
 constexpr int kFinPitch = 36;  // floats per staged row of 32: 16-byte reads of 8 rows fall in different banks
 constexpr int kFinStages = 2;
 
@@ -70,16 +68,21 @@ __global__ void __launch_bounds__(256) base_norms_kernel(const float* __restrict
     }
 }
 
-// One warp per query: its window w = 2 eps + delta (key_window_l2 / _ip).
-__global__ void __launch_bounds__(256) prune_windows_kernel(PruneArgs a) {
+// One warp per query: its window w = 2 eps + delta (key_window_l2 / _ip), its operand row and its counter.
+__global__ void __launch_bounds__(256) prune_queries_kernel(PruneArgs a, __nv_bfloat16* __restrict__ qb, int kpad) {
     const int q = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (q >= a.nq) return;
+    const bool l2 = a.metric == ANN_METRIC_L2;
     float s = 0.f, e = 0.f;
-    for (int d = lane; d < a.dim; d += 32) {
-        const float v = a.q[(int64_t)q * a.dpad + d];
-        const float t = v - __bfloat162float(__float2bfloat16_rn(v));
+    const float* __restrict__ x = a.q + (int64_t)q * a.dpad;
+    for (int d = lane; d < kpad; d += 32) {
+        const float v = d < a.dim ? x[d] : 0.f;
+        const __nv_bfloat16 b = __float2bfloat16_rn(v);
+        const float t = v - __bfloat162float(b);
         s = fmaf(v, v, s);
         e = fmaf(t, t, e);
+        qb[(int64_t)q * kpad + d] = l2 && d >= a.dim && d < a.dim + 3 ? __float2bfloat16_rn(1.f)
+                                                                      : __float2bfloat16_rn(l2 ? -2.f * v : -v);
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
@@ -88,18 +91,11 @@ __global__ void __launch_bounds__(256) prune_windows_kernel(PruneArgs a) {
     }
     if (lane != 0) return;
     const float qn = sqrtf(s), rq = sqrtf(e);
-    const float w = a.metric == ANN_METRIC_L2 ? key_window_l2(qn, rq, a.b.cmax, a.b.rmax, a.dim)
-                                              : key_window_ip(qn, rq, a.b.cmax, a.b.rmax, a.dim);
+    const float w = l2 ? key_window_l2(qn, rq, a.b.cmax, a.b.rmax, a.dim) : key_window_ip(qn, rq, a.b.cmax, a.b.rmax, a.dim);
     const bool ok = qn <= kPruneNormMax && (qn >= kPruneNormMin || s == 0.f);  // false for NaN
     a.win[q] = ok ? w : __int_as_float(0x7fffffff);
-}
-
-__global__ void prune_bars_kernel(PruneArgs a) {
-    const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q == 0) *a.count = 0;
-    if (q >= a.nq) return;
-    a.tauX[q] = __fadd_ru(a.tauF[q], a.win[q]);
     a.rcount[q] = 0;
+    if (q == 0) *a.count = 0;
 }
 
 // One block per query (file comment, step 3). Bound by the gather of the kept rows (about 500 rows of 1.5 KB a query
@@ -107,8 +103,11 @@ __global__ void prune_bars_kernel(PruneArgs a) {
 // its own stage, and each lane then sums its own row in the scan's order -- a row's terms are one serial chain, so
 // 32 rows a warp, not 32 lanes a row, keep the FP32 pipe fed.
 //   staged scan: one chain over d; streaming scan: 8 chains (floats 4o .. 4o + 3 of every 32), added pairwise.
-template <bool STREAM, int METRIC>
-__global__ void __launch_bounds__(kFinThreads) prune_finish_kernel(PruneArgs a) {
+// Warps: 8, two blocks per SM; 16 where a launch has no second block for an SM (launch_prune_finish): one query over
+// 1M x 384, 33 -> 25 us.
+template <bool STREAM, int METRIC, int kFinWarps>
+__global__ void __launch_bounds__(kFinWarps * 32) prune_finish_kernel(PruneArgs a) {
+    constexpr int kFinThreads = kFinWarps * 32;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int cap = a.cap, k = a.k, dpad = a.dpad;
     float* sX = reinterpret_cast<float*>(smem_raw);                                  // [warps][stages][32 pitch]
@@ -130,7 +129,7 @@ __global__ void __launch_bounds__(kFinThreads) prune_finish_kernel(PruneArgs a) 
         uint32_t prefix = 0, mask = 0;
         int rem = k;
         for (int shift = 24; shift >= 0; shift -= 8) {
-            sHist[tid] = 0;
+            if (tid < 256) sHist[tid] = 0;
             __syncthreads();
             for (int i = tid; i < cnt; i += kFinThreads)
                 if ((sO[i] & mask) == prefix) atomicAdd(&sHist[(sO[i] >> shift) & 255u], 1);
@@ -242,14 +241,24 @@ __global__ void prune_gather_kernel(const float* __restrict__ q, int dpad, const
         for (int d = threadIdx.x; d < dpad; d += blockDim.x) qg[(int64_t)j * dpad + d] = q[(int64_t)list[j] * dpad + d];
 }
 
-size_t finish_smem(int cap, int dpad) {
-    return sizeof(float) * ((size_t)kFinWarps * kFinStages * 32 * kFinPitch + dpad) + sizeof(unsigned long long) * cap;
+size_t finish_smem(int cap, int dpad, int warps) {
+    return sizeof(float) * ((size_t)warps * kFinStages * 32 * kFinPitch + dpad) + sizeof(unsigned long long) * cap;
+}
+template <int W>
+int run_finish(const PruneArgs& a, cudaStream_t st) {
+    auto kern = a.metric == ANN_METRIC_L2
+                    ? (a.stream_form ? prune_finish_kernel<true, ANN_METRIC_L2, W> : prune_finish_kernel<false, ANN_METRIC_L2, W>)
+                    : (a.stream_form ? prune_finish_kernel<true, ANN_METRIC_IP, W> : prune_finish_kernel<false, ANN_METRIC_IP, W>);
+    ANN_CUDA_TRY(smem_optin(reinterpret_cast<const void*>(kern)));
+    kern<<<a.nq, W * 32, finish_smem(a.cap, a.dpad, W), st>>>(a);
+    ANN_LAUNCH_CHECK();
+    return ANN_OK;
 }
 
 }  // namespace
 
 int prune_cap(int k) { return k <= 128 ? 4096 : 8192; }
-bool prune_fits(int k, int dpad) { return k <= 512 && finish_smem(prune_cap(k), dpad) <= 200 * 1024; }
+bool prune_fits(int k, int dpad) { return k <= 512 && finish_smem(prune_cap(k), dpad, 8) <= 200 * 1024; }
 
 int prune_bar_rank(int k, int64_t S, int64_t n) {
     // keys of the k best met in the sample: about Poisson(k S / n); the rank past its 1 - 1e-7 quantile
@@ -272,14 +281,8 @@ int launch_base_norms(const float* x, int64_t n, int dim, int64_t ld, unsigned* 
     return ANN_OK;
 }
 
-int launch_prune_windows(const PruneArgs& a, cudaStream_t st) {
-    prune_windows_kernel<<<(unsigned)ceil_div(a.nq, 8), 256, 0, st>>>(a);
-    ANN_LAUNCH_CHECK();
-    return ANN_OK;
-}
-
-int launch_prune_bars(const PruneArgs& a, cudaStream_t st) {
-    prune_bars_kernel<<<(unsigned)ceil_div(a.nq, 256), 256, 0, st>>>(a);
+int launch_prune_queries(const PruneArgs& a, __nv_bfloat16* qb, int kpad, cudaStream_t st) {
+    prune_queries_kernel<<<(unsigned)ceil_div(a.nq, 8), 256, 0, st>>>(a, qb, kpad);
     ANN_LAUNCH_CHECK();
     return ANN_OK;
 }
@@ -287,13 +290,8 @@ int launch_prune_bars(const PruneArgs& a, cudaStream_t st) {
 int launch_prune_finish(const PruneArgs& a, cudaStream_t st) {
     ANN_CHECK_ARG(a.k >= 1 && prune_fits(a.k, a.dpad) && a.dpad % 32 == 0 && a.cap == prune_cap(a.k),
                   "pruned scan: k=%d, padded dim %d", a.k, a.dpad);
-    auto kern = a.metric == ANN_METRIC_L2
-                    ? (a.stream_form ? prune_finish_kernel<true, ANN_METRIC_L2> : prune_finish_kernel<false, ANN_METRIC_L2>)
-                    : (a.stream_form ? prune_finish_kernel<true, ANN_METRIC_IP> : prune_finish_kernel<false, ANN_METRIC_IP>);
-    ANN_CUDA_TRY(smem_optin(reinterpret_cast<const void*>(kern)));
-    kern<<<a.nq, kFinThreads, finish_smem(a.cap, a.dpad), st>>>(a);
-    ANN_LAUNCH_CHECK();
-    return ANN_OK;
+    const bool wide = a.nq <= kNumSMs && finish_smem(a.cap, a.dpad, 16) <= 220 * 1024;
+    return wide ? run_finish<16>(a, st) : run_finish<8>(a, st);
 }
 
 int launch_prune_gather(const float* q, int dpad, const int* list, const int* count, int nq, float* qg, cudaStream_t st) {

@@ -1,5 +1,6 @@
 // Launch interfaces of the pruned exact scan (flat_prune.cu).
 #pragma once
+#include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -51,7 +52,6 @@ struct PruneArgs {
     PruneBounds b;
     float* win;         // [nq] window: 2 eps + delta (NaN: the query is not covered by the bound)
     const float* tauF;  // [nq] sampled bar
-    float* tauX;        // [nq] filter bar tauF + win
     int cap;            // survivors kept per query
     float* fkey;        // [nq, cap] survivors: key, position
     int* fcol;
@@ -67,9 +67,9 @@ bool prune_fits(int k, int dpad);
 // Rank of the sampled bar: with S of n keys sampled, the smallest rank r for which the k smallest keys lie at or
 // below the r-th smallest sampled key with probability of about 1 - 1e-7.
 int prune_bar_rank(int k, int64_t S, int64_t n);
-int launch_prune_windows(const PruneArgs& a, cudaStream_t st);  // win
-int launch_prune_bars(const PruneArgs& a, cudaStream_t st);     // tauX; rcount and count zeroed
-int launch_prune_finish(const PruneArgs& a, cudaStream_t st);   // results, list and count
+// win and the queries' operand rows qb [nq, kpad] (launch_tc_operand's); rcount and count zeroed.
+int launch_prune_queries(const PruneArgs& a, __nv_bfloat16* qb, int kpad, cudaStream_t st);
+int launch_prune_finish(const PruneArgs& a, cudaStream_t st);  // results, list and count
 // qg[j] = q[list[j]] for j < *count.
 int launch_prune_gather(const float* q, int dpad, const int* list, const int* count, int nq, float* qg, cudaStream_t st);
 

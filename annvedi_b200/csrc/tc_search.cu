@@ -183,25 +183,6 @@ __device__ uint32_t warp_kth_ord(const float* __restrict__ keys, int64_t n, int6
     return prefix;
 }
 
-// One warp per query: bar1 / bar2 = the r1-th / r2-th smallest of the query's keys[offs[q] .. + lens[q])
-// (+inf where the stream is shorter).
-__global__ void __launch_bounds__(256) warp_bars_kernel(const float* __restrict__ keys, const int64_t* __restrict__ offs,
-                                                        const int64_t* __restrict__ lens, int nq, int r1, int r2,
-                                                        float* __restrict__ bar1, float* __restrict__ bar2) {
-    __shared__ int sHist[8][256];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int q = blockIdx.x * 8 + warp;
-    if (q >= nq) return;  // the whole warp
-    const float* kq = keys + offs[q];
-    const int64_t n = lens[q];
-    const float b1 = r1 <= n ? from_ord(warp_kth_ord(kq, n, r1, sHist[warp])) : kInf;
-    const float b2 = r2 <= n ? from_ord(warp_kth_ord(kq, n, r2, sHist[warp])) : kInf;
-    if (lane == 0) {
-        bar1[q] = b1;
-        bar2[q] = b2;
-    }
-}
-
 // The digit of rank `rem` (1-based) in a 256-bin histogram and the count of keys below that digit, on
 // every lane of the warp.
 __device__ __forceinline__ void warp_hist_pick(const int* hist, int64_t rem, int* digit, int* before) {
@@ -289,13 +270,18 @@ __global__ void __launch_bounds__(kBarThreads) block_bars_kernel(const float* __
                                                                  const int64_t* __restrict__ offs,
                                                                  const int64_t* __restrict__ lens, int64_t ld, int nq,
                                                                  int r1, int r2, int staged, float* __restrict__ bar1,
-                                                                 float* __restrict__ bar2) {
+                                                                 float* __restrict__ bar2,
+                                                                 const float* __restrict__ add2) {
     extern __shared__ uint32_t smem_bars[];
     __shared__ int sHist[2][256];
     __shared__ int sPick[4];  // digit and count below it, per rank
     const int q = blockIdx.x;
     if (q >= nq) return;  // the whole block
     const int warp = threadIdx.x >> 5;
+    auto put = [&](float b1, float b2) {
+        bar1[q] = b1;
+        bar2[q] = add2 ? __fadd_ru(b2, add2[q]) : b2;
+    };
     const int64_t n = lens ? lens[q] : ld;
     const float* kq = keys + (offs ? offs[q] : q * ld);
     const bool in_smem = n <= staged;
@@ -337,10 +323,7 @@ __global__ void __launch_bounds__(kBarThreads) block_bars_kernel(const float* __
         const float lo = from_ord(sMinMax[0]), hi = from_ord(sMinMax[1]);
         const float scale = (float)kBarBins / (hi - lo);
         if (!(hi > lo) || !isfinite(scale)) {  // every key the same (or not finite): each rank's key is lo
-            if (threadIdx.x == 0 && hi == lo) {
-                bar1[q] = want1 ? lo : kInf;
-                bar2[q] = want2 ? lo : kInf;
-            }
+            if (threadIdx.x == 0 && hi == lo) put(want1 ? lo : kInf, want2 ? lo : kInf);
             if (hi == lo) return;
         } else {
             auto bin_of = [&](uint32_t o) { return min(kBarBins - 1, (int)((from_ord(o) - lo) * scale)); };
@@ -381,10 +364,7 @@ __global__ void __launch_bounds__(kBarThreads) block_bars_kernel(const float* __
                     }
                 }
                 __syncthreads();
-                if (threadIdx.x == 0) {
-                    bar1[q] = want1 ? sRes[0] : kInf;
-                    bar2[q] = want2 ? sRes[1] : kInf;
-                }
+                if (threadIdx.x == 0) put(want1 ? sRes[0] : kInf, want2 ? sRes[1] : kInf);
                 return;
             }
         }
@@ -423,10 +403,7 @@ __global__ void __launch_bounds__(kBarThreads) block_bars_kernel(const float* __
         }
         pmask |= 255u << shift;
     }
-    if (threadIdx.x == 0) {
-        bar1[q] = want1 ? from_ord(p1) : kInf;
-        bar2[q] = want2 ? from_ord(p2) : kInf;
-    }
+    if (threadIdx.x == 0) put(want1 ? from_ord(p1) : kInf, want2 ? from_ord(p2) : kInf);
 }
 
 // One warp per query: the R smallest of the query's (key, id) buffer [q * cap, + min(count[q], cap)) as a set:
@@ -998,18 +975,13 @@ int launch_max_int(const int* v, int n, int* out, cudaStream_t st) {
     return ANN_OK;
 }
 
-int launch_warp_bars(const float* keys, const int64_t* offs, const int64_t* lens, int nq, int r1, int r2, float* bar1,
-                     float* bar2, cudaStream_t st, int64_t max_len) {
+int launch_bars(const float* keys, const int64_t* offs, const int64_t* lens, int nq, int r1, int r2, float* bar1,
+                float* bar2, cudaStream_t st, int64_t max_len, const float* add2) {
     if (nq == 0) return ANN_OK;
-    ANN_CHECK_ARG(r1 >= 1 && r2 >= 1, "bars: ranks %d, %d", r1, r2);
-    ANN_CHECK_ARG(max_len > 0 || (offs && lens), "bars: streams without offsets need their length");
-    if (max_len > 0) {  // one block per query; streams of up to 8,192 keys (32 KB) staged in shared memory
-        const int staged = (int)std::min<int64_t>(max_len, 8192);
-        block_bars_kernel<<<(unsigned)nq, kBarThreads, (size_t)staged * 4, st>>>(keys, offs, lens, max_len, nq, r1, r2,
-                                                                                staged, bar1, bar2);
-    } else {
-        warp_bars_kernel<<<(unsigned)ceil_div(nq, 8), 256, 0, st>>>(keys, offs, lens, nq, r1, r2, bar1, bar2);
-    }
+    ANN_CHECK_ARG(r1 >= 1 && r2 >= 1 && max_len >= 1, "bars: ranks %d, %d of %lld keys", r1, r2, (long long)max_len);
+    const int staged = (int)std::min<int64_t>(max_len, 8192);  // 32 KB
+    block_bars_kernel<<<(unsigned)nq, kBarThreads, (size_t)staged * 4, st>>>(keys, offs, lens, max_len, nq, r1, r2, staged,
+                                                                            bar1, bar2, add2);
     ANN_LAUNCH_CHECK();
     return ANN_OK;
 }
