@@ -69,6 +69,29 @@ __device__ __forceinline__ SelectBound block_select_bound(At&& at, int m, int k,
     return b;
 }
 
+// Exclusive prefix of v over the block's 1,024 threads; *total = the sum. sWarp: 32 words.
+__device__ __forceinline__ int64_t block_prefix(int64_t v, int64_t* sWarp, int64_t* total) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int64_t incl = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int64_t y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += y;
+    }
+    if (lane == 31) sWarp[warp] = incl;
+    __syncthreads();
+    int64_t w = sWarp[lane];  // every warp sums the warps' totals
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int64_t y = __shfl_up_sync(0xffffffffu, w, o);
+        if (lane >= o) w += y;
+    }
+    *total = __shfl_sync(0xffffffffu, w, 31);
+    const int64_t before = __shfl_sync(0xffffffffu, w, warp > 0 ? warp - 1 : 0);
+    __syncthreads();  // sWarp is free
+    return (warp > 0 ? before : 0) + incl - v;
+}
+
 // Ascending bitonic sort of n words (a power of two) in shared memory by the block; starts and ends with a barrier.
 __device__ __forceinline__ void block_sort_u64(unsigned long long* w, int n) {
     __syncthreads();

@@ -1434,6 +1434,15 @@ static int ivf_query_device(ann_ivf* h, ann_workspace* ws, const IvfQueryCfg& c,
             ss.total_items = titem + h->C;
             ss.desc = titem_desc;
             ss.cap = items_cap;
+            if (nq * c.npc <= kSmallSetupRows) {
+                const TcOperands op = tc_operands(h, c, qb, q8, qfac, pfac);
+                ss.qrows = op.qrows;
+                ss.row_bytes = op.row_bytes;
+                ss.A = Apk;
+                ss.dbase = dbase;
+                ss.qfac = op.qfac;
+                ss.pfac = op.pfac;
+            }
             if ((rc = launch_tc_small_setup(a, ss, st))) return rc;
             tot[1] = c.small_keys;
         } else if (sampled) {
@@ -1455,7 +1464,8 @@ static int ivf_query_device(ann_ivf* h, ann_workspace* ws, const IvfQueryCfg& c,
                 const TcOperands op = tc_operands(h, c, qb, q8, qfac, pfac);
                 const int64_t max_pairs = (int64_t)nq * c.npc;
                 const int64_t* n_pairs = c.small_tc ? b.total_items : b.lq_off + h->C;
-                if ((rc = launch_tc_ivf_pairs(op.qrows, op.row_bytes, b.pair_vals, b.pair_lists, n_pairs, max_pairs, c.npc,
+                if (!(c.small_tc && nq * c.npc <= kSmallSetupRows) &&
+                    (rc = launch_tc_ivf_pairs(op.qrows, op.row_bytes, b.pair_vals, b.pair_lists, n_pairs, max_pairs, c.npc,
                                               b.cand_off, a.plan.seg_pref, h->list_off, Apk, dbase, st, op.qfac,
                                               op.pfac)))
                     return rc;
@@ -1735,7 +1745,7 @@ int ann_ivf_query(ann_ivf* h, ann_workspace* ws, const float* queries, int32_t n
     }
     // One CTA sets up a small tensor-core batch whose queries are sure to find k rows: up to 1,024 pairs and 64 MB of
     // stream keys, sized by the largest lists. One query x 4 lists at 1M x 384: 154 us a call by the batch's ten
-    // launches and a wait for their totals, 110 us.
+    // launches and a wait for their totals, 110 us (72 with 64 pairs' operand rows in the set-up and 32-warp re-ranks).
     // (A cap below k could end a stream short of k after all.)
     c.small_keys = (int64_t)qc * c.npc * h->sizes_desc[0];
     c.small_tc = c.tc && nq < h->sampled_min_queries && !c.fallback && (c.shard || c.max_c >= k) &&

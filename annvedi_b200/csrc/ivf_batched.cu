@@ -16,6 +16,7 @@
 // on the batch it came in: diff_d = fma(code_d, scale_d, -(q_d - offset_d)), the squares summed by fused
 // multiply-adds in dimension order separately over the two halves of the padded code row, then
 // low + high. The FP32 re-rank that follows decides the final order.
+#include "block_select.cuh"
 #include "common.cuh"
 #include "ivf.cuh"
 #include "ivf_batched.cuh"
@@ -63,36 +64,13 @@ __global__ void pair_rank_kernel(IvfPlan p, int* __restrict__ cnt, int32_t* __re
     t.slen[q] = run;
 }
 
-// Exclusive prefix of v over the block's 1,024 threads; *total = the sum.
-__device__ __forceinline__ int64_t prefix_1024(int64_t v, int64_t* sWarp, int64_t* total) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    int64_t incl = v;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int64_t y = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += y;
-    }
-    if (lane == 31) sWarp[warp] = incl;
-    __syncthreads();
-    int64_t w = sWarp[lane];  // every warp sums the warps' totals
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int64_t y = __shfl_up_sync(0xffffffffu, w, o);
-        if (lane >= o) w += y;
-    }
-    *total = __shfl_sync(0xffffffffu, w, 31);
-    const int64_t before = __shfl_sync(0xffffffffu, w, warp > 0 ? warp - 1 : 0);
-    __syncthreads();  // sWarp is free
-    return (warp > 0 ? before : 0) + incl - v;
-}
-
 // out[0..n] = the exclusive sums of v(0..n) by one block, a run of them a thread.
 template <class V>
 __device__ __forceinline__ int64_t block_offsets(int n, int64_t* out, int64_t* sWarp, V&& v) {
     const int per = (n + 1023) / 1024, i0 = min(n, (int)threadIdx.x * per), i1 = min(n, i0 + per);
     int64_t sum = 0, total;
     for (int i = i0; i < i1; ++i) sum += v(i);
-    int64_t run = prefix_1024(sum, sWarp, &total);
+    int64_t run = block_prefix(sum, sWarp, &total);
     for (int i = i0; i < i1; ++i) {
         out[i] = run;
         run += v(i);

@@ -811,25 +811,10 @@ int launch_tc_coarse(const float* keys, int64_t ldk, int nq, int C, int npc, int
 }
 
 namespace {
-// Exclusive prefix of v over the block's 1,024 threads; *total = the sum. sPart: 1,024 words.
-__device__ __forceinline__ int64_t block_prefix(int64_t v, int64_t* sPart, int64_t* total) {
-    sPart[threadIdx.x] = v;
-    __syncthreads();
-    for (int off = 1; off < 1024; off <<= 1) {
-        const int64_t y = threadIdx.x >= off ? sPart[threadIdx.x - off] : 0;
-        __syncthreads();
-        sPart[threadIdx.x] += y;
-        __syncthreads();
-    }
-    const int64_t r = sPart[threadIdx.x] - v;
-    *total = sPart[1023];
-    __syncthreads();
-    return r;
-}
-
 // One CTA: thread q plans query q, thread e is pair e, thread g is group (list) g. A call of a few queries is bound by
 // the chain of its launches, not by their work: this one takes the place of ten (plan, pairs, sort, list offsets, items
-// twice, two scans, descriptors: 45 us of a query's 118 us) and of a wait for their totals on the host.
+// twice, two scans, descriptors: 45 us of a query's 118 us) and of a wait for their totals on the host, and of the operand
+// rows' launch where they are few (s.A given).
 __global__ void __launch_bounds__(1024) tc_small_setup_kernel(IvfQueryArgs a, TcSmallSetup s) {
     __shared__ unsigned long long sKey[kSmallSetupPairs];
     __shared__ int64_t sPart[1024];
@@ -906,12 +891,25 @@ __global__ void __launch_bounds__(1024) tc_small_setup_kernel(IvfQueryArgs a, Tc
                                               (int)min((int64_t)256, nr - rt * 256));
         }
     }
+    // operand rows (as launch_tc_ivf_pairs): a warp per pair
+    for (int i = tid >> 5; s.A && i < n_valid; i += 32) {
+        const int v = (int)(unsigned)sKey[i], q = v / npc, j = v % npc, lane = tid & 31;
+        const uint4* src = reinterpret_cast<const uint4*>(static_cast<const char*>(s.qrows) + (size_t)q * s.row_bytes);
+        uint4* dst = reinterpret_cast<uint4*>(static_cast<char*>(s.A) + (size_t)i * s.row_bytes);
+        for (int c = lane; c < s.row_bytes / 16; c += 32) dst[c] = src[c];
+        if (lane == 0) {
+            if (s.pfac) s.pfac[i] = s.qfac[q];
+            // (cand_off and seg_pref were written by this block, before its barriers)
+            s.dbase[i] = s.cand_off[q] + p.seg_pref[(int64_t)q * (npc + 1) + j] - a.ix.list_off[(int)(sKey[i] >> 32)];
+        }
+    }
 }
 }  // namespace
 
 int launch_tc_small_setup(const IvfQueryArgs& a, const TcSmallSetup& s, cudaStream_t st) {
     ANN_CHECK_ARG(a.plan.nq >= 1 && (int64_t)a.plan.nq * a.plan.npc <= kSmallSetupPairs, "small set-up: %d queries x %d lists",
                   a.plan.nq, a.plan.npc);
+    ANN_CHECK_ARG(s.A == nullptr || (s.dbase && s.row_bytes % 16 == 0), "small set-up: operand rows of %d bytes", s.row_bytes);
     tc_small_setup_kernel<<<1, 1024, 0, st>>>(a, s);
     ANN_LAUNCH_CHECK();
     return ANN_OK;

@@ -40,7 +40,15 @@ struct TcSmallSetup {
     int64_t* total_items; // [1]
     int4* desc;           // [cap]
     int64_t cap;
+    // the pairs' operand rows as launch_tc_ivf_pairs lays them out (A null: left to it)
+    const void* qrows = nullptr;
+    int row_bytes = 0;
+    void* A = nullptr;
+    int64_t* dbase = nullptr;
+    const float* qfac = nullptr;
+    float* pfac = nullptr;
 };
+constexpr int kSmallSetupRows = 64;  // up to here the one CTA copies them in less than a launch
 int launch_tc_small_setup(const IvfQueryArgs& a, const TcSmallSetup& s, cudaStream_t st);
 // For each valid pair i (< lq_off[C]; pairs grouped by list, pair_vals = q * npc + j, pair_lists = the
 // list): A[i] = qb[q] (kpad BF16 columns) and dbase[i] = cand_off[q] + seg_pref[q][j] - list_off[list],
