@@ -18,8 +18,10 @@
 // segment's `lim` smallest distances are found on their own (compat_segments_kernel), merged into the heap the
 // reference holds at every segment's first row (compat_prefix_kernel), and one warp a segment walks its rows from
 // there, replaying insertions (rows with D < T, rare once T settles) and recording each row's threshold
-// (compat_threshold_kernel). As one walk of all rows by one warp this took 248 of a query's 436 us at 100k x 384; what
-// bounds it now is the first segment's walk, about 240 insertions of 290 clocks each (37 us).
+// (compat_threshold_kernel). As one walk of all rows by one warp this took 248 of a query's 436 us at 100k x 384. The
+// walk inserts 64 ln(b / a) rows of [a, b) on random data, 290 clocks each, so the first segment's alone is most of it
+// (240 insertions, 32 us of 163): it is cut again at 128, 256, 512 and 1024, five warps that make their own starting heap
+// from the rows before (a few chunks of 64, sorted and merged): 44 insertions each, 15 us.
 // Pass 3 (compat_values_kernel) picks v_i from D, P and T_i, and each segment's k best (v_i, i) by block; the k best of
 // those, sorted, are the result (compat_final_kernel).
 #include <cfloat>
@@ -141,10 +143,51 @@ __global__ void __launch_bounds__(256) compat_segments_kernel(CompatArgs a) {
     }
 }
 
+// The `lim` smallest of two ascending lists of 64 values (FLT_MAX: none), (lo, hi) and (b0, b1): lane l holds values l and
+// l + 32. min(a[i], b[63 - i]) are the 64 smallest, a bitonic sequence, which six exchange steps sort.
+__device__ __forceinline__ void heap_merge(float& lo, float& hi, float b0, float b1, int lim) {
+    const int lane = threadIdx.x & 31;
+    // value i meets value 63 - i: lane l's lo meets lane 31 - l's hi, and its hi meets that lane's lo
+    lo = fminf(lo, __shfl_xor_sync(0xffffffffu, b1, 31));
+    hi = fminf(hi, __shfl_xor_sync(0xffffffffu, b0, 31));
+    const float t = fminf(lo, hi);  // step 32
+    hi = fmaxf(lo, hi);
+    lo = t;
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) {
+        const float ol = __shfl_xor_sync(0xffffffffu, lo, d), oh = __shfl_xor_sync(0xffffffffu, hi, d);
+        const bool low = (lane & d) == 0;
+        lo = low ? fminf(lo, ol) : fmaxf(lo, ol);
+        hi = low ? fminf(hi, oh) : fmaxf(hi, oh);
+    }
+    if (lane >= lim) lo = FLT_MAX;
+    if (lane + 32 >= lim) hi = FLT_MAX;
+}
+
+// Ascending order of a warp's 64 values, lane l holding values l and l + 32.
+__device__ __forceinline__ void heap_sort(float& lo, float& hi) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int size = 2; size <= 64; size <<= 1) {
+        if (size == 64) {  // step 32
+            const float t = fminf(lo, hi);
+            hi = fmaxf(lo, hi);
+            lo = t;
+        }
+#pragma unroll
+        for (int d = size == 64 ? 16 : size >> 1; d > 0; d >>= 1) {
+            const float ol = __shfl_xor_sync(0xffffffffu, lo, d), oh = __shfl_xor_sync(0xffffffffu, hi, d);
+            const bool low = (lane & d) == 0;
+            const bool up_lo = (lane & size) == 0, up_hi = ((lane + 32) & size) == 0;  // ascending runs
+            lo = low == up_lo ? fminf(lo, ol) : fmaxf(lo, ol);
+            hi = low == up_hi ? fminf(hi, oh) : fmaxf(hi, oh);
+        }
+    }
+}
+
 // One warp per query: seg_heap[s] := the heap the reference holds at segment s's first row, the `lim` smallest of the
-// earlier segments' lists. Two ascending lists a, b of 64 values: min(a[i], b[63 - i]) are the 64 smallest, a bitonic
-// sequence, which six exchange steps sort. Lane l holds values l and l + 32. The lists are staged in shared memory by
-// the block first: a list's load from L2 takes longer than its merge.
+// earlier segments' lists. The lists are staged in shared memory by the block first: a list's load from L2 takes longer
+// than its merge.
 __global__ void __launch_bounds__(256) compat_prefix_kernel(CompatArgs a) {
     __shared__ float sL[kSelectSegs * 64];
     const int lane = threadIdx.x & 31, qi = blockIdx.x;
@@ -158,39 +201,44 @@ __global__ void __launch_bounds__(256) compat_prefix_kernel(CompatArgs a) {
         L[s * 64 + lane] = lo;
         L[s * 64 + lane + 32] = hi;
         if (s + 1 >= a.nseg) break;
-        const float b0 = sL[s * 64 + lane], b1 = sL[s * 64 + lane + 32];
-        // value i meets value 63 - i: lane l's lo meets lane 31 - l's hi, and its hi meets that lane's lo
-        lo = fminf(lo, __shfl_xor_sync(0xffffffffu, b1, 31));
-        hi = fminf(hi, __shfl_xor_sync(0xffffffffu, b0, 31));
-        const float t = fminf(lo, hi);  // step 32
-        hi = fmaxf(lo, hi);
-        lo = t;
-#pragma unroll
-        for (int d = 16; d > 0; d >>= 1) {
-            const float ol = __shfl_xor_sync(0xffffffffu, lo, d), oh = __shfl_xor_sync(0xffffffffu, hi, d);
-            const bool low = (lane & d) == 0;
-            lo = low ? fminf(lo, ol) : fmaxf(lo, ol);
-            hi = low ? fminf(hi, oh) : fmaxf(hi, oh);
-        }
-        if (lane >= lim) lo = FLT_MAX;
-        if (lane + 32 >= lim) hi = FLT_MAX;
+        heap_merge(lo, hi, sL[s * 64 + lane], sL[s * 64 + lane + 32], lim);
     }
 }
 
-// One warp per (segment, query): each row's threshold, from the segment's starting heap.
+// One warp per (segment, query), several for the first segment: each row's threshold, from the starting heap.
+constexpr int kFirstCuts = 5;  // the first segment's rows from 0, 128, 256, 512 and 1024
 __global__ void __launch_bounds__(32 * kCompatWarps) compat_threshold_kernel(CompatArgs a) {
-    const int s = blockIdx.x * kCompatWarps + (threadIdx.x >> 5), lane = threadIdx.x & 31, qi = blockIdx.y;
+    const int w = blockIdx.x * kCompatWarps + (threadIdx.x >> 5), lane = threadIdx.x & 31, qi = blockIdx.y;
+    const int s = w < kFirstCuts ? 0 : w - (kFirstCuts - 1);
     if (s >= a.nseg) return;  // the whole warp
+    const int lim = a.k < 64 ? a.k : 64;
+    const float* D = a.D + (int64_t)qi * a.n;
+    float* T = a.T + (int64_t)qi * a.n;
+    int64_t begin = (int64_t)s * a.seg_rows, end = min(a.n, begin + a.seg_rows);
     WarpHeap64 heap;
-    heap.init(a.k < 64 ? a.k : 64);
+    heap.init(lim);
     if (s > 0) {
         const float* L = a.seg_heap + ((int64_t)qi * a.nseg + s) * 64;
         heap.lo = L[lane];
         heap.hi = L[lane + 32];
+    } else {
+        if (w > 0) begin = (int64_t)64 << w;
+        if (begin >= end) return;  // the whole warp
+        if (w + 1 < kFirstCuts) end = min(end, (int64_t)128 << w);
+        if (w == 0 && lim == 64) {  // no threshold before 64 rows are seen
+            const int64_t m = min((int64_t)64, end);
+            if (lane < m) T[lane] = FLT_MAX;
+            if (lane + 32 < m) T[lane + 32] = FLT_MAX;
+            begin = 64;
+        }
+        for (int64_t r = 0; r < begin; r += 64) {
+            const float d0 = r + lane < end ? D[r + lane] : FLT_MAX, d1 = r + lane + 32 < end ? D[r + lane + 32] : FLT_MAX;
+            float b0 = d0 < FLT_MAX ? d0 : FLT_MAX, b1 = d1 < FLT_MAX ? d1 : FLT_MAX;  // inf, NaN: never held
+            heap_sort(b0, b1);
+            heap_merge(heap.lo, heap.hi, b0, b1, lim);
+        }
     }
-    const int64_t begin = (int64_t)s * a.seg_rows;
-    float* T = a.T + (int64_t)qi * a.n;
-    compat_walk(a.D + (int64_t)qi * a.n, begin, min(a.n, begin + a.seg_rows), heap, [&](int64_t i, float t, bool valid) {
+    compat_walk(D, begin, end, heap, [&](int64_t i, float t, bool valid) {
         if (valid) T[i] = t;
     });
 }
@@ -266,7 +314,7 @@ int launch_compat(CompatArgs a, int q_begin, int q_count, cudaStream_t st) {
     dim3 g1((unsigned)rblocks, (unsigned)ceil_div(q_count, kCompatQG));
     partials<<<g1, 256, smem, st>>>(a, q_begin);
     ANN_LAUNCH_CHECK();
-    const dim3 gw((unsigned)ceil_div(a.nseg, kCompatWarps), (unsigned)q_count);
+    const dim3 gw((unsigned)ceil_div(a.nseg + kFirstCuts - 1, kCompatWarps), (unsigned)q_count);
     if (a.nseg > 1) {
         compat_segments_kernel<<<dim3(a.nseg - 1, (unsigned)q_count), 256, 0, st>>>(a);
         ANN_LAUNCH_CHECK();
