@@ -185,23 +185,39 @@ __device__ __forceinline__ void heap_sort(float& lo, float& hi) {
     }
 }
 
-// One warp per query: seg_heap[s] := the heap the reference holds at segment s's first row, the `lim` smallest of the
-// earlier segments' lists. The lists are staged in shared memory by the block first: a list's load from L2 takes longer
-// than its merge.
+// One block per query: seg_heap[s] := the heap the reference holds at segment s's first row, the `lim` smallest of the
+// earlier segments' lists. Staged in shared memory: a list's load from L2 takes longer than its merge. Eight warps: each
+// merges its run of lists, then the runs before it, then those into its own heaps: 13 + 7 + 13 merges in a chain
+// instead of 97 (98 segments: 15.8 -> 7.8 us).
 __global__ void __launch_bounds__(256) compat_prefix_kernel(CompatArgs a) {
     __shared__ float sL[kSelectSegs * 64];
-    const int lane = threadIdx.x & 31, qi = blockIdx.x;
+    __shared__ float sRun[8 * 64];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, qi = blockIdx.x;
     const int lim = a.k < 64 ? a.k : 64;
     float* L = a.seg_heap + (int64_t)qi * a.nseg * 64;
     for (int i = threadIdx.x; i < (a.nseg - 1) * 64; i += 256) sL[i] = L[i];  // the last segment has no list
     __syncthreads();
-    if (threadIdx.x >= 32) return;
+    const int per = (a.nseg + 7) / 8, s0 = min(a.nseg, warp * per), s1 = min(a.nseg, s0 + per);
     float lo = FLT_MAX, hi = FLT_MAX;
-    for (int s = 0; s < a.nseg; ++s) {
-        L[s * 64 + lane] = lo;
-        L[s * 64 + lane + 32] = hi;
-        if (s + 1 >= a.nseg) break;
-        heap_merge(lo, hi, sL[s * 64 + lane], sL[s * 64 + lane + 32], lim);
+    for (int s = s0; s < s1; ++s) {  // the heap of the run's earlier lists, in place
+        float* l = sL + s * 64;
+        const bool has = s + 1 < a.nseg;
+        const float b0 = has ? l[lane] : FLT_MAX, b1 = has ? l[lane + 32] : FLT_MAX;
+        l[lane] = lo;
+        l[lane + 32] = hi;
+        heap_merge(lo, hi, b0, b1, lim);
+    }
+    sRun[warp * 64 + lane] = lo;
+    sRun[warp * 64 + lane + 32] = hi;
+    __syncthreads();
+    lo = hi = FLT_MAX;
+    for (int r = 0; r < warp; ++r) heap_merge(lo, hi, sRun[r * 64 + lane], sRun[r * 64 + lane + 32], lim);
+#pragma unroll 2
+    for (int s = s0; s < s1; ++s) {
+        float h0 = sL[s * 64 + lane], h1 = sL[s * 64 + lane + 32];
+        heap_merge(h0, h1, lo, hi, lim);
+        L[s * 64 + lane] = h0;
+        L[s * 64 + lane + 32] = h1;
     }
 }
 
@@ -273,8 +289,11 @@ __global__ void __launch_bounds__(256) compat_values_kernel(CompatArgs a) {
     segment_select(T, begin, m, a.k, a.seg_best + ((int64_t)qi * a.nseg + s) * a.k, sHist, sMisc, &sN);
 }
 
-// The k best of the segments' best, in order. One block per query.
-__global__ void __launch_bounds__(512) compat_final_kernel(CompatArgs a, int q_begin) {
+// The k best of the segments' best, in order. One block per query; the words are read once into shared memory where
+// they fit (98 segments of 100: 20 -> 13 us), which six passes over them follow.
+constexpr int kFinalThreads = 1024, kFinalStaged = 20480;
+__global__ void __launch_bounds__(kFinalThreads) compat_final_kernel(CompatArgs a, int q_begin) {
+    extern __shared__ __align__(16) unsigned long long sW[];
     __shared__ int sHist[256];
     __shared__ int sMisc[12];
     __shared__ int sN;
@@ -282,16 +301,20 @@ __global__ void __launch_bounds__(512) compat_final_kernel(CompatArgs a, int q_b
     const int qi = blockIdx.x;
     const unsigned long long* w = a.seg_best + (int64_t)qi * a.nseg * a.k;
     const int m = a.nseg * a.k;
+    if (m <= kFinalStaged) {
+        for (int i = threadIdx.x; i < m; i += kFinalThreads) sW[i] = w[i];
+        w = sW;
+    }
     if (threadIdx.x == 0) sN = 0;
     __syncthreads();
     const SelectBound b = block_select_bound([&](int i) { return w[i]; }, m, a.k, sHist, sMisc);
     const int p2 = pow2_ceil(a.k);
-    for (int i = threadIdx.x; i < m; i += 512)
+    for (int i = threadIdx.x; i < m; i += kFinalThreads)
         if (b.in(w[i])) sR[atomicAdd(&sN, 1)] = w[i];
-    for (int i = a.k + threadIdx.x; i < p2; i += 512) sR[i] = ~0ull;
+    for (int i = a.k + threadIdx.x; i < p2; i += kFinalThreads) sR[i] = ~0ull;
     block_sort_u64(sR, p2);
     const int64_t o = (int64_t)(q_begin + qi) * a.k;
-    for (int e = threadIdx.x; e < a.k; e += 512) {
+    for (int e = threadIdx.x; e < a.k; e += kFinalThreads) {
         if (a.out_ids) a.out_ids[o + e] = (int64_t)(unsigned)sR[e];
         if (a.out_dists) a.out_dists[o + e] = f32_ord((uint32_t)(sR[e] >> 32));
     }
@@ -325,7 +348,9 @@ int launch_compat(CompatArgs a, int q_begin, int q_count, cudaStream_t st) {
     ANN_LAUNCH_CHECK();
     compat_values_kernel<<<dim3(a.nseg, (unsigned)q_count), 256, 0, st>>>(a);
     ANN_LAUNCH_CHECK();
-    compat_final_kernel<<<(unsigned)q_count, 512, 0, st>>>(a, q_begin);
+    const int64_t words = (int64_t)a.nseg * a.k;
+    ANN_CUDA_TRY(smem_optin(reinterpret_cast<const void*>(compat_final_kernel)));
+    compat_final_kernel<<<(unsigned)q_count, kFinalThreads, words <= kFinalStaged ? words * 8 : 0, st>>>(a, q_begin);
     ANN_LAUNCH_CHECK();
     return ANN_OK;
 }
