@@ -1232,6 +1232,13 @@ def main():
     ap.add_argument("--no-cpu-baseline", action="store_true")
     args = ap.parse_args()
     args.warmup = max(3, args.warmup)
+    # the compiled reference (oracle/Makefile) needs the reference's sources, which a checkout need not have
+    no_ref = not os.path.isdir(os.path.join(ROOT, "oracle", "_ref"))
+    missing = "the compiled reference (oracle/_ref) is not built here"
+    if args.impl == "reference" and no_ref:
+        if int(os.environ.get("RANK", "0")) == 0:
+            print(json.dumps({"impl": "reference", "unavailable": missing}), flush=True)
+        return
     if args.impl == "reference":
         # host-only arm: rank 0 runs it, the other ranks exit without work (no process group needed)
         line = run_reference(args, int(os.environ.get("RANK", "0")), int(os.environ.get("WORLD_SIZE", "1")))
@@ -1239,7 +1246,11 @@ def main():
             print(json.dumps(line), flush=True)
         return
     rank, world, local = dist_setup()
+    want_baseline = not args.no_cpu_baseline
+    args.no_cpu_baseline = args.no_cpu_baseline or no_ref
     line = run_ours(args, rank, world, local)
+    if want_baseline and no_ref and line is not None and world == 1:
+        line["cpu_baseline"] = {"unavailable": missing}
     if rank == 0 and line is not None:
         print(json.dumps(line), flush=True)
     if world > 1:
