@@ -67,6 +67,7 @@ struct ann_ivf {
     bool codes_known = false;
     double prune_credit_us = 0.0;
     int prune_failed = 0;  // batches in a row that it could not settle
+    double cand_rate = 0;  // candidates a probe had in the latest exact batch (0: none yet)
     std::mutex tc_mu;
     int64_t query_count = 0;
     // query options (ann_ivf_set_option)
@@ -103,6 +104,7 @@ static void ivf_free_state(ann_ivf* h) {
     h->code_cmax = 0.f;
     h->codes_known = false;
     h->prune_failed = 0;
+    h->cand_rate = 0.0;
     h->prune_credit_us = 0.0;
     h->sq8_fac = nullptr;
     h->proj = h->projT = h->lsh_mean = nullptr;
@@ -1454,6 +1456,10 @@ static int ivf_query_device(ann_ivf* h, ann_workspace* ws, const IvfQueryCfg& c,
         }
         if (tot[2] != 0) sampled_done = false;
         if (plan_apart) every_row.resize((size_t)(int)tot[3]);  // the plan has listed them in every_list
+        if (!c.tc && tot[2] == 0) {
+            std::lock_guard<std::mutex> lk(h->tc_mu);
+            h->cand_rate = (double)tot[1] / ((double)nq * c.npc);
+        }
         done = sampled_done;
         if (tot[2] == 0 && !sampled_done) {  // no query fell back to scanning every row
             if ((rc = ws_reserve_big(ws, sizeof(float) * (size_t)std::max<int64_t>(tot[1], 1)))) return rc;
@@ -1709,16 +1715,22 @@ int ann_ivf_query(ann_ivf* h, ann_workspace* ws, const float* queries, int32_t n
             c.coarse_keys = h->cent_bounds.cmax >= kPruneNormMin && h->cent_bounds.cmax <= kPruneNormMax;
     }
     // The exact form's SQ8 selection by keys, where it is estimated to save 60 us: it takes the sum of every candidate
-    // off the FP32 units (1.3e-7 us a term at 1M x 384, of lists of the mean size), and adds its launches (60 us) and
-    // the distances formed apart (1.4e-4 us each of nq R). Measured, every distance / by keys, us a call: 1M x 384, 8 of
-    // 2,048 lists: 777 / 570 (1,000 queries, R = 100), 1130 / 933 (2,000, R = 400), 1726 / 988 (5,000, R = 100), and
-    // 2068 / 1008 (2,000, R = 400, list sizes by a power law); 2 probed: 1044 / 932 (5,000, R = 100), 770 / 848 (2,000,
-    // R = 400: not taken); 500k x 768, 8 of 1,024: 1844 / 938 (2,000, R = 100); 200k x 96, 8 of 512: 642 / 583 (5,000,
-    // R = 100), 402 / 442 (2,000: not taken).
+    // off the FP32 units (1.3e-7 us a term at 1M x 384; as many candidates a probe as the latest batch had, lists of the
+    // mean size before one), and adds its launches (60 us) and the distances formed apart (1.4e-4 us each of nq R).
+    // Measured, every distance / by keys, us a call. Lists of one size, 1M x 384, 8 of 2,048: 777 / 570 (1,000 queries,
+    // R = 100), 1130 / 933 (2,000, R = 400), 1726 / 988 (5,000, R = 100); 2 probed: 1044 / 932 (5,000, R = 100), 770 / 848
+    // (2,000, R = 400: not taken); 500k x 768, 8 of 1,024: 1844 / 938 (2,000, R = 100); 200k x 96, 8 of 512: 402 / 442
+    // (2,000, R = 100: not taken). Sizes by a power law, queries as the rows: 1M x 384, 2 of 2,048: 585 / 300 (200, R = 100),
+    // 1778 / 741 (2,000, R = 400), 5801 / 1282 (10,000, R = 100); 300k x 768, 8 of 256: 2841 / 661 (2,000, R = 100).
     const int64_t pairs = (int64_t)nq * c.npc;
-    c.saved_us = 1.3e-7 * (double)pairs * ((double)h->n / h->C) * h->dim - 60.0 - 1.4e-4 * (double)nq * c.R;
+    double rate = 0.0;
+    {
+        std::lock_guard<std::mutex> lk(h->tc_mu);
+        rate = h->cand_rate > 0.0 ? h->cand_rate : (double)h->n / h->C;
+    }
+    c.saved_us = 1.3e-7 * (double)pairs * rate * h->dim - 60.0 - 1.4e-4 * (double)nq * c.R;
     if (!c.ref && !c.tc && c.batched && c.saved_us >= 60.0 && ivf_prune_fits(c.R, c.npc, h->dpad8) &&
-        pairs * tc_kpad(h->dim, ANN_METRIC_L2) <= (int64_t)1 << 29 && pairs * ceil_div(h->sizes_desc[0], h->sample_div) <= (int64_t)1 << 28 &&
+        pairs * tc_kpad(h->dim, ANN_METRIC_L2) <= (int64_t)1 << 29 && pairs * ceil_div(h->sizes_desc[0], h->sample_div) <= (int64_t)1 << 29 &&
         (int64_t)nq * ivf_prune_cap(c.R) <= (int64_t)1 << 27 &&
         (rc0 = ivf_ensure_codes(h, c.saved_us, st, &c.pruned)))
         return rc0;
