@@ -307,7 +307,7 @@ __global__ void __launch_bounds__(kFinalThreads) compat_final_kernel(CompatArgs 
     }
     if (threadIdx.x == 0) sN = 0;
     __syncthreads();
-    const SelectBound b = block_select_bound([&](int i) { return w[i]; }, m, a.k, sHist, sMisc);
+    const SelectBound b = block_select_bound<true>([&](int i) { return w[i]; }, m, a.k, sHist, sMisc);
     const int p2 = pow2_ceil(a.k);
     for (int i = threadIdx.x; i < m; i += kFinalThreads)
         if (b.in(w[i])) sR[atomicAdd(&sN, 1)] = w[i];

@@ -124,23 +124,10 @@ __global__ void __launch_bounds__(kFinWarps * 32) prune_finish_kernel(PruneArgs 
     const int* fc = a.fcol + (int64_t)q * cap;
     bool fail = cnt > cap || cnt < k || !(w < kInf);
     float T = 0.f;
-    if (!fail) {  // the k-th smallest kept key: four 8-bit digits
+    if (!fail) {  // the k-th smallest kept key
         for (int i = tid; i < cnt; i += kFinThreads) sO[i] = ord_f32(fk[i]);
-        uint32_t prefix = 0, mask = 0;
-        int rem = k;
-        for (int shift = 24; shift >= 0; shift -= 8) {
-            if (tid < 256) sHist[tid] = 0;
-            __syncthreads();
-            for (int i = tid; i < cnt; i += kFinThreads)
-                if ((sO[i] & mask) == prefix) atomicAdd(&sHist[(sO[i] >> shift) & 255u], 1);
-            __syncthreads();
-            int d, before, own;
-            block_pick(sHist, rem, sMisc, &d, &before, &own);
-            rem -= before;
-            prefix |= (uint32_t)d << shift;
-            mask |= 255u << shift;
-        }
-        T = f32_ord(prefix);
+        __syncthreads();
+        T = f32_ord(block_kth([&](int i) { return sO[i]; }, cnt, k, sHist, sMisc));
         fail = !(T <= tauF);
     }
     if (fail) {  // uniform
@@ -216,7 +203,7 @@ __global__ void __launch_bounds__(kFinWarps * 32) prune_finish_kernel(PruneArgs 
             sE[g + lane] = ((unsigned long long)ord_f32((METRIC == ANN_METRIC_L2 ? v : -v) + 0.f) << 32) | (unsigned)row;
     }
     __syncthreads();
-    const SelectBound bound = block_select_bound([&](int i) { return sE[i]; }, m, k, sHist, sMisc);
+    const SelectBound bound = block_select_bound<true>([&](int i) { return sE[i]; }, m, k, sHist, sMisc);
     unsigned long long* sR = reinterpret_cast<unsigned long long*>(sX);  // the best k, then sorted
     const int p2 = pow2_ceil(k);
     if (tid == 0) sN = 0;

@@ -155,6 +155,7 @@ __global__ void __launch_bounds__(kThreads) ivf_prune_finish_kernel(IvfPruneArgs
     float* sQ = reinterpret_cast<float*>(sX + kWarps * kStages * 32 * kPitch);   // [dpad8] -(q - offset)
     float* sS = sQ + dpad8;                                                      // [dpad8] scale
     unsigned long long* sE = reinterpret_cast<unsigned long long*>(sS + dpad8);  // [mcap] (distance, position)
+    uint32_t* sO = reinterpret_cast<uint32_t*>(sE);  // [cap = 2 mcap] keys, before sE is filled
     __shared__ int sHist[256];
     __shared__ int sMisc[12];
     __shared__ int sN;
@@ -177,23 +178,9 @@ __global__ void __launch_bounds__(kThreads) ivf_prune_finish_kernel(IvfPruneArgs
     bool fail = ns < 0 || cnt > cap || cnt < need || !(w.x < kInf);
     float T = 0.f;
     if (!fail) {  // the need-th smallest kept key
-        uint32_t prefix = 0, mask = 0;
-        int rem = need;
-        for (int shift = 24; shift >= 0; shift -= 8) {
-            sHist[tid] = 0;
-            __syncthreads();
-            for (int i = tid; i < cnt; i += kThreads) {
-                const uint32_t o = ord_f32(fk[i]);
-                if ((o & mask) == prefix) atomicAdd(&sHist[(o >> shift) & 255u], 1);
-            }
-            __syncthreads();
-            int d, before, own;
-            block_pick(sHist, rem, sMisc, &d, &before, &own);
-            rem -= before;
-            prefix |= (uint32_t)d << shift;
-            mask |= 255u << shift;
-        }
-        T = f32_ord(prefix);
+        for (int i = tid; i < cnt; i += kThreads) sO[i] = ord_f32(fk[i]);
+        __syncthreads();
+        T = f32_ord(block_kth([&](int i) { return sO[i]; }, cnt, need, sHist, sMisc));
         fail = !(T <= tauF);
     }
     if (fail) {  // uniform
@@ -284,7 +271,7 @@ __global__ void __launch_bounds__(kThreads) ivf_prune_finish_kernel(IvfPruneArgs
         }
     }
     __syncthreads();
-    const SelectBound bound = block_select_bound([&](int i) { return sE[i]; }, m, need, sHist, sMisc);
+    const SelectBound bound = block_select_bound<true>([&](int i) { return sE[i]; }, m, need, sHist, sMisc);
     if (tid == 0) sN = 0;
     __syncthreads();
     for (int i = tid; i < m; i += kThreads) {
@@ -331,7 +318,7 @@ int launch_ivf_prune_bars(const IvfPruneArgs& a, cudaStream_t st) {
 }
 
 int launch_ivf_prune_finish(const IvfPruneArgs& a, cudaStream_t st) {
-    ANN_CHECK_ARG(a.R <= a.cap && ivf_prune_fits(a.R, a.plan.npc, a.ix.dpad8),
+    ANN_CHECK_ARG(a.R <= a.cap && a.cap <= 2 * formed_cap(a.R) && ivf_prune_fits(a.R, a.plan.npc, a.ix.dpad8),
                   "pruned SQ8 selection: R=%d, %d lists, code stride %d", a.R, a.plan.npc, a.ix.dpad8);
     ANN_CUDA_TRY(smem_optin(reinterpret_cast<const void*>(ivf_prune_finish_kernel)));
     ivf_prune_finish_kernel<<<a.plan.nq, kThreads, finish_smem(a.R, a.ix.dpad8), st>>>(a);
