@@ -64,7 +64,10 @@ struct ScanCfg {
 // PQ: the query tile comes from FlatScanArgs::qpair (query pairs interleaved element by element, negated for
 // L2), staged per chunk as BQ / 2 rows of 2 KC floats; thread query pairs (2 jj, 2 jj + 1) share each x element
 // through packed FP32 instructions (x - q as x + (-q), then fma, per half exactly the scalar steps)
-template <int BQ, int TQ, int TR, int STAGES, int METRIC, bool PQ>
+// One (query tile, split) per CTA; DEV: a batch whose size the device knows (nq_dev) runs on a fixed grid instead, each CTA
+// taking the tiles that exist in turn (apart: with the loop in the common kernel, 16 queries over 21k x 661 took 227 us, not
+// 215).
+template <int BQ, int TQ, int TR, int STAGES, int METRIC, bool PQ, bool DEV>
 __global__ void __launch_bounds__(256) flat_scan_kernel(FlatScanArgs a) {
     using C = ScanCfg<BQ, TQ, TR, STAGES, METRIC>;
     static_assert(!PQ || TQ % 2 == 0, "query pairs");
@@ -86,13 +89,12 @@ __global__ void __launch_bounds__(256) flat_scan_kernel(FlatScanArgs a) {
     const int tq = tid / C::WR;
     const int tr = tid % C::WR;
     const int k = a.k;
-    // one (query tile, split) per CTA; a batch whose size the device knows (nq_dev) runs on a fixed grid instead,
-    // each CTA taking the tiles that exist in turn
-    if (a.nq_dev) a.nq = min(a.nq, *a.nq_dev);
-    const int n_qt = a.nq_dev ? (a.nq + BQ - 1) / BQ : gridDim.x;
-    for (int item = blockIdx.y * gridDim.x + blockIdx.x; item < n_qt * a.nsplit; item += gridDim.x * gridDim.y) {
-    const int q0 = (item % n_qt) * BQ;
-    const int split = item / n_qt;
+    if (DEV) a.nq = min(a.nq, *a.nq_dev);
+    const int n_qt = DEV ? (a.nq + BQ - 1) / BQ : 1;
+    const int items = DEV ? n_qt * a.nsplit : 1;
+    for (int item = DEV ? blockIdx.x : 0; item < items; item += gridDim.x) {
+    const int q0 = (DEV ? item % n_qt : blockIdx.x) * BQ;
+    const int split = DEV ? item / n_qt : blockIdx.y;
     const int64_t row_begin = (int64_t)split * a.rows_per_split;
     int64_t row_end = row_begin + a.rows_per_split;
     if (row_end > a.n) row_end = a.n;
@@ -295,6 +297,7 @@ __global__ void __launch_bounds__(256) flat_scan_kernel(FlatScanArgs a) {
             oi[e] = e < cnt ? sId[ql * cap + e] : kNoId;
         }
     }
+    if (!DEV) break;
     __syncthreads();  // the next item reuses the stages and the buffers
     }
 }
@@ -585,7 +588,8 @@ static int dispatch_stream(const FlatScanArgs& a, int bq, int n_qtiles, cudaStre
 template <int BQ, int TQ, int TR, int STAGES, int METRIC, bool PQ = false>
 static int launch_scan_t(FlatScanArgs a, int n_qtiles, cudaStream_t st) {
     using C = ScanCfg<BQ, TQ, TR, STAGES, METRIC>;
-    auto kern = flat_scan_kernel<BQ, TQ, TR, STAGES, METRIC, PQ>;
+    auto kern = a.nq_dev ? flat_scan_kernel<BQ, TQ, TR, STAGES, METRIC, PQ, true>
+                         : flat_scan_kernel<BQ, TQ, TR, STAGES, METRIC, PQ, false>;
     const size_t smem = C::smem(a.cap);
     ANN_CHECK_ARG(smem <= 227 * 1024, "flat scan: %zu bytes of shared memory for k=%d", smem, a.k);
     ANN_CUDA_TRY(smem_optin(reinterpret_cast<const void*>(kern)));
