@@ -613,8 +613,8 @@ static int flat_check_err(ann_flat* h) {
 // element (1.7 ms at 1M x 384), a pruned call saves 40 us and up, so a base that is searched only once or twice
 // should not pay: the calls' estimated savings add up (prune_credit_us), and the copy is laid out by the call
 // that brings them to its cost -- at once for a large batch, after a dozen single queries otherwise. Measured, scan
-// / pruned, us a call: 1M x 384: 376 / 259 (1 query), 1121 / 256 (8), 45342 / 967 (1,000); 32768 x 64: 105 / 67
-// (1), 2550 / 172 (1,000). *ok = false (and no error) where the search keeps to the plain scan: not yet laid out,
+// / pruned, us a call: 1M x 384: 376 / 194 (1 query), 1121 / 213 (8), 45342 / 873 (1,000); 32768 x 64: 105 / 68
+// (1), 2550 / 130 (1,000). *ok = false (and no error) where the search keeps to the plain scan: not yet laid out,
 // a copy that would take more than half of the free memory, or rows that the bounds do not cover.
 static int flat_ensure_pruned(ann_flat* h, int nq, cudaStream_t st, bool* ok) {
     *ok = false;
@@ -668,7 +668,7 @@ static int flat_exact_pruned(ann_flat* h, ann_workspace* ws, const float* qdev, 
     *done = false;
     const int64_t n = h->n;
     const int dpad = h->dpad;
-    if (n < kPruneMinRows || n < 64 * (int64_t)kk || !prune_fits(kk, dpad)) return ANN_OK;
+    if (n < prune_min_rows(nq, kk) || n < 64 * (int64_t)kk || !prune_fits(kk, dpad)) return ANN_OK;
     bool ok = false;
     int rc = flat_ensure_pruned(h, nq, st, &ok);
     if (rc || !ok) return rc;

@@ -15,9 +15,12 @@ struct PruneBounds {
 // Norms outside this range leave the error bound's assumptions (no overflow, nothing lost to underflow).
 constexpr float kPruneNormMin = 1e-12f, kPruneNormMax = 1e15f;
 
-// Smaller bases are scanned: from here on every batch measured faster pruned (32768 x 64, one query: 67 us against
-// 105 us), and the sample (an eighth of a small base) still holds enough rows for the bar.
-constexpr int64_t kPruneMinRows = 32768;
+// Smaller bases are scanned. Measured over dims 64, 384, 768, both metrics, k = 10 and 100, scanned / pruned, us a call:
+// one query 6,000 rows 59 / 66 (k = 10, dim 384), 8,192 rows 0.97 to 1.11 times faster at k = 10 and 1.65 to 2 times at
+// k = 100, from 12,000 on 1.02 to 2.2 times; 3 queries 3,000 rows 89 / 66,
+// 8,192 rows 1.3 to 3.1 times; 8 and more 3,000 rows 1.04 to 3.1 times, 24,000 rows 1.2 to 21 times. The sample (an eighth
+// of a small base) still holds enough rows for the bar.
+inline int64_t prune_min_rows(int nq, int k) { return nq == 1 && k < 64 ? 12000 : (nq <= 4 ? 8192 : 4096); }
 
 // The window of the BF16 keys (tc_gemm.cuh) of vector q against rows x: 2 eps + delta. With x^, q^ the BF16 operands,
 //   |x.q - x^.q^| <= |x - x^| |q| + |x^| |q - q^| <= rmax |q| + (cmax + rmax) |q - q^|,
