@@ -161,10 +161,15 @@ __device__ __forceinline__ void block_sort_u64(unsigned long long* w, int n) {
         }
 }
 
-// The word of a distance and its row; NaN orders after +inf, -0 with +0.
+// The word of a distance and its row; NaN orders after +inf, -0 with +0. By the bits alone: with the NaN passed through
+// an FP32 addition the compiled word came out below every distance's.
 __device__ __forceinline__ unsigned long long select_word(float v, int64_t row) {
-    if (v != v) v = __int_as_float(0x7fffffff);
-    return ((unsigned long long)ord_f32(v + 0.f) << 32) | (unsigned)row;
+    uint32_t u = __float_as_uint(v);
+    if ((u & 0x7fffffffu) > 0x7f800000u)
+        u = 0x7fffffffu;
+    else if (u == 0x80000000u)
+        u = 0u;
+    return ((unsigned long long)((u & 0x80000000u) ? ~u : (u | 0x80000000u)) << 32) | (unsigned)row;
 }
 
 // Rows of a segment when n rows are selected from in up to kSelectSegs segments (a multiple of 1024).
