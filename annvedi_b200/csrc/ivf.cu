@@ -554,7 +554,8 @@ __global__ void __launch_bounds__(256) rows_segment_kernel(const float* __restri
 }
 
 // One block per list entry: the best k <= R of its segments' best, in no order, to row rows[entry] of out_key / out_id,
-// padded to R with (+inf, kNoId).
+// padded to R with (+inf, kNoId). Keys that are NaN are not kept, as the scan with fused selection keeps none: their words
+// order last, so where they are among the best k every number is too.
 __global__ void __launch_bounds__(512) rows_final_kernel(const unsigned long long* __restrict__ best, int m, int k, int R,
                                                          const int32_t* __restrict__ rows, float* __restrict__ out_key,
                                                          int* __restrict__ out_id) {
@@ -573,8 +574,9 @@ __global__ void __launch_bounds__(512) rows_final_kernel(const unsigned long lon
     for (int i = threadIdx.x; i < m; i += 512) {
         if (!b.in(w[i])) continue;
         const int at = atomicAdd(&sN, 1);
-        out_key[o + at] = f32_ord((uint32_t)(w[i] >> 32));
-        out_id[o + at] = (int)(unsigned)w[i];
+        const bool nan = (uint32_t)(w[i] >> 32) == 0xffffffffu;
+        out_key[o + at] = nan ? kInf : f32_ord((uint32_t)(w[i] >> 32));
+        out_id[o + at] = nan ? kNoId : (int)(unsigned)w[i];
     }
 }
 
