@@ -565,7 +565,11 @@ __device__ __forceinline__ void coarse_by_chunks(const float* __restrict__ kr, c
                 acc = fmaf(t3, t3, acc);
             }
         }
-        for (int j = 0; j < held; ++j) insert(__shfl_sync(0xffffffffu, acc, j), __shfl_sync(0xffffffffu, id, j));
+        for (int j = 0; j < held; ++j) {
+            const float d = __shfl_sync(0xffffffffu, acc, j);
+            const int cid = __shfl_sync(0xffffffffu, id, j);
+            if (d <= kInf) insert(d, cid);  // (uniform) NaN: the scan compares with none
+        }
         held = 0;
         __syncwarp();
     };

@@ -32,3 +32,9 @@ def _check(c, dim, nq, k, npc, R, sizes, seed):
 def test_nan_queries_that_scan_every_row(cuda, c, dim, nq, k, npc, R):
     """Lists of 5 rows among longer ones: a query of no list is one short of k, which scans every row."""
     _check(c, dim, nq, k, npc, R, [5, 5, 5] + [150] * (c - 3), c)
+
+
+@pytest.mark.parametrize("c,dim,nq,k,npc,R", [(256, 48, 64, 10, 4, 40), (300, 384, 200, 20, 8, 80), (2048, 33, 90, 5, 32, 20)])
+def test_nan_queries_ranked_by_centroid_keys(cuda, c, dim, nq, k, npc, R):
+    """256 lists and more: the batch's coarse ranking by keys."""
+    _check(c, dim, nq, k, npc, R, [21 + i % 7 for i in range(c)], c + dim)
