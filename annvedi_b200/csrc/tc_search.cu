@@ -525,9 +525,11 @@ __device__ __forceinline__ void coarse_by_chunks(const float* __restrict__ kr, c
         const float b1 = __shfl_sync(0xffffffffu, a1, s1 ? __ffs(s1) - 1 : 0);
         bar = s0 ? b0 : (s1 ? b1 : kInf);  // no rank npc - 1 only with NaN minima: every chunk
     }
-    const float qn = sqrtf(s2), w = key_window_l2(qn, sqrtf(e2), cmax, rmax, dim);
-    // a query that the bound does not cover (NaN, norms out of range) takes every centroid
-    const bool all = !(qn <= kPruneNormMax && (qn >= kPruneNormMin || s2 == 0.f) && w < kInf);
+    // Norms below kPruneNormMin count as that (their squares are inexact below 2^-126, the bound's share of them nil).
+    const float qn = fmaxf(sqrtf(s2), kPruneNormMin), w = key_window_l2(qn, fmaxf(sqrtf(e2), kPruneNormMin), cmax, rmax, dim);
+    // SCAN: a query that the bound does not cover (NaN, huge norms) takes every centroid. Otherwise its keys alone decide,
+    // and one that compares with none (NaN, an infinite component) probes list 0 npc times.
+    const bool all = SCAN && !(s2 < kInf && qn <= kPruneNormMax && w < kInf);
     const float lim = all ? kInf : __fadd_ru(bar, w);
     float bd = kInf;  // lane j < npc: the j-th best (distance, id) so far
     int bi = kNoId;
