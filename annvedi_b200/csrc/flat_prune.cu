@@ -90,9 +90,13 @@ __global__ void __launch_bounds__(256) prune_queries_kernel(PruneArgs a, __nv_bf
         e += __shfl_xor_sync(0xffffffffu, e, o);
     }
     if (lane != 0) return;
-    const float qn = sqrtf(s), rq = sqrtf(e);
-    const float w = l2 ? key_window_l2(qn, rq, a.b.cmax, a.b.rmax, a.dim) : key_window_ip(qn, rq, a.b.cmax, a.b.rmax, a.dim);
-    const bool ok = qn <= kPruneNormMax && (qn >= kPruneNormMin || s == 0.f);  // false for NaN
+    // Squares of components below 2^-74 are lost, so s = 0 does not say that the query is zero. Under L2 norms below
+    // kPruneNormMin count as that, their share of the window nil beside the rows' own; under inner product every term
+    // of the window is the query's, and such queries, zero among them (every key the same), are left to the scan.
+    const float qn = fmaxf(sqrtf(s), kPruneNormMin), rq = fmaxf(sqrtf(e), kPruneNormMin);
+    const float w = l2 ? key_window_l2(qn, rq, a.b.cmax, a.b.rmax, a.dim)
+                       : key_window_ip(sqrtf(s), sqrtf(e), a.b.cmax, a.b.rmax, a.dim);
+    const bool ok = s < kInf && qn <= kPruneNormMax && (l2 || sqrtf(s) >= kPruneNormMin);  // false for NaN
     a.win[q] = ok ? w : __int_as_float(0x7fffffff);
     a.rcount[q] = 0;
     if (q == 0) *a.count = 0;
