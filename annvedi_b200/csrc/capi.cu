@@ -753,9 +753,12 @@ static int flat_exact_pruned(ann_flat* h, ann_workspace* ws, const float* qdev, 
         sa.out_min = kA;
         sa.b_tile_stride = stride;
         sa.b_rows = n;
+        sa.wait_ns = h->wait_ns;
+        sa.test_no_loads = h->wait_ns > 0;
         if ((rc = launch_tc_sample(qb, h->base_bf16, sa, st))) return rc;
         if ((rc = launch_bars(kA, nullptr, nullptr, nc, rF, rF, tauF, tauX, st, S / 8, win))) return rc;
-        const TcFilterArgs fa{nc, (int)n, kpad, kTcBF16, tauX, fkey, fcol, cap, rcount, nullptr, nullptr, h->d_err};
+        const TcFilterArgs fa{nc, (int)n, kpad, kTcBF16, tauX, fkey, fcol, cap, rcount, nullptr, nullptr, h->d_err, h->wait_ns,
+                              h->wait_ns > 0};
         if ((rc = launch_tc_filter(qb, h->base_bf16, fa, st))) return rc;
         if ((rc = launch_prune_finish(p, st))) return rc;
         // the queries on the list, by the plain scan (none, nearly always: the kernels read the count and return)
@@ -794,6 +797,8 @@ int ann_flat_scores_tc(ann_flat* h, const float* queries, int32_t nq, int64_t ld
     float* tmp = reinterpret_cast<float*>(h->ws.big);
     if ((rc = flat_tc_queries(h, t, queries, nq, ldq, qb, rfac, st))) return rc;
     TcGemmArgs a{nq, (int)h->n, t.kpad, nullptr, tmp, h->n, h->d_err};
+    a.wait_ns = h->wait_ns;
+    a.test_no_loads = h->wait_ns > 0;
     a.kind = t.kind;
     a.col_fac = t.cfac;
     a.row_fac = t.kind == kTcE4M3 ? rfac : nullptr;
@@ -811,6 +816,11 @@ int ann_flat_set_option(ann_flat* h, int32_t option, int64_t value) {
             ANN_CHECK_ARG(value == 0 || value == 8 || value == 16 || value == 32,
                           "ann_flat_set_option: query tile %lld (0, 8, 16 or 32)", (long long)value);
             h->query_tile = (int)value;
+            return ANN_OK;
+        case ANN_FLAT_OPT_WAIT_SELFTEST:
+            ANN_CHECK_ARG(value == 0 || (value >= 1000 && value <= 2000000000LL), "ann_flat_set_option: wait limit %lld ns",
+                          (long long)value);
+            h->wait_ns = (uint64_t)value;
             return ANN_OK;
         default:
             set_error("ann_flat_set_option: unknown option %d", option);
@@ -947,13 +957,16 @@ int ann_flat_query_tc(ann_flat* h, ann_workspace* ws, const float* queries, int3
             sa.out_min = kA;
             sa.b_tile_stride = stride;
             sa.b_rows = n;
+            sa.wait_ns = h->wait_ns;
+            sa.test_no_loads = h->wait_ns > 0;
             if ((rc = launch_tc_sample(qbc, t.base, sa, st))) return rc;
             const int S8 = (int)(S / 8);
             if ((rc = launch_bars(kA, nullptr, nullptr, nc, rF, R, tauF, tauS, st, S8))) return rc;
             h->prof.mark(prec, st);
             auto filter = [&](const void* A, int M, const float* tau, const float* rf, int rcap) -> int {
                 ANN_CUDA_TRY(cudaMemsetAsync(rowcnt, 0, sizeof(int) * (size_t)M, st));
-                const TcFilterArgs fa{M, (int)n, kpad, t.kind, tau, fkey, fcol, rcap, rowcnt, t.cfac, rf, h->d_err};
+                const TcFilterArgs fa{M,    (int)n, kpad,   t.kind, tau, fkey,     fcol,
+                                      rcap, rowcnt, t.cfac, rf,     h->d_err, h->wait_ns, h->wait_ns > 0};
                 int r = launch_tc_filter(A, t.base, fa, st);
                 if (r) return r;
                 return launch_max_int(rowcnt, M, flags + 1, st);
@@ -1008,6 +1021,8 @@ int ann_flat_query_tc(ann_flat* h, ann_workspace* ws, const float* queries, int3
             float* keys = reinterpret_cast<float*>(ws->big);
             const int prec = h->prof.begin(st, 3);  // stage 3: the full key matrix, 4: its selection
             TcGemmArgs a{nf, (int)n, kpad, nullptr, keys, n, h->d_err};
+            a.wait_ns = h->wait_ns;
+            a.test_no_loads = h->wait_ns > 0;
             a.kind = t.kind;
             a.col_fac = t.cfac;
             a.row_fac = e4 ? rfc + f0 : nullptr;

@@ -73,6 +73,7 @@ struct ann_ivf {
     // query options (ann_ivf_set_option)
     int sample_div = 8;             // the sampled bars score the first ceil(size / sample_div) rows of a list
     int sampled_min_queries = 256;  // batches from this size take the sampled tensor-core path
+    uint64_t wait_ns = 0;           // > 0: the self-test of the bounded waits, with this limit
 
     IvfView view() const {
         IvfView v;
@@ -1147,6 +1148,8 @@ static int ivf_tc_sampled(ann_ivf* h, ann_workspace* ws, const IvfQueryCfg& c, c
     if ((rc = launch_tc_item_descs(descs, 2, C, b.lq_off, h->list_off, st))) return rc;
     // 1. sample pass: keys of the list heads into the sample streams; the two bars per query
     TcGemmArgs gs{(int)max_pairs, (int)h->n, op.K, nullptr, SK, 0, h->d_err};
+    gs.wait_ns = h->wait_ns;
+    gs.test_no_loads = h->wait_ns > 0;
     gs.kind = op.kind;
     gs.col_fac = op.col_fac;
     gs.row_fac = op.pfac;
@@ -1167,6 +1170,8 @@ static int ivf_tc_sampled(ann_ivf* h, ann_workspace* ws, const IvfQueryCfg& c, c
     // 2. filter pass over every row of the probed lists into the queries' buffers
     auto filter = [&](const float* tau, const int* skip_if_zero) -> int {
         TcGemmArgs g{(int)max_pairs, (int)h->n, op.K, nullptr, nullptr, 0, h->d_err};
+        g.wait_ns = h->wait_ns;
+        g.test_no_loads = h->wait_ns > 0;
         g.skip_if_zero = skip_if_zero;
         g.kind = op.kind;
         g.col_fac = op.col_fac;
@@ -1316,6 +1321,8 @@ static int ivf_query_device(ann_ivf* h, ann_workspace* ws, const IvfQueryCfg& c,
         // BF16 keys to every centroid, then the exact FP32 order of the best npc + 16
         if ((rc = launch_tc_operand(qdev, nq, h->dim, h->dpad, qb, h->kpad, kTcQuery, ANN_METRIC_L2, 0, st))) return rc;
         TcGemmArgs ca{nq, h->C, h->kpad, nullptr, ckeys, h->C, h->d_err};
+        ca.wait_ns = h->wait_ns;
+        ca.test_no_loads = h->wait_ns > 0;
         ca.out_cmin = ckmin;  // and each query's 32-centroid chunk minima, which let the ranking skip chunks
         if ((rc = launch_tc_gemm(qb, h->cent_bf16, ca, st))) return rc;
         if ((rc = launch_tc_coarse(ckeys, h->C, nq, h->C, c.npc, 16, qdev, h->centroids, h->dpad, probes, st,
@@ -1478,6 +1485,8 @@ static int ivf_query_device(ann_ivf* h, ann_workspace* ws, const IvfQueryCfg& c,
                 const TcItemDescs descs{titem, nullptr, titem_desc, items_cap};
                 if (!c.small_tc && (rc = launch_tc_item_descs(&descs, 1, h->C, b.lq_off, h->list_off, st))) return rc;
                 TcGemmArgs g{(int)max_pairs, (int)h->n, op.K, nullptr, D, 0, h->d_err};
+                g.wait_ns = h->wait_ns;
+                g.test_no_loads = h->wait_ns > 0;
                 g.kind = op.kind;
                 g.col_fac = op.col_fac;
                 g.row_fac = op.pfac;
@@ -1866,6 +1875,10 @@ int ann_ivf_set_option(ann_ivf* h, int32_t option, int64_t value) {
         case ANN_IVF_OPT_SAMPLED_MIN:
             ANN_CHECK_ARG(value >= 1 && value <= INT32_MAX, "sampled-path batch size %lld", (long long)value);
             h->sampled_min_queries = (int)value;
+            return ANN_OK;
+        case ANN_IVF_OPT_WAIT_SELFTEST:
+            ANN_CHECK_ARG(value == 0 || (value >= 1000 && value <= 2000000000LL), "wait limit %lld ns", (long long)value);
+            h->wait_ns = (uint64_t)value;
             return ANN_OK;
         default:
             set_error("ann_ivf_set_option: unknown option %d", option);

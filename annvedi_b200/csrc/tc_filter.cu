@@ -215,7 +215,7 @@ __global__ void __launch_bounds__(kFiThreads, 1) tc_filter_kernel(const __grid_c
     FilterWork work(sh, (int)blockIdx.x / CG, (int)gridDim.x / CG);
 
     if (warp == 0) {
-        if (lane == 0) {  // base rows (and, when not resident, the query rows of the same k-block)
+        if (lane == 0 && !a.test_no_loads) {  // base rows (and, when not resident, the query rows of the same k-block)
             RingPos pos;
             bool ok = true;
             const uint32_t a_bytes = (uint32_t)sh.a_box * kRowBytes;
@@ -232,14 +232,9 @@ __global__ void __launch_bounds__(kFiThreads, 1) tc_filter_kernel(const __grid_c
                     fi_tma<CG>(sB + (size_t)s * kBSize, &tmB, kb * kBlockK, brow, fb);
                 }
             }
-            if (!ok) {  // give the copies in flight time to land before the CTA ends
-                const uint64_t t0 = gtimer();
-                while (gtimer() - t0 < 5000000ull) {
-                }
-            }
         }
     } else if (warp == kFiWarpA) {
-        if (lane == 0 && resident) {  // the query tile of each run
+        if (lane == 0 && resident && !a.test_no_loads) {  // the query tile of each run
             int run = 0;
             bool ok = true;
             while (ok && work.next()) {
@@ -251,11 +246,6 @@ __global__ void __launch_bounds__(kFiThreads, 1) tc_filter_kernel(const __grid_c
                     fi_tma<CG>(sA + (size_t)kb * kABytes, &tmA, kb * kBlockK, work.m * CG * kBM + rank * kBM, fb);
                 }
                 ++run;
-            }
-            if (!ok) {
-                const uint64_t t0 = gtimer();
-                while (gtimer() - t0 < 5000000ull) {
-                }
             }
         }
     } else if (warp == 1) {
@@ -311,6 +301,7 @@ __global__ void __launch_bounds__(kFiThreads, 1) tc_filter_kernel(const __grid_c
             }
             if (leader) fi_commit<CG>(done);
             __syncwarp();
+            if (!ok) let_copies_land();  // (a producer may have issued its last copies and left without a wait)
         }
         bar_wait_warp(su32(done), 0, nullptr, 0);  // every MMA issued has completed before TMEM is released
     } else {  // epilogue
@@ -458,6 +449,7 @@ __global__ void __launch_bounds__(kFiThreads, 1) tc_filter_kernel(const __grid_c
             ++acc;
         }
         if (!SAMPLE) flush(nq);
+        if (KIND != kTcBF16) asm volatile("cp.async.wait_all;" ::: "memory");  // (left over where a wait gave up)
     }
     __syncthreads();
     if (CG == 2) cluster_sync();  // neither CTA's barriers or accumulators are in use any more

@@ -15,7 +15,8 @@ struct TcFilterArgs {
     const float2* col_fac; // E4M3: per B row, per A row (TcGemmArgs)
     const float* row_fac;
     int* err;              // device flag set (to 2) if a bounded wait gives up
-    uint64_t wait_ns = 0;
+    uint64_t wait_ns = 0;  // limit of the waits (0: 2 s)
+    int test_no_loads = 0; // self-test: the producers issue no copies, so that the waits run out with nothing in flight
     // Sample pass (launch_tc_sample): N sampled columns in whole tiles of 256, tile j holding B rows
     // j * 256 * b_tile_stride ..; out_min [M, N / 8] receives the smallest key of each 8 columns.
     float* out_min = nullptr;

@@ -209,6 +209,7 @@ __global__ void __launch_bounds__(epi_threads(EPI), 1) tc_gemm_kernel(const __gr
         if (leader) mma_commit(done);
         __syncwarp();
         bar_wait_warp(su32(done), 0, nullptr, 0);
+        if (!ok) let_copies_land();
     } else {  // epilogue warps 2..9
         const int lane_base = 32 * (warp & 3);
         const int ew = warp - 2;
@@ -467,6 +468,7 @@ __global__ void __launch_bounds__(epi_threads(EPI), 1) tc_gemm_kernel(const __gr
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             bar_arrive(&tempty[b]);
         }
+        if (kFilterOnly) asm volatile("cp.async.wait_all;" ::: "memory");  // (left over where a wait gave up)
     }
     __syncthreads();
     if (warp == 1) {

@@ -91,6 +91,13 @@ __device__ __forceinline__ bool bar_wait_warp(uint32_t b, uint32_t parity, int* 
         }
     return true;
 }
+// A warp that gave up holds its CTA (and with it the pair) for 5 ms before the CTA may end: copies in flight into its shared
+// memory take microseconds, and once the MMA issuer has given up nothing else waits for them.
+__device__ __forceinline__ void let_copies_land() {
+    const uint64_t t0 = gtimer();
+    while (gtimer() - t0 < 5000000ull) {
+    }
+}
 __device__ __forceinline__ void bar_arrive(uint64_t* b) {
     asm volatile("{\n .reg .b64 st;\n mbarrier.arrive.shared::cta.b64 st, [%0];\n}" ::"r"(su32(b)) : "memory");
 }

@@ -207,12 +207,13 @@ class IVFIndex:
                              "rerank": rerank},
                 "profiled_calls": int(out[6])}
 
-    OPTIONS = {"sample_div": 2, "sampled_min_queries": 3}
+    OPTIONS = {"sample_div": 2, "sampled_min_queries": 3, "wait_selftest": 4}
 
     def set_option(self, name: str, value: int) -> None:
         """Query options (ann_ivf_set_option): "sample_div" (the sampled bars score the first
         ceil(size / div) rows of each list), "sampled_min_queries" (batch size from which the tensor-core
-        forms take the sampled path). Neither changes results."""
+        forms take the sampled path), "wait_selftest" (ns; > 0: the tensor-core kernels copy nothing, so that their
+        waits give up; 0: off). The first two change no results."""
         if name not in self.OPTIONS:
             raise RuntimeError(f"unknown option {name!r}")
         _lib.check(self._lib.ann_ivf_set_option(self._h, self.OPTIONS[name], int(value)))

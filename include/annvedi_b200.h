@@ -145,6 +145,9 @@ int ann_flat_set_tc_precision(ann_flat* h, int32_t precision);
  *     tile sums a pair's terms in the same order and the splits merge by (distance, id)); the tile changes
  *     speed only, and autotune.tune_flat_tile picks it by timing. */
 #define ANN_FLAT_OPT_QUERY_TILE 1
+/*   ANN_FLAT_OPT_WAIT_SELFTEST: value > 0 (1e3..2e9): the tensor-core kernels of the index's searches issue no copies,
+ *     so that their bounded waits give up after `value` ns, as in ann_tc_wait_selftest; 0 (the default): off. */
+#define ANN_FLAT_OPT_WAIT_SELFTEST 2
 int ann_flat_set_option(ann_flat* h, int32_t option, int64_t value);
 
 /* Diagnostic: the tensor-core key matrix out_keys[nq][n] (device pointers; synchronous). */
@@ -277,6 +280,8 @@ int ann_ivf_profile(ann_ivf* h, double* out8);
  *   ANN_IVF_OPT_SAMPLED_MIN: batches of at least this many queries take the sampled path (default 256). */
 #define ANN_IVF_OPT_SAMPLE_DIV 2
 #define ANN_IVF_OPT_SAMPLED_MIN 3
+/*   ANN_IVF_OPT_WAIT_SELFTEST: as ANN_FLAT_OPT_WAIT_SELFTEST. */
+#define ANN_IVF_OPT_WAIT_SELFTEST 4
 int ann_ivf_set_option(ann_ivf* h, int32_t option, int64_t value);
 
 /* Single-kernel times of the same profiled calls (CUDA events around each launch, on the query stream):

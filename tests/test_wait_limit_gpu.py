@@ -1,0 +1,64 @@
+"""Searches whose device waits run out (the self-test option: no copies are issued): the kernels wind down, the status says so,
+and the same index answers the next call as before."""
+import ctypes
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+TIMEOUT = -5
+FLAT_OPT_WAIT_SELFTEST = 2
+
+
+def _flat(n, dim, nq, precision, rng):
+    import torch
+    from annvedi_b200.linear import LinearIndex
+    ix = LinearIndex(device=0, mode="exact")
+    ix.fit(torch.from_numpy(rng.standard_normal((n, dim)).astype(np.float32)).cuda())
+    ix.set_tc_precision(precision)
+    return ix, torch.from_numpy(rng.standard_normal((nq, dim)).astype(np.float32)).cuda()
+
+
+# 200,000 rows: the sampled form (tc_filter.cu, one CTA a tile and CTA pairs); 20,000: the key matrix (tc_gemm.cu)
+@pytest.mark.parametrize("n,dim,nq,precision", [(200000, 40, 3, "bf16"), (200000, 1000, 20, "bf16"), (200000, 64, 300, "bf16"),
+                                                (200000, 64, 300, "e4m3"), (20000, 64, 40, "bf16"), (300, 32, 2, "e4m3")])
+def test_flat_tensor_core_search(cuda, n, dim, nq, precision):
+    import torch
+    ix, q = _flat(n, dim, nq, precision, np.random.default_rng(nq))
+    lib = ix._lib
+    want = ix.search_tc(q, 10)
+    assert lib.ann_flat_device_status(ix._h) == 0
+    assert lib.ann_flat_set_option(ix._h, FLAT_OPT_WAIT_SELFTEST, ctypes.c_int64(100000)) == 0
+    ix.search_tc(q, 10)
+    torch.cuda.synchronize()
+    assert lib.ann_flat_device_status(ix._h) == TIMEOUT
+    assert lib.ann_flat_device_status(ix._h) == 0  # read and cleared
+    with pytest.raises(RuntimeError):
+        ix.search_tc(q.cpu().numpy(), 10)
+    assert lib.ann_flat_set_option(ix._h, FLAT_OPT_WAIT_SELFTEST, ctypes.c_int64(0)) == 0
+    got = ix.search_tc(q, 10)
+    assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+    assert lib.ann_flat_device_status(ix._h) == 0
+
+
+@pytest.mark.parametrize("mode", ["tc", "tc_sq8"])
+@pytest.mark.parametrize("nq", [1, 40, 400])
+def test_ivf_tensor_core_search(cuda, mode, nq):
+    import torch
+    from annvedi_b200.ivf import IVFIndex
+    rng = np.random.default_rng(nq)
+    x = rng.standard_normal((20000, 96)).astype(np.float32)
+    ix = IVFIndex(device=0, mode=mode)
+    ix.fit(x, 1, 0, 64, centroids=x[:64])
+    q = torch.from_numpy(rng.standard_normal((nq, 96)).astype(np.float32)).cuda()
+    want = ix.search(q, 10, 0, 4, 40)
+    assert ix._lib.ann_ivf_device_status(ix._h) == 0
+    ix.set_option("wait_selftest", 100000)
+    ix.search(q, 10, 0, 4, 40)
+    torch.cuda.synchronize()
+    assert ix._lib.ann_ivf_device_status(ix._h) == TIMEOUT
+    ix.set_option("wait_selftest", 0)
+    got = ix.search(q, 10, 0, 4, 40)
+    assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+    assert ix._lib.ann_ivf_device_status(ix._h) == 0
