@@ -311,7 +311,6 @@ extern "C" {
 
 static int flat_exact_pruned(ann_flat* h, ann_workspace* ws, const float* qdev, int nq, int kk, int64_t* ids_dev,
                              float* dists_dev, cudaStream_t st, bool* done);
-static int flat_check_err(ann_flat* h);
 
 int ann_flat_query(ann_flat* h, ann_workspace* ws, const float* queries, int32_t nq, int64_t ldq, int32_t k,
                    int32_t mode, int32_t mem, int64_t* out_ids, float* out_dists, void* stream) {
@@ -466,7 +465,6 @@ int ann_flat_query(ann_flat* h, ann_workspace* ws, const float* queries, int32_t
         if (out_dists)
             ANN_CUDA_TRY(cudaMemcpyAsync(out_dists, dists_dev, sizeof(float) * (size_t)nq * kk, cudaMemcpyDeviceToHost, st));
         ANN_CUDA_TRY(cudaStreamSynchronize(st));
-        if (pruned) return flat_check_err(h);
     }
     return ANN_OK;
 }
@@ -697,7 +695,7 @@ static int flat_exact_pruned(ann_flat* h, ann_workspace* ws, const float* qdev, 
     sz.take<float>((size_t)qc * cap);
     sz.take<int>((size_t)qc * cap);
     for (int i = 0; i < 2; ++i) sz.take<int>((size_t)qc);
-    sz.take<int>(1);
+    for (int i = 0; i < 2; ++i) sz.take<int>(1);
     sz.take<float>((size_t)qc * dpad);
     sz.take<float>((size_t)(qc + 1) / 2 * 2 * dpad);
     sz.take<float>((size_t)qc * nsplit * kk);
@@ -718,6 +716,7 @@ static int flat_exact_pruned(ann_flat* h, ann_workspace* ws, const float* qdev, 
     int* rcount = cv.take<int>((size_t)qc);
     int* list = cv.take<int>((size_t)qc);
     int* count = cv.take<int>(1);
+    int* err = cv.take<int>(1);
     float* qg = cv.take<float>((size_t)qc * dpad);
     float* qpair = cv.take<float>((size_t)(qc + 1) / 2 * 2 * dpad);
     float* skey = cv.take<float>((size_t)qc * nsplit * kk);
@@ -745,11 +744,12 @@ static int flat_exact_pruned(ann_flat* h, ann_workspace* ws, const float* qdev, 
         p.rcount = rcount;
         p.list = list;
         p.count = count;
+        p.err = err;
         p.out_ids = ids_dev + (size_t)q0 * kk;
         p.out_dists = dists_dev ? dists_dev + (size_t)q0 * kk : nullptr;
         if ((rc = launch_prune_queries(p, qb, kpad, st))) return rc;
         TcFilterArgs sa{nc, (int)S, kpad, kTcBF16};
-        sa.err = h->d_err;
+        sa.err = err;
         sa.out_min = kA;
         sa.b_tile_stride = stride;
         sa.b_rows = n;
@@ -757,7 +757,7 @@ static int flat_exact_pruned(ann_flat* h, ann_workspace* ws, const float* qdev, 
         sa.test_no_loads = h->wait_ns > 0;
         if ((rc = launch_tc_sample(qb, h->base_bf16, sa, st))) return rc;
         if ((rc = launch_bars(kA, nullptr, nullptr, nc, rF, rF, tauF, tauX, st, S / 8, win))) return rc;
-        const TcFilterArgs fa{nc, (int)n, kpad, kTcBF16, tauX, fkey, fcol, cap, rcount, nullptr, nullptr, h->d_err, h->wait_ns,
+        const TcFilterArgs fa{nc, (int)n, kpad, kTcBF16, tauX, fkey, fcol, cap, rcount, nullptr, nullptr, err, h->wait_ns,
                               h->wait_ns > 0};
         if ((rc = launch_tc_filter(qb, h->base_bf16, fa, st))) return rc;
         if ((rc = launch_prune_finish(p, st))) return rc;

@@ -14,7 +14,7 @@
 //      best k taken.
 // A query that the bound does not cover (norms out of range, NaN), whose bar was too low, or with more survivors
 // than fit goes to a list that the plain scan answers right after, its length read on the device: no step waits
-// for the host.
+// for the host. Every query does if a bounded wait of the passes gave up, since their keys may then be incomplete.
 #include "block_select.cuh"
 #include "common.cuh"
 #include "flat_prune.cuh"
@@ -99,7 +99,7 @@ __global__ void __launch_bounds__(256) prune_queries_kernel(PruneArgs a, __nv_bf
     const bool ok = s < kInf && qn <= kPruneNormMax && (l2 || sqrtf(s) >= kPruneNormMin);  // false for NaN
     a.win[q] = ok ? w : __int_as_float(0x7fffffff);
     a.rcount[q] = 0;
-    if (q == 0) *a.count = 0;
+    if (q == 0) *a.count = *a.err = 0;
 }
 
 // One block per query (file comment, step 3). Bound by the gather of the kept rows (about 500 rows of 1.5 KB a query
@@ -126,7 +126,7 @@ __global__ void __launch_bounds__(kFinWarps * 32) prune_finish_kernel(PruneArgs 
     const float w = a.win[q], tauF = a.tauF[q];
     const float* fk = a.fkey + (int64_t)q * cap;
     const int* fc = a.fcol + (int64_t)q * cap;
-    bool fail = cnt > cap || cnt < k || !(w < kInf);
+    bool fail = cnt > cap || cnt < k || !(w < kInf) || *a.err != 0;
     float T = 0.f;
     if (!fail) {  // the k-th smallest kept key
         for (int i = tid; i < cnt; i += kFinThreads) sO[i] = ord_f32(fk[i]);

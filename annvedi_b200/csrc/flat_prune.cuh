@@ -61,6 +61,7 @@ struct PruneArgs {
     int* rcount;        // [nq] survivors met
     int* list;          // [nq] queries left to the scan
     int* count;         // [1]
+    int* err;           // [1] set where a wait of the sample or filter pass gave up: every query is left to the scan
     int64_t* out_ids;   // [nq, k]
     float* out_dists;   // [nq, k] or null
 };
@@ -70,7 +71,7 @@ bool prune_fits(int k, int dpad);
 // Rank of the sampled bar: with S of n keys sampled, the smallest rank r for which the k smallest keys lie at or
 // below the r-th smallest sampled key with probability of about 1 - 1e-7.
 int prune_bar_rank(int k, int64_t S, int64_t n);
-// win and the queries' operand rows qb [nq, kpad] (launch_tc_operand's); rcount and count zeroed.
+// win and the queries' operand rows qb [nq, kpad] (launch_tc_operand's); rcount, count and err zeroed.
 int launch_prune_queries(const PruneArgs& a, __nv_bfloat16* qb, int kpad, cudaStream_t st);
 int launch_prune_finish(const PruneArgs& a, cudaStream_t st);  // results, list and count
 // qg[j] = q[list[j]] for j < *count.

@@ -62,3 +62,24 @@ def test_ivf_tensor_core_search(cuda, mode, nq):
     got = ix.search(q, 10, 0, 4, 40)
     assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
     assert ix._lib.ann_ivf_device_status(ix._h) == 0
+
+
+@pytest.mark.parametrize("metric", ["l2", "ip"])
+@pytest.mark.parametrize("n,dim,nq", [(60000, 64, 1), (60000, 64, 40), (40000, 100, 300)])
+def test_exact_search_falls_back_to_the_scan(cuda, metric, n, dim, nq):
+    """The exact search's tensor-core passes certify nothing where a wait gave up: the scan answers, and no error is left."""
+    import torch
+    from annvedi_b200.linear import LinearIndex
+    from tests.test_pruned_exact_gpu import _plain
+    rng = np.random.default_rng(nq)
+    ix = LinearIndex(device=0, metric=metric, mode="exact")
+    ix.fit(torch.from_numpy(rng.standard_normal((n, dim)).astype(np.float32)).cuda())
+    q = torch.from_numpy(rng.standard_normal((nq, dim)).astype(np.float32)).cuda()
+    ix.search_tc(q[:1], 1)  # the BF16 copy is there: the next exact search prunes
+    good = ix.search(q, 20)
+    wi, wd = _plain(ix, q, 20)
+    assert ix._lib.ann_flat_set_option(ix._h, FLAT_OPT_WAIT_SELFTEST, ctypes.c_int64(100000)) == 0
+    for ids, d in (good, ix.search(q, 20), ix.search(q.cpu().numpy(), 20)):
+        np.testing.assert_array_equal(np.asarray(ids.cpu() if torch.is_tensor(ids) else ids), wi)
+        np.testing.assert_array_equal(np.asarray(d.cpu() if torch.is_tensor(d) else d), wd)
+    assert ix._lib.ann_flat_device_status(ix._h) == 0
