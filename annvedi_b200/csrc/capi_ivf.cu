@@ -999,6 +999,7 @@ static size_t ivf_scratch(const ann_ivf* h, const IvfQueryCfg& c, int nq) {
     sz.take<int32_t>((size_t)nq);  // re-rank query order
     sz.take<int32_t>((size_t)nq);  // queries set apart (every row), and their count
     sz.take<int32_t>(1);
+    sz.take<int>(1);               // the exact form's key passes: a wait gave up
     sz.take<int64_t>(1);           // an every-row stream: its length
     sz.take<int32_t>(1);           // and its segment flag
     return sz.off;
@@ -1042,8 +1043,10 @@ constexpr int kRowCapFactor = 16;
 static int ivf_tc_sampled(ann_ivf* h, ann_workspace* ws, const IvfQueryCfg& c, const IvfQueryArgs& a,
                           IvfBatchArgs* bp, void* bscratch, int64_t* tot, const TcOperands& op, unsigned char* Apk,
                           int64_t* titem, int4* titem_desc, int64_t items_cap, float* keyR, int* idR, int prec,
-                          bool* done, cudaStream_t st, bool pruned = false) {
+                          bool* done, cudaStream_t st, int* key_err = nullptr) {
     *done = false;
+    const bool pruned = key_err != nullptr;
+    int* err = pruned ? key_err : h->d_err;
     const int nq = a.plan.nq, npc = c.npc, C = (int)h->C, R = c.R;
     const int64_t max_pairs = (int64_t)nq * npc;
     const int64_t largest = h->sizes_desc.empty() ? 1 : h->sizes_desc[0];
@@ -1147,7 +1150,7 @@ static int ivf_tc_sampled(ann_ivf* h, ann_workspace* ws, const IvfQueryCfg& c, c
     const TcItemDescs descs[2] = {{sitem, lcap, sitem_desc, scap}, {titem, nullptr, titem_desc, items_cap}};
     if ((rc = launch_tc_item_descs(descs, 2, C, b.lq_off, h->list_off, st))) return rc;
     // 1. sample pass: keys of the list heads into the sample streams; the two bars per query
-    TcGemmArgs gs{(int)max_pairs, (int)h->n, op.K, nullptr, SK, 0, h->d_err};
+    TcGemmArgs gs{(int)max_pairs, (int)h->n, op.K, nullptr, SK, 0, err};
     gs.wait_ns = h->wait_ns;
     gs.test_no_loads = h->wait_ns > 0;
     gs.kind = op.kind;
@@ -1169,7 +1172,7 @@ static int ivf_tc_sampled(ann_ivf* h, ann_workspace* ws, const IvfQueryCfg& c, c
     h->prof.kend(kt, kKernBars, st);
     // 2. filter pass over every row of the probed lists into the queries' buffers
     auto filter = [&](const float* tau, const int* skip_if_zero) -> int {
-        TcGemmArgs g{(int)max_pairs, (int)h->n, op.K, nullptr, nullptr, 0, h->d_err};
+        TcGemmArgs g{(int)max_pairs, (int)h->n, op.K, nullptr, nullptr, 0, err};
         g.wait_ns = h->wait_ns;
         g.test_no_loads = h->wait_ns > 0;
         g.skip_if_zero = skip_if_zero;
@@ -1200,10 +1203,11 @@ static int ivf_tc_sampled(ann_ivf* h, ann_workspace* ws, const IvfQueryCfg& c, c
         kt = h->prof.kbegin(st);
         if ((rc = launch_ivf_prune_finish(pa, st))) return rc;
         h->prof.kend(kt, kKernSelect, st);
-        int fails = 0;
+        int fails = 0, gave_up = 0;
         ANN_CUDA_TRY(cudaMemcpyAsync(&fails, pa.fails, sizeof(int), cudaMemcpyDeviceToHost, st));
+        ANN_CUDA_TRY(cudaMemcpyAsync(&gave_up, key_err, sizeof(int), cudaMemcpyDeviceToHost, st));
         ANN_CUDA_TRY(cudaStreamSynchronize(st));
-        *done = fails == 0;
+        *done = fails == 0 && gave_up == 0;
         return ANN_OK;
     }
     ANN_CUDA_TRY(cudaMemsetAsync(scount, 0, sizeof(int) * (size_t)nq, st));
@@ -1289,6 +1293,7 @@ static int ivf_query_device(ann_ivf* h, ann_workspace* ws, const IvfQueryCfg& c,
     int32_t* qorder = cv.take<int32_t>((size_t)nq);
     int32_t* apart = cv.take<int32_t>((size_t)nq);
     int32_t* apart_count = cv.take<int32_t>(1);
+    int* key_err = cv.take<int>(1);
     int64_t* every_len = cv.take<int64_t>(1);
     int32_t* every_seg = cv.take<int32_t>(1);
 
@@ -1310,7 +1315,10 @@ static int ivf_query_device(ann_ivf* h, ann_workspace* ws, const IvfQueryCfg& c,
     a.nsplit = c.nsplit;
     a.num_threads = c.num_threads;
     a.ndist = h->d_ndist;
-    a.err = h->d_err;
+    if (c.coarse_keys || c.pruned) {  // exact results: a call whose waits give up takes the scans instead
+        a.key_err = key_err;
+        ANN_CUDA_TRY(cudaMemsetAsync(key_err, 0, sizeof(int), st));
+    }
     a.out_ids = ids_dev;
     a.out_dists = dists_dev;
 
@@ -1320,7 +1328,7 @@ static int ivf_query_device(ann_ivf* h, ann_workspace* ws, const IvfQueryCfg& c,
     if (c.tc || c.coarse_keys) {
         // BF16 keys to every centroid, then the exact FP32 order of the best npc + 16
         if ((rc = launch_tc_operand(qdev, nq, h->dim, h->dpad, qb, h->kpad, kTcQuery, ANN_METRIC_L2, 0, st))) return rc;
-        TcGemmArgs ca{nq, h->C, h->kpad, nullptr, ckeys, h->C, h->d_err};
+        TcGemmArgs ca{nq, h->C, h->kpad, nullptr, ckeys, h->C, c.coarse_keys ? key_err : h->d_err};
         ca.wait_ns = h->wait_ns;
         ca.test_no_loads = h->wait_ns > 0;
         ca.out_cmin = ckmin;  // and each query's 32-centroid chunk minima, which let the ranking skip chunks
@@ -1412,20 +1420,20 @@ static int ivf_query_device(ann_ivf* h, ann_workspace* ws, const IvfQueryCfg& c,
     bool done = false;
     if (!c.ref && c.batched) {
         IvfBatchArgs b{};
-        int64_t tot_local[4] = {0, 0, 0, 0};
+        int64_t tot_local[5] = {0, 0, 0, 0, 0};
         int64_t* tot = tot_local;
         // The sampled path needs none of the set-up's totals to run: they land in page-locked words and are read
         // after its own synchronisation.
         const bool sampled = c.pruned || (c.tc && nq >= h->sampled_min_queries);
         if (sampled && (rc = ws_pinned(ws, &tot))) return rc;
-        tot[0] = tot[1] = tot[2] = tot[3] = 0;
+        for (int i = 0; i < 5; ++i) tot[i] = 0;
         auto run_sampled = [&](bool* ok) -> int {
             if (c.pruned) {
                 const int kpad = tc_kpad(h->dim, ANN_METRIC_L2);
                 const TcOperands op{nullptr, 2 * kpad, h->code_f16, kpad, kTcF16, nullptr, nullptr, nullptr};
                 const int64_t cap = tc_items_bound((int64_t)nq * c.npc, (int)h->C, h->sizes_desc[0]);
                 int r = ivf_tc_sampled(h, ws, c, a, &b, bscratch, tot, op, nullptr, nullptr, nullptr, cap, keyR, idR, prec,
-                                       ok, st, true);
+                                       ok, st, key_err);
                 if (r == ANN_ERR_NOMEM) {  // the batched pass may need less
                     clear_error();
                     r = batched_prepare(a, bscratch, &b, tot, st);
@@ -1460,6 +1468,13 @@ static int ivf_query_device(ann_ivf* h, ann_workspace* ws, const IvfQueryCfg& c,
             IvfBatchTiles tiles;
             tiles.titem = titem;
             if ((rc = batched_prepare(a, bscratch, &b, tot, st, true, tiles))) return rc;
+        }
+        if (c.coarse_keys && tot[4] != 0) {  // the probes may be wrong: again, ranked by the scan
+            const int64_t counted = tot[1] + (plan_apart ? tot[3] * h->n : 0);
+            if ((rc = launch_uncount(h->d_ndist, counted, st))) return rc;
+            IvfQueryCfg scan = c;
+            scan.coarse_keys = scan.pruned = false;
+            return ivf_query_device(h, ws, scan, base, qdev, nq, ids_dev, dists_dev, st);
         }
         if (tot[2] != 0) sampled_done = false;
         if (plan_apart) every_row.resize((size_t)(int)tot[3]);  // the plan has listed them in every_list

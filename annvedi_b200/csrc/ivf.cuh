@@ -74,7 +74,7 @@ struct IvfQueryArgs {
     float* P;                  // reference mode [nq, ncp, L]
     float* V;                  // reference mode [nq, L]
     unsigned long long* ndist; // device counter of candidates scanned (get_n_distances)
-    int* err;                  // device flag: a bounded wait gave up
+    const int* key_err;        // NULL, or the flag of the exact form's key passes: a bounded wait gave up
     int metric;                // re-rank metric: ANN_METRIC_L2 (default) or ANN_METRIC_IP
     int64_t* out_ids;          // [nq, k]
     float* out_dists;          // [nq, k]
@@ -116,6 +116,7 @@ int launch_set_every_row(const IvfPlan& plan, const int32_t* list, int count, in
 // neighbouring re-rank CTAs gather rows of the same lists; one CTA, C <= kQueryOrderMaxLists.
 constexpr int kQueryOrderMaxLists = 32768;
 int launch_query_order(const int32_t* probes, int npc, int nq, int C, int32_t* order, cudaStream_t st);
+int launch_uncount(unsigned long long* ndist, int64_t n, cudaStream_t st);  // *ndist -= n
 int launch_add_offset(int64_t* v, int64_t n, int64_t add, cudaStream_t st);  // v[i] += add
 // k-means of the reference (ivf_build.cu): certification of the fast two nearest centroids, the
 // reference arithmetic for the queued near-ties, and the ThreadPool-chunk-ordered update.

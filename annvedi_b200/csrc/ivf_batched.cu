@@ -83,7 +83,8 @@ __device__ __forceinline__ int64_t block_offsets(int n, int64_t* out, int64_t* s
 __global__ void __launch_bounds__(1024) batch_offsets_kernel(IvfPlan p, const int* __restrict__ cnt, int C,
                                                              const int64_t* __restrict__ list_off, int64_t* lq_off,
                                                              int64_t* item_off, int64_t* cand_off, const int* fallback,
-                                                             const int* apart_count, int64_t* totals, IvfBatchTiles t) {
+                                                             const int* apart_count, const int* key_err, int64_t* totals,
+                                                             IvfBatchTiles t) {
     __shared__ int64_t sWarp[32];
     auto rows = [&](int l) { return list_off[l + 1] - list_off[l]; };
     const bool first = threadIdx.x == 0;
@@ -97,6 +98,7 @@ __global__ void __launch_bounds__(1024) batch_offsets_kernel(IvfPlan p, const in
         if (first) {
             totals[0] = items;
             totals[2] = *fallback;
+            totals[4] = key_err ? *key_err : 0;
         }
     } else if (blockIdx.x == 2) {
         const int64_t cands = block_offsets(p.nq, cand_off, sWarp, [&](int q) { return p.n_cands[q]; });
@@ -349,7 +351,7 @@ size_t batched_scratch_bytes(int nq, int npc, int C) {
     sz.take<int64_t>((size_t)C + 1);                  // lq_off
     sz.take<int64_t>((size_t)C + 1);                  // item_off
     sz.take<int64_t>((size_t)nq + 1);                 // cand_off
-    sz.take<int64_t>(4);                              // totals
+    sz.take<int64_t>(5);                              // totals
     return sz.bytes();
 }
 
@@ -367,17 +369,17 @@ int batched_prepare(const IvfQueryArgs& a, void* scratch, IvfBatchArgs* out, int
     int64_t* lq_off = cv.take<int64_t>((size_t)C + 1);
     int64_t* item_off = cv.take<int64_t>((size_t)C + 1);
     int64_t* cand_off = cv.take<int64_t>((size_t)nq + 1);
-    int64_t* totals = cv.take<int64_t>(4);
+    int64_t* totals = cv.take<int64_t>(5);
     ANN_CUDA_TRY(cudaMemsetAsync(cnt, 0, sizeof(int) * ((size_t)C + 2), st));
     pair_rank_kernel<<<(unsigned)ceil_div(n, 256), 256, 0, st>>>(a.plan, cnt, rank, cnt + C, a.ix.list_off, tiles);
     ANN_LAUNCH_CHECK();
     batch_offsets_kernel<<<6, 1024, 0, st>>>(a.plan, cnt, C, a.ix.list_off, lq_off, item_off, cand_off, cnt + C,
-                                             a.apart ? a.apart_count : nullptr, totals, tiles);
+                                             a.apart ? a.apart_count : nullptr, a.key_err, totals, tiles);
     ANN_LAUNCH_CHECK();
     pair_place_kernel<<<(unsigned)std::min<int64_t>(ceil_div(n, 8), 16 * kNumSMs), 256, 0, st>>>(
         a.plan, rank, lq_off, a.ix.list_off, vals, lists, tiles);
     ANN_LAUNCH_CHECK();
-    ANN_CUDA_TRY(cudaMemcpyAsync(host_totals, totals, 4 * sizeof(int64_t), cudaMemcpyDeviceToHost, st));
+    ANN_CUDA_TRY(cudaMemcpyAsync(host_totals, totals, 5 * sizeof(int64_t), cudaMemcpyDeviceToHost, st));
     if (sync) ANN_CUDA_TRY(cudaStreamSynchronize(st));
     IvfBatchArgs b{};
     b.ix = a.ix;

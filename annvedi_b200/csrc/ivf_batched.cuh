@@ -46,8 +46,8 @@ struct IvfBatchTiles {
 
 // Scratch of batched_prepare for nq queries x npc probes over C lists.
 size_t batched_scratch_bytes(int nq, int npc, int C);
-// Groups the plan's probes by list (in no order within one), counts work items and candidate offsets; host_totals[0..3] =
-// {work items, total candidates, whether a query's stream is every row, queries set apart}. Synchronises the stream.
+// Groups the plan's probes by list (in no order within one), counts work items and candidate offsets; host_totals[0..4] =
+// {work items, total candidates, whether a query's stream is every row, queries set apart, *a.key_err}. Synchronises the stream.
 // With sync = false the totals are copied to host_totals (which must then be page-locked) without waiting: they
 // are valid after the caller's next synchronisation of st.
 int batched_prepare(const IvfQueryArgs& a, void* scratch, IvfBatchArgs* out, int64_t* host_totals, cudaStream_t st,

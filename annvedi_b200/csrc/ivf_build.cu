@@ -187,6 +187,14 @@ int launch_iota(int32_t* v, int64_t n, cudaStream_t st) {
     return ANN_OK;
 }
 
+__global__ void uncount_kernel(unsigned long long* ndist, unsigned long long n) { atomicAdd(ndist, 0ull - n); }
+
+int launch_uncount(unsigned long long* ndist, int64_t n, cudaStream_t st) {
+    uncount_kernel<<<1, 1, 0, st>>>(ndist, (unsigned long long)n);
+    ANN_LAUNCH_CHECK();
+    return ANN_OK;
+}
+
 int launch_add_offset(int64_t* v, int64_t n, int64_t add, cudaStream_t st) {
     if (n == 0) return ANN_OK;
     add_offset_kernel<<<(unsigned)std::min<int64_t>(ceil_div(n, 256), 16 * kNumSMs), 256, 0, st>>>(v, n, add);

@@ -83,3 +83,32 @@ def test_exact_search_falls_back_to_the_scan(cuda, metric, n, dim, nq):
         np.testing.assert_array_equal(np.asarray(ids.cpu() if torch.is_tensor(ids) else ids), wi)
         np.testing.assert_array_equal(np.asarray(d.cpu() if torch.is_tensor(d) else d), wd)
     assert ix._lib.ann_flat_device_status(ix._h) == 0
+
+
+@pytest.mark.parametrize("c,sizes,nq,k,npc", [(300, 40, 200, 10, 8), (300, 6, 64, 20, 2), (64, 1200, 600, 20, 8)])
+def test_exact_ivf_batch_takes_the_scans(cuda, c, sizes, nq, k, npc):
+    """The exact form's rankings by keys: where their waits give up, the batch has the small calls' results and count.
+    (300 lists: the coarse ranking; 64: the SQ8 selection, from the call on that has laid its operand out.)"""
+    import torch
+    from annvedi_b200.ivf import IVFIndex
+    rng = np.random.default_rng(c)
+    dim = 256
+    cen = rng.standard_normal((c, dim)).astype(np.float32)
+    assign = np.repeat(np.arange(c), sizes).astype(np.int32)
+    x = (cen[assign] + 0.3 * rng.standard_normal((len(assign), dim))).astype(np.float32)
+    ix = IVFIndex(device=0, mode="exact")
+    ix.fit(x, 1, 0, c, centroids=cen, assign=assign)
+    q = torch.from_numpy((cen[rng.integers(0, c, nq)] + 0.3 * rng.standard_normal((nq, dim))).astype(np.float32)).cuda()
+    for _ in range(8):
+        ix.search(q, k, 0, npc, 4 * k)
+    ix.reset_distances_count()
+    parts = [ix.search(q[s:s + 8].contiguous(), k, 0, npc, 4 * k) for s in range(0, nq, 8)]
+    torch.cuda.synchronize()
+    count = ix.total_distances_count()
+    ix.set_option("wait_selftest", 100000)
+    ix.reset_distances_count()
+    ids, d = ix.search(q, k, 0, npc, 4 * k)
+    torch.cuda.synchronize()
+    assert torch.equal(ids, torch.cat([p[0] for p in parts])) and torch.equal(d, torch.cat([p[1] for p in parts]))
+    assert ix.total_distances_count() == count
+    assert ix._lib.ann_ivf_device_status(ix._h) == 0
