@@ -225,6 +225,7 @@ int ann_flat_destroy(ann_flat* h) {
         if (h->base_e4m3) cudaFree(h->base_e4m3);
         if (h->fac_e4m3) cudaFree(h->fac_e4m3);
         if (h->d_err) cudaFree(h->d_err);
+        if (h->prune_word) cudaFreeHost(h->prune_word);  // (the frees above have waited for the device)
     }
     ws_release(&h->ws);
     delete h;
@@ -260,6 +261,8 @@ int ann_flat_fit(ann_flat* h, const float* data, int64_t n, int32_t dim, int64_t
     }
     h->bounds_known = false;
     h->prune_credit_us = 0.0;
+    h->prune_streak = h->prune_skip = 0;
+    h->prune_seen = h->prune_pass;
     const size_t bytes = sizeof(float) * (size_t)n * dpad;
     cudaError_t e = cudaMalloc(&h->base, bytes);
     if (e != cudaSuccess) {
@@ -614,16 +617,18 @@ static int flat_check_err(ann_flat* h) {
 // / pruned, us a call: 1M x 384: 376 / 194 (1 query), 1121 / 213 (8), 45342 / 873 (1,000); 32768 x 64: 105 / 68
 // (1), 2550 / 130 (1,000). *ok = false (and no error) where the search keeps to the plain scan: not yet laid out,
 // a copy that would take more than half of the free memory, or rows that the bounds do not cover.
+static bool flat_prune_open(ann_flat* h, bool capturing);
 static int flat_ensure_pruned(ann_flat* h, int nq, cudaStream_t st, bool* ok) {
     *ok = false;
     std::lock_guard<std::mutex> lk(h->tc_mu);
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    ANN_CUDA_TRY(cudaStreamIsCapturing(st, &cs));
+    const bool capturing = cs != cudaStreamCaptureStatusNone;
     if (!h->bounds_known) {
         const double elems = (double)h->n * h->dim;
         h->prune_credit_us += 40.0 + elems * (nq <= 4 ? 0.25e-6 + 0.2e-6 * (nq - 1) : 1.0e-7 * nq);
         if (!h->base_bf16 && h->prune_credit_us < 500.0 + 3.1e-6 * elems) return ANN_OK;
-        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-        ANN_CUDA_TRY(cudaStreamIsCapturing(st, &cs));
-        if (cs != cudaStreamCaptureStatusNone) return ANN_OK;
+        if (capturing) return ANN_OK;
         if (!h->base_bf16) {
             size_t mfree = 0, mtotal = 0;
             ANN_CUDA_TRY(cudaMemGetInfo(&mfree, &mtotal));
@@ -654,9 +659,47 @@ static int flat_ensure_pruned(ann_flat* h, int nq, cudaStream_t st, bool* ok) {
         h->bounds = PruneBounds{};
         if (c >= kPruneNormMin && c <= kPruneNormMax && r <= c) h->bounds = PruneBounds{c * 1.001f, r * 1.001f};
         h->bounds_known = true;
+        if (!h->prune_word) {
+            void* w = nullptr;
+            if (cudaHostAlloc(&w, sizeof(*h->prune_word), cudaHostAllocPortable | cudaHostAllocMapped) == cudaSuccess) {
+                h->prune_word = static_cast<unsigned long long*>(w);
+                *h->prune_word = (unsigned long long)h->prune_seen << 32;
+            } else {
+                cudaGetLastError();  // no back-off then
+            }
+        }
     }
-    *ok = h->bounds.cmax > 0.f;
+    *ok = h->bounds.cmax > 0.f && flat_prune_open(h, capturing);
     return ANN_OK;
+}
+
+// Whether this call tries the pruned form (under tc_mu). The window grows with |x| |q|, not with the rows' spread: over data
+// far from the origin, or with more copies of a row than survivors fit, the pass leaves the queries to the scan and was
+// for nothing (N(50, 0.01), 37 queries over 131,725 x 33, inner product: 328 us scanned, 902 with the pass). A pass that
+// left more than a quarter of its queries is followed by 4 calls of the scan alone, then 8, up to 1,024, until one does not.
+// The device writes the count; it is read here without a wait, so by a later call than the next where calls are queued.
+// A captured call keeps the form for every replay, and one bad pass may have been its queries' doing (a warm-up on zeros):
+// it is the scan from the second such pass on.
+static bool flat_prune_open(ann_flat* h, bool capturing) {
+    if (h->prune_word) {
+        const unsigned long long w = __atomic_load_n(h->prune_word, __ATOMIC_RELAXED);
+        if ((uint32_t)(w >> 32) != h->prune_seen) {
+            h->prune_seen = (uint32_t)(w >> 32);
+            const unsigned n = (unsigned)(w >> 16) & 0xffffu, left = (unsigned)w & 0xffffu;
+            if (4 * left > n) {
+                h->prune_skip = 4 << std::min(h->prune_streak, 8);
+                ++h->prune_streak;
+            } else {
+                h->prune_streak = h->prune_skip = 0;
+            }
+        }
+    }
+    if (capturing) return h->prune_streak < 2;
+    if (h->prune_skip > 0) {
+        --h->prune_skip;
+        return false;
+    }
+    return true;
 }
 
 // The pruned form of the exact scan (flat_prune.cu) for queries qdev [nq, dpad]; *done = false, and nothing
@@ -762,7 +805,12 @@ static int flat_exact_pruned(ann_flat* h, ann_workspace* ws, const float* qdev, 
         if ((rc = launch_tc_filter(qb, h->base_bf16, fa, st))) return rc;
         if ((rc = launch_prune_finish(p, st))) return rc;
         // the queries on the list, by the plain scan (none, nearly always: the kernels read the count and return)
-        if ((rc = launch_prune_gather(q, dpad, list, count, nc, qg, st))) return rc;
+        uint32_t pass;
+        {
+            std::lock_guard<std::mutex> lk(h->tc_mu);
+            pass = ++h->prune_pass;
+        }
+        if ((rc = launch_prune_gather(q, dpad, list, count, nc, qg, h->prune_word, pass, st))) return rc;
         FlatScanArgs a{h->base, n, dpad, qg, nc, h->metric, kk, rps, nsplit, skey, sid};
         a.qpair = qpair;
         a.nq_dev = count;
@@ -826,6 +874,18 @@ int ann_flat_set_option(ann_flat* h, int32_t option, int64_t value) {
             set_error("ann_flat_set_option: unknown option %d", option);
             return ANN_ERR_INVALID;
     }
+}
+
+int ann_flat_prune_stats(ann_flat* h, int64_t* out4) {
+    clear_error();
+    ANN_CHECK_ARG(h != nullptr && out4 != nullptr, "ann_flat_prune_stats: null argument");
+    std::lock_guard<std::mutex> lk(h->tc_mu);
+    const unsigned long long w = h->prune_word ? __atomic_load_n(h->prune_word, __ATOMIC_RELAXED) : 0;
+    out4[0] = h->prune_pass;
+    out4[1] = (int64_t)(w >> 16) & 0xffff;
+    out4[2] = (int64_t)w & 0xffff;
+    out4[3] = h->prune_skip;
+    return ANN_OK;
 }
 
 int ann_flat_set_tc_precision(ann_flat* h, int32_t precision) {

@@ -32,6 +32,13 @@ struct ann_flat {
     annb::PruneBounds bounds;            // of the BF16 copy's keys (cmax 0: the rows are not covered)
     bool bounds_known = false;
     double prune_credit_us = 0.0;        // what pruning would have saved the exact searches so far (estimated)
+    // how the latest pruned pass ended, written by the device (page-locked; pass << 32 | queries << 16 | queries left to
+    // the scan), and the back-off that follows from it (flat_prune_open)
+    unsigned long long* prune_word = nullptr;
+    uint32_t prune_pass = 0;             // passes launched
+    uint32_t prune_seen = 0;             // the latest whose end has been read
+    int prune_streak = 0;                // passes in a row that left too many queries
+    int prune_skip = 0;                  // calls that the scan still answers
 };
 
 namespace annb {

@@ -226,8 +226,10 @@ __global__ void __launch_bounds__(kFinWarps * 32) prune_finish_kernel(PruneArgs 
 }
 
 __global__ void prune_gather_kernel(const float* __restrict__ q, int dpad, const int* __restrict__ list,
-                                    const int* __restrict__ count, float* __restrict__ qg) {
+                                    const int* __restrict__ count, float* __restrict__ qg, int nq,
+                                    volatile unsigned long long* word, uint32_t pass) {
     const int n = *count;
+    if (word && blockIdx.x == 0 && threadIdx.x == 0) *word = ((unsigned long long)pass << 32) | ((unsigned)nq << 16) | (unsigned)n;
     for (int j = blockIdx.x; j < n; j += gridDim.x)
         for (int d = threadIdx.x; d < dpad; d += blockDim.x) qg[(int64_t)j * dpad + d] = q[(int64_t)list[j] * dpad + d];
 }
@@ -285,8 +287,10 @@ int launch_prune_finish(const PruneArgs& a, cudaStream_t st) {
     return wide ? run_finish<16>(a, st) : run_finish<8>(a, st);
 }
 
-int launch_prune_gather(const float* q, int dpad, const int* list, const int* count, int nq, float* qg, cudaStream_t st) {
-    prune_gather_kernel<<<(unsigned)std::min(nq, 2 * kNumSMs), 128, 0, st>>>(q, dpad, list, count, qg);
+int launch_prune_gather(const float* q, int dpad, const int* list, const int* count, int nq, float* qg,
+                        unsigned long long* word, uint32_t pass, cudaStream_t st) {
+    ANN_CHECK_ARG(nq <= 65535, "pruned scan: %d queries a pass", nq);
+    prune_gather_kernel<<<(unsigned)std::min(nq, 2 * kNumSMs), 128, 0, st>>>(q, dpad, list, count, qg, nq, word, pass);
     ANN_LAUNCH_CHECK();
     return ANN_OK;
 }

@@ -74,7 +74,9 @@ int prune_bar_rank(int k, int64_t S, int64_t n);
 // win and the queries' operand rows qb [nq, kpad] (launch_tc_operand's); rcount, count and err zeroed.
 int launch_prune_queries(const PruneArgs& a, __nv_bfloat16* qb, int kpad, cudaStream_t st);
 int launch_prune_finish(const PruneArgs& a, cudaStream_t st);  // results, list and count
-// qg[j] = q[list[j]] for j < *count.
-int launch_prune_gather(const float* q, int dpad, const int* list, const int* count, int nq, float* qg, cudaStream_t st);
+// qg[j] = q[list[j]] for j < *count; *word (page-locked host memory, optional) = pass << 32 | nq << 16 | *count
+// (nq <= 65,535).
+int launch_prune_gather(const float* q, int dpad, const int* list, const int* count, int nq, float* qg,
+                        unsigned long long* word, uint32_t pass, cudaStream_t st);
 
 }  // namespace annb

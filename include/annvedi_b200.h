@@ -150,6 +150,11 @@ int ann_flat_set_tc_precision(ann_flat* h, int32_t precision);
 #define ANN_FLAT_OPT_WAIT_SELFTEST 2
 int ann_flat_set_option(ann_flat* h, int32_t option, int64_t value);
 
+/* Diagnostic: the exact search's passes of tensor-core keys (queries whose result those certify skip the scan): out4 =
+ * {passes launched, queries of the latest finished pass, queries that it left to the scan, calls that the scan alone
+ * still answers because passes left too many}. A call takes one pass per 10,240 queries, or none. Does not synchronise. */
+int ann_flat_prune_stats(ann_flat* h, int64_t* out4);
+
 /* Diagnostic: the tensor-core key matrix out_keys[nq][n] (device pointers; synchronous). */
 int ann_flat_scores_tc(ann_flat* h, const float* queries, int32_t nq, int64_t ldq, float* out_keys, void* stream);
 
