@@ -261,6 +261,8 @@ int ann_flat_fit(ann_flat* h, const float* data, int64_t n, int32_t dim, int64_t
     }
     h->bounds_known = false;
     h->prune_credit_us = 0.0;
+    h->prune_refused = false;
+    h->prune_ws_refused = SIZE_MAX;
     h->prune_streak = h->prune_skip = 0;
     h->prune_seen = h->prune_pass;
     const size_t bytes = sizeof(float) * (size_t)n * dpad;
@@ -616,7 +618,7 @@ static int flat_check_err(ann_flat* h) {
 // that brings them to its cost -- at once for a large batch, after a dozen single queries otherwise. Measured, scan
 // / pruned, us a call: 1M x 384: 376 / 194 (1 query), 1121 / 213 (8), 45342 / 873 (1,000); 32768 x 64: 105 / 68
 // (1), 2550 / 130 (1,000). *ok = false (and no error) where the search keeps to the plain scan: not yet laid out,
-// a copy that would take more than half of the free memory, or rows that the bounds do not cover.
+// a copy that would take more than half of the free memory (asked once a fit), or rows that the bounds do not cover.
 static bool flat_prune_open(ann_flat* h, bool capturing);
 static int flat_ensure_pruned(ann_flat* h, int nq, cudaStream_t st, bool* ok) {
     *ok = false;
@@ -628,24 +630,15 @@ static int flat_ensure_pruned(ann_flat* h, int nq, cudaStream_t st, bool* ok) {
         const double elems = (double)h->n * h->dim;
         h->prune_credit_us += 40.0 + elems * (nq <= 4 ? 0.25e-6 + 0.2e-6 * (nq - 1) : 1.0e-7 * nq);
         if (!h->base_bf16 && h->prune_credit_us < 500.0 + 3.1e-6 * elems) return ANN_OK;
-        if (capturing) return ANN_OK;
-        if (!h->base_bf16) {
-            size_t mfree = 0, mtotal = 0;
-            ANN_CUDA_TRY(cudaMemGetInfo(&mfree, &mtotal));
-            if (sizeof(__nv_bfloat16) * (size_t)h->n * tc_kpad(h->dim, h->metric) > mfree / 2) return ANN_OK;
-        }
-        int rc = flat_ensure_bf16(h, st);
-        if (rc == ANN_ERR_NOMEM) {
-            clear_error();
-            return ANN_OK;
-        }
-        if (rc) return rc;
+        if (capturing || (h->prune_refused && !h->base_bf16)) return ANN_OK;
+        // the norms first: rows that the bounds do not cover need no copy
         unsigned *d2 = nullptr, h2[2] = {0, 0};
         if (cudaMalloc(&d2, sizeof(h2)) != cudaSuccess) {
             cudaGetLastError();
+            h->prune_refused = true;
             return ANN_OK;
         }
-        rc = launch_base_norms(h->base, h->n, h->dim, h->dpad, d2, st);
+        int rc = launch_base_norms(h->base, h->n, h->dim, h->dpad, d2, st);
         cudaError_t e = cudaSuccess;
         if (!rc) e = cudaMemcpyAsync(h2, d2, sizeof(h2), cudaMemcpyDeviceToHost, st);
         if (!rc && e == cudaSuccess) e = cudaStreamSynchronize(st);
@@ -656,8 +649,20 @@ static int flat_ensure_pruned(ann_flat* h, int nq, cudaStream_t st, bool* ok) {
         memcpy(&s2, &h2[0], 4);
         memcpy(&e2, &h2[1], 4);
         const float c = std::sqrt(s2), r = std::sqrt(e2);
-        h->bounds = PruneBounds{};
-        if (c >= kPruneNormMin && c <= kPruneNormMax && r <= c) h->bounds = PruneBounds{c * 1.001f, r * 1.001f};
+        const bool covered = c >= kPruneNormMin && c <= kPruneNormMax && r <= c;
+        if (covered && !h->base_bf16) {
+            size_t mfree = 0, mtotal = 0;
+            ANN_CUDA_TRY(cudaMemGetInfo(&mfree, &mtotal));
+            const bool fits = sizeof(__nv_bfloat16) * (size_t)h->n * tc_kpad(h->dim, h->metric) <= mfree / 2;
+            if (fits) rc = flat_ensure_bf16(h, st);
+            if (!fits || rc == ANN_ERR_NOMEM) {  // not asked for again: the query for free memory alone can stall a server
+                clear_error();
+                h->prune_refused = true;
+                return ANN_OK;
+            }
+            if (rc) return rc;
+        }
+        h->bounds = covered ? PruneBounds{c * 1.001f, r * 1.001f} : PruneBounds{};
         h->bounds_known = true;
         if (!h->prune_word) {
             void* w = nullptr;
@@ -743,9 +748,15 @@ static int flat_exact_pruned(ann_flat* h, ann_workspace* ws, const float* qdev, 
     sz.take<float>((size_t)(qc + 1) / 2 * 2 * dpad);
     sz.take<float>((size_t)qc * nsplit * kk);
     sz.take<int>((size_t)qc * nsplit * kk);
+    {
+        std::lock_guard<std::mutex> lk(h->tc_mu);
+        if (sz.bytes() >= h->prune_ws_refused && ws->big_cap < sz.bytes()) return ANN_OK;
+    }
     if ((rc = ws_reserve_big(ws, sz.bytes()))) {
         if (rc != ANN_ERR_NOMEM) return rc;
         clear_error();
+        std::lock_guard<std::mutex> lk(h->tc_mu);
+        h->prune_ws_refused = std::min(h->prune_ws_refused, sz.bytes());
         return ANN_OK;
     }
     Carver cv(ws->big);

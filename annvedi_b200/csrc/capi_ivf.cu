@@ -900,10 +900,10 @@ static int ivf_ensure_codes(ann_ivf* h, double saved_us, cudaStream_t st, bool* 
         size_t mfree = 0, mtotal = 0;
         ANN_CUDA_TRY(cudaMemGetInfo(&mfree, &mtotal));
         const size_t bytes = (sizeof(__nv_bfloat16) * (size_t)h->n * kpad + 255) / 256 * 256;
-        if (bytes > mfree / 2) return ANN_OK;
         char* cb = nullptr;  // the operand rows, then a word for their largest norm
-        if (cudaMalloc(&cb, bytes + 256) != cudaSuccess) {
+        if (bytes > mfree / 2 || cudaMalloc(&cb, bytes + 256) != cudaSuccess) {
             cudaGetLastError();
+            h->codes_known = true;  // not asked for again until the next fit
             return ANN_OK;
         }
         unsigned* d2 = reinterpret_cast<unsigned*>(cb + bytes);

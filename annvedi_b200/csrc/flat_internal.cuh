@@ -32,6 +32,8 @@ struct ann_flat {
     annb::PruneBounds bounds;            // of the BF16 copy's keys (cmax 0: the rows are not covered)
     bool bounds_known = false;
     double prune_credit_us = 0.0;        // what pruning would have saved the exact searches so far (estimated)
+    bool prune_refused = false;          // the BF16 copy for them did not fit beside what the card holds (until the next fit)
+    size_t prune_ws_refused = SIZE_MAX;  // scratch of this size did not fit
     // how the latest pruned pass ended, written by the device (page-locked; pass << 32 | queries << 16 | queries left to
     // the scan), and the back-off that follows from it (flat_prune_open)
     unsigned long long* prune_word = nullptr;

@@ -1,0 +1,80 @@
+"""The operand copies that the exact searches lay out for themselves: none for rows that the keys' bounds do not cover, and one
+that did not fit beside what the card holds is not asked for again until the next fit."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _free():
+    import torch
+    torch.cuda.synchronize()
+    return torch.cuda.mem_get_info()[0]
+
+
+class _Filled:
+    """All but `left` bytes of the card's free memory held."""
+
+    def __init__(self, left):
+        self.left = left
+
+    def __enter__(self):
+        import torch
+        torch.cuda.empty_cache()
+        self.block = torch.empty(_free() - self.left, dtype=torch.uint8, device="cuda")
+
+    def __exit__(self, *exc):
+        import torch
+        del self.block
+        torch.cuda.empty_cache()
+
+
+def test_uncovered_rows_get_no_copy(cuda):
+    import torch
+    from annvedi_b200.linear import LinearIndex
+    n, dim = 200_000, 256
+    x = torch.randn(n, dim, device="cuda")
+    x[5, 7] = float("inf")
+    ix = LinearIndex(device=0, mode="exact")
+    ix.fit(x)
+    q = torch.randn(500, dim, device="cuda")
+    ix.search(q, 10, mode="exact")  # (this call's estimated savings are beyond the copy's cost)
+    torch.cuda.empty_cache()
+    before = _free()
+    for _ in range(3):
+        ix.search(q, 10, mode="exact")
+    torch.cuda.empty_cache()
+    assert before - _free() < 64 << 20 and ix.get_prune_stats()["passes"] == 0
+    fresh = LinearIndex(device=0, mode="exact")
+    fresh.fit(x)
+    torch.cuda.empty_cache()
+    before = _free()
+    fresh.search(q, 10, mode="exact")
+    torch.cuda.empty_cache()
+    assert before - _free() < n * dim * 2  # the scan's scratch, no copy
+
+
+def test_refused_copy_is_not_asked_for_again(cuda):
+    import torch
+    from annvedi_b200.linear import LinearIndex
+    n, dim = 1_000_000, 512  # the copy: 1.06 GB
+    x = torch.randn(n, dim, device="cuda")
+    ix = LinearIndex(device=0, mode="exact")
+    ix.fit(x)
+    q = torch.randn(64, dim, device="cuda")
+    want = ix.search(q, 10, mode="exact", workspace=None)
+    ix.fit(x)  # (the copy that the call laid out is given back)
+    ix.search(q[:1], 10)  # the scan's scratch is there
+    with _Filled(1500 << 20):
+        for _ in range(3):
+            ids, d = ix.search(q, 10)
+        torch.cuda.synchronize()
+        assert torch.equal(ids, want[0]) and torch.equal(d, want[1])
+    for _ in range(3):
+        ix.search(q, 10)
+    assert ix.get_prune_stats()["passes"] == 1  # the first index state's
+    ix.fit(x)
+    ids, d = ix.search(q, 10)
+    torch.cuda.synchronize()
+    assert ix.get_prune_stats()["passes"] == 2
+    assert torch.equal(ids, want[0]) and torch.equal(d, want[1])
