@@ -406,7 +406,7 @@ int ann_flat_query(ann_flat* h, ann_workspace* ws, const float* queries, int32_t
     // ---- search ----
     const int prec = h->prof.begin(st);
     bool pruned = false;
-    if (mode == ANN_MODE_EXACT && h->query_tile == 0) {  // a set tile asks for the scan itself
+    if (mode == ANN_MODE_EXACT && h->prune) {
         if ((rc = flat_exact_pruned(h, ws, qdev, nq, kk, ids_dev, dists_dev, st, &pruned))) return rc;
     }
     if (pruned) {
@@ -718,7 +718,7 @@ static int flat_exact_pruned(ann_flat* h, ann_workspace* ws, const float* qdev, 
     bool ok = false;
     int rc = flat_ensure_pruned(h, nq, st, &ok);
     if (rc || !ok) return rc;
-    const int bq = std::min(flat_scan_bq(nq), flat_scan_max_bq(kk));
+    const int bq = std::min(h->query_tile > 0 ? h->query_tile : flat_scan_bq(nq), flat_scan_max_bq(kk));
     const bool stream_form = flat_stream_eligible(bq, kk, dpad);
     // a sample of about 64 tiles of 256 rows, an eighth of a small base
     const int64_t full_tiles = n / 256;
@@ -875,6 +875,10 @@ int ann_flat_set_option(ann_flat* h, int32_t option, int64_t value) {
             ANN_CHECK_ARG(value == 0 || value == 8 || value == 16 || value == 32,
                           "ann_flat_set_option: query tile %lld (0, 8, 16 or 32)", (long long)value);
             h->query_tile = (int)value;
+            return ANN_OK;
+        case ANN_FLAT_OPT_PRUNE:
+            ANN_CHECK_ARG(value == 0 || value == 1, "ann_flat_set_option: pruning %lld (0 or 1)", (long long)value);
+            h->prune = value != 0;
             return ANN_OK;
         case ANN_FLAT_OPT_WAIT_SELFTEST:
             ANN_CHECK_ARG(value == 0 || (value >= 1000 && value <= 2000000000LL), "ann_flat_set_option: wait limit %lld ns",

@@ -27,6 +27,7 @@ struct ann_flat {
     uint8_t* base_e4m3 = nullptr;        // [n, kpad8] E4M3 operand form, Weyl order, built on first use
     float2* fac_e4m3 = nullptr;          // [n] its per-row key factors
     int kpad8 = 0;                       // dim rounded up to 32
+    bool prune = true;                   // the exact search may prune by tensor-core keys
     uint64_t wait_ns = 0;                // > 0: the self-test of the bounded waits, with this limit
     std::mutex tc_mu;                    // serialises the first use of the operand forms above
     annb::PruneBounds bounds;            // of the BF16 copy's keys (cmax 0: the rows are not covered)

@@ -177,6 +177,11 @@ class LinearIndex:
         by the batch size. Results are the same for 8, 16 and 32; the tile changes speed only."""
         _lib.check(self._lib.ann_flat_set_option(self._h, 1, int(tile)))
 
+    def set_pruning(self, enabled: bool = True) -> None:
+        """Whether the exact search may prune the rows by tensor-core keys (ANN_FLAT_OPT_PRUNE; the default) or the scan
+        answers every query. The results are the scan's either way."""
+        _lib.check(self._lib.ann_flat_set_option(self._h, 3, int(bool(enabled))))
+
     def set_tc_precision(self, precision: str = "bf16") -> None:
         """Element kind of search_tc / scores_tc: "bf16" (default) or "e4m3" (scaled FP8: twice the tensor
         rate, a coarser key; pair it with a deeper refine_r)."""

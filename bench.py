@@ -268,6 +268,7 @@ def run_ours(args, rank, world, local):
         def flat_step():
             flat.search(queries, K_NN, mode="exact", out_ids=f_ids, out_dists=f_d)
 
+        flat.set_pruning(False)
         # the scan's query tile (a tile shape: queries sharing each staged row chunk) chosen by timing, so the
         # denominator is the plain scan at its best tile
         from annvedi_b200 import autotune

@@ -148,6 +148,9 @@ int ann_flat_set_tc_precision(ann_flat* h, int32_t precision);
 /*   ANN_FLAT_OPT_WAIT_SELFTEST: value > 0 (1e3..2e9): the tensor-core kernels of the index's searches issue no copies,
  *     so that their bounded waits give up after `value` ns, as in ann_tc_wait_selftest; 0 (the default): off. */
 #define ANN_FLAT_OPT_WAIT_SELFTEST 2
+/*   ANN_FLAT_OPT_PRUNE: 1 (the default): the exact search may prune the rows by tensor-core keys, whatever the query
+ *     tile; 0: the scan answers every query. The results are the scan's either way. */
+#define ANN_FLAT_OPT_PRUNE 3
 int ann_flat_set_option(ann_flat* h, int32_t option, int64_t value);
 
 /* Diagnostic: the exact search's passes of tensor-core keys (queries whose result those certify skip the scan): out4 =
