@@ -969,8 +969,10 @@ int ann_flat_query_tc(ann_flat* h, ann_workspace* ws, const float* queries, int3
     // n R / S keys pass it). The fast bar, the rF-th, lets n rF / S keys pass, rF just past the number of the
     // R best that a sample holds: fewer than R survivors, about 1 query in 10^7. The full pass keeps the keys
     // under the fast bar; a query with fewer than R survivors (the count is exact) is re-run under its
-    // safe bar, so every query ends with its best R keys among its survivors. Small bases, or a
-    // survivor overflow, use the full key matrix. (With every sampled key written and binned, a tenth of
+    // safe bar, so every query ends with its best R keys among its survivors. A query with more survivors than its
+    // buffer holds (thousands of copies of a row) is re-run under its fast bar with room for all of them: with the
+    // chunk's full key matrix in its place, 5 queries over 191,343 x 9, a third of the rows zero, took 1,145 us, 338 now.
+    // Small bases use the full key matrix. (With every sampled key written and binned, a tenth of
     // a 10,000-query call went to the bars: sample and bars 1.59 ms, 0.31 ms from the minima.)
     const int64_t n = h->n;
     const int64_t full_tiles = n / 256;
@@ -999,13 +1001,14 @@ int ann_flat_query_tc(ann_flat* h, ann_workspace* ws, const float* queries, int3
             // mixture), n R / S the safe bar of a re-run
             const int cap = (int)cap64;
             const int cap2 = (int)std::min<int64_t>(n, 2 * ceil_div((int64_t)R * n, S) + 1024);
-            const size_t ent = std::max((size_t)nc * cap, (size_t)std::min(nc, kRerunBatch) * cap2);
+            const size_t ent = std::max(std::max((size_t)nc * cap, (size_t)std::min(nc, kRerunBatch) * cap2),
+                                        (size_t)std::min<int64_t>(n, 1 << 24));  // one query's every row at least
             Sizer s2;
             s2.take<float>((size_t)nc * (S / 8));      // minima of 8 sampled keys
             s2.take<float>(ent);                       // survivors: key, position
             s2.take<int>(ent);
             for (int i = 0; i < 3; ++i) s2.take<float>((size_t)nc);  // fast, safe, gathered bars
-            for (int i = 0; i < 2; ++i) s2.take<int>((size_t)nc);    // row counts, re-run list
+            for (int i = 0; i < 3; ++i) s2.take<int>((size_t)nc);    // row counts, re-run lists
             s2.take<int>(4);                           // flags
             s2.take<unsigned char>((size_t)kRerunBatch * rowb);
             s2.take<float>((size_t)kRerunBatch);
@@ -1019,7 +1022,8 @@ int ann_flat_query_tc(ann_flat* h, ann_workspace* ws, const float* queries, int3
             float* tau2 = cb.take<float>((size_t)nc);
             int* rowcnt = cb.take<int>((size_t)nc);
             int* list = cb.take<int>((size_t)nc);
-            int* flags = cb.take<int>(4);
+            int* over = cb.take<int>((size_t)nc);
+            int* flags = cb.take<int>(4);  // queries in list and in over, most survivors of a query
             unsigned char* A2 = cb.take<unsigned char>((size_t)kRerunBatch * rowb);
             float* rfac2 = cb.take<float>((size_t)kRerunBatch);
 
@@ -1044,49 +1048,63 @@ int ann_flat_query_tc(ann_flat* h, ann_workspace* ws, const float* queries, int3
                                       rcap, rowcnt, t.cfac, rf,     h->d_err, h->wait_ns, h->wait_ns > 0};
                 int r = launch_tc_filter(A, t.base, fa, st);
                 if (r) return r;
-                return launch_max_int(rowcnt, M, flags + 1, st);
+                return launch_max_int(rowcnt, M, flags + 2, st);
             };
             if ((rc = filter(qbc, nc, tauF, rfc, cap))) return rc;
             h->prof.mark(prec, st);
             if (prec >= 0) h->prof.filter_launches += 1;
-            ANN_CUDA_TRY(cudaMemsetAsync(flags, 0, sizeof(int), st));
-            if ((rc = launch_tc_bar_check(rowcnt, nc, R, list, flags, st))) return rc;
-            int hf[2] = {0, 0};  // re-runs, most survivors of a query
+            ANN_CUDA_TRY(cudaMemsetAsync(flags, 0, 2 * sizeof(int), st));
+            if ((rc = launch_tc_bar_check(rowcnt, nc, R, list, flags, st, nullptr, nullptr, cap, over))) return rc;
+            int hf[3] = {0, 0, 0};
             ANN_CUDA_TRY(cudaMemcpyAsync(hf, flags, sizeof(hf), cudaMemcpyDeviceToHost, st));
             ANN_CUDA_TRY(cudaStreamSynchronize(st));
             int ngemm = 2;
-            if (hf[1] <= cap) {
-                RadixSelectArgs sv{};
-                sv.keys = fkey;
-                sv.ld = cap;
-                sv.lens32 = rowcnt;
-                sv.ids = fcol;
-                sv.R = R;
-                sv.out_key = keyRc;
-                sv.out_id = idRc;
-                if ((rc = launch_radix_select(sv, nc, st))) return rc;
-                done = true;
-                for (int j0 = 0; j0 < hf[0] && done; j0 += kRerunBatch) {
-                    const int nb = std::min(kRerunBatch, hf[0] - j0);
-                    if ((rc = launch_tc_gather(qbc, (int)rowb, list + j0, nb, tauS, A2, tau2, rfc, rfac2, st)))
-                        return rc;
-                    if ((rc = filter(A2, nb, tau2, e4 ? rfac2 : nullptr, cap2))) return rc;
-                    ++ngemm;
-                    int hmax = 0;
-                    ANN_CUDA_TRY(cudaMemcpyAsync(&hmax, flags + 1, sizeof(int), cudaMemcpyDeviceToHost, st));
-                    ANN_CUDA_TRY(cudaStreamSynchronize(st));
-                    if (hmax > cap2) {
+            RadixSelectArgs sv{};
+            sv.keys = fkey;
+            sv.ld = cap;
+            sv.lens32 = rowcnt;
+            sv.ids = fcol;
+            sv.R = R;
+            sv.out_key = keyRc;
+            sv.out_id = idRc;
+            if ((rc = launch_radix_select(sv, nc, st))) return rc;
+            done = true;
+            // queries rows[0..count) again under the bars tau, room for rcap survivors each, or for as many as one turns out
+            // to have; done = false where those exceed the buffer
+            auto redo = [&](const int* rows, int count, const float* tau, int rcap) -> int {
+                for (int j0 = 0; j0 < count && done;) {
+                    if ((size_t)rcap > ent) {
                         done = false;
                         break;
                     }
+                    const int nb = (int)std::min<size_t>(std::min(kRerunBatch, count - j0), ent / rcap);
+                    int r = launch_tc_gather(qbc, (int)rowb, rows + j0, nb, tau, A2, tau2, rfc, rfac2, st);
+                    if (r || (r = filter(A2, nb, tau2, e4 ? rfac2 : nullptr, rcap))) return r;
+                    ++ngemm;
+                    int hmax = 0;
+                    ANN_CUDA_TRY(cudaMemcpyAsync(&hmax, flags + 2, sizeof(int), cudaMemcpyDeviceToHost, st));
+                    ANN_CUDA_TRY(cudaStreamSynchronize(st));
+                    if (hmax > rcap) {
+                        rcap = hmax;
+                        continue;
+                    }
                     RadixSelectArgs sv2 = sv;
-                    sv2.ld = cap2;
-                    sv2.out_rows = list + j0;
-                    if ((rc = launch_radix_select(sv2, nb, st))) return rc;
+                    sv2.ld = rcap;
+                    sv2.out_rows = rows + j0;
+                    if ((r = launch_radix_select(sv2, nb, st))) return r;
+                    j0 += nb;
                 }
-                // positions of the operand copy -> rows
-                if (done && (rc = launch_tc_map_ids(idRc, (int64_t)nc * R, n, h->row_mult, st))) return rc;
-            }
+                return ANN_OK;
+            };
+            if ((rc = redo(list, hf[0], tauS, cap2))) return rc;
+            // a survivor taken this way costs about eight keys of the full matrix (1,000 queries over 1M x 384 with 200,000
+            // copies each: 33 ms, 20 by the matrix), and 8M of them no more than its selection of few queries
+            if ((int64_t)hf[1] * hf[2] > std::max<int64_t>((int64_t)nc * n / 10, 8 << 20))
+                done = false;
+            else if ((rc = redo(over, hf[1], tauF, hf[2])))
+                return rc;
+            // positions of the operand copy -> rows
+            if (done && (rc = launch_tc_map_ids(idRc, (int64_t)nc * R, n, h->row_mult, st))) return rc;
             h->prof.mark(prec, st);
             if (prec >= 0) h->prof.tc_launches += ngemm;
         }

@@ -25,13 +25,14 @@ __device__ __forceinline__ int pos_to_row(int64_t p, int64_t n, int64_t mult) {
 }
 
 __global__ void tc_bar_check_kernel(const int* rowcnt, int M, int R, int* list, int* flags, const int64_t* lens,
-                                    int* mark) {
+                                    int* mark, int cap, int* over) {
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= M) return;
     const int64_t need = lens ? min((int64_t)R, lens[q]) : (int64_t)R;
     const bool rerun = rowcnt[q] < need;
     if (rerun) list[atomicAdd(&flags[0], 1)] = q;
     if (mark) mark[q] = rerun;
+    if (over && rowcnt[q] > cap) over[atomicAdd(&flags[1], 1)] = q;
 }
 
 __global__ void tc_gather_kernel(const unsigned char* A, int row_bytes, const int* list, int nb, const float* tau,
@@ -937,9 +938,9 @@ int launch_tc_ivf_pairs(const void* qrows, int row_bytes, const int32_t* pair_va
 }
 
 int launch_tc_bar_check(const int* rowcnt, int M, int R, int* list, int* flags, cudaStream_t st, const int64_t* lens,
-                        int* mark) {
+                        int* mark, int cap, int* over) {
     if (M == 0) return ANN_OK;
-    tc_bar_check_kernel<<<(unsigned)ceil_div(M, 256), 256, 0, st>>>(rowcnt, M, R, list, flags, lens, mark);
+    tc_bar_check_kernel<<<(unsigned)ceil_div(M, 256), 256, 0, st>>>(rowcnt, M, R, list, flags, lens, mark, cap, over);
     ANN_LAUNCH_CHECK();
     return ANN_OK;
 }

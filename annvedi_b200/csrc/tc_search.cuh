@@ -14,9 +14,10 @@ namespace annb {
 int64_t tc_row_mult(int64_t n);
 
 // Rows with fewer than R survivors -- fewer than min(R, lens[row]) where lens is given -- go to list (count in
-// flags[0]); mark[row], if given, is 1 for them and 0 for the others.
+// flags[0]); mark[row], if given, is 1 for them and 0 for the others. Rows with more than cap survivors go to over, if given
+// (count in flags[1]).
 int launch_tc_bar_check(const int* rowcnt, int M, int R, int* list, int* flags, cudaStream_t st,
-                        const int64_t* lens = nullptr, int* mark = nullptr);
+                        const int64_t* lens = nullptr, int* mark = nullptr, int cap = 0, int* over = nullptr);
 // A2[j] = A[list[j]] (rows of row_bytes), tau2[j] = tau[list[j]] and, if given, rfac2[j] = rfac[list[j]].
 int launch_tc_gather(const void* A, int row_bytes, const int* list, int nb, const float* tau, void* A2, float* tau2,
                      const float* rfac, float* rfac2, cudaStream_t st);
