@@ -172,11 +172,20 @@ struct KmeansKeys {
     int32_t* amb = nullptr;          // [chunk] rows the keys' bound does not cover, and their count
     int* amb_count = nullptr;
     int* err = nullptr;
-    ~KmeansKeys() {
+    uint64_t wait_ns = 0;            // ann_ivf::wait_ns
+    void release() {
         for (void* p : {(void*)xb, (void*)cb, (void*)norms, (void*)max2, (void*)keys, (void*)cmin, (void*)amb,
                         (void*)amb_count, (void*)err})
             if (p) cudaFree(p);
+        ok = false;
+        xb = cb = nullptr;
+        norms = nullptr;
+        max2 = nullptr;
+        keys = cmin = nullptr;
+        amb = nullptr;
+        amb_count = err = nullptr;
     }
+    ~KmeansKeys() { release(); }
 };
 
 static bool prune_norm_ok(unsigned bits2) {
@@ -207,6 +216,7 @@ static int kmeans_keys_setup(KmeansKeys& k, const float* x, int64_t n, int dim, 
                      cudaMalloc(&k.err, sizeof(int)) == cudaSuccess;
     if (!mem) {
         cudaGetLastError();
+        k.release();
         return ANN_OK;
     }
     int rc = launch_base_norms(x, n, dim, dpad, k.max2, st, k.norms);
@@ -215,7 +225,10 @@ static int kmeans_keys_setup(KmeansKeys& k, const float* x, int64_t n, int dim, 
     ANN_CUDA_TRY(cudaMemsetAsync(k.err, 0, sizeof(int), st));
     ANN_CUDA_TRY(cudaMemcpyAsync(h, k.max2, sizeof(h), cudaMemcpyDeviceToHost, st));
     ANN_CUDA_TRY(cudaStreamSynchronize(st));
-    if (!prune_norm_ok(h[0]) || (given && !prune_norm_ok(h[2]))) return ANN_OK;
+    if (!prune_norm_ok(h[0]) || (given && !prune_norm_ok(h[2]))) {
+        k.release();
+        return ANN_OK;
+    }
     if ((rc = launch_tc_operand(x, n, dim, dpad, k.xb, k.kpad, kTcQuery, ANN_METRIC_L2, 0, st))) return rc;
     k.ok = true;
     return ANN_OK;
@@ -230,6 +243,8 @@ static int assign_rows_keys(KmeansKeys& k, const float* x, int64_t n, int dim, i
     for (int64_t r0 = 0; r0 < n; r0 += k.chunk) {
         const int nr = (int)std::min<int64_t>(k.chunk, n - r0);
         TcGemmArgs g{nr, C, k.kpad, nullptr, k.keys, C, k.err};
+        g.wait_ns = k.wait_ns;
+        g.test_no_loads = k.wait_ns > 0;
         g.out_cmin = k.cmin;
         if ((rc = launch_tc_gemm(k.xb + (size_t)r0 * k.kpad, k.cb, g, st))) return rc;
         ANN_CUDA_TRY(cudaMemsetAsync(k.amb_count, 0, sizeof(int), st));
@@ -411,12 +426,11 @@ int ann_ivf_fit(ann_ivf* h, const float* data, int64_t n, int32_t dim, int64_t l
             FIT_CUDA(cudaMemcpyAsync(seed_rows, seeds.data(), sizeof(int32_t) * 2 * C, cudaMemcpyHostToDevice, st));
             FIT_CUDA(cudaStreamSynchronize(st));
         }
-        if (centroids) {
+        if (centroids)
             FIT_CUDA(cudaMemcpy2DAsync(h->centroids, sizeof(float) * dpad, centroids, sizeof(float) * dim,
                                        sizeof(float) * dim, C, kind, st));
-        } else {
+        else
             FIT_TRY(launch_gather_rows(X, C, dpad, seed_rows, h->centroids, dpad, st));
-        }
         FIT_TRY(launch_iota(idx, n, st));  // the sort values
         // sort keys below C have few bits; a given assignment is sorted whole
         int c_bits = 1;
@@ -428,24 +442,36 @@ int ann_ivf_fit(ann_ivf* h, const float* data, int64_t n, int32_t dim, int64_t l
         FIT_CUDA(cudaMalloc(&tmp, tmp_bytes));
         const bool given_assign = assign != nullptr;
         const int iters = (centroids || given_assign) ? 0 : kmeans_iters;
+        kk.wait_ns = h->wait_ns;
         if (!given_assign) FIT_TRY(kmeans_keys_setup(kk, X, n, dim, dpad, h->centroids, C, centroids != nullptr, st));
         auto assign_round = [&]() -> int {
             if (kk.ok) return assign_rows_keys(kk, X, n, dim, dpad, h->centroids, C, a_raw, st);
             return assign_rows(X, n, dim, dpad, h->centroids, C, a_raw, &h->ws, st);
         };
-        for (int it = 0; it < iters; ++it) {
-            FIT_TRY(assign_round());
-            FIT_CUDA(cub::DeviceRadixSort::SortPairs(tmp, tmp_bytes, a_raw, a_sorted, idx, order, (int)n, 0, c_bits, st));
-            FIT_TRY(launch_list_offsets(a_sorted, n, C, h->list_off, st));
-            FIT_TRY(launch_kmeans_update(X, dpad, dim, order, h->list_off, C, h->centroids, dpad, seed_rows + C, n,
-                                         fit_threads, st));
-        }
-        // the lists: given assignment, else nearest to the current centroids (the last k-means
-        // assignment when iterating, as the reference's lists come from its last assign step)
-        if (given_assign) {
-            FIT_CUDA(cudaMemcpyAsync(a_raw, assign, sizeof(int32_t) * n, kind, st));
-        } else if (iters == 0) {
-            FIT_TRY(assign_round());
+        while (true) {
+            for (int it = 0; it < iters; ++it) {
+                FIT_TRY(assign_round());
+                FIT_CUDA(cub::DeviceRadixSort::SortPairs(tmp, tmp_bytes, a_raw, a_sorted, idx, order, (int)n, 0, c_bits, st));
+                FIT_TRY(launch_list_offsets(a_sorted, n, C, h->list_off, st));
+                FIT_TRY(launch_kmeans_update(X, dpad, dim, order, h->list_off, C, h->centroids, dpad, seed_rows + C, n,
+                                             fit_threads, st));
+            }
+            // the lists: given assignment, else nearest to the current centroids (the last k-means
+            // assignment when iterating, as the reference's lists come from its last assign step)
+            if (given_assign) {
+                FIT_CUDA(cudaMemcpyAsync(a_raw, assign, sizeof(int32_t) * n, kind, st));
+            } else if (iters == 0) {
+                FIT_TRY(assign_round());
+            }
+            if (!kk.ok) break;
+            // the keys' buffers are given back before the lists' rows are laid out; where one of their waits gave up, the
+            // rounds are run again by the scan
+            int gave_up = 0;
+            FIT_CUDA(cudaMemcpyAsync(&gave_up, kk.err, sizeof(int), cudaMemcpyDeviceToHost, st));
+            FIT_CUDA(cudaStreamSynchronize(st));
+            kk.release();
+            if (!gave_up) break;
+            if (!centroids) FIT_TRY(launch_gather_rows(X, C, dpad, seed_rows, h->centroids, dpad, st));
         }
         FIT_CUDA(cub::DeviceRadixSort::SortPairs(tmp, tmp_bytes, a_raw, a_sorted, idx, order, (int)n, 0,
                                                  given_assign ? 32 : c_bits, st));
@@ -470,15 +496,6 @@ int ann_ivf_fit(ann_ivf* h, const float* data, int64_t n, int32_t dim, int64_t l
         h->C = C;
         FIT_TRY(ivf_finish_lists(h, st));
         FIT_CUDA(cudaStreamSynchronize(st));
-        if (kk.ok) {
-            int gave_up = 0;
-            FIT_CUDA(cudaMemcpy(&gave_up, kk.err, sizeof(int), cudaMemcpyDeviceToHost));
-            if (gave_up) {
-                set_error("ann_ivf_fit: a device-side wait gave up after its time limit");
-                rc = ANN_ERR_TIMEOUT;
-                goto fail;
-            }
-        }
     }
 fail:
     for (void* p : {(void*)X, (void*)a_raw, (void*)a_sorted, (void*)idx, (void*)order, tmp, (void*)mn, (void*)mx,

@@ -78,3 +78,26 @@ def test_refused_copy_is_not_asked_for_again(cuda):
     torch.cuda.synchronize()
     assert ix.get_prune_stats()["passes"] == 2
     assert torch.equal(ids, want[0]) and torch.equal(d, want[1])
+
+
+def test_fit_gives_the_keys_buffers_back(cuda):
+    """A k-means fit of rows by tensor-core keys needs no more beside the rows and its state than the scan's: the keys' copy of
+    the rows is freed before the lists are laid out."""
+    import torch
+    from annvedi_b200.ivf import IVFIndex
+    n, dim, c = 1_000_000, 256, 256
+    x = torch.randn(n, dim, device="cuda")
+    want = None
+    for left in (None, (n * dim * 9) + (400 << 20)):  # the rows, the lists' rows and codes, and room for the sorts
+        ix = IVFIndex(device=0, mode="exact", num_threads=4)
+        if left is None:
+            ix.fit(x, 1, 0, c, kmeans_iters=1)
+        else:
+            with _Filled(left):
+                ix.fit(x, 1, 0, c, kmeans_iters=1)
+        st = ix.export_state()
+        ix.close()
+        if want is None:
+            want = st
+        for key in ("centroids", "reordered_to_original", "quantized_data"):
+            np.testing.assert_array_equal(st[key], want[key])

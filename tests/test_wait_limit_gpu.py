@@ -112,3 +112,19 @@ def test_exact_ivf_batch_takes_the_scans(cuda, c, sizes, nq, k, npc):
     assert torch.equal(ids, torch.cat([p[0] for p in parts])) and torch.equal(d, torch.cat([p[1] for p in parts]))
     assert ix.total_distances_count() == count
     assert ix._lib.ann_ivf_device_status(ix._h) == 0
+
+
+@pytest.mark.parametrize("given", [False, True])
+def test_fit_runs_its_rounds_by_the_scan(cuda, given):
+    """k-means assignments by keys: where their waits give up, the fit's centroids and lists are the same."""
+    from annvedi_b200.ivf import IVFIndex
+    rng = np.random.default_rng(3)
+    x = rng.standard_normal((9000, 40)).astype(np.float32)
+    states = []
+    for wait in (0, 100000):
+        ix = IVFIndex(device=0, mode="exact", num_threads=4)
+        ix.set_option("wait_selftest", wait)
+        ix.fit(x, 1, 0, 30, kmeans_iters=4, centroids=x[:30] if given else None)
+        states.append(ix.export_state())
+    for key in ("centroids", "reordered_to_original", "table_offsets", "quantized_data"):
+        np.testing.assert_array_equal(states[0][key], states[1][key])
