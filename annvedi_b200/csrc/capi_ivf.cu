@@ -1614,20 +1614,27 @@ static int ivf_query_device(ann_ivf* h, ann_workspace* ws, const IvfQueryCfg& c,
         // merge 346 us; the keys take 100 us, the selection 40 us.
         const size_t words_q = rows_select_words(h->n, c.R);
         const size_t per_q = sizeof(float) * (size_t)h->n + 8 * words_q;
-        const int group = (int)std::max<size_t>(1, std::min<size_t>(4096, ((size_t)256 << 20) / per_q));
-        for (size_t e0 = 0; e0 < every_row.size(); e0 += group) {
+        int group = (int)std::max<size_t>(1, std::min<size_t>(4096, ((size_t)256 << 20) / per_q));
+        for (size_t e0 = 0; e0 < every_row.size();) {
             const int ne = (int)std::min<size_t>(group, every_row.size() - e0);
             Sizer es;
             es.take<float>((size_t)ne * h->n);
             es.take<unsigned long long>((size_t)ne * words_q);
-            if ((rc = ws_reserve_big(ws, es.bytes()))) return rc;
+            if ((rc = ws_reserve_big(ws, es.bytes()))) {
+                if (rc != ANN_ERR_NOMEM || ne == 1) return rc;
+                clear_error();
+                group = ne / 2;
+                continue;
+            }
+            const size_t first = e0;
+            e0 += ne;
             Carver ec(ws->big);
             float* D = ec.take<float>((size_t)ne * h->n);
             unsigned long long* words = ec.take<unsigned long long>((size_t)ne * words_q);
             IvfQueryArgs b = a;
             b.plan.nq = ne;
             b.plan.cand_ids = nullptr;
-            b.qorder = every_list + e0;
+            b.qorder = every_list + first;
             if ((rc = launch_set_every_row(a.plan, b.qorder, ne, h->n, st))) return rc;
             if ((rc = launch_ivf_sq8_dists(b, D, h->n, st))) return rc;
             if ((rc = launch_rows_select(D, h->n, ne, c.R, b.qorder, words, keyR, idR, st))) return rc;
@@ -1812,7 +1819,21 @@ int ann_ivf_query(ann_ivf* h, ann_workspace* ws, const float* queries, int32_t n
     }
     const size_t head_bytes = (head.off + 255) / 256 * 256;
     int rc = ws_reserve_device(ws, head_bytes + ivf_scratch(h, c, qc) + 512);
+    if (rc == ANN_ERR_NOMEM && c.coarse_keys) {  // the centroid scan needs no keys
+        clear_error();
+        c.coarse_keys = false;
+        rc = ws_reserve_device(ws, head_bytes + ivf_scratch(h, c, qc) + 512);
+    }
     if (rc) return rc;
+    if (c.small_tc) {
+        rc = ws_reserve_big(ws, sizeof(float) * (size_t)std::max<int64_t>(c.small_keys, 1));
+        if (rc == ANN_ERR_NOMEM) {  // the batch's own set-up sizes the keys by its streams
+            clear_error();
+            c.small_tc = false;
+        } else if (rc) {
+            return rc;
+        }
+    }
     Carver cv(ws->dev);
     float* qdev = cv.take<float>((size_t)nq * dpad);
     int64_t* ids_dev = out_ids;

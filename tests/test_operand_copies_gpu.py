@@ -101,3 +101,35 @@ def test_fit_gives_the_keys_buffers_back(cuda):
             want = st
         for key in ("centroids", "reordered_to_original", "quantized_data"):
             np.testing.assert_array_equal(st[key], want[key])
+
+
+@pytest.mark.parametrize("mode,nq,c,sizes,npc,left", [
+    ("exact", 16000, 2048, [25] * 2048, 1, 90 << 20),            # 131 MB of coarse keys
+    ("tc", 150, 40, [100000] + [60] * 39, 1, 40 << 20),          # 60 MB of stream keys by the largest list
+    ("exact", 60, 40, [40000] * 30 + [3] * 10, 2, 20 << 20),     # 192 MB of keys of every row, 40 queries (8 MB of streams)
+])
+def test_batches_in_little_memory(cuda, mode, nq, c, sizes, npc, left):
+    """Batches whose faster form does not fit take the one that does, with the same results."""
+    import torch
+    from annvedi_b200.ivf import IVFIndex
+    rng = np.random.default_rng(nq)
+    dim, k = 32, 10
+    cen = (10 * rng.standard_normal((c, dim))).astype(np.float32)
+    cen[-10:] = cen[-1] + 0.01 * rng.standard_normal((10, dim)).astype(np.float32)
+    assign = np.repeat(np.arange(c), sizes).astype(np.int32)
+    x = (cen[assign] + 0.3 * rng.standard_normal((len(assign), dim))).astype(np.float32)
+    own = rng.integers(1, c - 10, nq)
+    if sizes[-1] < k:
+        own[:40] = c - 1
+    q = torch.from_numpy((cen[own] + 0.3 * rng.standard_normal((nq, dim))).astype(np.float32)).cuda()
+    out = [torch.empty(nq, k, dtype=torch.int64, device="cuda"), torch.empty(nq, k, device="cuda")]
+    ix = IVFIndex(device=0, mode=mode)
+    ix.fit(x, 1, 0, c, centroids=cen, assign=assign)
+    want = ix.search(q, k, 0, npc, 20)
+    other = IVFIndex(device=0, mode=mode)
+    other.fit(x, 1, 0, c, centroids=cen, assign=assign)
+    other.search(q[:1], k, 0, npc, 20)
+    with _Filled(left):
+        got = other.search(q, k, 0, npc, 20, out_ids=out[0], out_dists=out[1])
+        torch.cuda.synchronize()
+    assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
