@@ -172,9 +172,9 @@ __device__ __forceinline__ unsigned long long select_word(float v, int64_t row) 
     return ((unsigned long long)((u & 0x80000000u) ? ~u : (u | 0x80000000u)) << 32) | (unsigned)row;
 }
 
-// Rows of a segment when n rows are selected from in up to kSelectSegs segments (a multiple of 1024).
+// Rows of a segment when n rows are selected from in up to `segs` segments (a multiple of 1024).
 constexpr int kSelectSegs = 128;
-inline int64_t select_seg_rows(int64_t n) { return ceil_div(ceil_div(n, kSelectSegs), 1024) * 1024; }
+inline int64_t select_seg_rows(int64_t n, int segs = kSelectSegs) { return ceil_div(ceil_div(n, segs), 1024) * 1024; }
 
 // The segment's best min(k, m) of the values T[0..m) of rows row0.., as words in no order into out[0..k), the rest
 // filled with ~0. Whole block; sN: one int.

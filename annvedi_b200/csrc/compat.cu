@@ -34,7 +34,9 @@
 namespace annb {
 
 // grid: (row blocks, query groups); block: 256 threads = 16 rows x 16 lanes. PIECES: the row's 16-chunks held in
-// registers (dim <= 16 PIECES; 0: any dim), so that a row's loads are in flight together.
+// registers (dim <= 16 PIECES; 0: any dim), so that a row's loads are in flight together. As many as the dimension needs,
+// to a few: with 32 at every dimension up to 512, 127 queries over 46,245 x 4 took 818 us here, 313 by the loop before it
+// (a call: 971, 532; 473 now), and 500 over 100,000 x 100 8,335 us a call (7,290; 5,760 now).
 template <int PIECES>
 __global__ void __launch_bounds__(256) compat_partials_kernel(CompatArgs a, int q_begin) {
     extern __shared__ float sQ[];  // [QG][dim]
@@ -302,19 +304,19 @@ __global__ void __launch_bounds__(kFinalThreads) compat_final_kernel(CompatArgs 
     const unsigned long long* w = a.seg_best + (int64_t)qi * a.nseg * a.k;
     const int m = a.nseg * a.k;
     if (m <= kFinalStaged) {
-        for (int i = threadIdx.x; i < m; i += kFinalThreads) sW[i] = w[i];
+        for (int i = threadIdx.x; i < m; i += blockDim.x) sW[i] = w[i];
         w = sW;
     }
     if (threadIdx.x == 0) sN = 0;
     __syncthreads();
     const SelectBound b = block_select_bound<true>([&](int i) { return w[i]; }, m, a.k, sHist, sMisc);
     const int p2 = pow2_ceil(a.k);
-    for (int i = threadIdx.x; i < m; i += kFinalThreads)
+    for (int i = threadIdx.x; i < m; i += blockDim.x)
         if (b.in(w[i])) sR[atomicAdd(&sN, 1)] = w[i];
-    for (int i = a.k + threadIdx.x; i < p2; i += kFinalThreads) sR[i] = ~0ull;
+    for (int i = a.k + threadIdx.x; i < p2; i += blockDim.x) sR[i] = ~0ull;
     block_sort_u64(sR, p2);
     const int64_t o = (int64_t)(q_begin + qi) * a.k;
-    for (int e = threadIdx.x; e < a.k; e += kFinalThreads) {
+    for (int e = threadIdx.x; e < a.k; e += blockDim.x) {
         if (a.out_ids) a.out_ids[o + e] = (int64_t)(unsigned)sR[e];
         if (a.out_dists) a.out_dists[o + e] = f32_ord((uint32_t)(sR[e] >> 32));
     }
@@ -329,9 +331,20 @@ int launch_compat(CompatArgs a, int q_begin, int q_count, cudaStream_t st) {
     a.q_end = q_begin + q_count;
     const size_t smem = sizeof(float) * kCompatQG * a.dim;
     ANN_CHECK_ARG(a.k <= a.n, "reference mode: k=%d above n", a.k);
-    a.seg_rows = select_seg_rows(a.n);
+    // Many queries over few rows fill the chip by themselves, and a segment's lists only cost: one segment (1,000 queries over
+    // 10,000 x 100, k = 10: 28 us of a call less; 346 over 15,323 would take 28 us more).
+    a.seg_rows = select_seg_rows(a.n, q_count >= 256 && a.n <= 10240 ? 1 : kSelectSegs);
     a.nseg = (int)ceil_div(a.n, a.seg_rows);
-    auto partials = a.dim <= 512 ? compat_partials_kernel<32> : compat_partials_kernel<0>;
+    // the fewest registers that hold the row: the steps past its last piece are walked all the same
+    const int full16 = a.dim / 16;
+    auto partials = full16 <= 1    ? compat_partials_kernel<1>
+                    : full16 <= 2  ? compat_partials_kernel<2>
+                    : full16 <= 4  ? compat_partials_kernel<4>
+                    : full16 <= 8  ? compat_partials_kernel<8>
+                    : full16 <= 16 ? compat_partials_kernel<16>
+                    : full16 <= 24 ? compat_partials_kernel<24>
+                    : full16 <= 32 ? compat_partials_kernel<32>
+                                   : compat_partials_kernel<0>;
     ANN_CUDA_TRY(smem_optin(reinterpret_cast<const void*>(partials)));
     const int64_t rblocks = std::min<int64_t>(ceil_div(a.n, 16), kNumSMs * 8);
     dim3 g1((unsigned)rblocks, (unsigned)ceil_div(q_count, kCompatQG));
@@ -350,7 +363,8 @@ int launch_compat(CompatArgs a, int q_begin, int q_count, cudaStream_t st) {
     ANN_LAUNCH_CHECK();
     const int64_t words = (int64_t)a.nseg * a.k;
     ANN_CUDA_TRY(smem_optin(reinterpret_cast<const void*>(compat_final_kernel)));
-    compat_final_kernel<<<(unsigned)q_count, kFinalThreads, words <= kFinalStaged ? words * 8 : 0, st>>>(a, q_begin);
+    // (a few words a query are as soon done by 256 threads, of which eight blocks fit an SM)
+    compat_final_kernel<<<(unsigned)q_count, words <= 1024 ? 256 : kFinalThreads, words <= kFinalStaged ? words * 8 : 0, st>>>(a, q_begin);
     ANN_LAUNCH_CHECK();
     return ANN_OK;
 }
