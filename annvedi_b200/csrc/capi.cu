@@ -225,6 +225,7 @@ int ann_flat_destroy(ann_flat* h) {
         if (h->base_e4m3) cudaFree(h->base_e4m3);
         if (h->fac_e4m3) cudaFree(h->fac_e4m3);
         if (h->d_err) cudaFree(h->d_err);
+        if (h->d_prune_word) cudaFree(h->d_prune_word);
         if (h->prune_word) cudaFreeHost(h->prune_word);  // (the frees above have waited for the device)
     }
     ws_release(&h->ws);
@@ -665,12 +666,16 @@ static int flat_ensure_pruned(ann_flat* h, int nq, cudaStream_t st, bool* ok) {
         h->bounds = covered ? PruneBounds{c * 1.001f, r * 1.001f} : PruneBounds{};
         h->bounds_known = true;
         if (!h->prune_word) {
-            void* w = nullptr;
-            if (cudaHostAlloc(&w, sizeof(*h->prune_word), cudaHostAllocPortable | cudaHostAllocMapped) == cudaSuccess) {
+            void *w = nullptr, *d = nullptr;
+            if (cudaHostAlloc(&w, sizeof(*h->prune_word), cudaHostAllocPortable | cudaHostAllocMapped) == cudaSuccess &&
+                cudaMalloc(&d, sizeof(*h->d_prune_word)) == cudaSuccess) {
                 h->prune_word = static_cast<unsigned long long*>(w);
+                h->d_prune_word = static_cast<unsigned long long*>(d);
                 *h->prune_word = (unsigned long long)h->prune_seen << 32;
+                ANN_CUDA_TRY(cudaMemsetAsync(d, 0, sizeof(*h->d_prune_word), st));
             } else {
                 cudaGetLastError();  // no back-off then
+                if (w) cudaFreeHost(w);
             }
         }
     }
@@ -681,7 +686,8 @@ static int flat_ensure_pruned(ann_flat* h, int nq, cudaStream_t st, bool* ok) {
 // Whether this call tries the pruned form (under tc_mu). The window grows with |x| |q|, not with the rows' spread: over data
 // far from the origin, or with more copies of a row than survivors fit, the pass leaves the queries to the scan and was
 // for nothing (N(50, 0.01), 37 queries over 131,725 x 33, inner product: 328 us scanned, 902 with the pass). A pass that
-// left more than a quarter of its queries is followed by 4 calls of the scan alone, then 8, up to 1,024, until one does not.
+// left more than a quarter of its query tiles (any query, in batches of a tile) is followed by 4 calls of the scan alone,
+// then 8, up to 1,024, until one does not.
 // The device writes the count; it is read here without a wait, so by a later call than the next where calls are queued.
 // A captured call keeps the form for every replay, and one bad pass may have been its queries' doing (a warm-up on zeros):
 // it is the scan from the second such pass on.
@@ -690,8 +696,10 @@ static bool flat_prune_open(ann_flat* h, bool capturing) {
         const unsigned long long w = __atomic_load_n(h->prune_word, __ATOMIC_RELAXED);
         if ((uint32_t)(w >> 32) != h->prune_seen) {
             h->prune_seen = (uint32_t)(w >> 32);
-            const unsigned n = (unsigned)(w >> 16) & 0xffffu, left = (unsigned)w & 0xffffu;
-            if (4 * left > n) {
+            const int n = (int)((w >> 16) & 0xffffu), left = (int)(w & 0xffffu);
+            // the scan reads the base once per query tile, however few of a tile's queries are left
+            const int bq = h->query_tile > 0 ? h->query_tile : flat_scan_bq(n);
+            if (4 * ceil_div(left, bq) > ceil_div(n, bq)) {
                 h->prune_skip = 4 << std::min(h->prune_streak, 8);
                 ++h->prune_streak;
             } else {
@@ -714,7 +722,7 @@ static int flat_exact_pruned(ann_flat* h, ann_workspace* ws, const float* qdev, 
     *done = false;
     const int64_t n = h->n;
     const int dpad = h->dpad;
-    if (n < prune_min_rows(nq, kk) || n < 64 * (int64_t)kk || !prune_fits(kk, dpad)) return ANN_OK;
+    if (!prune_rows(n, nq, kk) || n < 64 * (int64_t)kk || !prune_fits(kk, dpad)) return ANN_OK;
     bool ok = false;
     int rc = flat_ensure_pruned(h, nq, st, &ok);
     if (rc || !ok) return rc;
@@ -748,6 +756,10 @@ static int flat_exact_pruned(ann_flat* h, ann_workspace* ws, const float* qdev, 
     sz.take<float>((size_t)(qc + 1) / 2 * 2 * dpad);
     sz.take<float>((size_t)qc * nsplit * kk);
     sz.take<int>((size_t)qc * nsplit * kk);
+    if (prune_split(qc)) {
+        sz.take<unsigned long long>((size_t)qc * cap);
+        sz.take<int2>((size_t)qc);
+    }
     {
         std::lock_guard<std::mutex> lk(h->tc_mu);
         if (sz.bytes() >= h->prune_ws_refused && ws->big_cap < sz.bytes()) return ANN_OK;
@@ -775,6 +787,8 @@ static int flat_exact_pruned(ann_flat* h, ann_workspace* ws, const float* qdev, 
     float* qpair = cv.take<float>((size_t)(qc + 1) / 2 * 2 * dpad);
     float* skey = cv.take<float>((size_t)qc * nsplit * kk);
     int* sid = cv.take<int>((size_t)qc * nsplit * kk);
+    unsigned long long* words = prune_split(qc) ? cv.take<unsigned long long>((size_t)qc * cap) : nullptr;
+    int2* joined = prune_split(qc) ? cv.take<int2>((size_t)qc) : nullptr;
     for (int q0 = 0; q0 < nq; q0 += qc) {
         const int nc = std::min(qc, nq - q0);
         const float* q = qdev + (size_t)q0 * dpad;
@@ -799,6 +813,8 @@ static int flat_exact_pruned(ann_flat* h, ann_workspace* ws, const float* qdev, 
         p.list = list;
         p.count = count;
         p.err = err;
+        p.words = words;
+        p.joined = joined;
         p.out_ids = ids_dev + (size_t)q0 * kk;
         p.out_dists = dists_dev ? dists_dev + (size_t)q0 * kk : nullptr;
         if ((rc = launch_prune_queries(p, qb, kpad, st))) return rc;
@@ -817,11 +833,14 @@ static int flat_exact_pruned(ann_flat* h, ann_workspace* ws, const float* qdev, 
         if ((rc = launch_prune_finish(p, st))) return rc;
         // the queries on the list, by the plain scan (none, nearly always: the kernels read the count and return)
         uint32_t pass;
+        int report;
         {
             std::lock_guard<std::mutex> lk(h->tc_mu);
             pass = ++h->prune_pass;
+            report = h->prune_streak > 0;
         }
-        if ((rc = launch_prune_gather(q, dpad, list, count, nc, qg, h->prune_word, pass, st))) return rc;
+        if ((rc = launch_prune_gather(q, dpad, list, count, nc, qg, h->d_prune_word, h->prune_word, pass, report, st)))
+            return rc;
         FlatScanArgs a{h->base, n, dpad, qg, nc, h->metric, kk, rps, nsplit, skey, sid};
         a.qpair = qpair;
         a.nq_dev = count;
@@ -895,7 +914,9 @@ int ann_flat_prune_stats(ann_flat* h, int64_t* out4) {
     clear_error();
     ANN_CHECK_ARG(h != nullptr && out4 != nullptr, "ann_flat_prune_stats: null argument");
     std::lock_guard<std::mutex> lk(h->tc_mu);
-    const unsigned long long w = h->prune_word ? __atomic_load_n(h->prune_word, __ATOMIC_RELAXED) : 0;
+    DeviceGuard g(h->device);
+    unsigned long long w = 0;
+    if (h->d_prune_word) ANN_CUDA_TRY(cudaMemcpy(&w, h->d_prune_word, sizeof(w), cudaMemcpyDeviceToHost));
     out4[0] = h->prune_pass;
     out4[1] = (int64_t)(w >> 16) & 0xffff;
     out4[2] = (int64_t)w & 0xffff;

@@ -35,9 +35,11 @@ struct ann_flat {
     double prune_credit_us = 0.0;        // what pruning would have saved the exact searches so far (estimated)
     bool prune_refused = false;          // the BF16 copy for them did not fit beside what the card holds (until the next fit)
     size_t prune_ws_refused = SIZE_MAX;  // scratch of this size did not fit
-    // how the latest pruned pass ended, written by the device (page-locked; pass << 32 | queries << 16 | queries left to
-    // the scan), and the back-off that follows from it (flat_prune_open)
+    // how the latest pruned pass ended, written by the device (pass << 32 | queries << 16 | queries left to the scan; in
+    // page-locked memory where queries were left or the host waits for a better end), and the back-off that follows from
+    // it (flat_prune_open)
     unsigned long long* prune_word = nullptr;
+    unsigned long long* d_prune_word = nullptr;
     uint32_t prune_pass = 0;             // passes launched
     uint32_t prune_seen = 0;             // the latest whose end has been read
     int prune_streak = 0;                // passes in a row that left too many queries

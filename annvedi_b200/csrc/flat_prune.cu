@@ -99,6 +99,7 @@ __global__ void __launch_bounds__(256) prune_queries_kernel(PruneArgs a, __nv_bf
     const bool ok = s < kInf && qn <= kPruneNormMax && (l2 || sqrtf(s) >= kPruneNormMin);  // false for NaN
     a.win[q] = ok ? w : __int_as_float(0x7fffffff);
     a.rcount[q] = 0;
+    if (a.joined) a.joined[q] = make_int2(0, 0);
     if (q == 0) *a.count = *a.err = 0;
 }
 
@@ -109,6 +110,10 @@ __global__ void __launch_bounds__(256) prune_queries_kernel(PruneArgs a, __nv_bf
 //   staged scan: one chain over d; streaming scan: 8 chains (floats 4o .. 4o + 3 of every 32), added pairwise.
 // Warps: 8, two blocks per SM; 16 where a launch has no second block for an SM (launch_prune_finish): one query over
 // 1M x 384, 33 -> 25 us.
+// With gridDim.y > 1 (few queries) a query's rows beyond those of one round of the warps go to further blocks, each taking
+// its run of the survivors; the block that ends last selects. A round is a chain of dim / 32 steps of about 1 us: clustered
+// data of many dimensions, whose windows hold thousands of rows, took up to eight rounds in one block (one query over
+// 20,000 x 2,048 normal / clustered: 118 / 152 us; 5 over 20,000 x 4,096: 216 / 880, scanned 438).
 template <bool STREAM, int METRIC, int kFinWarps>
 __global__ void __launch_bounds__(kFinWarps * 32) prune_finish_kernel(PruneArgs a) {
     constexpr int kFinThreads = kFinWarps * 32;
@@ -124,9 +129,11 @@ __global__ void __launch_bounds__(kFinWarps * 32) prune_finish_kernel(PruneArgs 
     const int q = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int cnt = a.rcount[q];
     const float w = a.win[q], tauF = a.tauF[q];
+    const int gave_up = *a.err;  // (with the loads above, not a round trip of its own behind them)
+    if (blockIdx.y > 0 && cnt <= (int)blockIdx.y * kFinThreads) return;  // no more than the blocks before take
     const float* fk = a.fkey + (int64_t)q * cap;
     const int* fc = a.fcol + (int64_t)q * cap;
-    bool fail = cnt > cap || cnt < k || !(w < kInf) || *a.err != 0;
+    bool fail = cnt > cap || cnt < k || !(w < kInf) || gave_up != 0;
     float T = 0.f;
     if (!fail) {  // the k-th smallest kept key
         for (int i = tid; i < cnt; i += kFinThreads) sO[i] = ord_f32(fk[i]);
@@ -135,17 +142,27 @@ __global__ void __launch_bounds__(kFinWarps * 32) prune_finish_kernel(PruneArgs 
         fail = !(T <= tauF);
     }
     if (fail) {  // uniform
-        if (tid == 0) a.list[atomicAdd(a.count, 1)] = q;
+        if (tid == 0 && blockIdx.y == 0) a.list[atomicAdd(a.count, 1)] = q;
         return;
     }
     const float lim = __fadd_ru(T, w);  // <= tauX: every key at or below it was kept
-    if (tid == 0) sN = 0;
-    __syncthreads();
     for (int d = tid; d < dpad; d += kFinThreads) sQ[d] = a.q[(int64_t)q * dpad + d];
-    for (int i = tid; i < cnt; i += kFinThreads)
-        if (fk[i] <= lim) sE[atomicAdd(&sN, 1)] = (unsigned)row_of_pos(fc[i], a.n, a.mult);
-    __syncthreads();
-    const int m = sN;  // >= k
+    auto collect = [&](int i0, int i1) {  // the rows of survivors [i0, i1) within the window; returns their number
+        if (tid == 0) sN = 0;
+        __syncthreads();
+        for (int i = i0 + tid; i < i1; i += kFinThreads)
+            if (fk[i] <= lim) sE[atomicAdd(&sN, 1)] = (unsigned)row_of_pos(fc[i], a.n, a.mult);
+        __syncthreads();
+        return sN;
+    };
+    const int total = collect(0, cnt);  // >= k, the same in every block of the query
+    const int blocks = min((int)gridDim.y, (total + kFinThreads - 1) / kFinThreads);
+    if ((int)blockIdx.y >= blocks) return;
+    int m = total;
+    if (blocks > 1) {
+        __syncthreads();
+        m = collect((int)((int64_t)cnt * blockIdx.y / blocks), (int)((int64_t)cnt * (blockIdx.y + 1) / blocks));
+    }
     float* myX = sX + warp * kFinStages * 32 * kFinPitch;
     const int nch = dpad / 32;
     for (int g = warp * 32; g < m; g += kFinWarps * 32) {
@@ -207,6 +224,22 @@ __global__ void __launch_bounds__(kFinWarps * 32) prune_finish_kernel(PruneArgs 
             sE[g + lane] = ((unsigned long long)ord_f32((METRIC == ANN_METRIC_L2 ? v : -v) + 0.f) << 32) | (unsigned)row;
     }
     __syncthreads();
+    if (blocks > 1) {
+        unsigned long long* gw = a.words + (int64_t)q * cap;
+        __shared__ int sAt;
+        if (tid == 0) sAt = atomicAdd(&a.joined[q].x, m);
+        __syncthreads();
+        for (int i = tid; i < m; i += kFinThreads) gw[sAt + i] = sE[i];
+        __threadfence();
+        __syncthreads();
+        if (tid == 0) sAt = atomicAdd(&a.joined[q].y, 1);
+        __syncthreads();
+        if (sAt != blocks - 1) return;  // uniform: another block of the query is still to come
+        __threadfence();
+        m = total;
+        for (int i = tid; i < m; i += kFinThreads) sE[i] = __ldcg(gw + i);
+        __syncthreads();
+    }
     const SelectBound bound = block_select_bound<true>([&](int i) { return sE[i]; }, m, k, sHist, sMisc);
     unsigned long long* sR = reinterpret_cast<unsigned long long*>(sX);  // the best k, then sorted
     const int p2 = pow2_ceil(k);
@@ -227,9 +260,14 @@ __global__ void __launch_bounds__(kFinWarps * 32) prune_finish_kernel(PruneArgs 
 
 __global__ void prune_gather_kernel(const float* __restrict__ q, int dpad, const int* __restrict__ list,
                                     const int* __restrict__ count, float* __restrict__ qg, int nq,
-                                    volatile unsigned long long* word, uint32_t pass) {
+                                    unsigned long long* dev_word, volatile unsigned long long* word, uint32_t pass,
+                                    int report) {
     const int n = *count;
-    if (word && blockIdx.x == 0 && threadIdx.x == 0) *word = ((unsigned long long)pass << 32) | ((unsigned)nq << 16) | (unsigned)n;
+    if (word && blockIdx.x == 0 && threadIdx.x == 0) {
+        const unsigned long long v = ((unsigned long long)pass << 32) | ((unsigned)nq << 16) | (unsigned)n;
+        *dev_word = v;
+        if (n > 0 || report) *word = v;  // over PCIe, and the kernels that follow wait for it
+    }
     for (int j = blockIdx.x; j < n; j += gridDim.x)
         for (int d = threadIdx.x; d < dpad; d += blockDim.x) qg[(int64_t)j * dpad + d] = q[(int64_t)list[j] * dpad + d];
 }
@@ -243,7 +281,8 @@ int run_finish(const PruneArgs& a, cudaStream_t st) {
                     ? (a.stream_form ? prune_finish_kernel<true, ANN_METRIC_L2, W> : prune_finish_kernel<false, ANN_METRIC_L2, W>)
                     : (a.stream_form ? prune_finish_kernel<true, ANN_METRIC_IP, W> : prune_finish_kernel<false, ANN_METRIC_IP, W>);
     ANN_CUDA_TRY(smem_optin(reinterpret_cast<const void*>(kern)));
-    kern<<<a.nq, W * 32, finish_smem(a.cap, a.dpad, W), st>>>(a);
+    const int blocks = a.words ? (int)std::min<int64_t>(ceil_div(a.cap, W * 32), std::max(1, kNumSMs / a.nq)) : 1;
+    kern<<<dim3(a.nq, blocks), W * 32, finish_smem(a.cap, a.dpad, W), st>>>(a);
     ANN_LAUNCH_CHECK();
     return ANN_OK;
 }
@@ -251,6 +290,7 @@ int run_finish(const PruneArgs& a, cudaStream_t st) {
 }  // namespace
 
 int prune_cap(int k) { return k <= 128 ? 4096 : 8192; }
+bool prune_split(int nq) { return nq <= kNumSMs / 2; }
 bool prune_fits(int k, int dpad) { return k <= 512 && finish_smem(prune_cap(k), dpad, 8) <= 200 * 1024; }
 
 int prune_bar_rank(int k, int64_t S, int64_t n) {
@@ -283,14 +323,15 @@ int launch_prune_queries(const PruneArgs& a, __nv_bfloat16* qb, int kpad, cudaSt
 int launch_prune_finish(const PruneArgs& a, cudaStream_t st) {
     ANN_CHECK_ARG(a.k >= 1 && prune_fits(a.k, a.dpad) && a.dpad % 32 == 0 && a.cap == prune_cap(a.k),
                   "pruned scan: k=%d, padded dim %d", a.k, a.dpad);
+    ANN_CHECK_ARG((a.words == nullptr) == (a.joined == nullptr), "pruned scan: shared rows need both arrays");
     const bool wide = a.nq <= kNumSMs && finish_smem(a.cap, a.dpad, 16) <= 220 * 1024;
     return wide ? run_finish<16>(a, st) : run_finish<8>(a, st);
 }
 
 int launch_prune_gather(const float* q, int dpad, const int* list, const int* count, int nq, float* qg,
-                        unsigned long long* word, uint32_t pass, cudaStream_t st) {
+                        unsigned long long* dev_word, unsigned long long* word, uint32_t pass, int report, cudaStream_t st) {
     ANN_CHECK_ARG(nq <= 65535, "pruned scan: %d queries a pass", nq);
-    prune_gather_kernel<<<(unsigned)std::min(nq, 2 * kNumSMs), 128, 0, st>>>(q, dpad, list, count, qg, nq, word, pass);
+    prune_gather_kernel<<<(unsigned)std::min(nq, 2 * kNumSMs), 128, 0, st>>>(q, dpad, list, count, qg, nq, dev_word, word, pass, report);
     ANN_LAUNCH_CHECK();
     return ANN_OK;
 }

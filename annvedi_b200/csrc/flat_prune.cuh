@@ -15,12 +15,16 @@ struct PruneBounds {
 // Norms outside this range leave the error bound's assumptions (no overflow, nothing lost to underflow).
 constexpr float kPruneNormMin = 1e-12f, kPruneNormMax = 1e15f;
 
-// Smaller bases are scanned. Measured over dims 64, 384, 768, both metrics, k = 10 and 100, scanned / pruned, us a call:
-// one query 6,000 rows 59 / 66 (k = 10, dim 384), 8,192 rows 0.97 to 1.11 times faster at k = 10 and 1.65 to 2 times at
-// k = 100, from 12,000 on 1.02 to 2.2 times; 3 queries 3,000 rows 89 / 66,
-// 8,192 rows 1.3 to 3.1 times; 8 and more 3,000 rows 1.04 to 3.1 times, 24,000 rows 1.2 to 21 times. The sample (an eighth
-// of a small base) still holds enough rows for the bar.
-inline int64_t prune_min_rows(int nq, int k) { return nq == 1 && k < 64 ? 12000 : (nq <= 4 ? 8192 : 4096); }
+// Bases that are scanned. Measured over dims 64 to 4,096, k = 10 and 100, scanned / pruned, us a call:
+// one query at k = 100 8,192 rows 1.6 to 1.9 times faster pruned; at k = 10 even up to 200,000 rows (50,000 x 768 93 / 105,
+// 100,000 x 384 80 / 78, 100,000 x 1,536 149 / 156, clustered data up to 25% slower), but for some 20,000, whose pass is one
+// tile an SM (70 / 70 at dim 384, 90 / 82 at 768, 152 / 118 at 2,048); 300,000 x 384 125 / 117, x 768 189 / 161;
+// 3 queries 3,000 rows 89 / 66, 8,192 rows 1.3 to 3.1 times; 8 and more 3,000 rows 1.04 to 3.1 times, 24,000 rows 1.2 to
+// 21 times. The sample (an eighth of a small base) still holds enough rows for the bar.
+inline bool prune_rows(int64_t n, int nq, int k) {
+    if (nq == 1 && k < 64) return n >= 200000 || (n >= 16384 && n < 32768);
+    return n >= (nq <= 4 ? 8192 : 4096);
+}
 
 // The window of the BF16 keys (tc_gemm.cuh) of vector q against rows x: 2 eps + delta. With x^, q^ the BF16 operands,
 //   |x.q - x^.q^| <= |x - x^| |q| + |x^| |q - q^| <= rmax |q| + (cmax + rmax) |q - q^|,
@@ -64,7 +68,12 @@ struct PruneArgs {
     int* err;           // [1] set where a wait of the sample or filter pass gave up: every query is left to the scan
     int64_t* out_ids;   // [nq, k]
     float* out_dists;   // [nq, k] or null
+    // few queries (prune_split(nq)): a query's rows shared by several blocks
+    unsigned long long* words;  // [nq, cap] the formed (distance, row)
+    int2* joined;               // [nq] words written, blocks done
 };
+// Whether a pass of nq queries uses words and joined (its blocks would leave most of the chip idle).
+bool prune_split(int nq);
 // Survivors kept per query, and whether their kernel's shared memory fits.
 int prune_cap(int k);
 bool prune_fits(int k, int dpad);
@@ -74,9 +83,9 @@ int prune_bar_rank(int k, int64_t S, int64_t n);
 // win and the queries' operand rows qb [nq, kpad] (launch_tc_operand's); rcount, count and err zeroed.
 int launch_prune_queries(const PruneArgs& a, __nv_bfloat16* qb, int kpad, cudaStream_t st);
 int launch_prune_finish(const PruneArgs& a, cudaStream_t st);  // results, list and count
-// qg[j] = q[list[j]] for j < *count; *word (page-locked host memory, optional) = pass << 32 | nq << 16 | *count
-// (nq <= 65,535).
+// qg[j] = q[list[j]] for j < *count; *dev_word = pass << 32 | nq << 16 | *count (nq <= 65,535) and, where *count > 0 or
+// report, *word (page-locked host memory) the same. Both words may be null together.
 int launch_prune_gather(const float* q, int dpad, const int* list, const int* count, int nq, float* qg,
-                        unsigned long long* word, uint32_t pass, cudaStream_t st);
+                        unsigned long long* dev_word, unsigned long long* word, uint32_t pass, int report, cudaStream_t st);
 
 }  // namespace annb

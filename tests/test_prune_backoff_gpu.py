@@ -58,8 +58,8 @@ def test_a_settled_pass_ends_it(cuda):
     assert (s["passes"], s["left"], s["skip"]) == (2, 0, 0)
     s = _run(ix, torch.from_numpy(q).cuda(), 10, 5)
     assert (s["passes"], s["left"]) == (7, 0)
-    # a quarter of the queries left is not a reason
-    mixed = q.copy()
+    # a few query tiles of many are not a reason (5 queries of 400 are one tile of 13 at most)
+    mixed = np.tile(q, (20, 1))
     mixed[:5] = np.nan
     s = _run(ix, torch.from_numpy(mixed).cuda(), 10, 3)
     assert (s["passes"], s["left"]) == (10, 5)
@@ -67,3 +67,13 @@ def test_a_settled_pass_ends_it(cuda):
     ix.fit(torch.from_numpy(x + 1).cuda())
     ix.search_tc(torch.from_numpy(q[:1]).cuda(), 1)
     assert _run(ix, torch.from_numpy(q).cuda(), 10, 2)["passes"] == 13
+
+
+def test_one_query_of_a_small_batch_is_its_whole_scan(cuda):
+    """The scan of one left query of 6 reads the base as for all six: such passes are backed off from."""
+    import torch
+    x, q = _data("normal", 30000, 64, 6, np.random.default_rng(5))
+    q[2] = np.nan
+    ix = _index(x)
+    s = _run(ix, torch.from_numpy(q).cuda(), 10, 7)
+    assert (s["passes"], s["left"], s["skip"]) == (2, 1, 7)  # calls 1 and 6; the seventh reads the sixth's end: 8 calls
