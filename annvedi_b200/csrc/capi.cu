@@ -9,6 +9,7 @@
 #include <cstring>
 #include <algorithm>
 #include <atomic>
+#include <optional>
 #include <vector>
 
 #include "block_select.cuh"
@@ -621,12 +622,9 @@ static int flat_check_err(ann_flat* h) {
 // (1), 2550 / 130 (1,000). *ok = false (and no error) where the search keeps to the plain scan: not yet laid out,
 // a copy that would take more than half of the free memory (asked once a fit), or rows that the bounds do not cover.
 static bool flat_prune_open(ann_flat* h, bool capturing);
-static int flat_ensure_pruned(ann_flat* h, int nq, cudaStream_t st, bool* ok) {
+static int flat_ensure_pruned(ann_flat* h, int nq, cudaStream_t st, bool capturing, bool* ok) {
     *ok = false;
     std::lock_guard<std::mutex> lk(h->tc_mu);
-    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    ANN_CUDA_TRY(cudaStreamIsCapturing(st, &cs));
-    const bool capturing = cs != cudaStreamCaptureStatusNone;
     if (!h->bounds_known) {
         const double elems = (double)h->n * h->dim;
         h->prune_credit_us += 40.0 + elems * (nq <= 4 ? 0.25e-6 + 0.2e-6 * (nq - 1) : 1.0e-7 * nq);
@@ -723,8 +721,13 @@ static int flat_exact_pruned(ann_flat* h, ann_workspace* ws, const float* qdev, 
     const int64_t n = h->n;
     const int dpad = h->dpad;
     if (!prune_rows(n, nq, kk) || n < 64 * (int64_t)kk || !prune_fits(kk, dpad)) return ANN_OK;
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    ANN_CUDA_TRY(cudaStreamIsCapturing(st, &cs));
+    const bool capturing = cs != cudaStreamCaptureStatusNone;
+    std::optional<CaptureRelax> relax;  // the first pruned call lays out, allocates and loads kernels
+    if (!capturing) relax.emplace();
     bool ok = false;
-    int rc = flat_ensure_pruned(h, nq, st, &ok);
+    int rc = flat_ensure_pruned(h, nq, st, capturing, &ok);
     if (rc || !ok) return rc;
     const int bq = std::min(h->query_tile > 0 ? h->query_tile : flat_scan_bq(nq), flat_scan_max_bq(kk));
     const bool stream_form = flat_stream_eligible(bq, kk, dpad);
@@ -760,16 +763,16 @@ static int flat_exact_pruned(ann_flat* h, ann_workspace* ws, const float* qdev, 
         sz.take<unsigned long long>((size_t)qc * cap);
         sz.take<int2>((size_t)qc);
     }
-    {
+    if (ws->big_cap < sz.bytes()) {
+        if (capturing) return ANN_OK;  // the scan's own scratch is there
         std::lock_guard<std::mutex> lk(h->tc_mu);
-        if (sz.bytes() >= h->prune_ws_refused && ws->big_cap < sz.bytes()) return ANN_OK;
-    }
-    if ((rc = ws_reserve_big(ws, sz.bytes()))) {
-        if (rc != ANN_ERR_NOMEM) return rc;
-        clear_error();
-        std::lock_guard<std::mutex> lk(h->tc_mu);
-        h->prune_ws_refused = std::min(h->prune_ws_refused, sz.bytes());
-        return ANN_OK;
+        if (sz.bytes() >= h->prune_ws_refused) return ANN_OK;
+        if ((rc = ws_reserve_big(ws, sz.bytes()))) {
+            if (rc != ANN_ERR_NOMEM) return rc;
+            clear_error();
+            h->prune_ws_refused = std::min(h->prune_ws_refused, sz.bytes());
+            return ANN_OK;
+        }
     }
     Carver cv(ws->big);
     __nv_bfloat16* qb = cv.take<__nv_bfloat16>((size_t)qc * kpad);

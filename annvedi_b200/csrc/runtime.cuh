@@ -35,6 +35,19 @@ struct DeviceGuard {
     }
 };
 
+// While it lives, this thread's allocations are allowed beside a stream capture of another thread (they would fail and
+// invalidate it): for what a search allocates on a later call than its first.
+struct CaptureRelax {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    bool ok;
+    CaptureRelax() { ok = cudaThreadExchangeStreamCaptureMode(&mode) == cudaSuccess; }
+    ~CaptureRelax() {
+        if (ok) cudaThreadExchangeStreamCaptureMode(&mode);
+    }
+    CaptureRelax(const CaptureRelax&) = delete;
+    CaptureRelax& operator=(const CaptureRelax&) = delete;
+};
+
 // Grows the workspace's device arena to at least `bytes` (drains the device first, since the old
 // block may be in use by earlier asynchronous work).
 int ws_reserve_device(ann_workspace* ws, size_t bytes);
