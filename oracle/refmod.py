@@ -102,6 +102,7 @@ def restate():
     lib.orc_sq8_train.argtypes = [_F, ctypes.c_int64, ctypes.c_int, _F, _F]
     lib.orc_sq8_encode.argtypes = [_F, ctypes.c_int64, ctypes.c_int, _F, _F, _U8]
     lib.orc_kmeans_order.argtypes = [ctypes.c_int64, _I32]
+    lib.orc_lsh_normals.argtypes = [ctypes.c_int64, _F]
     lib.orc_kmeans.restype = ctypes.c_int
     lib.orc_kmeans.argtypes = [_F, ctypes.c_int64, ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_int,
                                ctypes.c_int, ctypes.c_int, _F, _I32]
@@ -188,6 +189,25 @@ def kmeans_order(n: int) -> np.ndarray:
     """rand_indices of the reference's k-means: std::shuffle(iota(n), std::mt19937(1337))."""
     out = np.empty(n, np.int32)
     restate().orc_kmeans_order(n, _p(out, _I32))
+    return out
+
+
+def lsh_projections(n_tables: int, n_bits: int, dim: int) -> np.ndarray:
+    """The LSH projections restated (lsh_index_optimized.cpp:216-257): standard normals, each table's made orthonormal in
+    turn (Gram-Schmidt) where it has no more bits than dimensions. To FP32 rounding: the sums are FP64's."""
+    out = np.empty((n_tables * n_bits, dim), np.float32)
+    restate().orc_lsh_normals(out.size, _p(out, _F))
+    if n_bits > dim:
+        return out
+    for t in range(n_tables):
+        rows = out[t * n_bits:(t + 1) * n_bits].astype(np.float64)
+        for i in range(n_bits):
+            for j in range(i):
+                rows[i] -= (rows[i] @ rows[j]) * rows[j]
+            norm = np.sqrt(rows[i] @ rows[i])
+            if norm > 1e-8:
+                rows[i] /= norm
+        out[t * n_bits:(t + 1) * n_bits] = rows
     return out
 
 

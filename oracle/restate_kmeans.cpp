@@ -61,6 +61,14 @@ static void assign_range(const float *x, int64_t s, int64_t e, int dim, const fl
     }
 }
 
+/* The draws behind the projections (:216-225): `count` floats of std::normal_distribution over std::mt19937(42), both
+ * libstdc++'s, as for the shuffle above. */
+void orc_lsh_normals(int64_t count, float *out) {
+    std::mt19937 gen(42);
+    std::normal_distribution<float> normal(0.0f, 1.0f);
+    for (int64_t i = 0; i < count; ++i) out[i] = normal(gen);
+}
+
 /*
  * run_kmeans: `iters` rounds of assign + update over x [n, dim] with C lists and a ThreadPool of
  * `num_threads`. Writes the final centroids [C, dim] and the last round's assignment [n] (the
