@@ -67,6 +67,7 @@ struct ann_ivf {
     bool codes_known = false;
     double prune_credit_us = 0.0;
     int prune_failed = 0;  // batches in a row that it could not settle
+    int64_t prune_batches = 0, prune_settled = 0;  // batches that tried it, and that it settled
     double cand_rate = 0;  // candidates a probe had in the latest exact batch (0: none yet)
     std::mutex tc_mu;
     int64_t query_count = 0;
@@ -961,6 +962,8 @@ static void ivf_prune_settled(ann_ivf* h, bool settled, double saved_us) {
     std::lock_guard<std::mutex> lk(h->tc_mu);
     if (!settled) h->prune_credit_us = -16.0 * saved_us * (1 << std::min(h->prune_failed, 6));
     h->prune_failed = settled ? 0 : h->prune_failed + 1;
+    h->prune_batches += 1;
+    h->prune_settled += settled;
 }
 
 // Operand rows of the pairs: BF16 (kpad columns) or int8 weights (dpad8 bytes).
@@ -1937,6 +1940,15 @@ int ann_ivf_set_option(ann_ivf* h, int32_t option, int64_t value) {
             set_error("ann_ivf_set_option: unknown option %d", option);
             return ANN_ERR_INVALID;
     }
+}
+
+int ann_ivf_prune_stats(ann_ivf* h, int64_t* out2) {
+    clear_error();
+    ANN_CHECK_ARG(h != nullptr && out2 != nullptr, "ann_ivf_prune_stats: null argument");
+    std::lock_guard<std::mutex> lk(h->tc_mu);
+    out2[0] = h->prune_batches;
+    out2[1] = h->prune_settled;
+    return ANN_OK;
 }
 
 int ann_ivf_kernel_profile(ann_ivf* h, double* out8) {

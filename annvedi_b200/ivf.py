@@ -227,6 +227,13 @@ class IVFIndex:
         return {name: {"ms": float(out[i]), "launches": int(out[4 + i])}
                 for i, name in enumerate(("keys", "bars", "select", "rerank"))}
 
+    def get_prune_stats(self) -> dict:
+        """The exact form's SQ8 selection by tensor-core keys (ann_ivf_prune_stats): batches that tried it, and that it
+        settled."""
+        out = (ctypes.c_int64 * 2)()
+        _lib.check(self._lib.ann_ivf_prune_stats(self._h, out))
+        return {"batches": int(out[0]), "settled": int(out[1])}
+
     def reset_profile_results(self) -> None:
         _lib.check(self._lib.ann_ivf_reset_profile(self._h))
 

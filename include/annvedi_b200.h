@@ -292,6 +292,10 @@ int ann_ivf_profile(ann_ivf* h, double* out8);
 #define ANN_IVF_OPT_WAIT_SELFTEST 4
 int ann_ivf_set_option(ann_ivf* h, int32_t option, int64_t value);
 
+/* Diagnostic: the exact form's SQ8 selection by tensor-core keys: out2 = {batches that tried it, batches that it settled
+ * (the others ran the batched pass as well)}, over the index's life. */
+int ann_ivf_prune_stats(ann_ivf* h, int64_t* out2);
+
 /* Single-kernel times of the same profiled calls (CUDA events around each launch, on the query stream):
  * out8 = {list-keys kernel ms (the grouped tensor-core GEMM of the list rows, or the SQ8 batched
  * kernel), sampled-bar kernel ms, best-R selection kernel ms, FP32 re-rank kernel ms, then the launch
