@@ -877,7 +877,7 @@ int ann_flat_scores_tc(ann_flat* h, const float* queries, int32_t nq, int64_t ld
     float* rfac = cv.take<float>((size_t)nq);
     float* tmp = reinterpret_cast<float*>(h->ws.big);
     if ((rc = flat_tc_queries(h, t, queries, nq, ldq, qb, rfac, st))) return rc;
-    TcGemmArgs a{nq, (int)h->n, t.kpad, nullptr, tmp, h->n, h->d_err};
+    TcGemmArgs a{nq, (int)h->n, t.kpad, tmp, h->n, h->d_err};
     a.wait_ns = h->wait_ns;
     a.test_no_loads = h->wait_ns > 0;
     a.kind = t.kind;
@@ -1137,7 +1137,7 @@ int ann_flat_query_tc(ann_flat* h, ann_workspace* ws, const float* queries, int3
             if ((rc = ws_reserve_big(ws, sizeof(float) * (size_t)nf * n))) return rc;
             float* keys = reinterpret_cast<float*>(ws->big);
             const int prec = h->prof.begin(st, 3);  // stage 3: the full key matrix, 4: its selection
-            TcGemmArgs a{nf, (int)n, kpad, nullptr, keys, n, h->d_err};
+            TcGemmArgs a{nf, (int)n, kpad, keys, n, h->d_err};
             a.wait_ns = h->wait_ns;
             a.test_no_loads = h->wait_ns > 0;
             a.kind = t.kind;

@@ -243,7 +243,7 @@ static int assign_rows_keys(KmeansKeys& k, const float* x, int64_t n, int dim, i
     if ((rc = launch_tc_operand(cent, C, dim, dpad, k.cb, k.kpad, kTcBase, ANN_METRIC_L2, 0, st))) return rc;
     for (int64_t r0 = 0; r0 < n; r0 += k.chunk) {
         const int nr = (int)std::min<int64_t>(k.chunk, n - r0);
-        TcGemmArgs g{nr, C, k.kpad, nullptr, k.keys, C, k.err};
+        TcGemmArgs g{nr, C, k.kpad, k.keys, C, k.err};
         g.wait_ns = k.wait_ns;
         g.test_no_loads = k.wait_ns > 0;
         g.out_cmin = k.cmin;
@@ -1170,19 +1170,14 @@ static int ivf_tc_sampled(ann_ivf* h, ann_workspace* ws, const IvfQueryCfg& c, c
     const TcItemDescs descs[2] = {{sitem, lcap, sitem_desc, scap}, {titem, nullptr, titem_desc, items_cap}};
     if ((rc = launch_tc_item_descs(descs, 2, C, b.lq_off, h->list_off, st))) return rc;
     // 1. sample pass: keys of the list heads into the sample streams; the two bars per query
-    TcGemmArgs gs{(int)max_pairs, (int)h->n, op.K, nullptr, SK, 0, err};
+    TcGemmArgs gs{(int)max_pairs, (int)h->n, op.K, SK, 0, err};
     gs.wait_ns = h->wait_ns;
     gs.test_no_loads = h->wait_ns > 0;
     gs.kind = op.kind;
     gs.col_fac = op.col_fac;
     gs.row_fac = op.pfac;
-    gs.g_item_off = sitem;
-    gs.g_a_off = b.lq_off;
-    gs.g_b_off = h->list_off;
-    gs.g_b_len = lcap;
     gs.g_dbase = sdbase;
     gs.g_total = sitem + C;
-    gs.g_lists = C;
     gs.g_item_desc = sitem_desc;
     if ((rc = launch_tc_gemm(Apk, op.B, gs, st))) return rc;
     int kt = h->prof.kbegin(st);
@@ -1192,18 +1187,14 @@ static int ivf_tc_sampled(ann_ivf* h, ann_workspace* ws, const IvfQueryCfg& c, c
     h->prof.kend(kt, kKernBars, st);
     // 2. filter pass over every row of the probed lists into the queries' buffers
     auto filter = [&](const float* tau, const int* skip_if_zero) -> int {
-        TcGemmArgs g{(int)max_pairs, (int)h->n, op.K, nullptr, nullptr, 0, err};
+        TcGemmArgs g{(int)max_pairs, (int)h->n, op.K, nullptr, 0, err};
         g.wait_ns = h->wait_ns;
         g.test_no_loads = h->wait_ns > 0;
         g.skip_if_zero = skip_if_zero;
         g.kind = op.kind;
         g.col_fac = op.col_fac;
         g.row_fac = op.pfac;
-        g.g_item_off = titem;
-        g.g_a_off = b.lq_off;
-        g.g_b_off = h->list_off;
         g.g_total = titem + C;
-        g.g_lists = C;
         g.g_item_desc = titem_desc;
         g.g_row_query = rowq;
         g.tau = tau;
@@ -1348,7 +1339,7 @@ static int ivf_query_device(ann_ivf* h, ann_workspace* ws, const IvfQueryCfg& c,
     if (c.tc || c.coarse_keys) {
         // BF16 keys to every centroid, then the exact FP32 order of the best npc + 16
         if ((rc = launch_tc_operand(qdev, nq, h->dim, h->dpad, qb, h->kpad, kTcQuery, ANN_METRIC_L2, 0, st))) return rc;
-        TcGemmArgs ca{nq, h->C, h->kpad, nullptr, ckeys, h->C, c.coarse_keys ? key_err : h->d_err};
+        TcGemmArgs ca{nq, h->C, h->kpad, ckeys, h->C, c.coarse_keys ? key_err : h->d_err};
         ca.wait_ns = h->wait_ns;
         ca.test_no_loads = h->wait_ns > 0;
         ca.out_cmin = ckmin;  // and each query's 32-centroid chunk minima, which let the ranking skip chunks
@@ -1519,18 +1510,14 @@ static int ivf_query_device(ann_ivf* h, ann_workspace* ws, const IvfQueryCfg& c,
                     return rc;
                 const TcItemDescs descs{titem, nullptr, titem_desc, items_cap};
                 if (!c.small_tc && (rc = launch_tc_item_descs(&descs, 1, h->C, b.lq_off, h->list_off, st))) return rc;
-                TcGemmArgs g{(int)max_pairs, (int)h->n, op.K, nullptr, D, 0, h->d_err};
+                TcGemmArgs g{(int)max_pairs, (int)h->n, op.K, D, 0, h->d_err};
                 g.wait_ns = h->wait_ns;
                 g.test_no_loads = h->wait_ns > 0;
                 g.kind = op.kind;
                 g.col_fac = op.col_fac;
                 g.row_fac = op.pfac;
-                g.g_item_off = titem;
-                g.g_a_off = c.small_tc ? h->list_off : b.lq_off;  // (small: the descriptors alone are read)
-                g.g_b_off = h->list_off;
                 g.g_dbase = dbase;
                 g.g_total = titem + h->C;
-                g.g_lists = h->C;
                 g.g_item_desc = titem_desc;
                 const int kg = h->prof.kbegin(st);
                 if ((rc = launch_tc_gemm(Apk, op.B, g, st))) return rc;

@@ -38,32 +38,9 @@ struct GroupTile {
     int64_t a0, b0;
     int am, bn;
 };
-__device__ __forceinline__ GroupTile tile_of_desc(int4 d) { return GroupTile{d.x, d.y, d.z, d.w}; }
 __device__ __forceinline__ GroupTile group_tile(const TcGemmArgs& a, int64_t t) {
-    if (a.g_item_desc) return tile_of_desc(a.g_item_desc[t]);
-    int lo = 0, hi = a.g_lists - 1;
-    if (a.g_item_list) {
-        lo = a.g_item_list[t];  // one load, where a search would chain a dozen
-    } else {
-        while (lo < hi) {
-            const int mid = (lo + hi + 1) >> 1;
-            if (a.g_item_off[mid] <= t)
-                lo = mid;
-            else
-                hi = mid - 1;
-        }
-    }
-    const int64_t np = a.g_a_off[lo + 1] - a.g_a_off[lo];
-    const int64_t nr = a.g_b_len ? a.g_b_len[lo] : a.g_b_off[lo + 1] - a.g_b_off[lo];
-    const int64_t npt = (np + kBM - 1) / kBM;
-    const int64_t local = t - a.g_item_off[lo];
-    const int64_t g = local % npt, rt = local / npt;
-    GroupTile gt;
-    gt.a0 = a.g_a_off[lo] + g * kBM;
-    gt.b0 = a.g_b_off[lo] + rt * kBN;
-    gt.am = (int)min((int64_t)kBM, np - g * kBM);
-    gt.bn = (int)min((int64_t)kBN, nr - rt * kBN);
-    return gt;
+    const int4 d = a.g_item_desc[t];
+    return GroupTile{d.x, d.y, d.z, d.w};
 }
 
 // Epilogue warps of the key-matrix and grouped forms, and of the filter form; threads and shared memory
@@ -102,7 +79,7 @@ __global__ void __launch_bounds__(epi_threads(EPI), 1) tc_gemm_kernel(const __gr
     constexpr int kBlockK = KindOf<KIND>::kBlockK, kMmaK = KindOf<KIND>::kMmaK;
     const int mt = (int)ceil_div(a.M, kBM), nt = (int)ceil_div(a.N, kBN), kt = (int)ceil_div(a.K, kBlockK);
     const int k16_last = (a.K - (kt - 1) * kBlockK) / kMmaK;  // MMAs of the last k-block
-    const bool grouped = a.g_item_off != nullptr;
+    const bool grouped = a.g_item_desc != nullptr;
     const int64_t tiles = grouped ? *a.g_total : (int64_t)mt * nt;
 
     if (threadIdx.x == 0) {
@@ -134,23 +111,18 @@ __global__ void __launch_bounds__(epi_threads(EPI), 1) tc_gemm_kernel(const __gr
         if (lane == 0 && !a.test_no_loads) {
             int64_t it = 0;
             bool ok = true;
-            // with item descriptors, the next item's is loaded while this one's copies are issued
-            const bool pre = grouped && a.g_item_desc != nullptr;
-            int4 dnext = pre && (int64_t)blockIdx.x < tiles ? a.g_item_desc[blockIdx.x] : make_int4(0, 0, 0, 0);
+            // the next item's descriptor is loaded while this one's copies are issued
+            int4 dnext = grouped && (int64_t)blockIdx.x < tiles ? a.g_item_desc[blockIdx.x] : make_int4(0, 0, 0, 0);
             for (int64_t t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
                 int64_t arow, brow;
-                if (pre) {
+                if (grouped) {
                     const int4 d = dnext;
                     if (t + gridDim.x < tiles) dnext = a.g_item_desc[t + gridDim.x];
                     arow = d.x;
                     brow = d.y;
-                } else if (grouped) {
-                    const GroupTile gt = group_tile(a, t);
-                    arow = gt.a0;
-                    brow = gt.b0;
                 } else {
                     arow = (t % mt) * kBM;
-                    brow = (t / mt) * kBN * a.b_tile_stride;
+                    brow = (t / mt) * kBN;
                 }
                 for (int kb = 0; kb < kt; ++kb, ++it) {
                     const int s = (int)(it % kStages);
@@ -238,7 +210,6 @@ __global__ void __launch_bounds__(epi_threads(EPI), 1) tc_gemm_kernel(const __gr
                 cbase = gt.b0;
                 ncols = gt.bn;
             }
-            const float an = (a.normA && mvalid) ? a.normA[arow] : 0.f;
             const float rfac = (a.row_fac && mvalid) ? a.row_fac[arow] : 1.f;
             // rows past M or past a grouped item's pairs get a NaN bar, which no key passes (not even a -inf
             // key, which a -inf bar would let through)
@@ -255,10 +226,8 @@ __global__ void __launch_bounds__(epi_threads(EPI), 1) tc_gemm_kernel(const __gr
 #pragma unroll
                 for (int i = 0; i < kCols / 32; ++i) {
                     const int lcol = col0 + 32 * i + lane;  // column within the tile
-                    const int col = n0 + lcol;
-                    const int64_t nrow = grouped ? cbase + lcol : (int64_t)(col / kBN) * kBN * a.b_tile_stride + col % kBN;
                     const bool in = lcol < ncols;
-                    const float* src = reinterpret_cast<const float*>(a.col_fac + (in ? nrow : 0));
+                    const float* src = reinterpret_cast<const float*>(a.col_fac + (in ? cbase + lcol : 0));
                     cp_async4(sfx + 32 * i + lane, src, in);
                     cp_async4(sfy + 32 * i + lane, src + 1, in);
                 }
@@ -319,12 +288,11 @@ __global__ void __launch_bounds__(epi_threads(EPI), 1) tc_gemm_kernel(const __gr
                 asm volatile("cp.async.wait_all;" ::: "memory");
                 __syncwarp();
             }
-            const bool has_an = a.normA != nullptr;  // uniform
-            // filter keys of the 32 columns from col0 + c + 32 h (raw accumulators r): the row norm, the
-            // scale factors, NaN past the tile's valid columns
+            // filter keys of the 32 columns from col0 + c + 32 h (raw accumulators r): the scale factors, NaN past
+            // the tile's valid columns
             auto half_keys = [&](const uint32_t (&r)[32], int h, int c, float (&v)[32]) {
 #pragma unroll
-                for (int u = 0; u < 32; ++u) v[u] = acc_value<KIND>(r[u]) + (has_an ? an : 0.f);
+                for (int u = 0; u < 32; ++u) v[u] = acc_value<KIND>(r[u]);
                 if (staged) {
                     const float2 r2 = make_float2(rfac, rfac);
 #pragma unroll
@@ -426,19 +394,13 @@ __global__ void __launch_bounds__(epi_threads(EPI), 1) tc_gemm_kernel(const __gr
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
                     float v[32];
-                    if (has_an) {
 #pragma unroll
-                        for (int u = 0; u < 32; ++u) v[u] = acc_value<KIND>(h ? r1[u] : r0[u]) + an;
-                    } else {
-#pragma unroll
-                        for (int u = 0; u < 32; ++u) v[u] = acc_value<KIND>(h ? r1[u] : r0[u]);
-                    }
+                    for (int u = 0; u < 32; ++u) v[u] = acc_value<KIND>(h ? r1[u] : r0[u]);
                     const int nb = n0 + col0 + c + 32 * h;  // output column of v[0]
                     const int lb = col0 + c + 32 * h;       // its column within the tile
                     if (a.col_fac) {  // scaled operands: key = f.y + f.x * (row scale * accumulator)
-                        const int col = nb + lane;  // output column -> base row (strided sample of 256-row tiles)
-                        const int64_t nrow = (int64_t)(col / kBN) * kBN * a.b_tile_stride + col % kBN;
-                        const float2 f = col < a.N ? a.col_fac[nrow] : make_float2(0.f, 0.f);
+                        const int col = nb + lane;
+                        const float2 f = col < a.N ? a.col_fac[col] : make_float2(0.f, 0.f);
 #pragma unroll
                         for (int u = 0; u < 32; ++u)
                             v[u] = fmaf(__shfl_sync(0xffffffffu, f.x, u), rfac * v[u], __shfl_sync(0xffffffffu, f.y, u));
@@ -538,32 +500,26 @@ static cudaError_t run_tc_gemm(const CUtensorMap& tmA, const CUtensorMap& tmB, c
 int launch_tc_gemm(const void* A, const void* B, const TcGemmArgs& a, cudaStream_t st) {
     const int step = tc_16bit(a.kind) ? 16 : 32;
     ANN_CHECK_ARG(tc_16bit(a.kind) || a.kind == kTcE4M3 || a.kind == kTcI8, "tensor-core scan: element kind %d", a.kind);
-    ANN_CHECK_ARG(a.kind != kTcF16 || a.g_item_off, "tensor-core scan: FP16 operands are grouped");
+    ANN_CHECK_ARG(a.kind != kTcF16 || a.g_item_desc, "tensor-core scan: FP16 operands are grouped");
     ANN_CHECK_ARG(a.K % step == 0 && a.K > 0, "tensor-core scan: K=%d not a positive multiple of %d", a.K, step);
-    ANN_CHECK_ARG(tc_16bit(a.kind) || (a.col_fac && a.row_fac && (a.g_item_off == nullptr || a.kind == kTcI8)),
+    ANN_CHECK_ARG(tc_16bit(a.kind) || (a.col_fac && a.row_fac && (a.g_item_desc == nullptr || a.kind == kTcI8)),
                   "tensor-core scan: E4M3 / I8 operands need their scale factors (E4M3: no grouping)");
     ANN_CHECK_ARG((reinterpret_cast<uintptr_t>(A) & 15) == 0 && (reinterpret_cast<uintptr_t>(B) & 15) == 0,
                   "tensor-core scan: operands must be 16-byte aligned");
-    ANN_CHECK_ARG(a.out != nullptr || (a.g_item_off && a.tau && a.fkey && a.fcol && a.row_cap > 0 && a.rcount),
+    ANN_CHECK_ARG(a.out != nullptr || (a.g_item_desc && a.tau && a.fkey && a.fcol && a.row_cap > 0 && a.rcount),
                   "tensor-core scan: neither an output matrix nor a grouped filter");
-    ANN_CHECK_ARG(a.g_item_off == nullptr ||
-                      (a.g_a_off && a.g_b_off && a.g_total && a.g_lists > 0 &&
-                       ((a.out && a.g_dbase && a.tau == nullptr) || (a.out == nullptr && a.tau && a.g_row_query))),
+    ANN_CHECK_ARG(a.g_item_desc == nullptr ||
+                      (a.g_total && ((a.out && a.g_dbase && a.tau == nullptr) || (a.out == nullptr && a.tau && a.g_row_query))),
                   "tensor-core scan: incomplete grouping");
-    ANN_CHECK_ARG(a.b_tile_stride >= 1, "tensor-core scan: bad sample stride");
-    ANN_CHECK_ARG(a.out_cmin == nullptr || (a.out && a.g_item_off == nullptr && a.b_tile_stride == 1),
+    ANN_CHECK_ARG(a.out_cmin == nullptr || (a.out && a.g_item_desc == nullptr),
                   "tensor-core scan: chunk minima need the dense key-matrix mode");
     if (a.M == 0 || a.N == 0) return ANN_OK;
-    const int64_t b_rows = a.b_rows > 0 ? a.b_rows : a.N;
-    // the last sampled tile must start inside B
-    ANN_CHECK_ARG(a.g_item_off != nullptr || (ceil_div(a.N, kBN) - 1) * kBN * (int64_t)a.b_tile_stride < b_rows,
-                  "tensor-core scan: sample runs past the base");
     CUtensorMap tmA, tmB;
     int rc = tc_make_map(&tmA, A, a.M, a.K, kBM, a.kind);
     if (rc) return rc;
-    rc = tc_make_map(&tmB, B, b_rows, a.K, kBN, a.kind);
+    rc = tc_make_map(&tmB, B, a.N, a.K, kBN, a.kind);
     if (rc) return rc;
-    const int grid = a.g_item_off ? kNumSMs : tc_grid(a.M, a.N);  // grouped: persistent over the items
+    const int grid = a.g_item_desc ? kNumSMs : tc_grid(a.M, a.N);  // grouped: persistent over the items
     const bool filter = a.out == nullptr;
     cudaError_t e;
     if (a.kind == kTcBF16)
@@ -583,7 +539,7 @@ int launch_tc_gemm(const void* A, const void* B, const TcGemmArgs& a, cudaStream
 }
 
 namespace {
-// desc[t] for the items of list l = blockIdx.x (strided): the tile group_tile would derive for item t.
+// desc[t] for the items of list l = blockIdx.x (strided).
 __global__ void tc_item_descs_kernel(TcItemDescs s0, TcItemDescs s1, int C, const int64_t* __restrict__ a_off,
                                      const int64_t* __restrict__ b_off) {
     const TcItemDescs s = blockIdx.y ? s1 : s0;
@@ -621,7 +577,7 @@ int tc_wait_selftest(uint64_t wait_ns, int* flag_out) {
     if (e == cudaSuccess) e = cudaMemsetAsync(buf, 0, a_bytes + b_bytes + o_bytes + 256, st);
     if (e == cudaSuccess) {
         int* flag = reinterpret_cast<int*>(buf + a_bytes + b_bytes + o_bytes);
-        TcGemmArgs a{kBM, kBN, 64, nullptr, reinterpret_cast<float*>(buf + a_bytes + b_bytes), kBN, flag};
+        TcGemmArgs a{kBM, kBN, 64, reinterpret_cast<float*>(buf + a_bytes + b_bytes), kBN, flag};
         a.wait_ns = wait_ns;
         a.test_no_loads = 1;
         rc = launch_tc_gemm(buf, buf + a_bytes, a, st);

@@ -19,12 +19,9 @@ constexpr bool tc_16bit(int kind) { return kind == kTcBF16 || kind == kTcF16; }
 
 struct TcGemmArgs {
     int M, N, K;           // A [M, K], B [N, K] BF16 row-major; K a multiple of 16
-    const float* normA;    // [M] optional per-row addend (|a|^2 turns the L2 key into the squared distance)
     float* out;            // [M, ldo] keys; null in the grouped filter mode
     int64_t ldo;
     int* err;              // device flag set (to 2) if a bounded wait gives up
-    int b_tile_stride = 1; // B rows of output tile j start at row j * 256 * b_tile_stride (a strided sample)
-    int64_t b_rows = 0;    // rows of the B matrix when sampling (0: N)
     // Grouped filter mode (out == null): keys <= tau of a row's query are appended, as (key, column), to the query's
     // buffer: fkey / fcol [query * row_cap + slot] at slot = atomicAdd(&rcount[query], n) -- one atomic per lane per
     // 64 columns, n its survivors there -- and nothing is written at slots past row_cap (rcount may exceed it: the
@@ -34,24 +31,15 @@ struct TcGemmArgs {
     int* fcol = nullptr;
     int row_cap = 0;
     int* rcount = nullptr;
-    // Grouped mode (g_item_off != null; out receives the keys): tile t is work item t of a list-major
-    // grouping (an IVF batch). List l owns A rows [g_a_off[l], g_a_off[l+1]) (its (query, list) pairs)
-    // and B rows [g_b_off[l], g_b_off[l+1]) (its rows); its items are ceil(pairs/128) x ceil(rows/256)
-    // tiles, pair tiles fastest, numbered from g_item_off[l]; *g_total items in all (read on the
+    // Grouped mode (g_item_desc != null; out receives the keys): tile t is work item t of a list-major grouping (an IVF
+    // batch) of A rows, the (query, list) pairs, and B rows, the lists' rows: (first A row, first B row, A rows, B rows),
+    // one 16-byte load (launch_tc_item_descs), the next item's read ahead of its use; *g_total items in all (read on the
     // device). The key of pair i and list row r goes to out[g_dbase[i] + r].
-    const int64_t* g_item_off = nullptr;
-    const int64_t* g_a_off = nullptr;
-    const int64_t* g_b_off = nullptr;
+    const int4* g_item_desc = nullptr;
     const int64_t* g_dbase = nullptr;
     const int64_t* g_total = nullptr;
-    int g_lists = 0;
-    const int32_t* g_item_list = nullptr;  // optional: the list of each item (else a search of g_item_off)
-    // optional, in place of the two above: item t's tile as (first A row, first B row, A rows, B rows), one
-    // 16-byte load (launch_tc_item_descs); the roles read the next item's ahead of its use
-    const int4* g_item_desc = nullptr;
-    const int64_t* g_b_len = nullptr;      // optional: rows of list l taken (else g_b_off[l+1] - g_b_off[l])
     // Grouped filter mode (grouped, out == null): A row i belongs to query g_row_query[i]; its bar is
-    // tau[g_row_query[i]], and a survivor is recorded as (key, list row g_b_off[l] + r, that query).
+    // tau[g_row_query[i]], and a survivor is recorded as (key, list row, that query).
     const int32_t* g_row_query = nullptr;
     // Element kind of A and B. E4M3 and I8 operands carry factors per row: the key is
     // col_fac[n].y + col_fac[n].x * row_fac[m] * accumulator (key-matrix and filter modes; I8 also grouped,
