@@ -1017,9 +1017,8 @@ static size_t ivf_scratch(const ann_ivf* h, const IvfQueryCfg& c, int nq) {
         sz.take<int4>((size_t)tc_items_bound((int64_t)nq * c.npc, (int)h->C, h->sizes_desc[0]));
     }
     sz.take<int32_t>((size_t)nq);  // re-rank query order
-    sz.take<int32_t>((size_t)nq);  // queries set apart (every row), and their count
-    sz.take<int32_t>(1);
-    sz.take<int>(1);               // the exact form's key passes: a wait gave up
+    sz.take<int32_t>((size_t)nq);  // queries set apart (every row)
+    sz.take<int32_t>(2);           // their count, and whether a wait of the exact form's key passes gave up
     sz.take<int64_t>(1);           // an every-row stream: its length
     sz.take<int32_t>(1);           // and its segment flag
     return sz.off;
@@ -1140,6 +1139,7 @@ static int ivf_tc_sampled(ann_ivf* h, ann_workspace* ws, const IvfQueryCfg& c, c
         pa.frow = srow;
         pa.rcount = scount;
         pa.fails = flags;
+        pa.err = key_err;
         pa.keyR = keyR;
         pa.idR = idR;
         Apk = cv.take<unsigned char>((size_t)max_pairs * op.row_bytes);
@@ -1214,11 +1214,10 @@ static int ivf_tc_sampled(ann_ivf* h, ann_workspace* ws, const IvfQueryCfg& c, c
         kt = h->prof.kbegin(st);
         if ((rc = launch_ivf_prune_finish(pa, st))) return rc;
         h->prof.kend(kt, kKernSelect, st);
-        int fails = 0, gave_up = 0;
+        int fails = 0;
         ANN_CUDA_TRY(cudaMemcpyAsync(&fails, pa.fails, sizeof(int), cudaMemcpyDeviceToHost, st));
-        ANN_CUDA_TRY(cudaMemcpyAsync(&gave_up, key_err, sizeof(int), cudaMemcpyDeviceToHost, st));
         ANN_CUDA_TRY(cudaStreamSynchronize(st));
-        *done = fails == 0 && gave_up == 0;
+        *done = fails == 0;
         return ANN_OK;
     }
     ANN_CUDA_TRY(cudaMemsetAsync(scount, 0, sizeof(int) * (size_t)nq, st));
@@ -1303,8 +1302,8 @@ static int ivf_query_device(ann_ivf* h, ann_workspace* ws, const IvfQueryCfg& c,
     int4* titem_desc = c.tc ? cv.take<int4>((size_t)items_cap) : nullptr;
     int32_t* qorder = cv.take<int32_t>((size_t)nq);
     int32_t* apart = cv.take<int32_t>((size_t)nq);
-    int32_t* apart_count = cv.take<int32_t>(1);
-    int* key_err = cv.take<int>(1);
+    int32_t* apart_count = cv.take<int32_t>(2);
+    int* key_err = apart_count + 1;
     int64_t* every_len = cv.take<int64_t>(1);
     int32_t* every_seg = cv.take<int32_t>(1);
 
@@ -1326,10 +1325,8 @@ static int ivf_query_device(ann_ivf* h, ann_workspace* ws, const IvfQueryCfg& c,
     a.nsplit = c.nsplit;
     a.num_threads = c.num_threads;
     a.ndist = h->d_ndist;
-    if (c.coarse_keys || c.pruned) {  // exact results: a call whose waits give up takes the scans instead
-        a.key_err = key_err;
-        ANN_CUDA_TRY(cudaMemsetAsync(key_err, 0, sizeof(int), st));
-    }
+    if (c.coarse_keys || c.pruned) a.key_err = key_err;  // exact results: a call whose waits give up takes the scans instead
+    if (c.batched && !c.small_tc) ANN_CUDA_TRY(cudaMemsetAsync(apart_count, 0, 2 * sizeof(int32_t), st));
     a.out_ids = ids_dev;
     a.out_dists = dists_dev;
 
@@ -1372,7 +1369,6 @@ static int ivf_query_device(ann_ivf* h, ann_workspace* ws, const IvfQueryCfg& c,
     if (plan_apart) {
         a.apart = apart;
         a.apart_count = apart_count;
-        ANN_CUDA_TRY(cudaMemsetAsync(apart_count, 0, sizeof(int32_t), st));
     }
     // 2. plan: whole lists, or the LSH buckets' explicit streams (signatures first, their own stage)
     LshCandArgs la{};

@@ -164,6 +164,7 @@ __global__ void __launch_bounds__(kThreads) ivf_prune_finish_kernel(IvfPruneArgs
     const int cnt = a.rcount[q], ns = a.plan.n_seg[q];
     const float2 w = a.win[q];
     const float tauF = a.tauF[q];
+    const int gave_up = *a.err;
     const int64_t cands = a.plan.n_cands[q];
     const int need = (int)min((int64_t)R, cands);
     const float* fk = a.fkey + (int64_t)q * cap;
@@ -175,7 +176,7 @@ __global__ void __launch_bounds__(kThreads) ivf_prune_finish_kernel(IvfPruneArgs
         oi[e] = kNoId;
     }
     if (need == 0) return;  // an empty stream (a query set apart)
-    bool fail = ns < 0 || cnt > cap || cnt < need || !(w.x < kInf);
+    bool fail = ns < 0 || cnt > cap || cnt < need || !(w.x < kInf) || gave_up != 0;
     float T = 0.f;
     if (!fail) {  // the need-th smallest kept key
         for (int i = tid; i < cnt; i += kThreads) sO[i] = ord_f32(fk[i]);

@@ -32,6 +32,7 @@ struct IvfPruneArgs {
     const int* frow;
     int* rcount;         // [nq] survivors met
     int* fails;          // [1] queries that the pruned pass leaves
+    const int* err;      // [1] set where a wait of the key passes gave up: every query is left
     float* keyR;         // [nq, R] the best R (SQ8 distance, row), in no order, padded with (+inf, kNoId)
     int* idR;
 };
