@@ -1121,9 +1121,12 @@ int ann_flat_query_tc(ann_flat* h, ann_workspace* ws, const float* queries, int3
                 return ANN_OK;
             };
             if ((rc = redo(list, hf[0], tauS, cap2))) return rc;
-            // a survivor taken this way costs about eight keys of the full matrix (1,000 queries over 1M x 384 with 200,000
-            // copies each: 33 ms, 20 by the matrix), and 8M of them no more than its selection of few queries
-            if ((int64_t)hf[1] * hf[2] > std::max<int64_t>((int64_t)nc * n / 10, 8 << 20))
+            // Measured: a pass of its own 0.2 ms, its survivors 0.17 ns each; the full matrix 1 ms (its selection of whole
+            // rows) and 0.02 ns a key. 1,000 queries over 1M x 384 with 200,000 copies each: 33 ms by passes, 20 by the
+            // matrix; 70 of 184 over 184,924 x 70 with 74,000 copies, three to a pass: 4.8, 2.1.
+            const int64_t per_pass = std::max<int64_t>(1, std::min<int64_t>(kRerunBatch, (int64_t)ent / std::max(1, hf[2])));
+            const double passes_us = 200.0 * (double)ceil_div(hf[1], per_pass) + 1.7e-4 * (double)hf[1] * hf[2];
+            if (passes_us > 1000.0 + 2e-5 * (double)nc * (double)n)
                 done = false;
             else if ((rc = redo(over, hf[1], tauF, hf[2])))
                 return rc;
