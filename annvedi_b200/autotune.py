@@ -130,7 +130,8 @@ def tune_flat_tc(index, base, queries, kth, k: int = 100, target: float = 0.95, 
 def tune_flat_tile(index, queries, k: int = 100, tiles=(8, 16, 32), reps: int = 2, timer=None) -> dict:
     """Fastest query tile (queries per CTA) of a LinearIndex's exact scan for this batch, timed over `reps`
     calls after a warm-up call; the tile is left set on the index. Results do not depend on the tile, so no
-    recall is needed. Returns {"best": {...}, "table": [...]} with tile, ms_per_batch and qps."""
+    recall is needed. Searches that prune by tensor-core keys go on doing so, and differ by the tile only in the
+    queries that they leave to the scan (set_pruning(False) times the scan itself). Returns {"best": {...}, "table": [...]} with tile, ms_per_batch and qps."""
     import torch
     time_fn = _timer(timer)
     nq = queries.shape[0]

@@ -2,9 +2,13 @@
 
 At one to a few queries per call a search is a handful of short kernels, and launching them costs a
 visible share of the call. `GraphedSearch` captures one call of a search that makes no host
-synchronisation -- the plain exact scan (`LinearIndex.search`, mode "exact") and the IVF-SQ8 query for
+synchronisation -- the exact search (`LinearIndex.search`, mode "exact") and the IVF-SQ8 query for
 batches of fewer than 32 queries (`IVFIndex.search`, mode "exact"; larger batches group their (query,
 list) pairs on the host) -- and replays it for each new batch copied into its input buffer.
+
+A captured exact search keeps the form that it was captured in: the scan on an index that has not laid out its operand copy
+by then (the copy comes with the savings of a dozen single queries, of one large batch, or with `search_tc`), the form
+pruned by tensor-core keys afterwards. The results are the same.
 
 The captured launches bake in the addresses of their scratch memory, so a graphed search owns a
 workspace of its own: one eager call before the capture sizes it, and nothing else may use it. The
@@ -49,7 +53,7 @@ class GraphedSearch:
 
 
 def flat_exact(index, batch: int, k: int, device: int = 0) -> GraphedSearch:
-    """The plain exact scan of a LinearIndex for `batch` queries, captured."""
+    """The exact search of a LinearIndex for `batch` queries, captured."""
     def search(x, ids, dists, stream, ws):
         index.search(x, k, mode="exact", workspace=ws, out_ids=ids, out_dists=dists, stream=stream)
     return GraphedSearch(search, batch, index.dim, k, device)

@@ -346,10 +346,15 @@ def tc_route(name: str, index, refine_r: int = 400) -> Route:
 
 
 def flat_route(name: str, index) -> Route:
-    """The plain FP32 exact scan of a LinearIndex (ann_flat_query, exact mode)."""
+    """The exact search of a LinearIndex (ann_flat_query, exact mode): pruned by tensor-core keys where that saves time, with
+    the FP32 scan's results. The operand copy that it lays out belongs to the index, not to a call."""
     def search(x, k, stream, ws, out_ids=None, out_dists=None):
         return index.search(x, k, mode="exact", workspace=ws, stream=stream, out_ids=out_ids, out_dists=out_dists)
-    return Route(name, index.dim, search, lambda nq: nq * (200 * 8 * 100 + 8 * index.dim) + (16 << 20))
+    def scratch(nq):
+        # the scan's lists and queries; the pruned form's survivors, minima and operand rows, and its leftover lists
+        lists = 148 * 8 * 100
+        return nq * (200 * 8 * 100 + 8 * index.dim + 80_000 + 16 * index.dim) + min(256 << 20, nq * lists) + (16 << 20)
+    return Route(name, index.dim, search, scratch)
 
 
 def ivf_route(name: str, index, n_probe_clusters: int, refine_r: int = 300, max_list: int = 40_000,
