@@ -630,6 +630,7 @@ static int flat_ensure_pruned(ann_flat* h, int nq, cudaStream_t st, bool capturi
         h->prune_credit_us += 40.0 + elems * (nq <= 4 ? 0.25e-6 + 0.2e-6 * (nq - 1) : 1.0e-7 * nq);
         if (!h->base_bf16 && h->prune_credit_us < 500.0 + 3.1e-6 * elems) return ANN_OK;
         if (capturing || (h->prune_refused && !h->base_bf16)) return ANN_OK;
+        CaptureRelax relax;
         // the norms first: rows that the bounds do not cover need no copy
         unsigned *d2 = nullptr, h2[2] = {0, 0};
         if (cudaMalloc(&d2, sizeof(h2)) != cudaSuccess) {
@@ -724,11 +725,11 @@ static int flat_exact_pruned(ann_flat* h, ann_workspace* ws, const float* qdev, 
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     ANN_CUDA_TRY(cudaStreamIsCapturing(st, &cs));
     const bool capturing = cs != cudaStreamCaptureStatusNone;
-    std::optional<CaptureRelax> relax;  // the first pruned call lays out, allocates and loads kernels
-    if (!capturing) relax.emplace();
     bool ok = false;
     int rc = flat_ensure_pruned(h, nq, st, capturing, &ok);
     if (rc || !ok) return rc;
+    std::optional<CaptureRelax> relax;  // the first pass loads its kernels
+    if (!capturing && h->prune_pass == 0) relax.emplace();
     const int bq = std::min(h->query_tile > 0 ? h->query_tile : flat_scan_bq(nq), flat_scan_max_bq(kk));
     const bool stream_form = flat_stream_eligible(bq, kk, dpad);
     // a sample of about 64 tiles of 256 rows, an eighth of a small base
@@ -767,6 +768,7 @@ static int flat_exact_pruned(ann_flat* h, ann_workspace* ws, const float* qdev, 
         if (capturing) return ANN_OK;  // the scan's own scratch is there
         std::lock_guard<std::mutex> lk(h->tc_mu);
         if (sz.bytes() >= h->prune_ws_refused) return ANN_OK;
+        CaptureRelax allow;
         if ((rc = ws_reserve_big(ws, sz.bytes()))) {
             if (rc != ANN_ERR_NOMEM) return rc;
             clear_error();
