@@ -266,7 +266,7 @@ int ann_flat_fit(ann_flat* h, const float* data, int64_t n, int32_t dim, int64_t
     h->prune_refused = false;
     h->prune_ws_refused = SIZE_MAX;
     h->prune_streak = h->prune_skip = 0;
-    h->prune_seen = h->prune_pass;
+    if (h->prune_word) h->prune_seen = (uint32_t)(*h->prune_word >> 32);  // (the old base's passes are done: its end is not read)
     const size_t bytes = sizeof(float) * (size_t)n * dpad;
     cudaError_t e = cudaMalloc(&h->base, bytes);
     if (e != cudaSuccess) {

@@ -1,7 +1,7 @@
 // The exact scan of a query batch with its rows pruned by tensor-core keys.
 //
 // The exact scan (flat_scan.cu) forms every (query, row) distance on the FP32 units: 2 N dim instructions a query,
-// 45.3 ms for 1,000 queries over 1M x 384 with the tensor cores idle (0.87 ms pruned); a single query reads 4 bytes
+// 45.3 ms for 1,000 queries over 1M x 384 with the tensor cores idle (0.88 ms pruned); a single query reads 4 bytes
 // an element (0.37 ms, 0.19 ms pruned). Only about k distances a query are kept. Here the BF16 tensor-core keys
 // (tc_gemm.cuh) say which rows can be among them, and only those rows' FP32 distances are formed, with the scan's own
 // sums, so that ids and distances are the scan's bit for bit:

@@ -77,3 +77,23 @@ def test_one_query_of_a_small_batch_is_its_whole_scan(cuda):
     ix = _index(x)
     s = _run(ix, torch.from_numpy(q).cuda(), 10, 7)
     assert (s["passes"], s["left"], s["skip"]) == (2, 1, 7)  # calls 1 and 6; the seventh reads the sixth's end: 8 calls
+
+
+def test_a_new_fit_reads_no_old_end(cuda):
+    """Two passes under way, the first leaving every query and the second none, then a new base: its passes are its own."""
+    import torch
+    x, q = _data("normal", 30000, 64, 20, np.random.default_rng(6))
+    good, bad = torch.from_numpy(q).cuda(), torch.from_numpy(q * np.float32(1e17)).cuda()
+    ix = _index(x)
+    ix.search(good, 10)
+    torch.cuda.synchronize()
+    busy = torch.randn(8192, 8192, device="cuda")
+    for _ in range(8):
+        busy = busy @ busy * 1e-4  # the passes below are queued behind this
+    ix.search(bad, 10)
+    ix.search(good, 10)
+    assert ix.get_prune_stats()["passes"] == 3
+    ix.fit(torch.from_numpy(x + 1).cuda())
+    ix.search_tc(good[:1], 1)
+    s = _run(ix, good, 10, 3)
+    assert (s["passes"], s["left"], s["skip"]) == (6, 0, 0)
