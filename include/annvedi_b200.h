@@ -102,7 +102,8 @@ int ann_flat_fit(ann_flat* h, const float* data, int64_t n, int32_t dim, int64_t
  * stride `ldq`). Writes out_ids[nq][k'] (int64, -1 padded) and, if out_dists is not NULL, the
  * ranking values out_dists[nq][k'] (squared L2, or inner product for ANN_METRIC_IP), with
  * k' = min(k, n) as the reference clips k to n (linear_index.cpp:110). ANN_MODE_REFERENCE
- * reproduces the reference's own ranking (L2 only); ANN_MODE_EXACT returns the true top-k.
+ * reproduces the reference's own ranking (L2 only); ANN_MODE_EXACT returns the true top-k of the FP32 distances, pruned by
+ * tensor-core keys where that saves time (a pass whose device waits give up certifies nothing, and the scan answers).
  * Adds n per query to the distance counter (linear_index.cpp:108). */
 int ann_flat_query(ann_flat* h, ann_workspace* ws, const float* queries, int32_t nq, int64_t ldq, int32_t k,
                    int32_t mode, int32_t mem, int64_t* out_ids, float* out_dists, void* stream);
