@@ -226,7 +226,6 @@ int ann_flat_destroy(ann_flat* h) {
         if (h->base_e4m3) cudaFree(h->base_e4m3);
         if (h->fac_e4m3) cudaFree(h->fac_e4m3);
         if (h->d_err) cudaFree(h->d_err);
-        if (h->d_prune_word) cudaFree(h->d_prune_word);
         if (h->prune_word) cudaFreeHost(h->prune_word);  // (the frees above have waited for the device)
     }
     ws_release(&h->ws);
@@ -266,7 +265,10 @@ int ann_flat_fit(ann_flat* h, const float* data, int64_t n, int32_t dim, int64_t
     h->prune_refused = false;
     h->prune_ws_refused = SIZE_MAX;
     h->prune_streak = h->prune_skip = 0;
-    if (h->prune_word) h->prune_seen = (uint32_t)(*h->prune_word >> 32);  // (the old base's passes are done: its end is not read)
+    if (h->prune_word) {  // (the old base's passes are done: their end is not read)
+        h->prune_seen = (uint32_t)(h->prune_word[0] >> 32);
+        h->prune_word[1] = 0;
+    }
     const size_t bytes = sizeof(float) * (size_t)n * dpad;
     cudaError_t e = cudaMalloc(&h->base, bytes);
     if (e != cudaSuccess) {
@@ -665,16 +667,13 @@ static int flat_ensure_pruned(ann_flat* h, int nq, cudaStream_t st, bool capturi
         h->bounds = covered ? PruneBounds{c * 1.001f, r * 1.001f} : PruneBounds{};
         h->bounds_known = true;
         if (!h->prune_word) {
-            void *w = nullptr, *d = nullptr;
-            if (cudaHostAlloc(&w, sizeof(*h->prune_word), cudaHostAllocPortable | cudaHostAllocMapped) == cudaSuccess &&
-                cudaMalloc(&d, sizeof(*h->d_prune_word)) == cudaSuccess) {
+            void* w = nullptr;
+            if (cudaHostAlloc(&w, 2 * sizeof(*h->prune_word), cudaHostAllocPortable | cudaHostAllocMapped) == cudaSuccess) {
                 h->prune_word = static_cast<unsigned long long*>(w);
-                h->d_prune_word = static_cast<unsigned long long*>(d);
-                *h->prune_word = (unsigned long long)h->prune_seen << 32;
-                ANN_CUDA_TRY(cudaMemsetAsync(d, 0, sizeof(*h->d_prune_word), st));
+                h->prune_word[0] = (unsigned long long)h->prune_seen << 32;
+                h->prune_word[1] = 0;
             } else {
                 cudaGetLastError();  // no back-off then
-                if (w) cudaFreeHost(w);
             }
         }
     }
@@ -818,8 +817,11 @@ static int flat_exact_pruned(ann_flat* h, ann_workspace* ws, const float* qdev, 
         p.list = list;
         p.count = count;
         p.err = err;
-        p.words = words;
-        p.joined = joined;
+        // (a captured call is replayed on queries to come)
+        const bool shared = capturing || !h->prune_word || __atomic_load_n(&h->prune_word[1], __ATOMIC_RELAXED) != 0;
+        p.words = shared ? words : nullptr;
+        p.joined = shared ? joined : nullptr;
+        p.wide = words && !shared ? h->prune_word + 1 : nullptr;
         p.out_ids = ids_dev + (size_t)q0 * kk;
         p.out_dists = dists_dev ? dists_dev + (size_t)q0 * kk : nullptr;
         if ((rc = launch_prune_queries(p, qb, kpad, st))) return rc;
@@ -842,10 +844,10 @@ static int flat_exact_pruned(ann_flat* h, ann_workspace* ws, const float* qdev, 
         {
             std::lock_guard<std::mutex> lk(h->tc_mu);
             pass = ++h->prune_pass;
+            h->prune_nq = nc;
             report = h->prune_streak > 0;
         }
-        if ((rc = launch_prune_gather(q, dpad, list, count, nc, qg, h->d_prune_word, h->prune_word, pass, report, st)))
-            return rc;
+        if ((rc = launch_prune_gather(q, dpad, list, count, nc, qg, h->prune_word, pass, report, st))) return rc;
         FlatScanArgs a{h->base, n, dpad, qg, nc, h->metric, kk, rps, nsplit, skey, sid};
         a.qpair = qpair;
         a.nq_dev = count;
@@ -919,12 +921,10 @@ int ann_flat_prune_stats(ann_flat* h, int64_t* out4) {
     clear_error();
     ANN_CHECK_ARG(h != nullptr && out4 != nullptr, "ann_flat_prune_stats: null argument");
     std::lock_guard<std::mutex> lk(h->tc_mu);
-    DeviceGuard g(h->device);
-    unsigned long long w = 0;
-    if (h->d_prune_word) ANN_CUDA_TRY(cudaMemcpy(&w, h->d_prune_word, sizeof(w), cudaMemcpyDeviceToHost));
+    const unsigned long long w = h->prune_word ? __atomic_load_n(&h->prune_word[0], __ATOMIC_RELAXED) : 0;
     out4[0] = h->prune_pass;
-    out4[1] = (int64_t)(w >> 16) & 0xffff;
-    out4[2] = (int64_t)w & 0xffff;
+    out4[1] = h->prune_nq;
+    out4[2] = (uint32_t)(w >> 32) == h->prune_pass ? (int64_t)w & 0xffff : 0;  // (a pass that settled all need not write)
     out4[3] = h->prune_skip;
     return ANN_OK;
 }

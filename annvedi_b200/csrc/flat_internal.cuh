@@ -35,12 +35,12 @@ struct ann_flat {
     double prune_credit_us = 0.0;        // what pruning would have saved the exact searches so far (estimated)
     bool prune_refused = false;          // the BF16 copy for them did not fit beside what the card holds (until the next fit)
     size_t prune_ws_refused = SIZE_MAX;  // scratch of this size did not fit
-    // how the latest pruned pass ended, written by the device (pass << 32 | queries << 16 | queries left to the scan; in
-    // page-locked memory where queries were left or the host waits for a better end), and the back-off that follows from
-    // it (flat_prune_open)
-    unsigned long long* prune_word = nullptr;
-    unsigned long long* d_prune_word = nullptr;
+    // how the latest pruned pass ended, written by the device into page-locked memory where it left queries or the host waits
+    // for a better end (pass << 32 | queries << 16 | queries left to the scan), and the back-off that follows from it
+    // (flat_prune_open)
+    unsigned long long* prune_word = nullptr;  // two words: that, and whether a query had rows for several blocks (PruneArgs::wide)
     uint32_t prune_pass = 0;             // passes launched
+    int prune_nq = 0;                    // queries of the latest
     uint32_t prune_seen = 0;             // the latest whose end has been read
     int prune_streak = 0;                // passes in a row that left too many queries
     int prune_skip = 0;                  // calls that the scan still answers

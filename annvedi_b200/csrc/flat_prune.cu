@@ -113,8 +113,10 @@ __global__ void __launch_bounds__(256) prune_queries_kernel(PruneArgs a, __nv_bf
 // With gridDim.y > 1 (few queries) a query's rows beyond those of one round of the warps go to further blocks, each taking
 // its run of the survivors; the block that ends last selects. A round is a chain of dim / 32 steps of about 1 us: clustered
 // data of many dimensions, whose windows hold thousands of rows, took up to eight rounds in one block (one query over
-// 20,000 x 2,048 normal / clustered: 118 / 152 us; 5 over 20,000 x 4,096: 216 / 880, scanned 438).
-template <bool STREAM, int METRIC, int kFinWarps>
+// 20,000 x 2,048 normal / clustered: 118 / 152 us; 5 over 20,000 x 4,096: 216 / 880, scanned 438). The code and the blocks that
+// mostly have nothing to do cost a single query 2 us (a kernel of one block fetches its instructions anew each call), so an
+// index's passes have them (SPLIT) from the first query on that would use one.
+template <bool STREAM, int METRIC, int kFinWarps, bool SPLIT>
 __global__ void __launch_bounds__(kFinWarps * 32) prune_finish_kernel(PruneArgs a) {
     constexpr int kFinThreads = kFinWarps * 32;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -130,7 +132,7 @@ __global__ void __launch_bounds__(kFinWarps * 32) prune_finish_kernel(PruneArgs 
     const int cnt = a.rcount[q];
     const float w = a.win[q], tauF = a.tauF[q];
     const int gave_up = *a.err;  // (with the loads above, not a round trip of its own behind them)
-    if (blockIdx.y > 0 && cnt <= (int)blockIdx.y * kFinThreads) return;  // no more than the blocks before take
+    if (SPLIT && blockIdx.y > 0 && cnt <= (int)blockIdx.y * kFinThreads) return;  // no more than the blocks before take
     const float* fk = a.fkey + (int64_t)q * cap;
     const int* fc = a.fcol + (int64_t)q * cap;
     bool fail = cnt > cap || cnt < k || !(w < kInf) || gave_up != 0;
@@ -142,26 +144,28 @@ __global__ void __launch_bounds__(kFinWarps * 32) prune_finish_kernel(PruneArgs 
         fail = !(T <= tauF);
     }
     if (fail) {  // uniform
-        if (tid == 0 && blockIdx.y == 0) a.list[atomicAdd(a.count, 1)] = q;
+        if (tid == 0 && (!SPLIT || blockIdx.y == 0)) a.list[atomicAdd(a.count, 1)] = q;
         return;
     }
     const float lim = __fadd_ru(T, w);  // <= tauX: every key at or below it was kept
-    for (int d = tid; d < dpad; d += kFinThreads) sQ[d] = a.q[(int64_t)q * dpad + d];
-    auto collect = [&](int i0, int i1) {  // the rows of survivors [i0, i1) within the window; returns their number
+    auto collect = [&](int i0, int i1, bool first) {  // the rows of survivors [i0, i1) within the window; returns their number
         if (tid == 0) sN = 0;
         __syncthreads();
+        if (first)  // (behind the barrier, beside the survivors' loads)
+            for (int d = tid; d < dpad; d += kFinThreads) sQ[d] = a.q[(int64_t)q * dpad + d];
         for (int i = i0 + tid; i < i1; i += kFinThreads)
             if (fk[i] <= lim) sE[atomicAdd(&sN, 1)] = (unsigned)row_of_pos(fc[i], a.n, a.mult);
         __syncthreads();
         return sN;
     };
-    const int total = collect(0, cnt);  // >= k, the same in every block of the query
-    const int blocks = min((int)gridDim.y, (total + kFinThreads - 1) / kFinThreads);
-    if ((int)blockIdx.y >= blocks) return;
+    const int total = collect(0, cnt, true);  // >= k, the same in every block of the query
+    const int blocks = SPLIT ? min((int)gridDim.y, (total + kFinThreads - 1) / kFinThreads) : 1;
+    if (SPLIT && (int)blockIdx.y >= blocks) return;
+    if (!SPLIT && a.wide && total > kFinThreads && tid == 0) *static_cast<volatile unsigned long long*>(a.wide) = 1ull;
     int m = total;
-    if (blocks > 1) {
+    if (SPLIT && blocks > 1) {
         __syncthreads();
-        m = collect((int)((int64_t)cnt * blockIdx.y / blocks), (int)((int64_t)cnt * (blockIdx.y + 1) / blocks));
+        m = collect((int)((int64_t)cnt * blockIdx.y / blocks), (int)((int64_t)cnt * (blockIdx.y + 1) / blocks), false);
     }
     float* myX = sX + warp * kFinStages * 32 * kFinPitch;
     const int nch = dpad / 32;
@@ -224,7 +228,7 @@ __global__ void __launch_bounds__(kFinWarps * 32) prune_finish_kernel(PruneArgs 
             sE[g + lane] = ((unsigned long long)ord_f32((METRIC == ANN_METRIC_L2 ? v : -v) + 0.f) << 32) | (unsigned)row;
     }
     __syncthreads();
-    if (blocks > 1) {
+    if (SPLIT && blocks > 1) {
         unsigned long long* gw = a.words + (int64_t)q * cap;
         __shared__ int sAt;
         if (tid == 0) sAt = atomicAdd(&a.joined[q].x, m);
@@ -260,14 +264,10 @@ __global__ void __launch_bounds__(kFinWarps * 32) prune_finish_kernel(PruneArgs 
 
 __global__ void prune_gather_kernel(const float* __restrict__ q, int dpad, const int* __restrict__ list,
                                     const int* __restrict__ count, float* __restrict__ qg, int nq,
-                                    unsigned long long* dev_word, volatile unsigned long long* word, uint32_t pass,
-                                    int report) {
+                                    volatile unsigned long long* word, uint32_t pass, int report) {
     const int n = *count;
-    if (word && blockIdx.x == 0 && threadIdx.x == 0) {
-        const unsigned long long v = ((unsigned long long)pass << 32) | ((unsigned)nq << 16) | (unsigned)n;
-        *dev_word = v;
-        if (n > 0 || report) *word = v;  // over PCIe, and the kernels that follow wait for it
-    }
+    if (word && (n > 0 || report) && blockIdx.x == 0 && threadIdx.x == 0)  // over PCIe, and the kernels that follow wait for it
+        *word = ((unsigned long long)pass << 32) | ((unsigned)nq << 16) | (unsigned)n;
     for (int j = blockIdx.x; j < n; j += gridDim.x)
         for (int d = threadIdx.x; d < dpad; d += blockDim.x) qg[(int64_t)j * dpad + d] = q[(int64_t)list[j] * dpad + d];
 }
@@ -275,13 +275,13 @@ __global__ void prune_gather_kernel(const float* __restrict__ q, int dpad, const
 size_t finish_smem(int cap, int dpad, int warps) {
     return sizeof(float) * ((size_t)warps * kFinStages * 32 * kFinPitch + dpad) + sizeof(unsigned long long) * cap;
 }
-template <int W>
+template <int W, bool SPLIT>
 int run_finish(const PruneArgs& a, cudaStream_t st) {
     auto kern = a.metric == ANN_METRIC_L2
-                    ? (a.stream_form ? prune_finish_kernel<true, ANN_METRIC_L2, W> : prune_finish_kernel<false, ANN_METRIC_L2, W>)
-                    : (a.stream_form ? prune_finish_kernel<true, ANN_METRIC_IP, W> : prune_finish_kernel<false, ANN_METRIC_IP, W>);
+                    ? (a.stream_form ? prune_finish_kernel<true, ANN_METRIC_L2, W, SPLIT> : prune_finish_kernel<false, ANN_METRIC_L2, W, SPLIT>)
+                    : (a.stream_form ? prune_finish_kernel<true, ANN_METRIC_IP, W, SPLIT> : prune_finish_kernel<false, ANN_METRIC_IP, W, SPLIT>);
     ANN_CUDA_TRY(smem_optin(reinterpret_cast<const void*>(kern)));
-    const int blocks = a.words ? (int)std::min<int64_t>(ceil_div(a.cap, W * 32), std::max(1, kNumSMs / a.nq)) : 1;
+    const int blocks = SPLIT ? (int)std::min<int64_t>(ceil_div(a.cap, W * 32), std::max(1, kNumSMs / a.nq)) : 1;
     kern<<<dim3(a.nq, blocks), W * 32, finish_smem(a.cap, a.dpad, W), st>>>(a);
     ANN_LAUNCH_CHECK();
     return ANN_OK;
@@ -325,13 +325,14 @@ int launch_prune_finish(const PruneArgs& a, cudaStream_t st) {
                   "pruned scan: k=%d, padded dim %d", a.k, a.dpad);
     ANN_CHECK_ARG((a.words == nullptr) == (a.joined == nullptr), "pruned scan: shared rows need both arrays");
     const bool wide = a.nq <= kNumSMs && finish_smem(a.cap, a.dpad, 16) <= 220 * 1024;
-    return wide ? run_finish<16>(a, st) : run_finish<8>(a, st);
+    if (a.words) return wide ? run_finish<16, true>(a, st) : run_finish<8, true>(a, st);
+    return wide ? run_finish<16, false>(a, st) : run_finish<8, false>(a, st);
 }
 
 int launch_prune_gather(const float* q, int dpad, const int* list, const int* count, int nq, float* qg,
-                        unsigned long long* dev_word, unsigned long long* word, uint32_t pass, int report, cudaStream_t st) {
+                        unsigned long long* word, uint32_t pass, int report, cudaStream_t st) {
     ANN_CHECK_ARG(nq <= 65535, "pruned scan: %d queries a pass", nq);
-    prune_gather_kernel<<<(unsigned)std::min(nq, 2 * kNumSMs), 128, 0, st>>>(q, dpad, list, count, qg, nq, dev_word, word, pass, report);
+    prune_gather_kernel<<<(unsigned)std::min(nq, 2 * kNumSMs), 128, 0, st>>>(q, dpad, list, count, qg, nq, word, pass, report);
     ANN_LAUNCH_CHECK();
     return ANN_OK;
 }

@@ -68,11 +68,12 @@ struct PruneArgs {
     int* err;           // [1] set where a wait of the sample or filter pass gave up: every query is left to the scan
     int64_t* out_ids;   // [nq, k]
     float* out_dists;   // [nq, k] or null
-    // few queries (prune_split(nq)): a query's rows shared by several blocks
+    // few queries (prune_split(nq)): a query's rows shared by several blocks (null: by one)
     unsigned long long* words;  // [nq, cap] the formed (distance, row)
     int2* joined;               // [nq] words written, blocks done
+    unsigned long long* wide;   // optional, page-locked: set to 1 by a query that has rows for several blocks, where one forms them
 };
-// Whether a pass of nq queries uses words and joined (its blocks would leave most of the chip idle).
+// Whether a pass of nq queries may use words and joined (its blocks would leave most of the chip idle).
 bool prune_split(int nq);
 // Survivors kept per query, and whether their kernel's shared memory fits.
 int prune_cap(int k);
@@ -83,9 +84,9 @@ int prune_bar_rank(int k, int64_t S, int64_t n);
 // win and the queries' operand rows qb [nq, kpad] (launch_tc_operand's); rcount, count and err zeroed.
 int launch_prune_queries(const PruneArgs& a, __nv_bfloat16* qb, int kpad, cudaStream_t st);
 int launch_prune_finish(const PruneArgs& a, cudaStream_t st);  // results, list and count
-// qg[j] = q[list[j]] for j < *count; *dev_word = pass << 32 | nq << 16 | *count (nq <= 65,535) and, where *count > 0 or
-// report, *word (page-locked host memory) the same. Both words may be null together.
+// qg[j] = q[list[j]] for j < *count; where *count > 0 or report, *word (page-locked host memory, optional) =
+// pass << 32 | nq << 16 | *count (nq <= 65,535).
 int launch_prune_gather(const float* q, int dpad, const int* list, const int* count, int nq, float* qg,
-                        unsigned long long* dev_word, unsigned long long* word, uint32_t pass, int report, cudaStream_t st);
+                        unsigned long long* word, uint32_t pass, int report, cudaStream_t st);
 
 }  // namespace annb

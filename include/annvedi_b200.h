@@ -155,8 +155,8 @@ int ann_flat_set_tc_precision(ann_flat* h, int32_t precision);
 int ann_flat_set_option(ann_flat* h, int32_t option, int64_t value);
 
 /* Diagnostic: the exact search's passes of tensor-core keys (queries whose result those certify skip the scan): out4 =
- * {passes launched, queries of the latest finished pass, queries that it left to the scan, calls that the scan alone
- * still answers because passes left too many}. A call takes one pass per 10,240 queries, or none. */
+ * {passes launched, queries of the latest, queries that it left to the scan (once it is done), calls that the scan alone
+ * still answers because passes left too many}. A call takes one pass per 10,240 queries, or none. Does not synchronise. */
 int ann_flat_prune_stats(ann_flat* h, int64_t* out4);
 
 /* Diagnostic: the tensor-core key matrix out_keys[nq][n] (device pointers; synchronous). */
