@@ -219,7 +219,8 @@ class LinearIndex:
 
     def get_prune_stats(self) -> dict:
         """The exact search's tensor-core passes (ann_flat_prune_stats): how many were launched, the latest
-        one's queries and how many of them it left to the scan (once it is done), and the calls that the scan alone still answers."""
+        one's queries and how many of them it left to the scan (once it is done), and the calls that the scan alone
+        still answers."""
         out = (ctypes.c_int64 * 4)()
         _lib.check(self._lib.ann_flat_prune_stats(self._h, out))
         return {"passes": int(out[0]), "queries": int(out[1]), "left": int(out[2]), "skip": int(out[3])}
